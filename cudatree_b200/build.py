@@ -24,6 +24,7 @@ SOURCES = [
     "ct_api.cu",
     "ct_level.cu",
     "ct_fit.cu",
+    "ct_rows.cu",
     "ct_boot.cu",
     "ct_predict.cu",
     "ct_presort.cu",

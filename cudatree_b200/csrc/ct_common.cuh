@@ -91,12 +91,15 @@ __device__ __forceinline__ bool is_candidate(float x, float x_next) {
   return __dadd_rn((double)x, DIFF_THRESHOLD) < (double)x_next;
 }
 // is_candidate for sorted neighbours (x <= x_next) with the double test only
-// where it can matter: equal values never qualify, and a float gap above 1e-4
-// (true gap > 9.99e-5 after the subtraction's 2^-24 relative rounding) always
-// does, since the double sum x + 1e-5 exceeds x by less than that.
+// where it can matter: equal values never qualify; otherwise the float gap
+// x_next - x is off by at most 2^-24 of itself and the double sum x + 1e-5 by
+// 2^-53 of x (from |x| = 128 on every float gap is above 1.5e-5), so gaps that
+// differ from 1e-5 by more than one part in 10^5 decide it.
 __device__ __forceinline__ bool is_candidate_sorted(float x, float x_next) {
   if (!(x_next > x)) return false;
-  if (x_next - x > 1e-4f) return true;
+  const float gap = x_next - x;
+  if (gap > 1.00001e-5f) return true;
+  if (gap < 0.99999e-5f) return false;
   return is_candidate(x, x_next);
 }
 __device__ __forceinline__ double gini_part(int64_t sq_sum, double n_side, double n_total) {

@@ -124,7 +124,8 @@ void begin_level(Counters* c, cudaStream_t st) {
 // (a scanned entry that carries its label needs no label read).
 void account_level(const ct_problem* p, const View& view, const Counters& h) {
   Prof* pf = current_prof();
-  const double w = p->index_bytes, l = view.lab_shift ? 0.0 : p->label_bytes, v = sizeof(float);
+  // row-list growth: 32-bit row entries and 8-byte (value, label) sorted entries
+  const double w = view.rl[0] ? 4.0 : p->index_bytes, l = view.lab_shift ? 0.0 : p->label_bytes, v = sizeof(float);
   pf->stats.bytes[CT_K_SCAN] += (double)h.scan_elems * (w + l + v) + (double)h.vrows * (w + 8.0);
   pf->stats.bytes[CT_K_MARK] += (double)h.split_total * (w + 1.0);
   pf->stats.bytes[CT_K_PARTITION] += (double)h.part_elems * (2.0 * w + 1.0);  // chains actually partitioned
@@ -170,36 +171,93 @@ struct FitLayout {
   uint32_t mask_words;   // words of one node's mask
   LevelScratch s;
   struct LoopCtl* ctl;   // state of the graph-driven level loop
+  bool rows;             // row-list growth (ct_rows.cu)
+  uint32_t n_max;        // its most rows of any tree
+  uint2* pair;           // [n_features][n_rows] (rank, value bits), by row
+  uint2* ranked;         // [n_features][n_rows] (value bits, label), by rank, or NULL
+  uint32_t* rank;        // [n_features][n_rows] ranks alone, by row, or NULL
+  uint2* planes;         // its sorted lists, or NULL: they fit the caller's list buffers
   void* boot_ws;
   size_t boot_bytes;
   size_t bytes;
 };
 
-bool layout(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o, char* base, size_t size,
-            FitLayout* L) {
-  View v = make_view(p, nullptr);
+// Options common to the forms of a fit.
+void layout_options(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o, FitLayout* L) {
   const uint32_t slots = (o->mode == CT_FIT_PLAIN) ? 1u : n_trees;
   const uint64_t S = (uint64_t)slots * p->n_rows;
   const uint64_t cap_list64 = S / 2 + slots + 2;
+  *L = FitLayout{};
   L->n_slots = slots;
   L->cap_list = (uint32_t)std::min<uint64_t>(cap_list64, 0xffffffffull);
   L->chunk = std::min<uint32_t>(L->cap_list, o->step_nodes ? o->step_nodes : CHUNK_NODES_MAX);
-  if (virtual_possible(p) && !(o->flags & CT_FIT_NO_VIRTUAL)) {
-    // the per-node class counts of the virtual features stay within 1 GiB
-    const uint64_t per_node = (uint64_t)p->n_features * p->n_classes * sizeof(uint32_t);
-    L->chunk = std::min<uint32_t>(L->chunk, (uint32_t)std::max<uint64_t>(4096, (1ull << 30) / per_node));
-  }
   L->scan_piece = o->scan_piece ? o->scan_piece : DEFAULT_SCAN_PIECE;
-  // the warp subtree packs a row id into 27 bits of its sort key
-  L->subtree_cut = p->n_rows < (1u << 27) ? std::min<uint32_t>(o->subtree_cutoff, 128u) : 0u;
-  L->cap_small = L->subtree_cut ? 2 * L->chunk : 0u;
   L->host_loop = (o->flags & CT_FIT_HOST_LOOP) != 0;
   L->graph_samples = o->graph_samples == 0xffffffffu ? UINT64_MAX
                      : o->graph_samples               ? o->graph_samples
                                                       : DEFAULT_GRAPH_SAMPLES;
+  L->mask_words = mask_words(p->n_features);
+  L->mat16 = 16 * std::min(p->max_features, p->n_features);
+  L->n_max = p->n_rows;
+}
+
+// The virtual features' counts of a step stay within 1 GiB.
+void limit_virtual_chunk(const ct_problem* p, FitLayout* L) {
+  const uint64_t per_node = (uint64_t)p->n_features * p->n_classes * sizeof(uint32_t);
+  L->chunk = std::min<uint32_t>(L->chunk, (uint32_t)std::max<uint64_t>(4096, (1ull << 30) / per_node));
+}
+
+// Workspace of row-list growth (batched form; rows_possible).
+bool row_layout(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o, char* base, size_t size,
+                FitLayout* L) {
+  layout_options(p, n_trees, o, L);
+  L->rows = true;
+  const uint64_t S = (uint64_t)L->n_slots * p->n_rows;
+  L->virt = p->n_features >= 2 && p->n_features <= 64 && (uint64_t)p->n_features * p->n_classes <= 2048 &&
+            !(o->flags & CT_FIT_NO_VIRTUAL);
+  if (L->virt) limit_virtual_chunk(p, L);
+  L->subtree_cut = std::min<uint32_t>(o->subtree_cutoff, 32u);
+  L->cap_small = L->subtree_cut ? 2 * L->chunk : 0u;
+  View v = make_view(p, nullptr);
   Arena a{base, size, 0};
   L->small = L->cap_small ? a.take<ct_node>(L->cap_small) : nullptr;
-  L->small_bound = 0;
+  L->n_in = a.take<uint32_t>(L->n_slots);
+  L->fbin = a.take<uint32_t>((p->n_features + 31) / 32);
+  L->ffwork = a.take<char>(feature_flags_work_bytes(p->n_features));
+  L->vrow = L->virt ? a.take<uint64_t>(p->n_rows) : nullptr;
+  L->vval = a.take<float2>(p->n_features);
+  for (int i = 0; i < 2; ++i) {
+    L->list[i] = a.take<ct_node>(L->cap_list);
+    L->tot[i] = a.take<uint32_t>((size_t)L->cap_list * p->n_classes);
+    L->mask[i] = a.take<uint64_t>((size_t)L->cap_list * L->mask_words);
+  }
+  L->pair = a.take<uint2>((size_t)p->n_features * p->n_rows);
+  if (rows_have_large(p->n_rows)) {
+    L->ranked = a.take<uint2>((size_t)p->n_features * p->n_rows);
+    L->rank = a.take<uint32_t>((size_t)p->n_features * p->n_rows);
+  }
+  const uint32_t planes = rows_planes_needed(p);
+  L->planes = planes && !rows_planes_in_lists(p) ? a.take<uint2>((size_t)planes * S) : nullptr;
+  carve_row_scratch(a, v, LevelBounds{L->chunk, S}, step_piece(0, L->scan_piece, 1), &L->s, L->virt);
+  L->ctl = a.take<LoopCtl>(1);
+  L->bytes = a.used + 256;
+  return base != nullptr && a.ok();
+}
+
+// Workspace of list growth: the plain form, and batched fits that row-list
+// growth does not take.
+bool list_layout(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o, char* base, size_t size,
+                 FitLayout* L) {
+  View v = make_view(p, nullptr);
+  layout_options(p, n_trees, o, L);
+  const uint32_t slots = L->n_slots;
+  const uint64_t S = (uint64_t)slots * p->n_rows;
+  if (virtual_possible(p) && !(o->flags & CT_FIT_NO_VIRTUAL)) limit_virtual_chunk(p, L);
+  // the warp subtree packs a row id into 27 bits of its sort key
+  L->subtree_cut = p->n_rows < (1u << 27) ? std::min<uint32_t>(o->subtree_cutoff, 128u) : 0u;
+  L->cap_small = L->subtree_cut ? 2 * L->chunk : 0u;
+  Arena a{base, size, 0};
+  L->small = L->cap_small ? a.take<ct_node>(L->cap_small) : nullptr;
   L->n_in = a.take<uint32_t>(slots);
   L->fbin = a.take<uint32_t>((p->n_features + 31) / 32);
   L->ffwork = a.take<char>(feature_flags_work_bytes(p->n_features));
@@ -208,7 +266,6 @@ bool layout(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o, char
   L->vval = L->virt ? a.take<float2>(p->n_features) : nullptr;
   // the plain form moves nodes through the host, so only the batched form keeps masks
   const bool masks = o->mode == CT_FIT_BATCHED;
-  L->mask_words = mask_words(p->n_features);
   for (int i = 0; i < 2; ++i) {
     L->list[i] = a.take<ct_node>(L->cap_list);
     L->tot[i] = a.take<uint32_t>((size_t)L->cap_list * p->n_classes);
@@ -216,7 +273,6 @@ bool layout(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o, char
   }
   L->boot_bytes = bootstrap_scratch_bytes(p->n_rows, p->n_features, slots);
   L->boot_ws = a.take<char>(L->boot_bytes);
-  L->mat16 = 16 * std::min(p->max_features, p->n_features);
   LevelCaps caps = level_caps(v, step_piece(0, L->scan_piece, 1), LevelBounds{L->chunk, S});
   carve_level_scratch(a, v, caps, &L->s, L->virt);
   L->s.huge_rows = o->huge_rows ? o->huge_rows : HUGE_SEG;
@@ -268,6 +324,15 @@ void account_bootstrap(const ct_problem* p, uint64_t skip) {
   pf->launched(CT_K_BOOTSTRAP, p->bootstrap ? 3 : 1);
 }
 
+// Row-list growth: the presort and the values read and (rank, value) written
+// once per fit, the row lists written per tree.
+void account_row_roots(const ct_problem* p, uint32_t n_trees, uint64_t vmask) {
+  Prof* pf = current_prof();
+  const double n = p->n_rows, f = p->n_features - __builtin_popcountll(vmask);
+  pf->stats.bytes[CT_K_BOOTSTRAP] += n * f * (p->index_bytes + 12.0) + n_trees * n * (p->bootstrap ? 0.632 : 1.0) * 4.0;
+  pf->launched(CT_K_BOOTSTRAP, 2);
+}
+
 template <typename IdxT, typename LabT>
 int launch_root(const View& v, const FitLayout& L, uint32_t slot_lo, uint32_t n_slots, uint64_t seed,
                 uint32_t tree_lo, const TreeView& tv, int cur, cudaStream_t st) {
@@ -302,9 +367,13 @@ int root(const ct_problem* p, const View& v, const FitLayout& L, uint32_t slot_l
 // (disjoint) ranges.  Deferring them to one launch lets long subtrees overlap.
 int flush_subtrees(const ct_problem* p, const View& v, const FitLayout& L, const TreeView& tv, cudaStream_t st) {
   if (!L.subtree_cut || L.small_bound == 0) return CT_OK;
-  CT_TRY(launch_subtrees(v, p->index_bytes, p->label_bytes, L.small, L.cap_small,
-                         (uint32_t)std::min<uint64_t>(L.small_bound, L.cap_small), L.subtree_cut > 32, false, L.s, tv,
-                         st));
+  if (L.rows)
+    CT_TRY(launch_row_subtrees(v, L.small, L.cap_small, (uint32_t)std::min<uint64_t>(L.small_bound, L.cap_small), L.s,
+                               tv, st));
+  else
+    CT_TRY(launch_subtrees(v, p->index_bytes, p->label_bytes, L.small, L.cap_small,
+                           (uint32_t)std::min<uint64_t>(L.small_bound, L.cap_small), L.subtree_cut > 32, false, L.s,
+                           tv, st));
   CT_CUDA_TRY(cudaMemsetAsync(&L.s.ctr->n_small, 0, sizeof(uint32_t), st));
   L.small_bound = 0;
   return CT_OK;
@@ -332,6 +401,11 @@ int step(const ct_problem* p, const View& v, const FitLayout& L, const TreeView&
     const LevelBounds b{cn, total};
     if (L.subtree_cut && L.small_bound + 2ull * cn > L.cap_small) CT_TRY(flush_subtrees(p, v, L, tv, st));
     CT_TRY(launch_reset_step(L.s, cn, step_lists(L, cur, lo, C, total), st));
+    if (L.rows) {
+      CT_TRY(launch_row_step(v, L.s, b, L.n_max, tv, L.cap_list, L.subtree_cut, L.small, L.cap_small, st));
+      if (L.subtree_cut) L.small_bound += 2ull * cn;
+      continue;
+    }
     // Persistent split and children launches (at most the resident blocks):
     // their grids would otherwise be sized by the capacity bounds, most of
     // whose warps find no item.  The mark fill keeps one warp per piece.
@@ -531,15 +605,20 @@ int build_loop_graph(const ct_problem* p, const View& v, const FitLayout& L, con
   CT_TRY(capture_into(cp.conditional.phGraph_out[0], nullptr, st, [&]() -> int {
     k_loop_step<<<1, 1, 0, st>>>(L.ctl, L.s.ctr, L.s.step, ll, L.chunk, C, L.scan_piece, L.mat16);
     pf->launched(CT_K_CHILDREN);
-    CT_TRY(launch_split(v, ib, lb, L.s, b, L.scan_piece, true, st));
-    CT_TRY(launch_partition(v, ib, lb, L.s, b, tv, true, st));
-    CT_TRY(launch_children(v, ib, lb, L.s, b, tv, L.cap_list, L.subtree_cut, L.small, L.cap_small, true, st));
+    if (L.rows) {
+      CT_TRY(launch_row_step(v, L.s, b, L.n_max, tv, L.cap_list, L.subtree_cut, L.small, L.cap_small, st));
+    } else {
+      CT_TRY(launch_split(v, ib, lb, L.s, b, L.scan_piece, true, st));
+      CT_TRY(launch_partition(v, ib, lb, L.s, b, tv, true, st));
+      CT_TRY(launch_children(v, ib, lb, L.s, b, tv, L.cap_list, L.subtree_cut, L.small, L.cap_small, true, st));
+    }
     k_loop_end<<<1, 1, 0, st>>>(L.ctl, L.s.ctr, L.chunk, L.cap_list, h);
     pf->launched(CT_K_CHILDREN);
     return CT_OK;
   }));
   const ct_kernel_stats s2 = pf->stats;
   CT_TRY(capture_into(lg.graph, &loop, st, [&]() -> int {
+    if (L.rows) return launch_row_subtrees(v, L.small, L.cap_small, L.cap_small, L.s, tv, st);
     return launch_subtrees(v, ib, lb, L.small, L.cap_small, L.cap_small, L.subtree_cut > 32, true, L.s, tv, st);
   }));
   const ct_kernel_stats s3 = pf->stats;
@@ -579,6 +658,8 @@ int graph_level_loop(const ct_problem* p, const View& v, const FitLayout& L, con
   key_add(key, L.scan_piece);
   key_add(key, L.mat16);
   key_add(key, L.subtree_cut);
+  key_add(key, L.rows);
+  key_add(key, L.n_max);
   LoopGraph& lg = t_loop_graph;
   if (!lg.exec || lg.key != key) {
     lg.reset();
@@ -656,6 +737,26 @@ View fit_view(const ct_problem* p, const ct_lists* l, const FitLayout& L) {
   return v;
 }
 
+// The view of row-list growth: 32-bit row lists at the front of the caller's
+// list buffers, the sorted planes behind them (or in the workspace).
+View row_view(const ct_problem* p, const ct_lists* l, const FitLayout& L, uint2* pair, uint2* ranked,
+              uint32_t* rank, uint2* planes) {
+  View v = make_view(p, l);
+  v.lab_shift = p->n_rows > 1 ? 32u - (uint32_t)__builtin_clz(p->n_rows - 1) : 1u;
+  v.row_mask = (1u << v.lab_shift) - 1u;
+  v.fbin = L.fbin;
+  v.rl[0] = reinterpret_cast<uint32_t*>(l->si0);
+  v.rl[1] = reinterpret_cast<uint32_t*>(l->si1);
+  v.pair = pair;
+  v.ranked = ranked;
+  v.rank = rank;
+  const size_t off = ((size_t)l->n_slots * l->stride * sizeof(uint32_t) + 15) & ~size_t(15);
+  v.planes0 = planes ? rows_planes_needed(p) : rows_planes_in_lists(p);
+  v.sorted0 = planes ? planes : reinterpret_cast<uint2*>(reinterpret_cast<char*>(l->si0) + off);
+  v.sorted1 = planes ? planes : reinterpret_cast<uint2*>(reinterpret_cast<char*>(l->si1) + off);
+  return v;
+}
+
 // Per-feature preparation of a fit call: the two-valued features; when the
 // fit can have virtual features, which ones are (every two-valued feature
 // but feature 0, whose lists give the leaf labels) and their rows' value
@@ -666,8 +767,8 @@ View fit_view(const ct_problem* p, const ct_lists* l, const FitLayout& L) {
 // Two-valued features stand for the few-valued ones: masks are kept when at
 // least one feature in eight is two-valued.
 int prepare_features(const ct_problem* p, FitLayout* L, View* v, cudaStream_t st) {
-  CT_TRY(feature_flags(p->x_fm, p->n_rows, p->n_features, L->fbin, L->virt ? L->vval : nullptr, L->ffwork, st));
-  if (L->mask[0] && p->n_features > 64) {
+  CT_TRY(feature_flags(p->x_fm, p->n_rows, p->n_features, L->fbin, L->vval, L->ffwork, st));
+  if (!L->rows && L->mask[0] && p->n_features > 64) {
     std::vector<uint32_t> fb((p->n_features + 31) / 32);
     CT_CUDA_TRY(cudaMemcpyAsync(fb.data(), L->fbin, fb.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CT_CUDA_TRY(cudaStreamSynchronize(st));
@@ -703,24 +804,8 @@ int seed_source(const ct_problem* p, const ct_lists* l, const View& v, const voi
   return CT_OK;
 }
 
-int fit_batched(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uint32_t n_trees,
-                const FitLayout& L0, const ct_tree_buffers* trees, cudaStream_t st) {
-  FitLayout L = L0;
-  View v = fit_view(p, l, L);
-  TreeView tv = tree_view(trees, 0);
-  CT_TRY(prepare_features(p, &L, &v, st));
-  CT_CUDA_TRY(cudaMemsetAsync(L.s.ctr, 0, sizeof(Counters), st));
-  CT_CUDA_TRY(cudaMemsetAsync(L.boot_ws, 0, 16, st));
-  current_prof()->begin(CT_K_BOOTSTRAP);
-  const void* src = nullptr;
-  CT_TRY(seed_source(p, l, v, &src, st));
-  CT_TRY(bootstrap_many(p, l, 0, n_trees, first_tree, src, v.row_mask, virtual_skip(v), L.n_in, L.boot_ws,
-                        L.boot_bytes, st));
-  current_prof()->end();
-  for (uint32_t s = 0; s < n_trees; ++s) account_bootstrap(p, virtual_skip(v));
-  CT_TRY(check_boot_error(L, st));
-  begin_level(L.s.ctr, st);
-  CT_TRY(root(p, v, L, 0, n_trees, first_tree, tv, 0, st));
+// The levels of a batched fit whose roots are in list 0.
+int grow_levels(const ct_problem* p, const View& v, const FitLayout& L, const TreeView& tv, cudaStream_t st) {
   Counters h;
   if (!current_prof()->timing && !L.host_loop) {
     // Levels holding more than graph_samples samples run from the host (one
@@ -753,6 +838,36 @@ int fit_batched(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uin
     CT_TRY(read_counters(L, &h, st));
   }
   return CT_OK;
+}
+
+int fit_batched(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uint32_t n_trees,
+                const FitLayout& L0, const ct_tree_buffers* trees, cudaStream_t st) {
+  FitLayout L = L0;
+  View v = L.rows ? row_view(p, l, L, L.pair, L.ranked, L.rank, L.planes) : fit_view(p, l, L);
+  TreeView tv = tree_view(trees, 0);
+  CT_TRY(prepare_features(p, &L, &v, st));
+  CT_CUDA_TRY(cudaMemsetAsync(L.s.ctr, 0, sizeof(Counters), st));
+  if (L.rows) {
+    current_prof()->begin(CT_K_BOOTSTRAP);
+    CT_TRY(launch_row_pairs(v, p, L.pair, L.ranked, L.rank, st));
+    CT_TRY(launch_row_roots(v, p, 0, n_trees, first_tree, L.n_in, tv, L.list[0], L.tot[0], L.cap_list, L.s.ctr,
+                            L.mask[0], L.vval, st));
+    current_prof()->end();
+    account_row_roots(p, n_trees, v.vmask);
+    return grow_levels(p, v, L, tv, st);
+  }
+  CT_CUDA_TRY(cudaMemsetAsync(L.boot_ws, 0, 16, st));
+  current_prof()->begin(CT_K_BOOTSTRAP);
+  const void* src = nullptr;
+  CT_TRY(seed_source(p, l, v, &src, st));
+  CT_TRY(bootstrap_many(p, l, 0, n_trees, first_tree, src, v.row_mask, virtual_skip(v), L.n_in, L.boot_ws,
+                        L.boot_bytes, st));
+  current_prof()->end();
+  for (uint32_t s = 0; s < n_trees; ++s) account_bootstrap(p, virtual_skip(v));
+  CT_TRY(check_boot_error(L, st));
+  begin_level(L.s.ctr, st);
+  CT_TRY(root(p, v, L, 0, n_trees, first_tree, tv, 0, st));
+  return grow_levels(p, v, L, tv, st);
 }
 
 int fit_plain(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uint32_t n_trees,
@@ -967,10 +1082,16 @@ int autotune(const ct_problem* p, const ct_lists* l, uint32_t n_trees, uint32_t 
   return CT_OK;
 }
 
+// The larger of the two growth forms' workspaces: a fit takes the one it can.
 size_t fit_workspace_bytes(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o) {
-  FitLayout L;
-  layout(p, n_trees, o, nullptr, 0, &L);
-  return L.bytes;
+  FitLayout L{};
+  list_layout(p, n_trees, o, nullptr, 0, &L);
+  size_t bytes = L.bytes;
+  if (o->mode == CT_FIT_BATCHED && rows_possible(p)) {
+    row_layout(p, n_trees, o, nullptr, 0, &L);
+    bytes = std::max(bytes, L.bytes);
+  }
+  return bytes;
 }
 
 int fit(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uint32_t n_trees,
@@ -990,8 +1111,13 @@ int fit(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uint32_t n_
   CT_ARG_CHECK(l->stride >= p->n_rows, "list stride must be >= n_rows");
   const uint32_t need_slots = (o->mode == CT_FIT_PLAIN) ? 1u : n_trees;
   CT_ARG_CHECK(l->n_slots >= need_slots, "lists hold too few tree slots");
-  FitLayout L;
-  if (!layout(p, n_trees, o, reinterpret_cast<char*>(ws), wsb, &L)) {
+  // Row-list growth where the problem, the lists' alignment and the workspace
+  // allow it; a workspace sized for list growth alone still takes that.
+  FitLayout L{};
+  char* base = reinterpret_cast<char*>(ws);
+  const bool aligned = (((uintptr_t)l->si0 | (uintptr_t)l->si1) & 15u) == 0;
+  if (!(o->mode == CT_FIT_BATCHED && aligned && rows_possible(p) && row_layout(p, n_trees, o, base, wsb, &L)) &&
+      !list_layout(p, n_trees, o, base, wsb, &L)) {
     set_last_error("fit workspace too small");
     return CT_ERR_OOM;
   }
@@ -1259,7 +1385,7 @@ bool layout_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options*
 }  // namespace
 
 size_t fit_queue_workspace_bytes(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o) {
-  FitLayout L;
+  FitLayout L{};
   View* vd = nullptr;
   uint32_t* sj = nullptr;
   layout_queue(jobs, n_jobs, o, nullptr, 0, &L, &vd, &sj);
@@ -1296,7 +1422,7 @@ int check_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o
 int fit_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o, const ct_tree_buffers* trees,
               void* ws, size_t wsb, cudaStream_t st) {
   CT_TRY(check_queue(jobs, n_jobs, o, trees));
-  FitLayout L;
+  FitLayout L{};
   View* views_dev = nullptr;
   uint32_t* slot_job_dev = nullptr;
   if (!layout_queue(jobs, n_jobs, o, reinterpret_cast<char*>(ws), wsb, &L, &views_dev, &slot_job_dev)) {

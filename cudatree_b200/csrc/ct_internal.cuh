@@ -84,6 +84,28 @@ struct PartPiece {
   uint32_t npieces;
   uint32_t status;        // status column of this piece (npieces > 1)
 };
+// Row-list growth: one piece of a sorted list, its best candidate, a split.
+struct RowPiece {
+  uint32_t node;
+  uint32_t slot;          // selected slot of the node
+  uint32_t j;
+  uint32_t npieces;
+};
+struct RowBest {
+  double score;
+  uint32_t pos;
+  uint32_t pure;          // bit 0: the left side holds one class; bit 1: the right side
+  float xl;               // values at pos and pos + 1
+  float xr;
+};
+struct RowSplit {
+  uint32_t node;
+  uint32_t feature;
+  uint32_t nl;            // rows of the left child
+  uint32_t children;      // raw id of the left child
+  float xl;               // a row goes left when its value is at most xl
+  uint32_t pure;
+};
 struct Counters {
   uint32_t n_nodes;       // nodes in the current chunk
   uint32_t n_scan_pieces;
@@ -120,7 +142,7 @@ struct Counters {
 // and its loop graph, not per step (subtrees run after the level loop).
 enum : uint32_t {
   ITEM_SELECT, ITEM_HIST, ITEM_CARRY, ITEM_SCAN, ITEM_TWO_VALUED, ITEM_REDUCE, ITEM_PLAN, ITEM_FILL,
-  ITEM_CHILDREN, ITEM_VPIECES, ITEM_VCOUNT, ITEM_STEP_SLOTS, ITEM_SUBTREE = ITEM_STEP_SLOTS,
+  ITEM_CHILDREN, ITEM_VPIECES, ITEM_VCOUNT, ITEM_MOVE, ITEM_BITS, ITEM_STEP_SLOTS, ITEM_SUBTREE = ITEM_STEP_SLOTS,
   ITEM_SUBTREE_WIDE
 };
 __device__ __forceinline__ void reset_step_counters(Counters* c, uint32_t n_nodes) {
@@ -254,6 +276,24 @@ struct View {
   uint32_t slot_base;
   uint32_t sel_stride;
   uint32_t mask_stride;
+  // Row-list growth (ct_rows.cu): a tree keeps one list, its rows in row
+  // order (entries row | label << lab_shift, 32 bits whatever the problem's
+  // index width), and a node's sorted order of a feature is made only when
+  // the node selects that feature, from the feature's ranks.  rl[b]: the row
+  // lists of buffer b, [n_slots][stride]; pair[f * n_rows + row] = (position
+  // of row in feature f's presort, bits of x[f][row]) and ranked[f * n_rows +
+  // p] = (bits of the p-th smallest value, its row's label), not written for
+  // virtual features; sorted plane k ([n_slots][stride] (value bits, label))
+  // holds the sorted lists of the nodes' k-th selected features: planes
+  // [0, planes0) at sorted0, the others at sorted1.  rl[0] NULL: the lists
+  // of every feature are kept (list growth).
+  uint32_t* rl[2];
+  const uint2* pair;
+  const uint2* ranked;
+  const uint32_t* rank;   // the ranks alone, [n_features][n_rows] by row
+  uint2* sorted0;
+  uint2* sorted1;
+  uint32_t planes0;
 };
 // `const View& V`: the view of the job that owns tree slot SLOT.  In a
 // kernel instantiated for a queue (template flag Q) it is that job's entry
@@ -307,6 +347,16 @@ __device__ __forceinline__ float ld_keep(const float* p, uint64_t pol) {
   return v;
 }
 
+// the row list of a node (row-list growth)
+__device__ __forceinline__ uint32_t* row_list(const View& v, uint32_t buf, uint32_t slot) {
+  return v.rl[buf] + (size_t)(slot - v.slot_base) * v.stride;
+}
+// the sorted list of a node's k-th selected feature (row-list growth)
+__device__ __forceinline__ uint2* sorted_list(const View& v, uint32_t slot, uint32_t k) {
+  uint2* base = k < v.planes0 ? v.sorted0 : v.sorted1;
+  const size_t plane = k < v.planes0 ? k : k - v.planes0;
+  return base + (plane * v.n_slots + (slot - v.slot_base)) * v.stride;
+}
 template <typename IdxT>
 __device__ __forceinline__ IdxT* list_ptr(const View& v, uint32_t buf, uint32_t slot, uint32_t f) {
   IdxT* base = reinterpret_cast<IdxT*>(buf ? v.si1 : v.si0);
@@ -395,6 +445,33 @@ struct LevelScratch {
   uint32_t* vcls;         // [cap_nodes][n_features][n_classes] those rows by class
   uint2* vpieces;         // [cap_vpieces] (node, piece) of the nodes' row lists
   uint32_t cap_vpieces;
+  // Row-list growth (carve_row_scratch), else NULL / 0.  Counters fields it
+  // counts with: n_small_segs (warp items), n_carry (order items),
+  // n_scan_pieces (pieces), n_part_pieces (one-piece splits), n_status (mpart),
+  // n_big_segs (big_nodes), n_tv (bunits), n_tiles (bzero), n_huge_segs (gsmall),
+  // n_hchains (glarge), n_bchains (citems).
+  uint2* witems;          // [cap_w] (node, selected slot) of nodes of at most WARP_ROWS rows
+  uint32_t cap_w;
+  uint2* gsmall;          // [cap_order] (node, selected slot) of k_row_group's smaller and larger nodes
+  uint2* glarge;
+  uint2* oitems;          // [cap_order] (node, selected slot) whose sorted list k_row_order makes
+  uint32_t cap_order;
+  uint4* bunits;          // [cap_units] (node, selected slot, slice | slices << 16, first piece) of the rank bitmaps k_row_bits makes
+  uint32_t cap_units;
+  uint4* bzero;           // [cap_order] (node, selected slot, first piece, pieces) whose bitmap several slices
+                          // share: zeroed first
+  uint2* citems;          // [cap_order] (first piece, pieces) of every list of several pieces
+  RowPiece* rpieces;      // [cap_scan] pieces of sorted lists and bitmaps; carry rows are indexed alike
+  RowBest* rbest;         // [cap_nodes][sel_stride] best of the warp items, then [cap_scan] of the pieces
+  uint32_t* node_q;       // [cap_nodes] bits of the largest gain known of the node's candidates (seq_scan)
+  RowSplit* rsplits;      // [cap_nodes]
+  PartPiece* mpart;       // [cap_mpart] row pieces of splits of more than PART_PIECE rows
+  uint32_t* mbits;        // [cap_mpart][PART_ROUNDS] their left flags
+  uint32_t* mleft;        // [cap_mpart] their left counts
+  uint32_t* msup;         // [cap_mpart] left counts of 32 pieces together (entry base + j / 32)
+  uint32_t cap_mpart;
+  uint32_t* big_nodes;    // [cap_big] nodes k_row_select_big selects for
+  uint32_t cap_big;
 };
 __device__ __forceinline__ bool masked(uint64_t m, uint32_t f) { return f < 64 && ((m >> f) & 1u); }
 // words of one node's constant-feature mask
@@ -539,6 +616,29 @@ int launch_subtrees(const View& v, uint32_t ib, uint32_t lb, const ct_node* smal
 int launch_seg_partition(uint32_t index_bytes, const PartWork& w, uint64_t bound_small, uint64_t bound_tiles,
                          cudaStream_t st);
 PartWork level_part_work(const View& v, const LevelScratch& s);
+
+// Row-list growth (ct_rows.cu).  Whether a problem's trees can grow that way,
+// and whether its sorted lists fit behind the row lists in the caller's list
+// buffers (else they take row_planes_bytes of workspace).
+bool rows_possible(const ct_problem* p);
+uint32_t rows_planes_in_lists(const ct_problem* p);
+uint32_t rows_planes_needed(const ct_problem* p);
+bool carve_row_scratch(Arena& a, const View& v, LevelBounds b, uint32_t scan_piece, LevelScratch* s, bool virt);
+int launch_row_pairs(const View& v, const ct_problem* p, uint2* pair, uint2* ranked, uint32_t* rank, cudaStream_t st);
+bool rows_have_large(uint32_t n_rows);  // some node may take a bitmap or an order item (rank and ranked are needed)
+int launch_row_roots(const View& v, const ct_problem* p, uint32_t slot_lo, uint32_t n_slots, uint32_t tree_lo,
+                     uint32_t* n_in, const TreeView& tv, ct_node* out, uint32_t* out_tot, uint32_t cap, Counters* ctr,
+                     uint64_t* out_mask, const float2* vals, cudaStream_t st);
+// One level step: selection, split search, split of the row lists, children.
+// n_max: the most rows of any tree (a step whose nodes all fit a warp item
+// launches no order and piece kernels).
+int launch_row_step(const View& v, const LevelScratch& s, LevelBounds b, uint32_t n_max,
+                    const TreeView& tv, uint32_t cap_next, uint32_t small_cut, ct_node* small, uint32_t cap_small,
+                    cudaStream_t st);
+int launch_row_subtrees(const View& v, const ct_node* small, uint32_t cap_small, uint32_t bound, const LevelScratch& s,
+                        const TreeView& tv, cudaStream_t st);
+// Virtual-feature counts of a step's nodes (ct_level.cu).
+int launch_virtual_counts(const View& v, const LevelScratch& s, uint64_t nodes, uint64_t vpieces, cudaStream_t st);
 
 // Start of a step (device-side, stream ordered): per-step counters reset,
 // n_nodes and the step's lists set.

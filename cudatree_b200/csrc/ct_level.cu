@@ -22,47 +22,13 @@
 #include <algorithm>
 #include <cfloat>
 
-#include "ct_internal.cuh"
+#include "ct_items.cuh"
 
 namespace ct {
 
 namespace {
 
 constexpr uint32_t SCAN_BATCH = 4;  // rounds of 32 whose loads are issued together
-
-__device__ __forceinline__ double dinf() { return __longlong_as_double(0x7ff0000000000000ll); }
-
-__device__ __forceinline__ uint32_t global_warp() {
-  return (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-}
-__device__ __forceinline__ uint32_t total_warps() { return (gridDim.x * blockDim.x) >> 5; }
-
-// Items of a warp-per-item launch.  A warp takes item global_warp() first;
-// when the grid does not cover every item (a persistent launch), it then
-// claims the items past the grid in order from a counter, so uneven items
-// balance as they do with one warp per item.  Warp-collective.
-template <typename F>
-__device__ __forceinline__ void for_items(uint32_t count, uint32_t* claim, F item) {
-  const uint32_t nw = total_warps();
-  uint32_t w = global_warp();
-  while (w < count) {
-    item(w);
-    __syncwarp();
-    if (nw >= count) break;
-    uint32_t k = 0;
-    if (lane_id() == 0) k = atomicAdd(claim, 1u);
-    w = nw + __shfl_sync(FULL, k, 0);
-  }
-}
-
-__device__ __forceinline__ uint32_t read_error(const Counters* c) {
-  return *reinterpret_cast<const volatile uint32_t*>(&c->error);
-}
-// Work-list count clamped to its capacity; 0 once an earlier kernel of the
-// step flagged an error, so no kernel reads a record that was not written.
-__device__ __forceinline__ uint32_t live_count(const LevelScratch& s, uint32_t count, uint32_t cap) {
-  return read_error(s.ctr) ? 0u : min(count, cap);
-}
 
 // (score, pos) lexicographic minimum across the warp.
 __device__ __forceinline__ void warp_argmin2(double& score, uint32_t& pos, float& p, float& q) {
@@ -130,7 +96,9 @@ __device__ __forceinline__ void vcount_item(const View& v, const StepLists& list
   const uint32_t C = v.n_classes, fc = v.n_features * C;
   const uint2 pc = s.vpieces[pi];
   const ct_node nd = lists.nodes[pc.x];
-  const IdxT* rl = list_ptr<IdxT>(v, nd.buf, nd.slot, v.vslot) + nd.start;
+  const IdxT* rl =
+      (v.rl[0] ? reinterpret_cast<const IdxT*>(row_list(v, nd.buf, nd.slot)) : list_ptr<IdxT>(v, nd.buf, nd.slot, v.vslot)) +
+      nd.start;
   const uint32_t lo = pc.y * VPIECE;
   const uint32_t hi = min(lo + VPIECE, nd.n);
   for (uint32_t i = lane; i < fc; i += 32) cnt[i] = 0;
@@ -1575,22 +1543,6 @@ __global__ void k_reset_step(Counters* c, uint32_t n_nodes, StepLists* step, Ste
 
 inline uint32_t clamp32(uint64_t x) { return x > 0xffffffffull ? 0xffffffffu : (uint32_t)x; }
 
-// Blocks of a warp-per-item launch: one warp per item, or, for a launch that
-// must not depend on the item count (persistent), at most the blocks that
-// are resident at once, whose warps then loop over the items.
-template <typename K>
-uint32_t grid_for(K kernel, uint64_t warps, size_t smem, bool persistent) {
-  uint32_t cap = 0;
-  if (persistent) {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, THREADS_PER_BLOCK, smem);
-    cap = (uint32_t)std::max(1, sms) * (uint32_t)std::max(1, per);
-  }
-  return item_blocks(warps, cap);
-}
-
 template <typename IdxT, typename LabT, bool Q>
 void split_impl(const View& v, const LevelScratch& s, const LevelCaps& caps, uint32_t scan_piece, bool persistent,
                 cudaStream_t st) {
@@ -1718,6 +1670,14 @@ static size_t carve_or_size(Arena& a, const View& v, const LevelCaps& c, LevelSc
   t.vcls = virt ? a.take<uint32_t>((size_t)c.nodes * v.n_features * C) : nullptr;
   t.vpieces = virt ? a.take<uint2>(c.vpieces) : nullptr;
   t.cap_vpieces = virt ? c.vpieces : 0u;
+  t.witems = nullptr;
+  t.oitems = nullptr;
+  t.rpieces = nullptr;
+  t.rbest = nullptr;
+  t.rsplits = nullptr;
+  t.mpart = nullptr;
+  t.mbits = t.mleft = t.msup = t.big_nodes = nullptr;
+  t.cap_w = t.cap_order = t.cap_mpart = t.cap_big = 0;
   if (s) *s = t;
   return a.used;
 }
@@ -1807,6 +1767,16 @@ int launch_children(const View& v, uint32_t ib, uint32_t lb, const LevelScratch&
                     cudaStream_t st) {
   return v.jobs ? launch_children_q<true>(v, ib, lb, s, b, tv, cap_next, small_cut, small, cap_small, persistent, st)
                 : launch_children_q<false>(v, ib, lb, s, b, tv, cap_next, small_cut, small, cap_small, persistent, st);
+}
+
+// Row-list growth's virtual counts: entries are 32 bits and carry the label.
+int launch_virtual_counts(const View& v, const LevelScratch& s, uint64_t nodes, uint64_t vpieces, cudaStream_t st) {
+  const size_t smv = (size_t)WARPS_PER_BLOCK * v.n_features * v.n_classes * sizeof(uint32_t);
+  k_vpieces<<<grid_for(k_vpieces, nodes, 0, true), THREADS_PER_BLOCK, 0, st>>>(v, s);
+  k_vcount<uint32_t, uint8_t><<<grid_for(k_vcount<uint32_t, uint8_t>, vpieces, smv, true), THREADS_PER_BLOCK, smv, st>>>(
+      v, s);
+  CT_CUDA_TRY(cudaGetLastError());
+  return CT_OK;
 }
 
 template <bool Q>
@@ -2009,6 +1979,12 @@ View make_view(const ct_problem* p, const ct_lists* l) {
   v.slot_base = 0;
   v.sel_stride = p->max_features;
   v.mask_stride = mask_words(p->n_features);
+  v.rl[0] = v.rl[1] = nullptr;
+  v.pair = nullptr;
+  v.ranked = nullptr;
+  v.rank = nullptr;
+  v.sorted0 = v.sorted1 = nullptr;
+  v.planes0 = 0;
   return v;
 }
 

@@ -1,0 +1,2437 @@
+// Row-list growth: the batched fit's level step without per-feature lists.
+//
+// A tree keeps one list, its rows in row order.  A node splits on one of the
+// m features it selects, so keeping every feature's list sorted per node
+// (list growth, ct_level.cu + ct_partition.cu) moves F lists per level for m
+// that are scanned.  Here a node's sorted order of a feature is made when the
+// node selects it, from the row's rank in the feature's presort (View::pair,
+// built once per fit), and only the row list is partitioned.
+//
+//   k_row_pairs    (rank, value) of every (feature, row)
+//   k_row_roots    in-bag rows of each tree, its row list and root node
+//                  (reference bootstrap_fill.cu + bootstrap_reshuffle.cu)
+//   k_row_select   feature subset of each node: constancy from the node's rows
+//   k_row_select_big  the same for large nodes with features that look constant
+//   k_row_warp     nodes of at most WARP_ROWS rows: one warp sorts one
+//                  (node, feature) in registers and scans it
+//   k_row_group    nodes of at most GROUP_ROWS rows: the same by one CTA
+//   k_row_bits     larger nodes, by a bitmap over the feature's ranks, which
+//                  stands for the sorted list of a node with one row in 64
+//   k_row_order    larger nodes that are sparser: their list, from such a bitmap
+//   k_row_hist, k_row_carry, k_row_scan  the Gini scan of those lists and bitmaps
+//                  in pieces (reference compute_2d, dfs_module.cu:310-443)
+//   k_row_reduce   best candidate of each node; node record, children, work list
+//   k_row_mark     left flags and class counts; moves the rows of small splits
+//   k_row_move     stable split of the row lists of larger ones
+//   k_row_children child records for the next step
+//   k_row_subtree  subtrees of at most 32 rows, one warp each
+//
+// Measured on one B200 (ct_fit): 581,012 x 54 covtype-shaped rows, 100 trees
+// 62.5 -> 42.6 ms; 10,000 x 3,000 rows, 100 classes, 200 trees 202 -> 46.7 ms
+// (the lists of 3,000 features were partitioned per level for 55 scanned); 200,003 x
+// 28 continuous columns, 50 trees 14.2 -> 8.0 ms; 1,797 x 64, 50 trees 1.44 ->
+// 0.67 ms.  What bounds each kernel stands at it.
+//
+// Rows of equal value may come in any order in a sorted list: no candidate
+// lies between them, and a candidate's class counts depend only on the set of
+// rows up to it, so the splits are those of the presorted lists.
+#include <algorithm>
+#include <cfloat>
+
+#include "ct_items.cuh"
+
+namespace ct {
+
+namespace {
+
+constexpr uint32_t WARP_ROWS = 512;      // nodes up to this size: one warp per (node, feature)
+constexpr uint32_t WARP_ROWS_BITS = 9;
+constexpr uint32_t GROUP_ROWS = 9216;    // nodes up to this size: one CTA per (node, feature)
+constexpr uint32_t GROUP_SMALL_ROWS = 2048;  // the smaller of these nodes take a smaller CTA
+constexpr int GROUP_SMALL_WARPS = 8;
+constexpr int GROUP_WARPS = 16;
+constexpr uint32_t SELECT_ROWS = 2048;   // a selecting warp checks at most this many rows of a larger node
+constexpr int ORDER_THREADS = 512;
+constexpr uint32_t ORDER_SMEM_MAX = 224u * 1024u;
+
+// Shared memory of k_row_order: the rank bitmap, then a prefix count per word
+// (16 bits) or per four words (32 bits) in as many bytes.
+__host__ __device__ __forceinline__ uint32_t order_words(uint32_t n_rows) { return ((n_rows + 127) / 128) * 4; }
+__host__ __device__ __forceinline__ size_t order_smem(uint32_t n_rows) { return (size_t)order_words(n_rows) * 6; }
+
+// Nodes whose rank bitmap (over all ranks) stands for their sorted list: those
+// with at least about one row in 64, so that the bitmap takes no more room
+// than the list would (it is kept in the list's place) and a scan meets a row
+// in every other word.  Their pieces are runs of ranks.
+__host__ __device__ __forceinline__ bool row_dense(uint32_t n, uint32_t n_rows) {
+  return n > GROUP_ROWS && 8u * (size_t)n >= (size_t)order_words(n_rows) * 4 + 16;
+}
+// Ranks of one piece of a bitmap: a power of two of about as many rows as a
+// list's piece, at least a 1,024-rank window, at most what 16 bits can list.
+__device__ __forceinline__ uint32_t dense_chunk(uint32_t n, uint32_t n_rows, uint32_t scan_piece) {
+  const uint64_t ranks = (uint64_t)scan_piece * n_rows / n;
+  return ranks >= 32768u ? 32768u : ranks <= 1024u ? 1024u : 1u << (31 - __clz((int)ranks));
+}
+constexpr uint32_t BITS_SLICE = 32768;   // rows per k_row_bits unit
+constexpr int BITS_THREADS = 512;
+constexpr uint32_t BITS_COUNTS = 4096;   // pieces x classes that k_row_bits counts itself (else k_row_hist does)
+
+__device__ __forceinline__ uint32_t* rank_bits(const View& v, const ct_node& nd, uint32_t slot) {
+  return reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(sorted_list(v, nd.slot, slot) + nd.start) + 15) &
+                                     ~uintptr_t(15));
+}
+
+constexpr uint32_t SEQ_CLASSES = 8;  // most classes of the lane-sequential scan (seq_scan)
+
+// A candidate's gain n / (nl nr) sum_c (L_c - nl T_c / n)^2 is what its split
+// takes off n times the node's Gini impurity: the score is (const - gain) / n,
+// so the order of the gains is that of the scores.  Kept as 1 + gain in a
+// positive float (whose bits order as it does).  An estimate is off by less
+// than 6e-7 of itself (conversions and approximate reciprocals in fp32) plus
+// 4e-15 n^2 (fp64 rounding of sums of up to n^2 that cancel).
+__device__ __forceinline__ float gain_bound(float known, uint32_t n) {
+  return known * (1.0f - 2e-6f) - 8e-15f * (float)n * (float)n;
+}
+__device__ __forceinline__ float gain_of(double d, float nl, float nr, float n) {
+  return 1.0f + (float)d * __fdividef(n, nl * nr);
+}
+// At a position with `left` class counts, nl rows in all.
+__device__ __forceinline__ float gain_at(const uint32_t* left, const uint32_t* total, uint32_t C, uint32_t nl,
+                                         uint32_t n) {
+  const double t = (double)nl / (double)n;
+  double d = 0.0;
+  for (uint32_t c = 0; c < C; ++c) {
+    const double u = (double)left[c] - t * (double)total[c];
+    d += u * u;
+  }
+  return gain_of(d, (float)nl, (float)(n - nl), (float)n);
+}
+
+// Lane holding the warp's lowest (score, pos): two 32-bit minima over the
+// score's bits (scores are >= 0 or +inf, so their bits order as they do), one
+// over the positions.  All lanes get the lane id; NONE when no lane has a
+// finite score.
+__device__ __forceinline__ uint32_t warp_best_lane(double score, uint32_t pos) {
+  const uint64_t b = (uint64_t)__double_as_longlong(score);
+  const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
+  const uint32_t mhi = __reduce_min_sync(FULL, hi);
+  if (mhi >= 0x7ff00000u) return NONE;
+  const uint32_t mlo = __reduce_min_sync(FULL, hi == mhi ? lo : 0xffffffffu);
+  const bool tie = hi == mhi && lo == mlo;
+  const uint32_t mp = __reduce_min_sync(FULL, tie ? pos : 0xffffffffu);
+  return (uint32_t)__ffs(__ballot_sync(FULL, tie && pos == mp)) - 1;
+}
+
+// Exact score of a candidate (the scan's arithmetic, ct_level.cu).
+struct Scored {
+  double score;
+  uint32_t pure;
+};
+__device__ __forceinline__ Scored score_at(int64_t sl, int64_t sr, uint32_t nl, double nn) {
+  const double l = (double)nl;
+  const double gl = gini_part(sl, l, nn);
+  const double gr = gini_part(sr, __dsub_rn(nn, l), nn);
+  return Scored{__dadd_rn(gl, gr), (gl == 0.0 ? 1u : 0u) | (gr == 0.0 ? 2u : 0u)};
+}
+
+// ------------------------------------------------------------------------
+// (rank, value bits) by row and (value bits, label) by rank, of the features
+// that keep a presort order.
+template <typename IdxT, typename LabT>
+__global__ void k_row_pairs(const IdxT* __restrict__ presort, const float* __restrict__ x_fm,
+                            const LabT* __restrict__ labels, uint32_t n, uint64_t vmask, uint2* __restrict__ pair,
+                            uint2* __restrict__ ranked, uint32_t* __restrict__ rank) {
+  const uint32_t f = blockIdx.y;
+  if (f < 64 && ((vmask >> f) & 1ull)) return;
+  const size_t off = (size_t)f * n;
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
+    const uint32_t row = presort[off + p];
+    const uint32_t x = __float_as_uint(__ldg(x_fm + off + row));
+    pair[off + row] = make_uint2(p, x);
+    if (rank) rank[off + row] = p;
+    if (ranked) ranked[off + p] = make_uint2(x, (uint32_t)__ldg(labels + row));
+  }
+}
+
+// Class of the first row, in feature 0's order, of `n` listed rows: the leaf
+// rule.  Warp-collective.
+__device__ __forceinline__ uint32_t first_row_class(const View& v, const uint32_t* rows, uint32_t n) {
+  uint64_t best = ~0ull;
+  for (uint32_t i0 = 0; i0 < n; i0 += 32 * 8) {
+    uint32_t e[8], k[8];
+#pragma unroll
+    for (uint32_t r = 0; r < 8; ++r) {
+      const uint32_t i = i0 + r * 32 + lane_id();
+      e[r] = i < n ? rows[i] : NONE;
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < 8; ++r) k[r] = i0 + r * 32 + lane_id() < n ? v.pair[entry_row(v, e[r])].x : NONE;
+#pragma unroll
+    for (uint32_t r = 0; r < 8; ++r)
+      if (i0 + r * 32 + lane_id() < n) best = min(best, ((uint64_t)k[r] << 32) | (e[r] >> v.lab_shift));
+  }
+  const uint32_t hi = (uint32_t)(best >> 32);
+  const uint32_t m = __reduce_min_sync(FULL, hi);
+  return __reduce_min_sync(FULL, hi == m ? (uint32_t)best : NONE);
+}
+
+__device__ __forceinline__ void write_leaf(const TreeView& tv, size_t at, uint32_t value) {
+  tv.left[at] = 0;
+  tv.right[at] = 0;
+  tv.feature[at] = 0;
+  tv.threshold[at] = 0.f;
+  tv.value[at] = value;
+}
+
+// One CTA per tree: the in-bag rows as a bitmap in shared memory (a draw is
+// one atomic there), then the row list in row order, the root's class counts
+// and its record (a leaf if it holds fewer than min_samples_split rows).
+template <typename LabT>
+__global__ void __launch_bounds__(1024) k_row_roots(View v, uint64_t seed, uint32_t bootstrap, uint32_t slot_lo,
+                                                    uint32_t tree_lo, uint32_t* n_in, TreeView tv, ct_node* out,
+                                                    uint32_t* out_tot, uint32_t cap, Counters* ctr,
+                                                    uint64_t* out_mask, const float2* vals) {
+  extern __shared__ __align__(16) uint32_t root_smem[];
+  __shared__ uint32_t s_wcnt[32];
+  __shared__ uint32_t s_idx, s_min;
+  const uint32_t slot = slot_lo + blockIdx.x, N = v.n_rows, C = v.n_classes;
+  const uint32_t words = (N + 31) / 32;
+  uint32_t* bm = root_smem;
+  uint32_t* hist = root_smem + words;
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const LabT* labels = reinterpret_cast<const LabT*>(v.labels);
+  for (uint32_t w = threadIdx.x; w < words; w += blockDim.x)
+    bm[w] = bootstrap ? 0u : (w * 32 + 32 <= N ? FULL : (1u << (N & 31)) - 1u);
+  for (uint32_t c = threadIdx.x; c < C; c += blockDim.x) hist[c] = 0;
+  __syncthreads();
+  const uint64_t tkey = tree_key(seed, tree_lo + blockIdx.x);
+  if (bootstrap) {
+    const uint64_t bk = boot_key(tkey);
+    for (uint32_t i = threadIdx.x; i < N; i += blockDim.x) {
+      const uint32_t r = boot_draw(bk, i, N);
+      atomicOr(&bm[r >> 5], 1u << (r & 31));
+    }
+    __syncthreads();
+  }
+  const uint32_t per = ceil_div(words, nwarps);
+  const uint32_t wlo = min(warp * per, words), whi = min(wlo + per, words);
+  uint32_t c = 0;
+  for (uint32_t w = wlo + lane; w < whi; w += 32) c += __popc(bm[w]);
+  c = __reduce_add_sync(FULL, c);
+  if (lane == 0) s_wcnt[warp] = c;
+  __syncthreads();
+  uint32_t pos = 0, n = 0;
+  for (uint32_t k = 0; k < nwarps; ++k) {
+    pos += k < warp ? s_wcnt[k] : 0u;
+    n += s_wcnt[k];
+  }
+  uint32_t* rows = row_list(v, 0, slot);
+  const unsigned lt = lanemask_lt();
+  for (uint32_t w0 = wlo; w0 < whi; w0 += 4) {
+    uint32_t lab[4], bits[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      bits[k] = w0 + k < whi ? bm[w0 + k] : 0u;
+      lab[k] = (bits[k] >> lane) & 1u ? (uint32_t)labels[(w0 + k) * 32 + lane] : NONE;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      const unsigned grp = __match_any_sync(FULL, lab[k]);
+      if (lab[k] != NONE) {
+        rows[pos + __popc(bits[k] & lt)] = ((w0 + k) * 32 + lane) | (lab[k] << v.lab_shift);
+        if ((grp & lt) == 0u) atomicAdd(&hist[lab[k]], (uint32_t)__popc(grp));
+      }
+      pos += __popc(bits[k]);
+    }
+  }
+  if (threadIdx.x == 0) {
+    s_idx = NONE;
+    s_min = NONE;
+    n_in[slot] = n;
+    tv.n_nodes[slot + tv.slot_base] = 1;
+    if (n >= v.mss && n > 0) {
+      const uint32_t idx = atomicAdd(&ctr->n_next, 1u);
+      if (idx < cap) {
+        ct_node nd;
+        nd.slot = slot;
+        nd.start = 0;
+        nd.n = n;
+        nd.raw_id = 0;
+        nd.key = root_key(tkey);
+        nd.impurity = 1.0f;
+        nd.buf = 0;
+        out[idx] = nd;
+        atomicAdd(&ctr->next_total, (unsigned long long)n);
+        s_idx = idx;
+      } else {
+        atomicOr(&ctr->error, DEV_ERR_CAPACITY);
+      }
+    }
+  }
+  __syncthreads();
+  if (s_idx != NONE) {
+    for (uint32_t k = threadIdx.x; k < C; k += blockDim.x) out_tot[(size_t)s_idx * C + k] = hist[k];
+    if (out_mask)  // features constant over the whole data
+      for (uint32_t k = threadIdx.x; k < mask_words(v.n_features); k += blockDim.x) {
+        uint64_t m = 0;
+        for (uint32_t f = k * 64; f < min(k * 64 + 64, v.n_features); ++f)
+          m |= (uint64_t)(vals[f].x == vals[f].y) << (f & 63);
+        out_mask[(size_t)s_idx * v.mask_stride + k] = m;
+      }
+  } else if (n < v.mss || n == 0) {  // a leaf: the class of its first row in feature 0's order
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) atomicMin(&s_min, v.pair[entry_row(v, rows[i])].x);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
+      if (v.pair[entry_row(v, rows[i])].x == s_min)
+        write_leaf(tv, (size_t)(slot + tv.slot_base) * tv.capacity, rows[i] >> v.lab_shift);
+    if (n == 0 && threadIdx.x == 0) write_leaf(tv, (size_t)(slot + tv.slot_base) * tv.capacity, 0u);
+  }
+}
+
+// ------------------------------------------------------------------------
+// Selection.  The first m non-constant features of the node's permutation
+// (the rule of k_select); a feature varies in a node when two of its rows
+// differ in it.  A lane takes one feature and compares four of the node's
+// rows, which settles nearly every feature that varies; the others are read
+// row by row (CTA: by the whole block) until two values differ.  Features
+// found constant go into the node's mask, which its descendants inherit.
+template <bool CTA>
+__device__ __forceinline__ bool rows_vary(const View& v, const uint32_t* rows, const float* xf, uint32_t n, float x0) {
+  const uint32_t tid = CTA ? threadIdx.x : lane_id(), nt = CTA ? blockDim.x : 32u;
+  for (uint32_t i0 = 0; i0 < n; i0 += nt * 4) {
+    bool d = false;
+    uint32_t r[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+      const uint32_t i = i0 + k * nt + tid;
+      r[k] = i < n ? entry_row(v, rows[i]) : NONE;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) d |= r[k] != NONE && __ldg(xf + (r[k] != NONE ? r[k] : 0u)) != x0;
+    if (CTA ? __syncthreads_or(d) : __any_sync(FULL, d)) return true;
+  }
+  return false;
+}
+
+// Zeroes a bitmap that several slices fill, and its pieces' class counts.
+__device__ __forceinline__ void zero_bits(const View& v, const ct_node& nd, uint32_t slot, uint32_t* counts, uint32_t nc,
+                                          uint32_t tid, uint32_t nt) {
+  uint4* b4 = reinterpret_cast<uint4*>(rank_bits(v, nd, slot));
+  for (uint32_t g = tid; g < order_words(v.n_rows) / 4; g += nt) b4[g] = make_uint4(0u, 0u, 0u, 0u);
+  if (nc <= BITS_COUNTS)
+    for (uint32_t i = tid; i < nc; i += nt) counts[i] = 0;
+}
+
+// CTA: every warp of the block selects alike, warp 0 writes.
+template <bool Q, bool CTA>
+__device__ __forceinline__ void row_select_item(const View& vb, const StepLists& lists, const LevelScratch& s,
+                                                uint32_t w) {
+  const uint32_t lane = lane_id();
+  const ct_node nd = lists.nodes[w];
+  CT_JOB_VIEW(v, vb, nd.slot);
+  const uint32_t m = v.max_features, n = nd.n;
+  const bool writer = !CTA || threadIdx.x < 32;
+  uint64_t* cmask = lists.node_mask ? const_cast<uint64_t*>(lists.node_mask) + (size_t)w * v.mask_stride : nullptr;
+  const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
+  const uint32_t limit = CTA || n <= SELECT_ROWS ? n : SELECT_ROWS;
+  uint32_t taken = 0;
+  uint64_t vsel = 0;  // selected slots that hold virtual features (m <= 64 when there are any)
+  if (n >= 2) {
+    uint32_t r[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) r[j] = entry_row(v, rows[(uint64_t)j * (n - 1) / 3]);
+    for (uint32_t i0 = 0; i0 < v.n_features && taken < m; i0 += 32) {
+      const uint32_t i = i0 + lane;
+      bool usable = false, virt = false, unknown = false;
+      uint32_t f = 0;
+      if (i < v.n_features) {
+        f = feature_perm(i, v.n_features, nd.key, v.feistel_h);
+        virt = is_virtual(v, f);
+        if (virt) {  // some but not all rows take the high value
+          const uint32_t nb = s.vcnt[(size_t)w * 64 + f];
+          usable = nb > 0 && nb < n;
+        } else if (!mask_bit(cmask, f)) {
+          const float* xf = v.x_fm + (size_t)f * v.n_rows;
+          const float x0 = xf[r[0]];
+          usable = xf[r[1]] != x0 || xf[r[2]] != x0 || xf[r[3]] != x0;
+          unknown = !usable && n > 4;
+        }
+      }
+      unsigned ok = __ballot_sync(FULL, usable);
+      for (unsigned um = __ballot_sync(FULL, unknown); um; um &= um - 1) {
+        const uint32_t u = (uint32_t)__ffs(um) - 1;
+        if (taken + __popc(ok & ((1u << u) - 1u)) >= m) break;
+        const uint32_t fu = __shfl_sync(FULL, f, u);
+        const float* xf = v.x_fm + (size_t)fu * v.n_rows;
+        if (rows_vary<CTA>(v, rows, xf, limit, xf[r[0]])) {
+          ok |= 1u << u;
+        } else if (limit < n) {  // undecided: the block form selects for this node
+          if (lane == 0) {
+            const uint32_t b = atomicAdd(&s.ctr->n_big_segs, 1u);
+            if (b < s.cap_big) s.big_nodes[b] = w;
+            else atomicOr(&s.ctr->error, DEV_ERR_CAPACITY);
+          }
+          return;
+        } else if (cmask && writer && lane == 0) {
+          cmask[fu >> 6] |= 1ull << (fu & 63);
+        }
+      }
+      usable = (ok >> lane) & 1u;
+      const uint32_t rank = __popc(ok & lanemask_lt());
+      const bool keep = usable && taken + rank < m;
+      if (keep && writer) s.sel[(size_t)w * v.sel_stride + taken + rank] = f;
+      const uint64_t b = (keep && virt) ? 1ull << ((taken + rank) & 63) : 0ull;
+      vsel |= ((uint64_t)__reduce_or_sync(FULL, (uint32_t)(b >> 32)) << 32) | __reduce_or_sync(FULL, (uint32_t)b);
+      taken += min((uint32_t)__popc(ok), m - taken);
+    }
+  }
+  if (!writer) return;
+  // work items of the slots that need a sorted order (virtual ones are scored from counts)
+  const uint32_t tmat = taken - (uint32_t)__popcll(vsel);
+  const bool small = n <= WARP_ROWS, group = !small && n <= GROUP_ROWS, dense = row_dense(n, v.n_rows);
+  const bool narrow = n <= GROUP_SMALL_ROWS;
+  const uint32_t pps = small || group ? 1u : dense ? ceil_div(v.n_rows, dense_chunk(n, v.n_rows, lists.scan_piece)) : ceil_div(n, lists.scan_piece);
+  const uint32_t slices = dense ? ceil_div(n, BITS_SLICE) : 0u;
+  // the largest gain of the node's virtual candidates: a start for its scans' bound
+  uint32_t q0 = 0;
+  if (vsel && !small && vb.n_classes <= SEQ_CLASSES) {
+    __syncwarp();  // the slots' features, written by other lanes
+    for (uint32_t q = lane; q < taken; q += 32) {
+      if (!((vsel >> q) & 1ull)) continue;
+      const uint32_t f = s.sel[(size_t)w * v.sel_stride + q];
+      if (!is_candidate_sorted(v.vval[f].x, v.vval[f].y)) continue;
+      // from the high-value rows' counts: the gain is the same from either side
+      const float e = gain_at(s.vcls + ((size_t)w * v.n_features + f) * v.n_classes,
+                                 lists.tot + (size_t)w * v.n_classes, v.n_classes, s.vcnt[(size_t)w * 64 + f], n);
+      q0 = max(q0, __float_as_uint(e));
+    }
+    q0 = __reduce_max_sync(FULL, q0);
+  }
+  uint32_t base = 0, obase = 0, zbase = 0, cbase = 0, ok = 1;
+  if (lane == 0) {
+    if (tmat) {
+      atomicAdd(&s.ctr->scan_elems, (unsigned long long)tmat * n);
+      if (small) {
+        base = atomicAdd(&s.ctr->n_small_segs, tmat);
+        ok = base + (uint64_t)tmat <= s.cap_w;
+      } else if (group) {
+        base = atomicAdd(narrow ? &s.ctr->n_huge_segs : &s.ctr->n_hchains, tmat);
+        ok = base + (uint64_t)tmat <= s.cap_order;
+      } else {
+        base = atomicAdd(&s.ctr->n_scan_pieces, tmat * pps);
+        ok = base + (uint64_t)tmat * pps <= s.cap_scan;
+        atomicAdd(&s.ctr->part_elems, (unsigned long long)tmat * n);
+        if (pps > 1) {
+          cbase = atomicAdd(&s.ctr->n_bchains, tmat);
+          ok = ok && cbase + (uint64_t)tmat <= s.cap_order;
+        }
+        if (dense) {
+          obase = atomicAdd(&s.ctr->n_tv, tmat * slices);
+          if (!CTA && slices > 1) zbase = atomicAdd(&s.ctr->n_tiles, tmat);
+          ok = ok && obase + (uint64_t)tmat * slices <= s.cap_units && zbase + (uint64_t)tmat <= s.cap_order;
+        } else {
+          obase = atomicAdd(&s.ctr->n_carry, tmat);
+          ok = ok && obase + (uint64_t)tmat <= s.cap_order;
+        }
+      }
+      if (!ok) atomicOr(&s.ctr->error, DEV_ERR_CAPACITY);
+    }
+    s.nsel[w] = taken;
+    s.node_q[w] = q0;
+    s.piece_base[w] = base;
+    s.piece_cnt[w] = small || group || !ok ? 0u : tmat * pps;
+  }
+  base = __shfl_sync(FULL, base, 0);
+  obase = __shfl_sync(FULL, obase, 0);
+  zbase = __shfl_sync(FULL, zbase, 0);
+  cbase = __shfl_sync(FULL, cbase, 0);
+  ok = __shfl_sync(FULL, ok, 0);
+  if (!ok) return;
+  for (uint32_t k = 0; k < tmat; ++k) {  // k-th slot with a list
+    uint32_t slot = k;
+    if (vsel) {
+      slot = 0;
+      for (uint32_t left = k;; ++slot)
+        if (!((vsel >> slot) & 1ull) && left-- == 0) break;
+    }
+    if (small) {
+      if (lane == (k & 31u)) s.witems[base + k] = make_uint2(w, slot);
+      continue;
+    }
+    if (group) {
+      if (lane == (k & 31u)) (narrow ? s.gsmall : s.glarge)[base + k] = make_uint2(w, slot);
+      continue;
+    }
+    const uint32_t pb = base + k * pps;  // its first piece
+    for (uint32_t j = lane; j < pps; j += 32) s.rpieces[pb + j] = RowPiece{w, slot, j, pps};
+    if (pps > 1 && lane == 0) s.citems[cbase + k] = make_uint2(pb, pps);
+    if (dense) {
+      for (uint32_t j = lane; j < slices; j += 32)
+        s.bunits[obase + k * slices + j] = make_uint4(w, slot, j | (slices << 16), pb);
+      if (slices > 1 && lane == 0 && !CTA) s.bzero[zbase + k] = make_uint4(w, slot, pb, pps);
+      if (slices > 1 && CTA)  // a node the block form selects for: zeroed here
+        zero_bits(v, nd, slot, s.carry + (size_t)pb * vb.n_classes, pps * vb.n_classes, lane, 32);
+    } else if (lane == 0) {
+      s.oitems[obase + k] = make_uint2(w, slot);
+    }
+  }
+}
+
+template <bool Q>
+__global__ void __launch_bounds__(THREADS_PER_BLOCK) k_row_select(View v, LevelScratch s) {
+  const uint32_t count = min(s.ctr->n_nodes, s.cap_nodes);
+  const StepLists sl = *s.step;
+  for_items(count, &s.ctr->claim[ITEM_SELECT], [&](uint32_t w) { row_select_item<Q, false>(v, sl, s, w); });
+}
+
+template <bool Q>
+__global__ void __launch_bounds__(512) k_row_select_big(View v, LevelScratch s) {
+  const uint32_t count = live_count(s, s.ctr->n_big_segs, s.cap_big);
+  const StepLists sl = *s.step;
+  for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+    row_select_item<Q, true>(v, sl, s, s.big_nodes[i]);
+    __syncthreads();
+  }
+  // bitmaps that several slices fill
+  const uint32_t zeros = live_count(s, s.ctr->n_tiles, s.cap_order);
+  for (uint32_t i = blockIdx.x; i < zeros; i += gridDim.x) {
+    const uint4 z = s.bzero[i];
+    const ct_node nd = sl.nodes[z.x];
+    CT_JOB_VIEW(vj, v, nd.slot);
+    zero_bits(vj, nd, z.y, s.carry + (size_t)z.z * v.n_classes, z.w * v.n_classes, threadIdx.x, blockDim.x);
+  }
+}
+
+// ------------------------------------------------------------------------
+// Rank bitmap of a dense (node, feature): one CTA per slice of the node's rows
+// sets their rank's bits in shared memory, and counts the classes of each
+// piece's rows there.  A node of one slice stores its words and counts; the
+// slices of a larger one merge theirs into the zeroed bitmap and counts with
+// one coalesced atomic per non-empty word.  Bound by the gather of the ranks: a
+// 32-byte sector serves 8 rows in row order, 1 to 5 of them in the node.  The
+// classes counted here replace a pass over the sorted rows: covtype-shaped, 100
+// trees, 9.0 ms with ranks gathered from the (rank, value) pairs plus 5.8 ms of
+// counting -> 4.9 ms.
+__host__ __device__ __forceinline__ uint32_t bits_words(uint32_t n_rows) { return order_words(n_rows) + BITS_COUNTS; }
+
+template <bool Q>
+__global__ void __launch_bounds__(BITS_THREADS, 2) k_row_bits(View vb, LevelScratch s, uint32_t n_max) {
+  extern __shared__ __align__(16) uint32_t bits_sm[];
+  __shared__ uint32_t s_item;
+  const uint32_t count = live_count(s, s.ctr->n_tv, s.cap_units);
+  const StepLists lists = *s.step;
+  constexpr uint32_t T = BITS_THREADS, U = 8;
+  const uint32_t C = vb.n_classes;
+  uint4* bm4 = reinterpret_cast<uint4*>(bits_sm);
+  uint32_t* hist = bits_sm + order_words(n_max);
+  while (true) {
+    __syncthreads();  // the previous unit is done with the bitmap and s_item
+    if (threadIdx.x == 0) s_item = atomicAdd(&s.ctr->claim[ITEM_BITS], 1u);
+    __syncthreads();
+    if (s_item >= count) break;
+    const uint4 unit = s.bunits[s_item];
+    const uint32_t slice = unit.z & 0xffffu, slices = unit.z >> 16;
+    const ct_node nd = lists.nodes[unit.x];
+    CT_JOB_VIEW(v, vb, nd.slot);
+    const uint32_t f = s.sel[(size_t)unit.x * v.sel_stride + unit.y];
+    const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
+    const uint32_t* rf = v.rank + (size_t)f * v.n_rows;
+    const uint32_t groups = order_words(v.n_rows) / 4;
+    const uint32_t chunk = dense_chunk(nd.n, v.n_rows, lists.scan_piece), csh = 31 - __clz((int)chunk);
+    const uint32_t nc = ceil_div(v.n_rows, chunk) * C;
+    const bool counts = nc <= BITS_COUNTS;
+    const uint32_t lo = slice * BITS_SLICE, hi = min(lo + BITS_SLICE, nd.n);
+    for (uint32_t g = threadIdx.x; g < groups; g += T) bm4[g] = make_uint4(0u, 0u, 0u, 0u);
+    if (counts)
+      for (uint32_t i = threadIdx.x; i < nc; i += T) hist[i] = 0;
+    __syncthreads();
+    for (uint32_t i0 = lo + threadIdx.x; i0 < hi; i0 += T * U) {
+      uint32_t e[U], r[U];
+#pragma unroll
+      for (uint32_t k = 0; k < U; ++k) e[k] = i0 + k * T < hi ? rows[i0 + k * T] : 0u;
+#pragma unroll
+      for (uint32_t k = 0; k < U; ++k) r[k] = i0 + k * T < hi ? __ldg(rf + entry_row(v, e[k])) : 0u;
+#pragma unroll
+      for (uint32_t k = 0; k < U; ++k)
+        if (i0 + k * T < hi) {
+          atomicOr(&bits_sm[r[k] >> 5], 1u << (r[k] & 31));
+          if (counts) atomicAdd(&hist[(r[k] >> csh) * C + (e[k] >> v.lab_shift)], 1u);
+        }
+    }
+    __syncthreads();
+    uint4* out = reinterpret_cast<uint4*>(rank_bits(v, nd, unit.y));
+    uint32_t* oc = s.carry + (size_t)unit.w * C;
+    if (slices == 1) {
+      for (uint32_t g = threadIdx.x; g < groups; g += T) out[g] = bm4[g];
+      if (counts)
+        for (uint32_t i = threadIdx.x; i < nc; i += T) oc[i] = hist[i];
+    } else {
+      uint32_t* ow = reinterpret_cast<uint32_t*>(out);
+      for (uint32_t w = threadIdx.x; w < groups * 4; w += T)
+        if (const uint32_t b = bits_sm[w]) atomicOr(ow + w, b);
+      if (counts)
+        for (uint32_t i = threadIdx.x; i < nc; i += T)
+          if (const uint32_t t = hist[i]) atomicAdd(oc + i, t);
+    }
+  }
+}
+
+// ------------------------------------------------------------------------
+// Small nodes: one warp per (node, feature).  Sort keys are the row's rank in
+// the feature's presort above its index in the node (ranks are distinct), in
+// 32 bits; element e sits in register e / 32 of lane e % 32.
+template <int K>
+__device__ __forceinline__ void warp_sort_keys(uint32_t (&v)[K], uint32_t lane) {
+#pragma unroll
+  for (uint32_t size = 2; size <= 32u * K; size <<= 1) {
+#pragma unroll
+    for (uint32_t j = size >> 1; j > 0; j >>= 1) {
+      if (j >= 32) {
+        const uint32_t kj = j >> 5;
+#pragma unroll
+        for (uint32_t k = 0; k < (uint32_t)K; ++k) {
+          if (k & kj) continue;
+          const bool up = ((32 * k) & size) == 0u;
+          const uint32_t a = v[k], b = v[k | kj];
+          v[k] = up ? min(a, b) : max(a, b);
+          v[k | kj] = up ? max(a, b) : min(a, b);
+        }
+      } else {
+#pragma unroll
+        for (uint32_t k = 0; k < (uint32_t)K; ++k) {
+          const uint32_t o = __shfl_xor_sync(FULL, v[k], j);
+          const bool lower = (((lane + 32 * k) & size) == 0u) == ((lane & j) == 0u);
+          v[k] = lower ? min(v[k], o) : max(v[k], o);
+        }
+      }
+    }
+  }
+}
+
+// Shared memory of one warp: value bits and (label | class total << 16) of the
+// node's rows, then the running class counts (16 bits).
+__host__ __device__ __forceinline__ uint32_t warp_item_words(uint32_t n_classes) {
+  return 2 * WARP_ROWS + (n_classes + 1) / 2;
+}
+
+template <int K>
+__device__ __forceinline__ void row_warp_scan(const View& v, const uint32_t* tot, const uint32_t* rows, uint32_t n,
+                                              const uint2* pf, uint32_t* smem, RowBest* out) {
+  const uint32_t lane = lane_id();
+  float* xs = reinterpret_cast<float*>(smem);
+  uint32_t* lts = smem + WARP_ROWS;
+  uint16_t* cnt = reinterpret_cast<uint16_t*>(smem + 2 * WARP_ROWS);
+  uint32_t key[K];
+  uint32_t tsum = 0;
+  {
+    uint32_t e[K];
+    uint2 pr[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const uint32_t i = 32 * k + lane;
+      e[k] = i < n ? rows[i] : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) pr[k] = 32 * k + lane < n ? __ldg(pf + entry_row(v, e[k])) : make_uint2(0u, 0u);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const uint32_t i = 32 * k + lane;
+      key[k] = NONE;
+      if (i < n) {
+        const uint32_t lab = e[k] >> v.lab_shift, t = __ldg(tot + lab);
+        key[k] = (pr[k].x << WARP_ROWS_BITS) | i;
+        xs[i] = __uint_as_float(pr[k].y);
+        lts[i] = lab | (t << 16);
+        tsum += t;
+      }
+    }
+  }
+  for (uint32_t c = lane; c < v.n_classes; c += 32) cnt[c] = 0;
+  const int32_t st2 = (int32_t)__reduce_add_sync(FULL, tsum);  // sum of squared class totals
+  __syncwarp();
+  warp_sort_keys<K>(key, lane);
+  const double nn = (double)n;
+  const unsigned lt = lanemask_lt();
+  int32_t sl = 0, a = 0;  // sum of squared left counts; sum of left count x total
+  double best = dinf();
+  uint32_t bpos = NONE, bpure = 0;
+  float bxl = 0.f, bxr = 0.f;
+  float x = xs[key[0] & (WARP_ROWS - 1)];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (32u * k >= n) break;
+    const uint32_t p = 32 * k + lane;
+    const bool valid = p < n;
+    const uint32_t ltv = lts[key[k] & (WARP_ROWS - 1)];
+    const float x_nx = k + 1 < K ? xs[key[k + 1 < K ? k + 1 : k] & (WARP_ROWS - 1)] : 0.f;
+    float xn = __shfl_down_sync(FULL, x, 1);
+    const float first = __shfl_sync(FULL, x_nx, 0);
+    if (lane == 31) xn = first;
+    const uint32_t c = valid ? ltv & 0xffffu : NONE;
+    const unsigned grp = __match_any_sync(FULL, c);
+    uint32_t packed = 0;
+    if (valid) packed = (2u * (cnt[c] + (uint32_t)__popc(grp & lt)) + 1u) | (ltv & 0xffff0000u);
+    __syncwarp();
+    if (valid && (grp >> lane) == 1u) cnt[c] += (uint16_t)__popc(grp);
+    __syncwarp();
+    // 32 x (2 x 512 + 1) and 32 x 512 both stay below 2^16
+    const uint32_t incl = (uint32_t)warp_incl_scan_i32((int32_t)packed);
+    const uint32_t total = __shfl_sync(FULL, incl, 31);
+    const int32_t SL = sl + (int32_t)(incl & 0xffffu);
+    const int32_t SR = st2 - 2 * (a + (int32_t)(incl >> 16)) + SL;
+    sl += (int32_t)(total & 0xffffu);
+    a += (int32_t)(total >> 16);
+    if (valid && p + 1 < n && is_candidate_sorted(x, xn)) {
+      const Scored sc = score_at(SL, SR, p + 1, nn);
+      if (sc.score < best) {
+        best = sc.score;
+        bpos = p;
+        bpure = sc.pure;
+        bxl = x;
+        bxr = xn;
+      }
+    }
+    x = x_nx;
+  }
+  const uint32_t win = warp_best_lane(best, bpos);
+  if (win == NONE ? lane == 0 : lane == win) *out = RowBest{best, bpos, bpure, bxl, bxr};
+}
+
+template <bool Q>
+__device__ __forceinline__ void row_warp_item(const View& vb, const StepLists& lists, const LevelScratch& s,
+                                              uint32_t* smem, uint32_t i) {
+  const uint2 it = s.witems[i];
+  const ct_node nd = lists.nodes[it.x];
+  CT_JOB_VIEW(v, vb, nd.slot);
+  const uint32_t f = s.sel[(size_t)it.x * v.sel_stride + it.y];
+  const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
+  const uint2* pf = v.pair + (size_t)f * v.n_rows;
+  const uint32_t* tot = lists.tot + (size_t)it.x * vb.n_classes;
+  RowBest* out = s.rbest + (size_t)it.x * v.sel_stride + it.y;
+  if (nd.n <= 32) row_warp_scan<1>(v, tot, rows, nd.n, pf, smem, out);
+  else if (nd.n <= 64) row_warp_scan<2>(v, tot, rows, nd.n, pf, smem, out);
+  else if (nd.n <= 128) row_warp_scan<4>(v, tot, rows, nd.n, pf, smem, out);
+  else if (nd.n <= 256) row_warp_scan<8>(v, tot, rows, nd.n, pf, smem, out);
+  else row_warp_scan<16>(v, tot, rows, nd.n, pf, smem, out);
+}
+
+template <bool Q>
+__global__ void __launch_bounds__(THREADS_PER_BLOCK, 8) k_row_warp(View v, LevelScratch s) {
+  extern __shared__ uint32_t smem[];
+  uint32_t* ws = smem + (threadIdx.x >> 5) * warp_item_words(v.n_classes);
+  const uint32_t count = live_count(s, s.ctr->n_small_segs, s.cap_w);
+  const StepLists sl = *s.step;
+  for_items(count, &s.ctr->claim[ITEM_PLAN], [&](uint32_t i) { row_warp_item<Q>(v, sl, s, ws, i); });
+}
+
+// ------------------------------------------------------------------------
+// Scan of a run of at most SEQ_ROWS sorted rows with at most SEQ_CLASSES
+// classes: the rows lie in shared memory so that lane l walks the l-th piece
+// of 2^k consecutive ones.  First every lane counts its rows' classes in 8-bit
+// fields of two registers; a prefix over the lanes gives each its left class
+// counts and sums at its first row; then each updates them row by row, with no
+// exchange between lanes.  The exact score costs more than the rest of a step,
+// so a step only estimates the candidate's gain (see Gain) and the walk keeps
+// the largest.  Only a lane whose largest gain reaches the best known for the
+// node within the estimate's error walks again, and there the candidates
+// within that error are scored exactly: one further below can neither win nor
+// tie.
+constexpr uint32_t SEQ_ROWS = 512;
+
+// A run of `count` rows, 2^sh per lane: row i sits at (i >> sh) lanes of
+// 2^sh + 1 entries (no bank conflicts between lanes).
+__device__ __forceinline__ uint32_t seq_shift(uint32_t count) {  // count <= SEQ_ROWS
+  return count <= 32 ? 0u : 27u - (uint32_t)__clz((int)(count - 1));
+}
+__device__ __forceinline__ uint32_t seq_at(uint32_t i, uint32_t sh) { return i + (i >> sh); }
+constexpr uint32_t SEQ_SLOTS = SEQ_ROWS + 32;    // entries of a run, at the most
+// Shared memory of one warp, in words: 2 L + 1 per (class, lane), the class
+// totals as doubles, the class counts before the run, the class totals.
+constexpr uint32_t SEQ_TAB = SEQ_CLASSES * 32;
+constexpr uint32_t SEQ_BEFORE = SEQ_TAB + 2 * SEQ_CLASSES;
+constexpr uint32_t SEQ_WORDS = SEQ_BEFORE + 2 * SEQ_CLASSES;
+
+struct SeqBest {
+  double score;
+  uint32_t pos;
+  uint32_t pure;
+  float xl;
+  float xr;
+};
+
+// An entry: (value bits, 8 x label).
+__device__ __forceinline__ uint2 seq_entry(uint32_t x, uint32_t label) { return make_uint2(x, label << 3); }
+
+// 1 << s, 0 for s >= 32 (also when s wrapped below 0).
+__device__ __forceinline__ uint32_t shl_clamp(uint32_t s) {
+  uint32_t r;
+  asm("shl.b32 %0, 1, %1;" : "=r"(r) : "r"(s));
+  return r;
+}
+
+// This lane's class counts as 8-bit fields, spread over pairs of 16-bit
+// fields: word h of class c is (c >> 2) * 2 + (c & 1), its half (c >> 1) & 1.
+__device__ __forceinline__ void seq_count(const uint2* run, uint32_t m, uint32_t (&w)[4]) {
+  uint32_t lo = 0, hi = 0;
+#pragma unroll 4
+  for (uint32_t j = 0; j < m; ++j) {
+    const uint32_t c8 = run[j].y;
+    lo += shl_clamp(c8);
+    hi += shl_clamp(c8 - 32);
+  }
+  w[0] = lo & 0x00ff00ffu;
+  w[1] = (lo >> 8) & 0x00ff00ffu;
+  w[2] = hi & 0x00ff00ffu;
+  w[3] = (hi >> 8) & 0x00ff00ffu;
+}
+__device__ __forceinline__ uint32_t seq_field(const uint32_t (&w)[4], uint32_t c) {
+  return (w[(c >> 2) * 2 + (c & 1u)] >> (((c >> 1) & 1u) * 16)) & 0xffffu;
+}
+
+// The class totals of the node, for seq_scan; before[] is the caller's.
+__device__ __forceinline__ void seq_totals(uint32_t* sq, const uint32_t* tot, uint32_t C) {
+  const uint32_t lane = lane_id();
+  if (lane < SEQ_CLASSES) {
+    const uint32_t t = lane < C ? tot[lane] : 0u;
+    reinterpret_cast<double*>(sq + SEQ_TAB)[lane] = (double)t;
+    sq[SEQ_BEFORE + SEQ_CLASSES + lane] = t;
+  }
+}
+
+// The largest gain any order of rows could reach at a position among them or
+// at their ends, a[] and b[] being the class counts before and after them: the
+// gain is a convex function of the left class counts, so it is largest where
+// every class's rows lie all left or all right.  One such corner per lane and
+// round.  Warp-collective.
+__device__ __forceinline__ float gain_limit(const uint32_t* a, const uint32_t* b, const uint32_t* total, uint32_t C,
+                                            uint32_t n) {
+  const uint32_t lane = lane_id();
+  const double inv = 1.0 / (double)n;
+  float best = 0.f;
+  for (uint32_t m = lane; m < (1u << C); m += 32) {
+    uint32_t nl = 0;
+#pragma unroll
+    for (uint32_t c = 0; c < SEQ_CLASSES; ++c)
+      if (c < C) nl += (m >> c) & 1u ? b[c] : a[c];
+    if (nl == 0 || nl >= n) continue;
+    const double t = (double)nl * inv;
+    double d = 0.0;
+#pragma unroll
+    for (uint32_t c = 0; c < SEQ_CLASSES; ++c) {
+      if (c >= C) break;
+      const double u = (double)((m >> c) & 1u ? b[c] : a[c]) - t * (double)total[c];
+      d += u * u;
+    }
+    best = fmaxf(best, gain_of(d, (float)nl, (float)(n - nl), (float)n));
+  }
+  return __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(best)));
+}
+
+// The scan of a run at positions p0.. of the node's order.  run: this lane's
+// m rows; w: their counts (seq_count); sq: the warp's tables, with the totals
+// and the class counts before the run set; the latter are advanced past the
+// run here.  xp: the value before the lane's first row (its own value when
+// there is none).  node_q: the largest gain known for the node, kept by all of
+// its scans.
+__device__ __forceinline__ void seq_scan(const uint2* run, uint32_t m, uint32_t sh, const uint32_t (&w)[4], uint32_t* sq,
+                                         uint32_t C, float xp, uint32_t p0, uint32_t n, uint32_t* node_q, SeqBest& bb) {
+  const uint32_t lane = lane_id();
+  uint32_t* tab = sq + lane;
+  const double* tt = reinterpret_cast<const double*>(sq + SEQ_TAB);
+  uint32_t* before = sq + SEQ_BEFORE;
+  const uint32_t* total = before + SEQ_CLASSES;
+  uint32_t ex[4], tot[4];
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {  // words 0 and 1 hold classes 0-3, 2 and 3 classes 4-7
+    ex[h] = tot[h] = 0;
+    if (h < 2 || C > 4) {
+      const uint32_t incl = (uint32_t)warp_incl_scan_i32((int32_t)w[h]);
+      ex[h] = incl - w[h];
+      tot[h] = __shfl_sync(FULL, incl, 31);
+    }
+  }
+  int64_t sl = 0, a = 0, st2 = 0;  // sums of L^2, L T, T^2
+#pragma unroll
+  for (uint32_t c = 0; c < SEQ_CLASSES; ++c) {
+    if (c >= C) break;
+    const uint32_t l = before[c] + seq_field(ex, c), t = total[c];
+    tab[c * 32] = 2 * l + 1;
+    sl += (int64_t)l * l;
+    a += (int64_t)l * t;
+    st2 += (int64_t)t * t;
+  }
+  __syncwarp();
+  if (lane < C) before[lane] += seq_field(tot, lane);
+  const uint32_t k0 = p0 + (lane << sh);
+  const double inv = 1.0 / (double)n, std2 = (double)st2;
+  const float nf = (float)n;
+  float gmax = 0.f;
+  {
+    double s = (double)sl, a2 = -2.0 * (double)a, nl = (double)k0;
+    float nlf = (float)k0, nrf = nf - nlf, x0 = xp;  // exact: n < 2^24
+#pragma unroll 2
+    for (uint32_t j = 0; j < m; ++j) {
+      const uint2 e = run[j];
+      const float x = __uint_as_float(e.x);
+      uint32_t* t = tab + (e.y << 2);
+      const uint32_t d = *t;
+      const double r = nl * inv;
+      const float g = gain_of(fma(r, fma(r, std2, a2), s), nlf, nrf, nf);
+      if (is_candidate_sorted(x0, x)) gmax = fmaxf(gmax, g);
+      *t = d + 2;
+      s += (double)d;
+      a2 = fma(-2.0, tt[e.y >> 3], a2);
+      nl += 1.0;
+      nlf += 1.f;
+      nrf -= 1.f;
+      x0 = x;
+    }
+  }
+  const uint32_t gw = __reduce_max_sync(FULL, __float_as_uint(gmax));
+  uint32_t known = 0;
+  if (lane == 0 && gw) known = atomicMax(node_q, gw);
+  known = max(__shfl_sync(FULL, known, 0), gw);
+  const float bound = gain_bound(__uint_as_float(known), n);
+  if (gmax > 0.f && gmax >= bound) {  // this lane holds such a candidate
+    for (uint32_t j = m; j > 0; --j) tab[run[j - 1].y << 2] -= 2;  // the counts at the lane's first row again
+    const double nn = (double)n;
+    for (uint32_t j = 0; j < m; ++j) {
+      const uint2 e = run[j];
+      const float x = __uint_as_float(e.x);
+      uint32_t* t = tab + (e.y << 2);
+      const uint32_t d = *t, k = k0 + j;
+      if (is_candidate_sorted(xp, x)) {
+        const double r = (double)k * inv;
+        const float g = gain_of(fma(r, fma(r, std2, -2.0 * (double)a), (double)sl), (float)k, nf - (float)k, nf);
+        if (g >= bound) {
+          const Scored sc = score_at(sl, st2 - 2 * a + sl, k, nn);
+          if (sc.score < bb.score) bb = SeqBest{sc.score, k - 1, sc.pure, xp, x};
+        }
+      }
+      *t = d + 2;
+      sl += d;
+      a += total[e.y >> 3];
+      xp = x;
+    }
+  }
+  __syncwarp();
+}
+
+// ------------------------------------------------------------------------
+// Nodes of WARP_ROWS + 1 .. GROUP_ROWS rows: one CTA per (node, feature).  The
+// rows set their rank's bit in a bitmap over all ranks and count themselves in
+// their group of 128 ranks; a prefix over the groups and the set bits below a
+// row's own give its sorted position, where its value and label are stored.
+// Only the words a node touched are cleared after it, so an item costs its
+// rows and the groups, not the ranks.  Each warp then scans a run of the
+// sorted rows, from the class counts of the warps before it.  Bound by latency
+// (two CTAs per SM at covtype's 581,012 ranks, barriers between the phases); a
+// bitonic sort of the ranks in registers took 13.7 ms per 100 covtype-shaped
+// trees against 8.5 ms.
+__host__ __device__ __forceinline__ uint32_t group_count_words(uint32_t n_rows) {  // two 16-bit counts per word
+  return ((order_words(n_rows) / 4 + 7) / 8) * 4;
+}
+// Shared memory, in words: (value bits, 8 x label or label | class total << 16)
+// by position, bitmap, group counts, the warps' class counts or seq tables.
+// With up to SEQ_CLASSES classes a warp's run is padded for seq_scan.
+template <int W>
+__host__ __device__ __forceinline__ uint32_t group_rows_words() {
+  return 2 * ((W == GROUP_SMALL_WARPS ? GROUP_SMALL_ROWS : GROUP_ROWS) + W * 34);
+}
+__host__ __device__ __forceinline__ uint32_t group_class_words(uint32_t n_classes) {
+  return n_classes <= SEQ_CLASSES ? SEQ_WORDS : (n_classes + 3u) & ~3u;
+}
+template <int W>
+__host__ __device__ __forceinline__ uint32_t group_words(uint32_t n_classes, uint32_t n_rows) {
+  return group_rows_words<W>() + order_words(n_rows) + group_count_words(n_rows) + W * group_class_words(n_classes);
+}
+
+template <bool Q, int W>
+__device__ __forceinline__ void row_group_item(const View& vb, const StepLists& lists, const LevelScratch& s,
+                                               uint32_t* smem, uint32_t n_max, RowBest* s_best, uint32_t* s_wsum,
+                                               uint2 item) {
+  constexpr uint32_t T = W * 32, K = (W == GROUP_SMALL_WARPS ? GROUP_SMALL_ROWS : GROUP_ROWS) / T;
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5, C = vb.n_classes;
+  const ct_node nd = lists.nodes[item.x];
+  CT_JOB_VIEW(v, vb, nd.slot);
+  const uint32_t n = nd.n;
+  const uint32_t f = s.sel[(size_t)item.x * v.sel_stride + item.y];
+  const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
+  const uint2* pf = v.pair + (size_t)f * v.n_rows;
+  const uint32_t* tot = lists.tot + (size_t)item.x * C;
+  uint2* ent = reinterpret_cast<uint2*>(smem);
+  uint32_t* bm = smem + group_rows_words<W>();
+  uint32_t* gc = bm + order_words(n_max);
+  uint32_t* cls = gc + group_count_words(n_max);
+  uint32_t* cnt = cls + warp * group_class_words(C);
+  const bool seq = C <= SEQ_CLASSES;
+  const uint32_t units = group_count_words(v.n_rows) / 4;  // of 8 groups
+  // rows of one warp's run, and where position p is kept: runs of 32 << sh
+  // rows padded for seq_scan, else runs without padding
+  const uint32_t sh = seq_shift(ceil_div(n, (uint32_t)W));
+  const uint32_t len = seq ? 32u << sh : ceil_div(ceil_div(n, 32u), (uint32_t)W) * 32;
+  auto at = [&](uint32_t p) { return seq ? p + (p >> sh) : p; };
+  uint32_t rk[K], lb[K];
+  float xv[K];
+#pragma unroll
+  for (uint32_t k = 0; k < K; ++k) lb[k] = k * T + threadIdx.x < n ? rows[k * T + threadIdx.x] : 0u;
+  for (uint32_t g = threadIdx.x; g < units; g += T) reinterpret_cast<uint4*>(gc)[g] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+  for (uint32_t k = 0; k < K; ++k) {
+    rk[k] = 0;
+    xv[k] = 0.f;
+    if (k * T + threadIdx.x < n) {
+      const uint2 pr = __ldg(pf + entry_row(v, lb[k]));
+      rk[k] = pr.x;
+      xv[k] = __uint_as_float(pr.y);
+    }
+  }
+  if (!seq)
+    for (uint32_t c = lane; c < C; c += 32) cnt[c] = 0;
+  __syncthreads();
+#pragma unroll
+  for (uint32_t k = 0; k < K; ++k)
+    if (k * T + threadIdx.x < n) {
+      atomicOr(&bm[rk[k] >> 5], 1u << (rk[k] & 31));
+      atomicAdd(&gc[rk[k] >> 8], 1u << ((rk[k] >> 3) & 16));
+    }
+  __syncthreads();
+  // exclusive prefix of the groups' counts (at most 8,192: 16 bits)
+  const uint32_t per_w = ceil_div(ceil_div(units, 32u), (uint32_t)W) * 32;
+  const uint32_t ulo = min(warp * per_w, units), uhi = min(ulo + per_w, units);
+  uint32_t sum = 0;
+  for (uint32_t u = ulo + lane; u < uhi; u += 32) {
+    const uint4 q = reinterpret_cast<const uint4*>(gc)[u];
+    const uint32_t t = q.x + q.y + q.z + q.w;  // 16-bit fields: at most 512 each
+    sum += (t & 0xffffu) + (t >> 16);
+  }
+  sum = __reduce_add_sync(FULL, sum);
+  if (lane == 0) s_wsum[warp] = sum;
+  __syncthreads();
+  uint32_t run = __reduce_add_sync(FULL, lane < warp ? s_wsum[lane & (W - 1)] : 0u);
+  for (uint32_t u0 = ulo; u0 < uhi; u0 += 32) {
+    const uint32_t u = u0 + lane;
+    const uint4 q = u < uhi ? reinterpret_cast<const uint4*>(gc)[u] : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t t4 = q.x + q.y + q.z + q.w, t = (t4 & 0xffffu) + (t4 >> 16);
+    const uint32_t incl = (uint32_t)warp_incl_scan_i32((int32_t)t);
+    uint32_t b = run + incl - t;
+    uint4 o;
+    // each word holds the groups 2 i (low half) and 2 i + 1
+    o.x = b | ((b + (q.x & 0xffffu)) << 16);
+    b += (q.x & 0xffffu) + (q.x >> 16);
+    o.y = b | ((b + (q.y & 0xffffu)) << 16);
+    b += (q.y & 0xffffu) + (q.y >> 16);
+    o.z = b | ((b + (q.z & 0xffffu)) << 16);
+    b += (q.z & 0xffffu) + (q.z >> 16);
+    o.w = b | ((b + (q.w & 0xffffu)) << 16);
+    if (u < uhi) reinterpret_cast<uint4*>(gc)[u] = o;
+    run += __shfl_sync(FULL, incl, 31);
+  }
+  __syncthreads();
+#pragma unroll
+  for (uint32_t k = 0; k < K; ++k)
+    if (k * T + threadIdx.x < n) {
+      const uint32_t r = rk[k], in = (r >> 5) & 3u, below = (1u << (r & 31)) - 1u;
+      const uint4 q = reinterpret_cast<const uint4*>(bm)[r >> 7];
+      const uint32_t pos = reinterpret_cast<const uint16_t*>(gc)[r >> 7] + __popc(q.x & (in > 0 ? FULL : below)) +
+                           __popc(q.y & (in > 1 ? FULL : in == 1 ? below : 0u)) +
+                           __popc(q.z & (in > 2 ? FULL : in == 2 ? below : 0u)) + __popc(q.w & (in == 3 ? below : 0u));
+      const uint32_t lab = lb[k] >> v.lab_shift;
+      ent[at(pos)] = seq ? seq_entry(__float_as_uint(xv[k]), lab)
+                         : make_uint2(__float_as_uint(xv[k]), lab | (__ldg(tot + lab) << 16));
+    }
+  __syncthreads();
+#pragma unroll
+  for (uint32_t k = 0; k < K; ++k)  // every row is placed: clear the words it touched
+    if (k * T + threadIdx.x < n) bm[rk[k] >> 5] = 0u;
+  // this warp's run of sorted rows
+  const uint32_t w0 = min(warp * len, n), w1 = min(w0 + len, n);
+  RowBest rb{dinf(), NONE, 0u, 0.f, 0.f};
+  if (seq) {
+    uint32_t* before = cnt + SEQ_BEFORE;
+    const uint32_t i0 = min(w0 + (lane << sh), w1), m = min(w1 - i0, 1u << sh);
+    const uint2* run = ent + at(i0);
+    uint32_t w[4], t[4];
+    seq_count(run, m, w);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) t[h] = __reduce_add_sync(FULL, w[h]);
+    if (lane < SEQ_CLASSES) before[lane] = seq_field(t, lane);
+    seq_totals(cnt, tot, C);
+    __syncthreads();
+    uint32_t mine = 0;
+    if (lane < SEQ_CLASSES)
+      for (uint32_t k = 0; k < warp; ++k) mine += cls[k * SEQ_WORDS + SEQ_BEFORE + lane];
+    __syncthreads();
+    if (lane < SEQ_CLASSES) before[lane] = mine;
+    __syncwarp();
+    if (w0 < w1) {
+      SeqBest bb{dinf(), NONE, 0u, 0.f, 0.f};
+      const float xp = __uint_as_float(ent[at(i0 < w1 ? (i0 ? i0 - 1 : 0u) : w0)].x);
+      seq_scan(run, m, sh, w, cnt, C, xp, w0, n, s.node_q + item.x, bb);
+      rb = RowBest{bb.score, bb.pos, bb.pure, bb.xl, bb.xr};
+    }
+  } else {
+    for (uint32_t i = w0 + lane; i < w1; i += 32) atomicAdd(&cnt[ent[i].y & 0xffffu], 1u);
+    __syncthreads();
+    for (uint32_t c = threadIdx.x; c < C; c += T) {
+      uint32_t before = 0;
+#pragma unroll
+      for (uint32_t k = 0; k < W; ++k) {
+        const uint32_t t = cls[k * group_class_words(C) + c];
+        cls[k * group_class_words(C) + c] = before;
+        before += t;
+      }
+    }
+    __syncthreads();
+    // sums of squares stay at or below 2^26 (at most 8,192 rows)
+    uint32_t sl = 0, a = 0, st2 = 0;
+    for (uint32_t c = lane; c < C; c += 32) {
+      const uint32_t k = cnt[c], t = __ldg(tot + c);
+      sl += k * k;
+      a += k * t;
+      st2 += t * t;
+    }
+    sl = __reduce_add_sync(FULL, sl);
+    a = __reduce_add_sync(FULL, a);
+    st2 = __reduce_add_sync(FULL, st2);
+    __syncwarp();
+    const double nn = (double)n;
+    const unsigned lt = lanemask_lt();
+    float x_last = __uint_as_float(ent[w0 ? w0 - 1 : 0u].x);
+    for (uint32_t p0 = w0; p0 < w1; p0 += 32) {
+      const uint32_t p = p0 + lane;
+      const bool valid = p < w1;
+      const uint2 en = valid ? ent[p] : make_uint2(0u, 0u);
+      const uint32_t ltv = en.y;
+      const float x = __uint_as_float(en.x);
+      float xp = __shfl_up_sync(FULL, x, 1);
+      if (lane == 0) xp = x_last;
+      x_last = __shfl_sync(FULL, x, 31);
+      const uint32_t c = valid ? ltv & 0xffffu : NONE;
+      const unsigned grp = __match_any_sync(FULL, c);
+      uint32_t dl = 0, dt = 0;
+      if (valid) {
+        dl = 2 * (cnt[c] + (uint32_t)__popc(grp & lt)) + 1;
+        dt = ltv >> 16;
+      }
+      __syncwarp();
+      if (valid && (grp >> lane) == 1u) cnt[c] += __popc(grp);
+      __syncwarp();
+      const uint32_t il = (uint32_t)warp_incl_scan_i32((int32_t)dl), it = (uint32_t)warp_incl_scan_i32((int32_t)dt);
+      const uint32_t SL = sl + (il - dl);  // of the rows before this one
+      const uint32_t SR = st2 - 2 * (a + (it - dt)) + SL;
+      sl += __shfl_sync(FULL, il, 31);
+      a += __shfl_sync(FULL, it, 31);
+      if (valid && p > 0 && is_candidate_sorted(xp, x)) {
+        const Scored sc = score_at((int64_t)SL, (int64_t)SR, p, nn);
+        if (sc.score < rb.score) rb = RowBest{sc.score, p - 1, sc.pure, xp, x};
+      }
+    }
+  }
+  const uint32_t win = warp_best_lane(rb.score, rb.pos);
+  if (win == NONE ? lane == 0 : lane == win) s_best[warp] = rb;
+  __syncthreads();
+  if (warp == 0) {
+    rb = lane < W ? s_best[lane] : RowBest{dinf(), NONE, 0u, 0.f, 0.f};
+    const uint32_t wl = warp_best_lane(rb.score, rb.pos);
+    if (wl == NONE ? lane == 0 : lane == wl) s.rbest[(size_t)item.x * v.sel_stride + item.y] = rb;
+  }
+}
+
+template <bool Q, int W>
+__global__ void __launch_bounds__(W * 32, 2) k_row_group(View v, LevelScratch s, uint32_t n_max) {
+  extern __shared__ __align__(16) uint32_t group_sm[];
+  __shared__ RowBest s_best[W];
+  __shared__ uint32_t s_wsum[W];
+  __shared__ uint32_t s_item;
+  const uint32_t count = live_count(s, W == GROUP_SMALL_WARPS ? s.ctr->n_huge_segs : s.ctr->n_hchains, s.cap_order);
+  const uint2* list = W == GROUP_SMALL_WARPS ? s.gsmall : s.glarge;
+  uint32_t* claim = W == GROUP_SMALL_WARPS ? &s.ctr->ticket : &s.ctr->ticket_huge;
+  const StepLists sl = *s.step;
+  uint32_t i = blockIdx.x;
+  if (i >= count) return;
+  uint4* bm4 = reinterpret_cast<uint4*>(group_sm + group_rows_words<W>());
+  for (uint32_t g = threadIdx.x; g < order_words(n_max) / 4; g += W * 32) bm4[g] = make_uint4(0u, 0u, 0u, 0u);
+  while (i < count) {
+    if (threadIdx.x == 0) s_item = gridDim.x + atomicAdd(claim, 1u);  // the next item, claimed ahead
+    row_group_item<Q, W>(v, sl, s, group_sm, n_max, s_best, s_wsum, list[i]);
+    __syncthreads();
+    i = s_item;
+    __syncthreads();
+  }
+}
+
+// ------------------------------------------------------------------------
+// Larger nodes: one CTA per (node, feature).  The node's rows set their rank's
+// bit in a bitmap over all ranks; a row's sorted position is then the count
+// of set bits before its own (a prefix per word, or per four words when the
+// node has more than 65,535 rows), where its value and label are stored.
+template <bool Q>
+__global__ void __launch_bounds__(ORDER_THREADS, 2) k_row_order(View vb, LevelScratch s) {
+  extern __shared__ __align__(16) uint32_t order_sm[];
+  __shared__ uint32_t s_wsum[ORDER_THREADS / 32];
+  __shared__ uint32_t s_item;
+  const uint32_t count = live_count(s, s.ctr->n_carry, s.cap_order);
+  const StepLists lists = *s.step;
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  constexpr uint32_t T = ORDER_THREADS, NW = T / 32;
+  while (true) {
+    __syncthreads();  // the previous item is done with the bitmap and s_item
+    if (threadIdx.x == 0) s_item = atomicAdd(&s.ctr->claim[ITEM_TWO_VALUED], 1u);
+    __syncthreads();
+    const uint32_t it = s_item;
+    if (it >= count) break;
+    const uint2 item = s.oitems[it];
+    const ct_node nd = lists.nodes[item.x];
+    CT_JOB_VIEW(v, vb, nd.slot);
+    const uint32_t n = nd.n;
+    const uint32_t f = s.sel[(size_t)item.x * v.sel_stride + item.y];
+    const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
+    const uint2* pf = v.pair + (size_t)f * v.n_rows;
+    uint2* out = sorted_list(v, nd.slot, item.y) + nd.start;
+    const uint32_t words = order_words(v.n_rows), groups = words / 4;
+    uint32_t* bm = order_sm;
+    uint4* bm4 = reinterpret_cast<uint4*>(order_sm);
+    uint16_t* pre16 = reinterpret_cast<uint16_t*>(order_sm + words);
+    uint32_t* pre32 = order_sm + words;
+    for (uint32_t g = threadIdx.x; g < groups; g += T) bm4[g] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    for (uint32_t i0 = threadIdx.x; i0 < n; i0 += T * 4) {
+      uint32_t r[4];
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) r[k] = i0 + k * T < n ? rows[i0 + k * T] : NONE;
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k)
+        if (i0 + k * T < n) r[k] = __ldg(&pf[entry_row(v, r[k])].x);
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k)
+        if (i0 + k * T < n) atomicOr(&bm[r[k] >> 5], 1u << (r[k] & 31));
+    }
+    __syncthreads();
+    // exclusive prefix: each warp sums, then scans, a run of groups
+    const uint32_t per = ceil_div(ceil_div(groups, 32u), NW) * 32;
+    const uint32_t glo = min(warp * per, groups), ghi = min(glo + per, groups);
+    uint32_t sum = 0;
+    for (uint32_t g = glo + lane; g < ghi; g += 32) {
+      const uint4 q = bm4[g];
+      sum += __popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w);
+    }
+    sum = __reduce_add_sync(FULL, sum);
+    if (lane == 0) s_wsum[warp] = sum;
+    __syncthreads();
+    uint32_t run = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < NW; ++k) run += k < warp ? s_wsum[k] : 0u;
+    const bool wide = n > 0xffffu;
+    for (uint32_t g0 = glo; g0 < ghi; g0 += 32) {
+      const uint32_t g = g0 + lane;
+      const uint4 q = g < ghi ? bm4[g] : make_uint4(0u, 0u, 0u, 0u);
+      const uint32_t c0 = __popc(q.x), c1 = __popc(q.y), c2 = __popc(q.z), c3 = __popc(q.w);
+      const uint32_t t = c0 + c1 + c2 + c3;
+      const uint32_t incl = (uint32_t)warp_incl_scan_i32((int32_t)t);
+      const uint32_t b = run + incl - t;
+      if (g < ghi) {
+        if (wide) {
+          pre32[g] = b;
+        } else {
+          reinterpret_cast<uint2*>(pre16)[g] =
+              make_uint2(b | ((b + c0) << 16), (b + c0 + c1) | ((b + c0 + c1 + c2) << 16));
+        }
+      }
+      run += __shfl_sync(FULL, incl, 31);
+    }
+    __syncthreads();
+    for (uint32_t i0 = threadIdx.x; i0 < n; i0 += T * 4) {
+      uint32_t e[4];
+      uint2 pr[4];
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) e[k] = i0 + k * T < n ? __ldcs(rows + i0 + k * T) : 0u;
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k)
+        if (i0 + k * T < n) pr[k] = __ldg(pf + entry_row(v, e[k]));
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) {
+        if (i0 + k * T >= n) continue;
+        const uint32_t wd = pr[k].x >> 5, below = (1u << (pr[k].x & 31)) - 1u;
+        uint32_t pos;
+        if (wide) {
+          const uint4 q = bm4[wd >> 2];
+          const uint32_t in = wd & 3u;
+          pos = pre32[wd >> 2] + __popc(q.x & (in > 0 ? FULL : below)) + (in > 0 ? __popc(q.y & (in > 1 ? FULL : below)) : 0) +
+                (in > 1 ? __popc(q.z & (in > 2 ? FULL : below)) : 0) + (in > 2 ? __popc(q.w & below) : 0);
+        } else {
+          pos = pre16[wd] + __popc(bm[wd] & below);
+        }
+        if (pos < n) out[pos] = make_uint2(pr[k].y, e[k] >> v.lab_shift);
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------------
+// The elements of a piece, in sorted order, as (value bits, label).  A sorted
+// list's piece is its positions [lo, hi); a bitmap's is a run of ranks, whose
+// set bits are listed in shared memory a batch at a time (each lane takes a
+// word of a 1,024-rank window and writes its bits behind the lower lanes').
+constexpr uint32_t ROW_BATCH = 4;
+constexpr uint32_t LIST_FILL = 512;              // a batch ends with the window that reaches this
+constexpr uint32_t LIST_CAP = LIST_FILL + 1024;
+
+struct PieceStream {
+  const uint2* base;      // element i of the batch: base[dense ? list[i] : i]
+  const uint32_t* words;  // dense: bitmap words of the piece
+  uint16_t* list;
+  uint32_t n_words;
+  uint32_t next;          // first word (dense) or batch (list) not listed yet
+  uint32_t count;         // elements of the batch
+  bool dense;
+  __device__ __forceinline__ bool more() const { return dense && next < n_words; }
+  __device__ __forceinline__ uint2 load(uint32_t i) const { return dense ? __ldg(base + list[i]) : __ldcs(base + i); }
+  // Lists the next batch behind the last `keep` elements of this one, which
+  // are still to be read; false at the end of the piece.  Warp-collective.
+  __device__ __forceinline__ bool fill(uint32_t keep = 0) {
+    if (!dense) return next++ == 0 && count > 0;
+    const uint32_t lane = lane_id();
+    __syncwarp();
+    if (keep) {
+      for (uint32_t i0 = 0; i0 < keep; i0 += 32) {
+        const uint16_t e = i0 + lane < keep ? list[count - keep + i0 + lane] : (uint16_t)0;
+        __syncwarp();
+        if (i0 + lane < keep) list[i0 + lane] = e;
+        __syncwarp();
+      }
+    }
+    count = keep;
+    while (next < n_words && count < LIST_FILL) {
+      uint32_t b = next + lane < n_words ? __ldg(words + next + lane) : 0u;
+      const uint32_t c = __popc(b);
+      const uint32_t incl = (uint32_t)warp_incl_scan_i32((int32_t)c);
+      uint32_t pos = count + incl - c;
+      const uint32_t r0 = (next + lane) * 32 - 1;
+      for (; b; b &= b - 1) list[pos++] = (uint16_t)(r0 + __ffs(b));
+      count += __shfl_sync(FULL, incl, 31);
+      next += 32;
+    }
+    __syncwarp();
+    return count > 0;
+  }
+};
+
+// Shared memory of one warp of k_row_hist and k_row_scan, in words.
+__host__ __device__ __forceinline__ uint32_t hist_words(uint32_t n_classes) { return LIST_CAP / 2 + n_classes; }
+__host__ __device__ __forceinline__ uint32_t scan_words(uint32_t n_classes) {
+  return LIST_CAP / 2 + (n_classes <= SEQ_CLASSES ? 2 * SEQ_SLOTS + SEQ_WORDS : 2 * n_classes);
+}
+
+__device__ __forceinline__ PieceStream piece_stream(const View& v, const ct_node& nd, const RowPiece& pc, uint32_t f,
+                                                    uint32_t scan_piece, uint32_t* smem) {
+  PieceStream ps;
+  ps.list = reinterpret_cast<uint16_t*>(smem);
+  ps.next = 0;
+  ps.dense = row_dense(nd.n, v.n_rows);
+  if (ps.dense) {
+    const uint32_t chunk = dense_chunk(nd.n, v.n_rows, scan_piece), r0 = pc.j * chunk;
+    ps.base = v.ranked + (size_t)f * v.n_rows + r0;
+    ps.words = rank_bits(v, nd, pc.slot) + r0 / 32;
+    ps.n_words = min(chunk / 32, order_words(v.n_rows) - r0 / 32);
+    ps.count = 0;
+  } else {
+    const uint32_t lo = pc.j * scan_piece;
+    ps.base = sorted_list(v, nd.slot, pc.slot) + nd.start + lo;
+    ps.words = nullptr;
+    ps.n_words = 0;
+    ps.count = min(scan_piece, nd.n - lo);
+  }
+  return ps;
+}
+
+// Class counts of all but the last piece of a multi-piece list (carry rows
+// are indexed by piece).
+template <bool Q>
+__device__ __forceinline__ void row_hist_item(const View& vb, const StepLists& lists, const LevelScratch& s,
+                                              uint32_t* smem, uint32_t pi) {
+  const uint32_t C = vb.n_classes, lane = lane_id();
+  const RowPiece pc = s.rpieces[pi];
+  if (pc.j + 1 >= pc.npieces) return;
+  const ct_node nd = lists.nodes[pc.node];
+  CT_JOB_VIEW(v, vb, nd.slot);
+  if (row_dense(nd.n, v.n_rows) && pc.npieces * C <= BITS_COUNTS) return;  // k_row_bits counted them
+  const uint32_t f = s.sel[(size_t)pc.node * v.sel_stride + pc.slot];
+  PieceStream ps = piece_stream(v, nd, pc, f, lists.scan_piece, smem);
+  uint32_t* cnt = smem + LIST_CAP / 2;
+  uint32_t* out = s.carry + (size_t)pi * C;
+  for (uint32_t c = lane; c < C; c += 32) cnt[c] = 0;
+  __syncwarp();
+  while (ps.fill()) {
+    for (uint32_t b0 = 0; b0 < ps.count; b0 += 32 * 128) {  // at most 128 entries per lane
+      const uint32_t b1 = min(b0 + 32 * 128, ps.count);
+      uint64_t pk = 0;  // up to 8 classes: 8-bit field per class
+      for (uint32_t b = b0; b < b1; b += 32 * ROW_BATCH) {
+        uint32_t c[ROW_BATCH];
+#pragma unroll
+        for (uint32_t r = 0; r < ROW_BATCH; ++r) c[r] = b + r * 32 + lane < b1 ? ps.load(b + r * 32 + lane).y : NONE;
+#pragma unroll
+        for (uint32_t r = 0; r < ROW_BATCH; ++r) {
+          if (c[r] == NONE) continue;
+          if (C <= 8) pk += 1ull << (8 * c[r]);
+          else atomicAdd(&cnt[c[r]], 1u);
+        }
+      }
+      if (C <= 8) {
+        const uint32_t fh[2] = {(uint32_t)pk, (uint32_t)(pk >> 32)};
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+          const uint32_t ev = __reduce_add_sync(FULL, fh[h] & 0x00ff00ffu);
+          const uint32_t od = __reduce_add_sync(FULL, (fh[h] >> 8) & 0x00ff00ffu);
+          const uint32_t val = (lane & 1u ? od : ev) >> ((lane & 2u) * 8) & 0xffffu;
+          if (lane < 4 && 4 * h + lane < C) cnt[4 * h + lane] += val;
+        }
+      }
+    }
+  }
+  __syncwarp();
+  for (uint32_t c = lane; c < C; c += 32) out[c] = cnt[c];
+}
+
+template <bool Q>
+__global__ void __launch_bounds__(THREADS_PER_BLOCK) k_row_hist(View v, LevelScratch s) {
+  extern __shared__ uint32_t smem[];
+  uint32_t* ws = smem + (threadIdx.x >> 5) * hist_words(v.n_classes);
+  const uint32_t count = live_count(s, s.ctr->n_scan_pieces, s.cap_scan);
+  const StepLists sl = *s.step;
+  for_items(count, &s.ctr->claim[ITEM_HIST], [&](uint32_t i) { row_hist_item<Q>(v, sl, s, ws, i); });
+}
+
+// Exclusive prefix of the class counts over a list's pieces: one warp per
+// (list, class), 128 pieces per round.
+__global__ void __launch_bounds__(THREADS_PER_BLOCK) k_row_carry(LevelScratch s, uint32_t C) {
+  const uint32_t count = live_count(s, s.ctr->n_bchains, s.cap_order);
+  const uint32_t lane = lane_id();
+  for_items(count * C, &s.ctr->claim[ITEM_CARRY], [&](uint32_t i) {
+    const uint2 ci = s.citems[i / C];
+    uint32_t* h = s.carry + (size_t)ci.x * C + i % C;
+    uint32_t run = 0;
+    for (uint32_t j0 = 0; j0 < ci.y; j0 += 128) {
+      uint32_t t[4];
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) {  // the last piece's count is not needed, and not always there
+        const uint32_t j = j0 + k * 32 + lane;
+        t[k] = j + 1 < ci.y ? h[(size_t)j * C] : 0u;
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k) {
+        const uint32_t j = j0 + k * 32 + lane;
+        const uint32_t incl = (uint32_t)warp_incl_scan_i32((int32_t)t[k]);
+        if (j < ci.y) h[(size_t)j * C] = run + incl - t[k];
+        run += __shfl_sync(FULL, incl, 31);
+      }
+    }
+  });
+}
+
+// A start for the bound of the nodes' scans (seq_scan): the estimated gain at
+// every piece's first position that is a candidate.  One thread per piece.
+template <bool Q>
+__global__ void __launch_bounds__(256) k_row_bound(View vb, LevelScratch s) {
+  const uint32_t count = live_count(s, s.ctr->n_scan_pieces, s.cap_scan), C = vb.n_classes;
+  const StepLists lists = *s.step;
+  for (uint32_t pi = blockIdx.x * blockDim.x + threadIdx.x; pi < count; pi += gridDim.x * blockDim.x) {
+    const RowPiece pc = s.rpieces[pi];
+    if (pc.j == 0) continue;
+    const ct_node nd = lists.nodes[pc.node];
+    CT_JOB_VIEW(v, vb, nd.slot);
+    const uint32_t* left = s.carry + (size_t)pi * C;
+    uint32_t nl = 0;
+    for (uint32_t c = 0; c < C; ++c) nl += left[c];
+    if (nl == 0 || nl >= nd.n) continue;
+    float xa, xb;
+    if (row_dense(nd.n, v.n_rows)) {
+      const uint32_t f = s.sel[(size_t)pc.node * v.sel_stride + pc.slot];
+      const uint32_t w0 = pc.j * dense_chunk(nd.n, v.n_rows, lists.scan_piece) / 32;
+      const uint32_t* bits = rank_bits(v, nd, pc.slot);
+      uint32_t wa = w0, wb = w0, ba = 0, bb = 0;  // the nearest set bits on both sides, if near
+      for (uint32_t k = 0; k < 64 && wa > 0 && !ba; ++k) ba = __ldg(bits + --wa);
+      for (uint32_t k = 0; k < 64 && wb < order_words(v.n_rows) && !bb; ++k) bb = __ldg(bits + wb++);
+      if (!ba || !bb) continue;
+      const uint2* rk = v.ranked + (size_t)f * v.n_rows;
+      xa = __uint_as_float(__ldg(&rk[wa * 32 + 31 - __clz((int)ba)].x));
+      xb = __uint_as_float(__ldg(&rk[(wb - 1) * 32 + __ffs((int)bb) - 1].x));
+    } else {
+      const uint2* lst = sorted_list(v, nd.slot, pc.slot) + nd.start + pc.j * lists.scan_piece;
+      xa = __uint_as_float(lst[-1].x);
+      xb = __uint_as_float(lst[0].x);
+    }
+    if (!is_candidate_sorted(xa, xb)) continue;
+    atomicMax(s.node_q + pc.node, __float_as_uint(gain_at(left, lists.tot + (size_t)pc.node * C, C, nl, nd.n)));
+  }
+}
+
+// Value bits of the element before the piece (the last set bit before a
+// run of ranks).  The piece is not the node's first with elements.
+__device__ __forceinline__ uint32_t value_before(const View& v, const PieceStream& ps, const ct_node& nd,
+                                                 const RowPiece& pc, uint32_t f, uint32_t scan_piece) {
+  if (!ps.dense) return ps.base[-1].x;
+  const uint32_t lane = lane_id();
+  const uint32_t r0 = pc.j * dense_chunk(nd.n, v.n_rows, scan_piece);
+  const uint32_t* bits = ps.words - r0 / 32;
+  for (uint32_t w = r0 / 32; w > 0;) {  // 32 words at a time, the nearest on lane 0
+    const uint32_t b = lane < w ? __ldg(bits + w - 1 - lane) : 0u;
+    const unsigned any = __ballot_sync(FULL, b != 0u);
+    if (any) {
+      const uint32_t l = (uint32_t)__ffs(any) - 1;
+      const uint32_t bw = __shfl_sync(FULL, b, l);
+      return __ldg(&v.ranked[(size_t)f * v.n_rows + (w - 1 - l) * 32 + 31 - __clz(bw)].x);
+    }
+    w = w > 32 ? w - 32 : 0;
+  }
+  return 0u;
+}
+
+// Gini scan of one piece.  The candidate between two neighbours is judged
+// when the upper one is met, so only the value before the piece comes from
+// outside it.  A piece whose values all equal that one has no candidate, and
+// with up to SEQ_CLASSES classes neither is a piece scanned whose gain_limit
+// is below the best known (three rows in four on covtype-shaped data).  Per
+// 100 covtype-shaped trees: class match and warp scans per round 19.4 ms,
+// lane-sequential 21.3, with gain_limit 13.5, with estimates precise enough
+// that few lanes score exactly 9.3.
+template <bool Q>
+__device__ __forceinline__ void row_scan_item(const View& vb, const StepLists& lists, const LevelScratch& s,
+                                              uint32_t* smem, uint32_t pi) {
+  const uint32_t C = vb.n_classes, lane = lane_id();
+  uint32_t* cnt = smem + LIST_CAP / 2;
+  uint32_t* T = cnt + C;
+  const RowPiece pc = s.rpieces[pi];
+  const ct_node nd = lists.nodes[pc.node];
+  CT_JOB_VIEW(v, vb, nd.slot);
+  const uint32_t* carry = pc.npieces > 1 ? s.carry + (size_t)pi * C : nullptr;
+  const uint32_t* tot = lists.tot + (size_t)pc.node * C;
+  const uint32_t n = nd.n;
+  RowBest* out = s.rbest + (size_t)s.cap_nodes * vb.sel_stride + pi;
+  const uint32_t f = s.sel[(size_t)pc.node * v.sel_stride + pc.slot];
+  PieceStream ps = piece_stream(v, nd, pc, f, lists.scan_piece, smem);
+  if (C <= SEQ_CLASSES) {
+    // staged in shared memory, SEQ_ROWS at a time, for the lane-sequential scan
+    uint2* ent = reinterpret_cast<uint2*>(smem + LIST_CAP / 2);
+    uint32_t* sq = smem + LIST_CAP / 2 + 2 * SEQ_SLOTS;
+    uint32_t* before = sq + SEQ_BEFORE;
+    const uint32_t mine = lane < C && carry ? carry[lane] : 0u;
+    const uint32_t last = lane >= C ? 0u : pc.j + 1 < pc.npieces ? carry[C + lane] : tot[lane];  // counts after the piece
+    const float known = __uint_as_float(*reinterpret_cast<volatile uint32_t*>(s.node_q + pc.node));
+    if (lane < SEQ_CLASSES) {
+      before[lane] = mine;
+      sq[lane] = last;
+    }
+    seq_totals(sq, tot, C);
+    uint32_t p0 = __reduce_add_sync(FULL, mine);
+    const bool empty = !__any_sync(FULL, last != mine);
+    __syncwarp();
+    // no candidate of the piece can reach the best known: nothing to scan
+    if (empty || gain_limit(before, sq, before + SEQ_CLASSES, C, n) < gain_bound(known, n)) {
+      if (lane == 0) *out = RowBest{dinf(), NONE, 0u, 0.f, 0.f};
+      return;
+    }
+    __syncwarp();
+    SeqBest bb{dinf(), NONE, 0u, 0.f, 0.f};
+    float x_last = 0.f;
+    bool first = true;
+    uint32_t keep = 0;
+    while (ps.fill(keep)) {
+      if (first && p0 > 0) {
+        x_last = __uint_as_float(value_before(v, ps, nd, pc, f, lists.scan_piece));
+        if (!ps.dense && __uint_as_float(ps.base[ps.count - 1].x) == x_last) break;  // no candidate in the piece
+      }
+      keep = 0;
+      for (uint32_t b = 0; b < ps.count; b += SEQ_ROWS) {
+        const uint32_t k = min(SEQ_ROWS, ps.count - b);
+        if (k < SEQ_ROWS && ps.more()) {  // with the next batch
+          keep = k;
+          break;
+        }
+        const uint32_t sh = seq_shift(k);
+#pragma unroll 4
+        for (uint32_t i = lane; i < k; i += 32) {
+          const uint2 e = ps.load(b + i);
+          ent[seq_at(i, sh)] = seq_entry(e.x, e.y);
+        }
+        __syncwarp();
+        if (first && p0 == 0) x_last = __uint_as_float(ent[0].x);  // no candidate before the node's first row
+        first = false;
+        const uint32_t i0 = min(lane << sh, k), m = min(k - i0, 1u << sh);
+        const uint2* run = ent + seq_at(i0, sh);
+        uint32_t w[4];
+        seq_count(run, m, w);
+        const float x_end = __uint_as_float(ent[seq_at(k - 1, sh)].x);
+        const float xp = i0 > 0 && m > 0 ? __uint_as_float(ent[seq_at(i0 - 1, sh)].x) : x_last;
+        seq_scan(run, m, sh, w, sq, C, xp, p0, n, s.node_q + pc.node, bb);
+        x_last = x_end;
+        p0 += k;
+      }
+    }
+    const uint32_t win = warp_best_lane(bb.score, bb.pos);
+    if (win == NONE ? lane == 0 : lane == win) *out = RowBest{bb.score, bb.pos, bb.pure, bb.xl, bb.xr};
+    return;
+  }
+  int64_t sl = 0, st2 = 0, a = 0;
+  uint32_t before = 0;
+  for (uint32_t c = lane; c < C; c += 32) {
+    const uint32_t k = carry ? carry[c] : 0u;
+    const uint32_t t = tot[c];
+    cnt[c] = k;
+    T[c] = t;
+    before += k;
+    sl += (int64_t)k * k;
+    st2 += (int64_t)t * t;
+    a += (int64_t)k * t;
+  }
+  sl = warp_sum_i64(sl);
+  st2 = warp_sum_i64(st2);
+  a = warp_sum_i64(a);
+  uint32_t p0 = __reduce_add_sync(FULL, before);  // the batch's first position
+  __syncwarp();
+  const double nn = (double)n;
+  double best = dinf();
+  uint32_t bpos = NONE, bpure = 0;
+  float bxl = 0.f, bxr = 0.f;
+  const unsigned lt = lanemask_lt();
+  constexpr uint32_t B = 32 * ROW_BATCH;
+  uint32_t x_last = 0;
+  bool first = true;
+  while (ps.fill()) {
+    if (first && p0 > 0) {
+      x_last = value_before(v, ps, nd, pc, f, lists.scan_piece);
+      // all of this batch equals the value before it: when the batch is the
+      // whole piece, it has no candidate
+      if (!ps.dense && __uint_as_float(ps.base[ps.count - 1].x) == __uint_as_float(x_last)) break;
+    }
+    uint2 cur[ROW_BATCH];
+#pragma unroll
+    for (uint32_t r = 0; r < ROW_BATCH; ++r)
+      cur[r] = r * 32 + lane < ps.count ? ps.load(r * 32 + lane) : make_uint2(0u, NONE);
+    if (first && p0 == 0) x_last = __shfl_sync(FULL, cur[0].x, 0);  // no candidate before the node's first row
+    first = false;
+    for (uint32_t base = 0; base < ps.count; base += B) {
+      uint2 nxt[ROW_BATCH];
+#pragma unroll
+      for (uint32_t r = 0; r < ROW_BATCH; ++r) {
+        const uint32_t i = base + B + r * 32 + lane;
+        nxt[r] = i < ps.count ? ps.load(i) : make_uint2(0u, NONE);
+      }
+#pragma unroll
+      for (uint32_t r = 0; r < ROW_BATCH; ++r) {
+        if (base + r * 32 >= ps.count) break;
+        const uint32_t i = base + r * 32 + lane;
+        const bool valid = i < ps.count;
+        const uint32_t c = cur[r].y;
+        uint32_t xpb = __shfl_up_sync(FULL, cur[r].x, 1);
+        if (lane == 0) xpb = x_last;
+        x_last = __shfl_sync(FULL, cur[r].x, min(31u, ps.count - 1 - (base + r * 32)));
+        const float x = __uint_as_float(cur[r].x), xp = __uint_as_float(xpb);
+        const unsigned grp = __match_any_sync(FULL, c);
+        int32_t dl = 0, dt = 0;
+        if (valid) {
+          dl = 2 * (int32_t)(cnt[c] + __popc(grp & lt)) + 1;
+          dt = (int32_t)T[c];
+        }
+        __syncwarp();
+        if (valid && (grp >> lane) == 1u) cnt[c] += __popc(grp);
+        __syncwarp();
+        // |partial sums| <= 32 (2 n + 1) < 2^31: n <= 2^22 here
+        const int32_t il = warp_incl_scan_i32(dl), it = warp_incl_scan_i32(dt);
+        const int64_t SL = sl + (il - dl);  // of the rows before this one
+        const int64_t SR = st2 - 2 * (a + (it - dt)) + SL;
+        sl += __shfl_sync(FULL, il, 31);
+        a += __shfl_sync(FULL, it, 31);
+        if (valid && is_candidate_sorted(xp, x)) {
+          const Scored sc = score_at(SL, SR, p0 + i, nn);
+          if (sc.score < best) {
+            best = sc.score;
+            bpos = p0 + i - 1;
+            bpure = sc.pure;
+            bxl = xp;
+            bxr = x;
+          }
+        }
+      }
+#pragma unroll
+      for (uint32_t r = 0; r < ROW_BATCH; ++r) cur[r] = nxt[r];
+    }
+    p0 += ps.count;
+  }
+  const uint32_t win = warp_best_lane(best, bpos);
+  if (win == NONE ? lane == 0 : lane == win) *out = RowBest{best, bpos, bpure, bxl, bxr};
+}
+
+template <bool Q>
+__global__ void __launch_bounds__(THREADS_PER_BLOCK, 7) k_row_scan(View v, LevelScratch s) {
+  extern __shared__ uint32_t smem[];
+  uint32_t* ws = smem + (threadIdx.x >> 5) * scan_words(v.n_classes);
+  const uint32_t count = live_count(s, s.ctr->n_scan_pieces, s.cap_scan);
+  const StepLists sl = *s.step;
+  for_items(count, &s.ctr->claim[ITEM_SCAN], [&](uint32_t i) { row_scan_item<Q>(v, sl, s, ws, i); });
+}
+
+// ------------------------------------------------------------------------
+// Best candidate of a node (lowest score, then feature, then position), its
+// record in the tree, and the pieces of its rows' split.
+template <bool Q>
+__device__ __forceinline__ void row_reduce_item(const View& vb, const StepLists& lists, const LevelScratch& s,
+                                                const TreeView& tv, uint32_t w) {
+  const uint32_t lane = lane_id();
+  const ct_node nd = lists.nodes[w];
+  CT_JOB_VIEW(v, vb, nd.slot);
+  const uint32_t C = v.n_classes, nsel = s.nsel[w], n = nd.n;
+  const uint32_t* sel = s.sel + (size_t)w * v.sel_stride;
+  RowBest bb{dinf(), NONE, 0u, 0.f, 0.f};
+  uint32_t bf = NONE;
+  auto take = [&](const RowBest& rb, uint32_t f) {
+    if (rb.score < bb.score || (rb.score == bb.score && (f < bf || (f == bf && rb.pos < bb.pos)))) {
+      bb = rb;
+      bf = f;
+    }
+  };
+  if (n <= GROUP_ROWS) {
+    for (uint32_t q = lane; q < nsel; q += 32)
+      if (!is_virtual(v, sel[q])) take(s.rbest[(size_t)w * v.sel_stride + q], sel[q]);
+  } else {
+    const uint32_t pb = s.piece_base[w], pn = s.piece_cnt[w];
+    const RowBest* best = s.rbest + (size_t)s.cap_nodes * vb.sel_stride;
+    for (uint32_t q = lane; q < pn; q += 32) take(best[pb + q], sel[s.rpieces[pb + q].slot]);
+  }
+  if (v.vmask) {
+    // a virtual feature's one candidate (the last low-value row), scored from
+    // the class counts of its high-value rows; one selected slot per lane
+    for (uint32_t q = lane; q < nsel; q += 32) {
+      const uint32_t f = sel[q];
+      if (!is_virtual(v, f)) continue;
+      const float2 lh = v.vval[f];
+      if (!is_candidate_sorted(lh.x, lh.y)) continue;
+      const uint32_t* hc = s.vcls + ((size_t)w * v.n_features + f) * C;
+      const uint32_t* tc = lists.tot + (size_t)w * C;
+      int64_t sl = 0, sr = 0;
+      for (uint32_t c = 0; c < C; ++c) {
+        const int64_t r = hc[c], l = (int64_t)tc[c] - r;
+        sl += l * l;
+        sr += r * r;
+      }
+      const uint32_t nl = n - s.vcnt[(size_t)w * 64 + f];
+      const Scored sc = score_at(sl, sr, nl, (double)n);
+      take(RowBest{sc.score, nl - 1, sc.pure, lh.x, lh.y}, f);
+    }
+  }
+  // lowest (score, feature, position) over the lanes
+  const uint64_t sb = (uint64_t)__double_as_longlong(bb.score);
+  const uint32_t mhi = __reduce_min_sync(FULL, (uint32_t)(sb >> 32));
+  const uint32_t mlo = __reduce_min_sync(FULL, (uint32_t)(sb >> 32) == mhi ? (uint32_t)sb : NONE);
+  bool tie = (uint32_t)(sb >> 32) == mhi && (uint32_t)sb == mlo;
+  const uint32_t mf = __reduce_min_sync(FULL, tie ? bf : NONE);
+  tie = tie && bf == mf;
+  const uint32_t mp = __reduce_min_sync(FULL, tie ? bb.pos : NONE);
+  tie = tie && bb.pos == mp;
+  const uint32_t win = (uint32_t)__ffs(__ballot_sync(FULL, tie)) - 1;
+  uint32_t split = mhi < 0x7ff00000u;
+  const size_t at = (size_t)(nd.slot + tv.slot_base) * tv.capacity + nd.raw_id;
+  const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
+  const uint32_t npp = ceil_div(n, PART_PIECE);
+  uint32_t sidx = 0, base = 0, children = 0;
+  if (split && lane == win) {
+    children = atomicAdd(&tv.n_nodes[nd.slot + tv.slot_base], 2u);
+    if (children + 2ull > tv.capacity) {
+      atomicOr(&s.ctr->error, DEV_ERR_CAPACITY);
+      split = 0;
+    } else {
+      tv.left[at] = children;
+      tv.right[at] = children + 1;
+      tv.feature[at] = bf;
+      tv.threshold[at] = midpoint(bb.xl, bb.xr);
+      tv.value[at] = 0;
+      sidx = atomicAdd(&s.ctr->n_splits, 1u);
+      atomicAdd(&s.ctr->split_total, (unsigned long long)n);
+      atomicAdd(&s.ctr->part_elems, (unsigned long long)n);
+      base = npp == 1 ? atomicAdd(&s.ctr->n_part_pieces, 1u) : atomicAdd(&s.ctr->n_status, npp);
+      if (sidx >= s.cap_nodes || (npp == 1 ? base >= s.cap_part : base + (uint64_t)npp > s.cap_mpart)) {
+        atomicOr(&s.ctr->error, DEV_ERR_CAPACITY);
+        split = 0;
+      } else {
+        s.rsplits[sidx] = RowSplit{w, bf, bb.pos + 1, children, bb.xl, bb.pure};
+      }
+    }
+  }
+  const uint32_t src = win & 31u;
+  const bool leaf = mhi >= 0x7ff00000u;
+  split = __shfl_sync(FULL, split, src);
+  if (leaf) {
+    const uint32_t value = first_row_class(v, rows, n);
+    if (lane == 0) write_leaf(tv, at, value);
+    return;
+  }
+  if (!split) return;
+  sidx = __shfl_sync(FULL, sidx, src);
+  base = __shfl_sync(FULL, base, src);
+  for (uint32_t c = lane; c < C; c += 32) s.split_left[(size_t)sidx * C + c] = 0;
+  PartPiece* list = npp == 1 ? s.part : s.mpart;
+  for (uint32_t j = lane; j < npp; j += 32) {
+    list[base + j] = PartPiece{sidx, j, npp, 0};
+    if (npp > 1) s.msup[base + j] = 0;
+  }
+}
+
+template <bool Q>
+__global__ void __launch_bounds__(THREADS_PER_BLOCK) k_row_reduce(View v, LevelScratch s, TreeView tv) {
+  const uint32_t count = live_count(s, s.ctr->n_nodes, s.cap_nodes);
+  const StepLists sl = *s.step;
+  for_items(count, &s.ctr->claim[ITEM_REDUCE], [&](uint32_t w) { row_reduce_item<Q>(v, sl, s, tv, w); });
+}
+
+// ------------------------------------------------------------------------
+// Left flags of a piece of a split node's rows: a row goes left when its
+// value is at most the split's xl, in the presort's order (a virtual feature:
+// when it has the low value).  Counts the left rows' classes.  A split of one piece moves its
+// rows at once; a longer one keeps the flags and counts for k_row_move.
+template <bool Q>
+__device__ __forceinline__ void row_mark_item(const View& vb, const StepLists& lists, const LevelScratch& s,
+                                              uint32_t* cnt, uint32_t nm, uint32_t i) {
+  const uint32_t C = vb.n_classes, lane = lane_id();
+  const bool multi = i < nm;
+  const PartPiece pp = multi ? s.mpart[i] : s.part[i - nm];
+  const RowSplit sr = s.rsplits[pp.split];
+  const ct_node nd = lists.nodes[sr.node];
+  CT_JOB_VIEW(v, vb, nd.slot);
+  const bool virt = is_virtual(v, sr.feature);
+  const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
+  const float* xf = v.x_fm + (size_t)sr.feature * v.n_rows;
+  const uint32_t lo = pp.j * PART_PIECE, hi = min(lo + PART_PIECE, nd.n);
+  const uint32_t xl = f32_order(sr.xl);
+  const unsigned lt = lanemask_lt();
+  uint32_t e[PART_ROUNDS];
+  unsigned lm[PART_ROUNDS];
+#pragma unroll
+  for (uint32_t r = 0; r < PART_ROUNDS; ++r) {
+    const uint32_t p = lo + r * 32 + lane;
+    e[r] = p < hi ? __ldcs(rows + p) : 0u;
+  }
+  uint32_t left = 0;  // bit r: this lane's row of round r goes left
+  if (virt) {
+#pragma unroll
+    for (uint32_t r = 0; r < PART_ROUNDS; ++r)
+      if (lo + r * 32 + lane < hi)
+        left |= (uint32_t)(!((__ldg(v.vrow + entry_row(v, e[r])) >> sr.feature) & 1ull)) << r;
+  } else {
+#pragma unroll
+    for (uint32_t r = 0; r < PART_ROUNDS; ++r)
+      if (lo + r * 32 + lane < hi) left |= (uint32_t)(f32_order(__ldg(xf + entry_row(v, e[r]))) <= xl) << r;
+  }
+  uint32_t nleft = 0;
+#pragma unroll
+  for (uint32_t r = 0; r < PART_ROUNDS; ++r) {
+    lm[r] = __ballot_sync(FULL, (left >> r) & 1u);
+    nleft += __popc(lm[r]);
+  }
+  uint32_t* out = s.split_left + (size_t)pp.split * C;
+  if (C <= 8) {
+    uint64_t pk = 0;  // 8-bit field per class, at most 16 rows per lane
+#pragma unroll
+    for (uint32_t r = 0; r < PART_ROUNDS; ++r)
+      if ((left >> r) & 1u) pk += 1ull << (8 * (e[r] >> v.lab_shift));
+    const uint32_t fh[2] = {(uint32_t)pk, (uint32_t)(pk >> 32)};
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+      if (4 * h >= C) break;
+      const uint32_t ev = __reduce_add_sync(FULL, fh[h] & 0x00ff00ffu), od = __reduce_add_sync(FULL, (fh[h] >> 8) & 0x00ff00ffu);
+      const uint32_t val = (lane & 1u ? od : ev) >> ((lane & 2u) * 8) & 0xffffu;
+      if (lane < 4 && 4 * h + lane < C && val) atomicAdd(&out[4 * h + lane], val);
+    }
+  } else {
+    for (uint32_t c = lane; c < C; c += 32) cnt[c] = 0;
+    __syncwarp();
+#pragma unroll
+    for (uint32_t r = 0; r < PART_ROUNDS; ++r) {
+      if (lo + r * 32 >= hi) break;
+      const uint32_t c = (left >> r) & 1u ? e[r] >> v.lab_shift : NONE;
+      const unsigned grp = __match_any_sync(FULL, c);
+      if (c != NONE && (grp >> lane) == 1u) cnt[c] += __popc(grp);
+      __syncwarp();
+    }
+    for (uint32_t c = lane; c < C; c += 32)
+      if (cnt[c]) atomicAdd(&out[c], cnt[c]);
+  }
+  if (multi) {
+    uint32_t mine = 0;
+#pragma unroll
+    for (uint32_t r = 0; r < PART_ROUNDS; ++r)
+      if (lane == r) mine = lm[r];
+    if (lane < PART_ROUNDS) s.mbits[(size_t)i * PART_ROUNDS + lane] = mine;
+    if (lane == 0) {
+      s.mleft[i] = nleft;
+      atomicAdd(&s.msup[i - pp.j + pp.j / 32], nleft);
+    }
+    return;
+  }
+  if (nleft != sr.nl) {  // the scan and the rows disagree
+    if (lane == 0) atomicOr(&s.ctr->error, DEV_ERR_INTERNAL);
+    return;
+  }
+  uint32_t* dst = row_list(v, nd.buf ^ 1u, nd.slot) + nd.start;
+  uint32_t run = 0;
+#pragma unroll
+  for (uint32_t r = 0; r < PART_ROUNDS; ++r) {
+    const uint32_t p = r * 32 + lane;
+    const uint32_t rl = run + __popc(lm[r] & lt);
+    if (p < hi) dst[(left >> r) & 1u ? rl : sr.nl + (p - rl)] = e[r];
+    run += __popc(lm[r]);
+  }
+}
+
+template <bool Q>
+__global__ void __launch_bounds__(THREADS_PER_BLOCK) k_row_mark(View v, LevelScratch s) {
+  extern __shared__ uint32_t smem[];
+  uint32_t* cnt = smem + (threadIdx.x >> 5) * v.n_classes;
+  const uint32_t nm = live_count(s, s.ctr->n_status, s.cap_mpart);
+  const uint32_t count = nm + live_count(s, s.ctr->n_part_pieces, s.cap_part);
+  const StepLists sl = *s.step;
+  for_items(count, &s.ctr->claim[ITEM_FILL], [&](uint32_t i) { row_mark_item<Q>(v, sl, s, cnt, nm, i); });
+}
+
+template <bool Q>
+__global__ void __launch_bounds__(THREADS_PER_BLOCK) k_row_move(View vb, LevelScratch s) {
+  const uint32_t count = live_count(s, s.ctr->n_status, s.cap_mpart);
+  const StepLists lists = *s.step;
+  const uint32_t lane = lane_id();
+  const unsigned lt = lanemask_lt();
+  for_items(count, &s.ctr->claim[ITEM_MOVE], [&](uint32_t i) {
+    const PartPiece pp = s.mpart[i];
+    const RowSplit sr = s.rsplits[pp.split];
+    const ct_node nd = lists.nodes[sr.node];
+    CT_JOB_VIEW(v, vb, nd.slot);
+    const uint32_t lo = pp.j * PART_PIECE, hi = min(lo + PART_PIECE, nd.n);
+    const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
+    uint32_t* dst = row_list(v, nd.buf ^ 1u, nd.slot) + nd.start;
+    uint32_t e[PART_ROUNDS];
+#pragma unroll
+    for (uint32_t r = 0; r < PART_ROUNDS; ++r) {
+      const uint32_t p = lo + r * 32 + lane;
+      e[r] = p < hi ? __ldcs(rows + p) : 0u;
+    }
+    const uint32_t mine = lane < PART_ROUNDS ? s.mbits[(size_t)i * PART_ROUNDS + lane] : 0u;
+    // left rows of the split's earlier pieces: whole runs of 32 pieces, then
+    // the pieces of this one's run
+    const uint32_t first = i - pp.j, blk = pp.j / 32;
+    uint32_t before = 0;
+    for (uint32_t k = lane; k < blk; k += 32) before += s.msup[first + k];
+    if (blk * 32 + lane < pp.j) before += s.mleft[first + blk * 32 + lane];
+    uint32_t run = __reduce_add_sync(FULL, before);
+#pragma unroll
+    for (uint32_t r = 0; r < PART_ROUNDS; ++r) {
+      const uint32_t p = lo + r * 32 + lane;
+      const unsigned m = __shfl_sync(FULL, mine, r);
+      const uint32_t rl = run + __popc(m & lt);
+      if (p < hi) {
+        const uint32_t d = (m >> lane) & 1u ? rl : sr.nl + (p - rl);
+        if (d < nd.n) dst[d] = e[r];
+      }
+      run += __popc(m);
+    }
+    if (pp.j + 1 == pp.npieces && run != sr.nl && lane == 0) atomicOr(&s.ctr->error, DEV_ERR_INTERNAL);
+  });
+}
+
+// ------------------------------------------------------------------------
+// Children of the step's splits: leaves, subtree roots, and the next level's
+// nodes with their class totals and constant-feature masks.
+template <bool Q>
+__device__ __forceinline__ void row_children_item(const View& vb, const StepLists& lists, const LevelScratch& s,
+                                                  const TreeView& tv, uint32_t cap_next, uint32_t small_cut,
+                                                  ct_node* small, uint32_t cap_small, uint32_t w) {
+  const uint32_t lane = lane_id();
+  const RowSplit sr = s.rsplits[w];
+  const ct_node nd = lists.nodes[sr.node];
+  CT_JOB_VIEW(v, vb, nd.slot);
+  const uint32_t C = v.n_classes;
+  for (uint32_t side = 0; side < 2; ++side) {
+    ct_node ch;
+    ch.slot = nd.slot;
+    ch.n = side ? nd.n - sr.nl : sr.nl;
+    ch.start = side ? nd.start + sr.nl : nd.start;
+    ch.raw_id = sr.children + side;
+    ch.key = child_key(nd.key, (int)side);
+    ch.impurity = 1.0f;
+    ch.buf = nd.buf ^ 1u;
+    const bool pure = (sr.pure >> side) & 1u;
+    if (pure || ch.n < v.mss) {
+      const uint32_t* rows = row_list(v, ch.buf, ch.slot) + ch.start;
+      const uint32_t value = pure ? rows[0] >> v.lab_shift : first_row_class(v, rows, ch.n);
+      if (lane == 0) write_leaf(tv, (size_t)(nd.slot + tv.slot_base) * tv.capacity + ch.raw_id, value);
+      continue;
+    }
+    if (small_cut != 0 && ch.n <= small_cut) {
+      uint32_t placed = 0;
+      if (lane == 0) {
+        const uint32_t idx = atomicAdd(&s.ctr->n_small, 1u);
+        if (idx < cap_small) {
+          small[idx] = ch;
+          atomicAdd(&s.ctr->small_total, (unsigned long long)ch.n);
+          placed = 1;
+        }
+      }
+      if (__shfl_sync(FULL, placed, 0)) continue;
+      // the subtree list is full: the level steps split this child
+    }
+    uint32_t idx = 0;
+    if (lane == 0) {
+      idx = atomicAdd(&s.ctr->n_next, 1u);
+      if (idx < cap_next) {
+        lists.next[idx] = ch;
+        atomicAdd(&s.ctr->next_total, (unsigned long long)ch.n);
+      } else {
+        atomicOr(&s.ctr->error, DEV_ERR_CAPACITY);
+      }
+    }
+    idx = __shfl_sync(FULL, idx, 0);
+    if (idx >= cap_next) continue;
+    for (uint32_t c = lane; c < C; c += 32) {
+      const uint32_t left = s.split_left[(size_t)w * C + c];
+      lists.next_tot[(size_t)idx * C + c] = side ? lists.tot[(size_t)sr.node * C + c] - left : left;
+    }
+    if (lists.next_mask) {
+      // the parent's constant features; a two-valued split feature is constant in both children
+      const uint32_t mw = mask_words(v.n_features);
+      const uint64_t* pm = lists.node_mask + (size_t)sr.node * v.mask_stride;
+      uint64_t* cm = lists.next_mask + (size_t)idx * v.mask_stride;
+      const bool tv2 = two_valued(v, sr.feature);
+      for (uint32_t k = lane; k < mw; k += 32)
+        cm[k] = pm[k] | (tv2 && (sr.feature >> 6) == k ? 1ull << (sr.feature & 63) : 0ull);
+    }
+  }
+}
+
+template <bool Q>
+__global__ void __launch_bounds__(THREADS_PER_BLOCK)
+k_row_children(View v, LevelScratch s, TreeView tv, uint32_t cap_next, uint32_t small_cut, ct_node* small,
+               uint32_t cap_small) {
+  const uint32_t count = live_count(s, s.ctr->n_splits, s.cap_nodes);
+  const StepLists sl = *s.step;
+  for_items(count, &s.ctr->claim[ITEM_CHILDREN], [&](uint32_t w) {
+    row_children_item<Q>(v, sl, s, tv, cap_next, small_cut, small, cap_small, w);
+  });
+}
+
+// ------------------------------------------------------------------------
+// Subtrees of at most 32 rows, one warp each, one row per lane (lanes in
+// feature-0 order, so a node's leaf label is its lowest lane's).  A virtual
+// feature needs no gather (its rows' value bits are read once per subtree)
+// and no sort: its one candidate separates the lanes by their bit.  Another
+// feature is sorted by 32-bit keys, rank above lane.
+struct RowSub {
+  uint32_t mask;
+  uint32_t raw;
+  uint64_t key;
+};
+
+__device__ __forceinline__ uint32_t warp_sort_u32(uint32_t v, uint32_t lane) {
+  uint32_t a[1] = {v};
+  warp_sort_keys<1>(a, lane);
+  return a[0];
+}
+
+__device__ __forceinline__ void grow_rows(const View& v, const LevelScratch& s, const TreeView& tv, uint32_t tslot,
+                                          uint32_t row, uint32_t lab, uint64_t vbits, RowSub cur, RowSub* stack,
+                                          uint32_t lane) {
+  const uint32_t F = v.n_features, m = v.max_features;
+  const size_t toff = (size_t)tslot * tv.capacity;
+  const unsigned lt = lanemask_lt();
+  int sp = 0;
+  while (true) {
+    const uint32_t mask = cur.mask;
+    const uint32_t n = __popc(mask);
+    const bool in = (mask >> lane) & 1u;
+    const unsigned same = __match_any_sync(FULL, in ? lab : NONE);  // lanes of this lane's class
+    const int32_t tcls = (int32_t)__popc(same);
+    const int32_t st2 = (int32_t)__reduce_add_sync(FULL, in ? (uint32_t)tcls : 0u);
+    const double nn = (double)n;
+    double best = dinf();
+    uint32_t bf = NONE, bmask = 0, bpure = 0;
+    float bthr = 0.f;
+    uint32_t taken = 0;
+    uint32_t perm = feature_perm(min(lane, F - 1), F, cur.key, v.feistel_h);  // permutation positions [0, 32)
+    uint32_t f_nx = __shfl_sync(FULL, perm, 0);
+    bool v_nx = is_virtual(v, f_nx);
+    uint2 pr_nx = in && !v_nx ? __ldg(v.pair + (size_t)f_nx * v.n_rows + row) : make_uint2(0u, 0u);
+    for (uint32_t i = 0; i < F && taken < m; ++i) {
+      const uint32_t f = f_nx;
+      const bool virt = v_nx;
+      const uint2 pr = pr_nx;
+      if (i + 1 < F) {  // the next feature's values are gathered while this one is sorted and scanned
+        if (((i + 1) & 31u) == 0u) perm = feature_perm(min(i + 1 + lane, F - 1), F, cur.key, v.feistel_h);
+        f_nx = __shfl_sync(FULL, perm, (i + 1) & 31u);
+        v_nx = is_virtual(v, f_nx);
+        if (in && !v_nx) pr_nx = __ldg(v.pair + (size_t)f_nx * v.n_rows + row);
+      }
+      if (virt) {
+        const unsigned hm = __ballot_sync(FULL, in && ((vbits >> f) & 1ull));
+        if (hm == 0u || hm == mask) continue;
+        ++taken;
+        const float2 lh = v.vval[f];
+        if (!is_candidate_sorted(lh.x, lh.y)) continue;
+        const unsigned lo_m = mask & ~hm;
+        // sums of squared class counts, as sums over the side's rows of their class's count there
+        const bool low = (lo_m >> lane) & 1u;
+        const uint32_t k = in ? (uint32_t)__popc(same & (low ? lo_m : hm)) : 0u;
+        const uint32_t both = __reduce_add_sync(FULL, low ? k : k << 16);  // each at most 32 x 32
+        const Scored sc = score_at((int64_t)(both & 0xffffu), (int64_t)(both >> 16), (uint32_t)__popc(lo_m), nn);
+        if (sc.score < best || (sc.score == best && f < bf)) {
+          best = sc.score;
+          bf = f;
+          bpure = sc.pure;
+          bmask = lo_m;
+          bthr = midpoint(lh.x, lh.y);
+        }
+        continue;
+      }
+      const float xv = __uint_as_float(pr.y);
+      const uint32_t ord = f32_order(xv);
+      const uint32_t o0 = __shfl_sync(FULL, ord, __ffs(mask) - 1);
+      if (!__any_sync(FULL, in && ord != o0)) continue;
+      ++taken;
+      const uint32_t sk = warp_sort_u32(in ? (pr.x << 5) | lane : NONE, lane);  // lane p holds sorted position p
+      const bool valid = lane < n;
+      const uint32_t src = sk & 31u;
+      const float x = __shfl_sync(FULL, xv, src);
+      const uint32_t cl = __shfl_sync(FULL, lab, src);
+      const int32_t tc = __shfl_sync(FULL, tcls, src);
+      const float xn = __shfl_down_sync(FULL, x, 1);
+      const unsigned grp = __match_any_sync(FULL, valid ? cl : NONE);
+      const uint32_t packed = valid ? (2u * (uint32_t)__popc(grp & lt) + 1u) | ((uint32_t)tc << 16) : 0u;
+      const uint32_t incl = (uint32_t)warp_incl_scan_i32((int32_t)packed);
+      const int32_t SL = (int32_t)(incl & 0xffffu);
+      const int32_t SR = st2 - 2 * (int32_t)(incl >> 16) + SL;
+      Scored sc{dinf(), 0u};
+      if (valid && lane + 1 < n && is_candidate_sorted(x, xn)) sc = score_at(SL, SR, lane + 1, nn);
+      const uint32_t win = warp_best_lane(sc.score, lane);
+      if (win == NONE) continue;
+      const double ws = __shfl_sync(FULL, sc.score, win);
+      if (ws < best || (ws == best && f < bf)) {
+        best = ws;
+        bf = f;
+        bpure = __shfl_sync(FULL, sc.pure, win);
+        bmask = __reduce_or_sync(FULL, (valid && lane <= win) ? (1u << src) : 0u);
+        bthr = midpoint(__shfl_sync(FULL, x, win), __shfl_sync(FULL, xn, win));
+      }
+    }
+    bool split = bf != NONE;
+    uint32_t c0 = 0;
+    if (split && lane == 0) {
+      c0 = atomicAdd(&tv.n_nodes[tslot], 2u);
+      if (c0 + 2ull > tv.capacity) {
+        atomicOr(&s.ctr->error, DEV_ERR_CAPACITY);
+        split = false;
+      }
+    }
+    split = __shfl_sync(FULL, split, 0);
+    c0 = __shfl_sync(FULL, c0, 0);
+    if (!split) {
+      const uint32_t value = __shfl_sync(FULL, lab, __ffs(mask) - 1);
+      if (lane == 0) write_leaf(tv, toff + cur.raw, value);
+    } else {
+      if (lane == 0) {
+        tv.left[toff + cur.raw] = c0;
+        tv.right[toff + cur.raw] = c0 + 1;
+        tv.feature[toff + cur.raw] = bf;
+        tv.threshold[toff + cur.raw] = bthr;
+        tv.value[toff + cur.raw] = 0;
+      }
+      for (uint32_t side = 0; side < 2; ++side) {
+        const uint32_t cm = side ? mask & ~bmask : bmask;
+        if (((bpure >> side) & 1u) || (uint32_t)__popc(cm) < v.mss) {
+          const uint32_t value = __shfl_sync(FULL, lab, __ffs(cm) - 1);
+          if (lane == 0) write_leaf(tv, toff + c0 + side, value);
+        } else if (sp < 33) {
+          if (lane == 0) stack[sp] = RowSub{cm, c0 + side, child_key(cur.key, (int)side)};
+          ++sp;
+        } else {
+          if (lane == 0) atomicOr(&s.ctr->error, DEV_ERR_INTERNAL);
+        }
+      }
+    }
+    __syncwarp();
+    if (sp == 0) break;
+    --sp;
+    cur = stack[sp];
+    __syncwarp();
+  }
+}
+
+template <bool Q>
+__global__ void __launch_bounds__(THREADS_PER_BLOCK)
+k_row_subtree(View vb, const ct_node* __restrict__ small, LevelScratch s, TreeView tv, uint32_t cap_small) {
+  __shared__ RowSub stack_all[WARPS_PER_BLOCK][33];
+  const uint32_t lane = lane_id();
+  const uint32_t count = live_count(s, s.ctr->n_small, cap_small);
+  for_items(count, &s.ctr->claim[ITEM_SUBTREE], [&](uint32_t w) {
+    const ct_node nd = small[w];
+    CT_JOB_VIEW(v, vb, nd.slot);
+    const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
+    const bool have = lane < nd.n;
+    uint32_t e = have ? rows[lane] : 0u;
+    // lanes in feature-0 order
+    const uint32_t k0 = have ? (__ldg(&v.pair[entry_row(v, e)].x) << 5) | lane : NONE;
+    const uint32_t sk = warp_sort_u32(k0, lane);
+    e = __shfl_sync(FULL, e, sk & 31u);
+    const uint32_t row = have ? entry_row(v, e) : 0u;
+    const uint32_t lab = have ? e >> v.lab_shift : NONE;
+    const uint64_t vbits = have && v.vmask ? __ldg(v.vrow + row) : 0ull;
+    const RowSub cur{nd.n >= 32 ? FULL : ((1u << nd.n) - 1u), nd.raw_id, nd.key};
+    grow_rows(v, s, tv, nd.slot + tv.slot_base, row, lab, vbits, cur, stack_all[threadIdx.x >> 5], lane);
+  });
+}
+
+uint32_t sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return (uint32_t)std::max(1, sms);
+}
+
+inline uint32_t clamp32(uint64_t x) { return x > 0xffffffffull ? 0xffffffffu : (uint32_t)x; }
+
+// A kernel of CTAs that claim bitmap work: as many as are resident at once.
+template <typename K, typename... A>
+int launch_bitmap(K kernel, int threads, size_t smem, uint32_t items, cudaStream_t st, const A&... args) {
+  CT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ORDER_SMEM_MAX));
+  int per = 1;
+  CT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem));
+  kernel<<<std::min<uint32_t>(items, sm_count() * (uint32_t)std::max(1, per)), threads, smem, st>>>(args...);
+  CT_CUDA_TRY(cudaGetLastError());
+  return CT_OK;
+}
+
+template <bool Q>
+int row_step(const View& v, const LevelScratch& s, LevelBounds b, uint32_t n_max, const TreeView& tv,
+             uint32_t cap_next, uint32_t small_cut, ct_node* small, uint32_t cap_small, cudaStream_t st) {
+  Prof* pf = current_prof();
+  const uint32_t C = v.n_classes;
+  const size_t sm1 = (size_t)WARPS_PER_BLOCK * C * sizeof(uint32_t);
+  const uint64_t nodes = std::min<uint64_t>(b.nodes, s.cap_nodes);
+  const uint32_t sms = sm_count();
+  if (v.vmask) {
+    pf->begin(CT_K_SCAN);
+    CT_TRY(launch_virtual_counts(v, s, nodes, s.cap_vpieces, st));
+    pf->end();
+    pf->launched(CT_K_SCAN, 2);
+  }
+  pf->begin(CT_K_SELECT);
+  k_row_select<Q><<<grid_for(k_row_select<Q>, nodes, 0, true), THREADS_PER_BLOCK, 0, st>>>(v, s);
+  pf->launched(CT_K_SELECT);
+  if (n_max > SELECT_ROWS) {  // (a bitmap of several slices needs more rows than that)
+    k_row_select_big<Q><<<std::min(s.cap_big, sms), 512, 0, st>>>(v, s);
+    pf->launched(CT_K_SELECT);
+  }
+  pf->end();
+  if (n_max > GROUP_ROWS) {
+    pf->begin(CT_K_PARTITION);
+    CT_TRY(launch_bitmap(k_row_bits<Q>, BITS_THREADS, (size_t)bits_words(n_max) * 4, s.cap_units, st, v, s, n_max));
+    pf->launched(CT_K_PARTITION);
+    if (!row_dense(GROUP_ROWS + 1, n_max)) {  // some nodes above the group size may be sparse
+      CT_TRY(launch_bitmap(k_row_order<Q>, ORDER_THREADS, order_smem(n_max), s.cap_order, st, v, s));
+      pf->launched(CT_K_PARTITION);
+    }
+    pf->end();
+  }
+  pf->begin(CT_K_SCAN);
+  if (n_max > WARP_ROWS) {
+    CT_TRY(launch_bitmap(k_row_group<Q, GROUP_SMALL_WARPS>, 32 * GROUP_SMALL_WARPS,
+                         group_words<GROUP_SMALL_WARPS>(C, n_max) * sizeof(uint32_t), s.cap_order, st, v, s, n_max));
+    pf->launched(CT_K_SCAN);
+  }
+  if (n_max > GROUP_SMALL_ROWS) {
+    CT_TRY(launch_bitmap(k_row_group<Q, GROUP_WARPS>, 32 * GROUP_WARPS,
+                         group_words<GROUP_WARPS>(C, n_max) * sizeof(uint32_t), s.cap_order, st, v, s, n_max));
+    pf->launched(CT_K_SCAN);
+  }
+  if (n_max > GROUP_ROWS) {
+    const size_t smh = (size_t)WARPS_PER_BLOCK * hist_words(C) * sizeof(uint32_t);
+    const size_t sms2 = (size_t)WARPS_PER_BLOCK * scan_words(C) * sizeof(uint32_t);
+    // every list is a bitmap whose classes k_row_bits counts, unless some are
+    // sparse or the shortest pieces are too many for it
+    const bool hist = !row_dense(GROUP_ROWS + 1, n_max) || (uint64_t)ceil_div(n_max, 1024) * C > BITS_COUNTS;
+    if (hist) k_row_hist<Q><<<grid_for(k_row_hist<Q>, s.cap_scan, smh, true), THREADS_PER_BLOCK, smh, st>>>(v, s);
+    k_row_carry<<<grid_for(k_row_carry, (uint64_t)s.cap_order * C, 0, true), THREADS_PER_BLOCK, 0, st>>>(s, C);
+    if (C <= SEQ_CLASSES) {
+      k_row_bound<Q><<<sms * 8, 256, 0, st>>>(v, s);
+      pf->launched(CT_K_SCAN);
+    }
+    k_row_scan<Q><<<grid_for(k_row_scan<Q>, s.cap_scan, sms2, true), THREADS_PER_BLOCK, sms2, st>>>(v, s);
+    pf->launched(CT_K_SCAN, hist ? 3 : 2);
+  }
+  const size_t smw = (size_t)WARPS_PER_BLOCK * warp_item_words(C) * sizeof(uint32_t);
+  k_row_warp<Q><<<grid_for(k_row_warp<Q>, s.cap_w, smw, true), THREADS_PER_BLOCK, smw, st>>>(v, s);
+  pf->end();
+  pf->launched(CT_K_SCAN);
+  pf->begin(CT_K_REDUCE);
+  k_row_reduce<Q><<<grid_for(k_row_reduce<Q>, nodes, 0, true), THREADS_PER_BLOCK, 0, st>>>(v, s, tv);
+  pf->end();
+  pf->launched(CT_K_REDUCE);
+  pf->begin(CT_K_MARK);
+  k_row_mark<Q><<<grid_for(k_row_mark<Q>, (uint64_t)s.cap_mpart + s.cap_part, sm1, true), THREADS_PER_BLOCK, sm1, st>>>(
+      v, s);
+  pf->end();
+  pf->launched(CT_K_MARK);
+  if (n_max > PART_PIECE) {
+    pf->begin(CT_K_PARTITION);
+    k_row_move<Q><<<grid_for(k_row_move<Q>, s.cap_mpart, 0, true), THREADS_PER_BLOCK, 0, st>>>(v, s);
+    pf->end();
+    pf->launched(CT_K_PARTITION);
+  }
+  pf->begin(CT_K_CHILDREN);
+  k_row_children<Q><<<grid_for(k_row_children<Q>, nodes, 0, true), THREADS_PER_BLOCK, 0, st>>>(
+      v, s, tv, cap_next, small_cut, small, cap_small);
+  pf->end();
+  pf->launched(CT_K_CHILDREN);
+  CT_CUDA_TRY(cudaGetLastError());
+  return CT_OK;
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------------
+// Sorted planes (8 bytes per row and slot) that fit behind the row list in
+// each of the two list buffers (4 bytes per row and slot of n_features *
+// index_bytes).
+static uint32_t planes_per_buffer(const ct_problem* p) {
+  const uint64_t per_row = (uint64_t)p->n_features * p->index_bytes;
+  return per_row < 16 ? 0u : (uint32_t)std::min<uint64_t>((per_row - 8) / 8, 1u << 20);
+}
+bool rows_have_large(uint32_t n_rows) { return n_rows > GROUP_ROWS; }
+uint32_t rows_planes_needed(const ct_problem* p) {
+  return rows_have_large(p->n_rows) ? std::min(p->max_features, p->n_features) : 0u;
+}
+uint32_t rows_planes_in_lists(const ct_problem* p) {
+  const uint32_t k = planes_per_buffer(p);
+  return 2 * k >= rows_planes_needed(p) ? k : 0u;
+}
+
+// A row id and a label share 32 bits, the row list fits a list buffer, and the
+// rank bitmap fits shared memory.
+bool rows_possible(const ct_problem* p) {
+  const uint32_t row_bits = p->n_rows > 1 ? 32u - (uint32_t)__builtin_clz(p->n_rows - 1) : 1u;
+  const uint32_t lab_bits = p->n_classes > 1 ? 32u - (uint32_t)__builtin_clz(p->n_classes - 1) : 0u;
+  return row_bits + lab_bits <= 32 && row_bits <= 22 && (uint64_t)p->n_features * p->index_bytes >= 4 &&
+         order_smem(p->n_rows) <= ORDER_SMEM_MAX && (size_t)bits_words(p->n_rows) * 4 <= ORDER_SMEM_MAX &&
+         (p->n_rows <= WARP_ROWS ||
+          group_words<GROUP_SMALL_WARPS>(p->n_classes, p->n_rows) * sizeof(uint32_t) <= ORDER_SMEM_MAX) &&
+         (p->n_rows <= GROUP_SMALL_ROWS ||
+          group_words<GROUP_WARPS>(p->n_classes, p->n_rows) * sizeof(uint32_t) <= ORDER_SMEM_MAX) &&
+         p->n_features < 65535u;
+}
+
+bool carve_row_scratch(Arena& a, const View& v, LevelBounds b, uint32_t scan_piece, LevelScratch* s, bool virt) {
+  const size_t C = v.n_classes, m = v.sel_stride;
+  LevelScratch& t = *s;
+  t = LevelScratch{};
+  t.cap_nodes = clamp32(b.nodes);
+  // A sparse node makes at most n / piece + 1 pieces per slot, a dense one at
+  // most 2 n / piece + 1 (its runs of ranks hold half a piece at the least) or,
+  // at the longest run and 64 n >= n_rows, n / 512 + 1.
+  const uint64_t large = b.samples / (WARP_ROWS + 1);  // nodes above the warp size
+  t.cap_scan = clamp32(m * (2 * b.samples / scan_piece + b.samples / 512 + large) + 1);
+  t.cap_order = clamp32(m * large + 1);
+  t.cap_units = clamp32(m * (b.samples / BITS_SLICE + large) + 1);
+  t.cap_w = clamp32(m * b.nodes + 1);
+  t.cap_part = t.cap_nodes;
+  t.cap_mpart = clamp32(b.samples / PART_PIECE + b.samples / (PART_PIECE + 1) + 1);
+  t.cap_big = clamp32(b.samples / SELECT_ROWS + 1);
+  t.cap_vpieces = virt ? clamp32(b.samples / VPIECE + b.nodes + 1) : 0u;
+  t.ctr = a.take<Counters>(1);
+  t.step = a.take<StepLists>(1);
+  t.sel = a.take<uint32_t>(t.cap_nodes * m);
+  t.nsel = a.take<uint32_t>(t.cap_nodes);
+  t.node_q = a.take<uint32_t>(t.cap_nodes);
+  t.piece_base = a.take<uint32_t>(t.cap_nodes);
+  t.piece_cnt = a.take<uint32_t>(t.cap_nodes);
+  t.witems = a.take<uint2>(t.cap_w);
+  t.oitems = a.take<uint2>(t.cap_order);
+  t.bunits = a.take<uint4>(t.cap_units);
+  t.bzero = a.take<uint4>(t.cap_order);
+  t.citems = a.take<uint2>(t.cap_order);
+  t.gsmall = a.take<uint2>(t.cap_order);
+  t.glarge = a.take<uint2>(t.cap_order);
+  t.rpieces = a.take<RowPiece>(t.cap_scan);
+  t.rbest = a.take<RowBest>((size_t)t.cap_nodes * m + t.cap_scan);
+  t.carry = a.take<uint32_t>((size_t)t.cap_scan * C);
+  t.rsplits = a.take<RowSplit>(t.cap_nodes);
+  t.split_left = a.take<uint32_t>((size_t)t.cap_nodes * C);
+  t.part = a.take<PartPiece>(t.cap_part);
+  t.mpart = a.take<PartPiece>(t.cap_mpart);
+  t.mbits = a.take<uint32_t>((size_t)t.cap_mpart * PART_ROUNDS);
+  t.mleft = a.take<uint32_t>(t.cap_mpart);
+  t.msup = a.take<uint32_t>(t.cap_mpart);
+  t.big_nodes = a.take<uint32_t>(t.cap_big);
+  t.vcnt = virt ? a.take<uint32_t>((size_t)t.cap_nodes * 64) : nullptr;
+  t.vcls = virt ? a.take<uint32_t>((size_t)t.cap_nodes * v.n_features * C) : nullptr;
+  t.vpieces = virt ? a.take<uint2>(t.cap_vpieces) : nullptr;
+  return a.ok();
+}
+
+template <typename IdxT, typename LabT>
+static void row_pairs(const View& v, const ct_problem* p, uint2* pair, uint2* ranked, uint32_t* rank,
+                      cudaStream_t st) {
+  const dim3 grid(std::min<uint32_t>(ceil_div(p->n_rows, 1024), 512u), p->n_features);
+  k_row_pairs<IdxT, LabT><<<grid, 256, 0, st>>>(reinterpret_cast<const IdxT*>(p->presort), p->x_fm,
+                                                reinterpret_cast<const LabT*>(p->labels), p->n_rows, v.vmask, pair,
+                                                ranked, rank);
+}
+int launch_row_pairs(const View& v, const ct_problem* p, uint2* pair, uint2* ranked, uint32_t* rank, cudaStream_t st) {
+  if (p->index_bytes == 2 && p->label_bytes == 1) row_pairs<uint16_t, uint8_t>(v, p, pair, ranked, rank, st);
+  else if (p->index_bytes == 2) row_pairs<uint16_t, uint16_t>(v, p, pair, ranked, rank, st);
+  else if (p->label_bytes == 1) row_pairs<uint32_t, uint8_t>(v, p, pair, ranked, rank, st);
+  else row_pairs<uint32_t, uint16_t>(v, p, pair, ranked, rank, st);
+  CT_CUDA_TRY(cudaGetLastError());
+  return CT_OK;
+}
+
+int launch_row_roots(const View& v, const ct_problem* p, uint32_t slot_lo, uint32_t n_slots, uint32_t tree_lo,
+                     uint32_t* n_in, const TreeView& tv, ct_node* out, uint32_t* out_tot, uint32_t cap, Counters* ctr,
+                     uint64_t* out_mask, const float2* vals, cudaStream_t st) {
+  const size_t smem = ((size_t)(p->n_rows + 31) / 32 + v.n_classes) * sizeof(uint32_t);
+  const uint32_t threads = p->n_rows >= 8192 ? 1024u : p->n_rows >= 1024 ? 512u : 128u;
+  if (p->label_bytes == 1) {
+    static const cudaError_t configured =
+        cudaFuncSetAttribute(k_row_roots<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ORDER_SMEM_MAX);
+    CT_CUDA_TRY(configured);
+    k_row_roots<uint8_t><<<n_slots, threads, smem, st>>>(v, p->seed, p->bootstrap, slot_lo, tree_lo, n_in, tv, out,
+                                                         out_tot, cap, ctr, out_mask, vals);
+  } else {
+    static const cudaError_t configured =
+        cudaFuncSetAttribute(k_row_roots<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ORDER_SMEM_MAX);
+    CT_CUDA_TRY(configured);
+    k_row_roots<uint16_t><<<n_slots, threads, smem, st>>>(v, p->seed, p->bootstrap, slot_lo, tree_lo, n_in, tv, out,
+                                                          out_tot, cap, ctr, out_mask, vals);
+  }
+  CT_CUDA_TRY(cudaGetLastError());
+  return CT_OK;
+}
+
+int launch_row_step(const View& v, const LevelScratch& s, LevelBounds b, uint32_t n_max, const TreeView& tv,
+                    uint32_t cap_next, uint32_t small_cut, ct_node* small, uint32_t cap_small, cudaStream_t st) {
+  return v.jobs ? row_step<true>(v, s, b, n_max, tv, cap_next, small_cut, small, cap_small, st)
+                : row_step<false>(v, s, b, n_max, tv, cap_next, small_cut, small, cap_small, st);
+}
+
+int launch_row_subtrees(const View& v, const ct_node* small, uint32_t cap_small, uint32_t bound, const LevelScratch& s,
+                        const TreeView& tv, cudaStream_t st) {
+  if (cap_small == 0 || bound == 0) return CT_OK;
+  Prof* pf = current_prof();
+  pf->begin(CT_K_SUBTREE);
+  const uint32_t items = std::min(bound, cap_small);
+  if (v.jobs)
+    k_row_subtree<true><<<grid_for(k_row_subtree<true>, items, 0, true), THREADS_PER_BLOCK, 0, st>>>(v, small, s, tv,
+                                                                                                      cap_small);
+  else
+    k_row_subtree<false><<<grid_for(k_row_subtree<false>, items, 0, true), THREADS_PER_BLOCK, 0, st>>>(v, small, s, tv,
+                                                                                                        cap_small);
+  pf->end();
+  pf->launched(CT_K_SUBTREE);
+  CT_CUDA_TRY(cudaGetLastError());
+  return CT_OK;
+}
+
+}  // namespace ct
