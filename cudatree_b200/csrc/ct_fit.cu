@@ -1382,6 +1382,66 @@ bool layout_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options*
   return base != nullptr && a.ok();
 }
 
+// Row-list growth of a queue: the jobs' own arrays, by offset from the
+// workspace's base.
+struct QueueRows {
+  std::vector<uint2*> pair, ranked, planes;
+  std::vector<uint32_t*> rank;
+  std::vector<float2*> vals;
+};
+
+bool queue_rows_possible(const ct_fit_job* jobs, uint32_t n_jobs) {
+  const QueueShape q = queue_shape(jobs, n_jobs);
+  const ct_problem pb = batch_problem(jobs, q);  // the kernels' shared memory is sized by the batch's largest N and C
+  if (!rows_possible(&pb)) return false;
+  for (uint32_t j = 0; j < n_jobs; ++j)
+    if (!rows_possible(&jobs[j].problem) || (((uintptr_t)jobs[j].lists.si0 | (uintptr_t)jobs[j].lists.si1) & 15u))
+      return false;
+  return true;
+}
+
+bool layout_queue_rows(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o, char* base, size_t size,
+                       FitLayout* L, View** views_dev, uint32_t** slot_job_dev, QueueRows* qr) {
+  const QueueShape q = queue_shape(jobs, n_jobs);
+  const ct_problem pb = batch_problem(jobs, q);
+  layout_options(&pb, q.slots, o, L);
+  L->rows = true;
+  L->cap_list = (uint32_t)std::min<uint64_t>(q.samples / 2 + q.slots + 2, 0xffffffffull);
+  L->chunk = std::min<uint32_t>(L->cap_list, o->step_nodes ? o->step_nodes : CHUNK_NODES_MAX);
+  L->subtree_cut = std::min<uint32_t>(o->subtree_cutoff, 32u);
+  L->cap_small = L->subtree_cut ? 2 * L->chunk : 0u;
+  Arena a{base, size, 0};
+  L->small = L->cap_small ? a.take<ct_node>(L->cap_small) : nullptr;
+  L->n_in = a.take<uint32_t>(q.slots);
+  L->fbin = a.take<uint32_t>(q.fbin_words);
+  L->ffwork = a.take<char>(q.ff_bytes);
+  for (int i = 0; i < 2; ++i) {
+    L->list[i] = a.take<ct_node>(L->cap_list);
+    L->tot[i] = a.take<uint32_t>((size_t)L->cap_list * q.c_max);
+    L->mask[i] = a.take<uint64_t>((size_t)L->cap_list * L->mask_words);
+  }
+  for (uint32_t j = 0; j < n_jobs; ++j) {
+    const ct_problem& p = jobs[j].problem;
+    const size_t cells = (size_t)p.n_features * p.n_rows;
+    const bool large = rows_have_large(p.n_rows);
+    const uint32_t planes = rows_planes_needed(&p);
+    qr->pair.push_back(a.take<uint2>(cells));
+    qr->ranked.push_back(large ? a.take<uint2>(cells) : nullptr);
+    qr->rank.push_back(large ? a.take<uint32_t>(cells) : nullptr);
+    qr->planes.push_back(planes && !rows_planes_in_lists(&p)
+                             ? a.take<uint2>((size_t)planes * jobs[j].lists.n_slots * jobs[j].lists.stride)
+                             : nullptr);
+    qr->vals.push_back(a.take<float2>(p.n_features));
+  }
+  View v = make_view(&pb, nullptr);
+  carve_row_scratch(a, v, LevelBounds{L->chunk, q.samples}, step_piece(0, L->scan_piece, 1), &L->s, false);
+  L->ctl = a.take<LoopCtl>(1);
+  *views_dev = a.take<View>(n_jobs);
+  *slot_job_dev = a.take<uint32_t>(q.slots);
+  L->bytes = a.used + 256;
+  return base != nullptr && a.ok();
+}
+
 }  // namespace
 
 size_t fit_queue_workspace_bytes(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o) {
@@ -1389,7 +1449,13 @@ size_t fit_queue_workspace_bytes(const ct_fit_job* jobs, uint32_t n_jobs, const 
   View* vd = nullptr;
   uint32_t* sj = nullptr;
   layout_queue(jobs, n_jobs, o, nullptr, 0, &L, &vd, &sj);
-  return L.bytes;
+  size_t bytes = L.bytes;
+  if (queue_rows_possible(jobs, n_jobs)) {
+    QueueRows qr;
+    layout_queue_rows(jobs, n_jobs, o, nullptr, 0, &L, &vd, &sj, &qr);
+    bytes = std::max(bytes, L.bytes);
+  }
+  return bytes;
 }
 
 int check_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o, const ct_tree_buffers* trees) {
@@ -1425,7 +1491,11 @@ int fit_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o, 
   FitLayout L{};
   View* views_dev = nullptr;
   uint32_t* slot_job_dev = nullptr;
-  if (!layout_queue(jobs, n_jobs, o, reinterpret_cast<char*>(ws), wsb, &L, &views_dev, &slot_job_dev)) {
+  QueueRows qr;
+  char* base = reinterpret_cast<char*>(ws);
+  if (!(queue_rows_possible(jobs, n_jobs) &&
+        layout_queue_rows(jobs, n_jobs, o, base, wsb, &L, &views_dev, &slot_job_dev, &qr)) &&
+      !layout_queue(jobs, n_jobs, o, base, wsb, &L, &views_dev, &slot_job_dev)) {
     set_last_error("queue fit workspace too small");
     return CT_ERR_OOM;
   }
@@ -1444,7 +1514,8 @@ int fit_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o, 
     uint32_t slot = 0, fw = 0;
     for (uint32_t j = 0; j < n_jobs; ++j) {
       const ct_fit_job& jb = jobs[j];
-      View vj = fit_view(&jb.problem, &jb.lists, L);
+      View vj = L.rows ? row_view(&jb.problem, &jb.lists, L, qr.pair[j], qr.ranked[j], qr.rank[j], qr.planes[j])
+                       : fit_view(&jb.problem, &jb.lists, L);
       vj.fbin = L.fbin + fw;
       vj.n_classes = q.c_max;
       vj.slot_base = slot;
@@ -1453,8 +1524,8 @@ int fit_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o, 
       views[j] = vj;
       first_slot[j] = slot;
       for (uint32_t t = 0; t < jb.n_trees; ++t) slot_job[slot + t] = j;
-      CT_TRY(feature_flags(jb.problem.x_fm, jb.problem.n_rows, jb.problem.n_features, L.fbin + fw, nullptr,
-                           L.ffwork, st));
+      CT_TRY(feature_flags(jb.problem.x_fm, jb.problem.n_rows, jb.problem.n_features, L.fbin + fw,
+                           L.rows ? qr.vals[j] : nullptr, L.ffwork, st));
       slot += jb.n_trees;
       fw += (jb.problem.n_features + 31) / 32;
     }
@@ -1473,6 +1544,19 @@ int fit_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o, 
     vb.row_mask = views[0].row_mask;
     TreeView tv = tree_view(trees, 0);
     CT_CUDA_TRY(cudaMemsetAsync(L.s.ctr, 0, sizeof(Counters), st));
+    if (L.rows) {
+      vb.rl[0] = views[0].rl[0];  // (marks the batch view as row-list growth; the jobs' own are used)
+      current_prof()->begin(CT_K_BOOTSTRAP);
+      for (uint32_t j = 0; j < n_jobs; ++j) {
+        const ct_fit_job& jb = jobs[j];
+        CT_TRY(launch_row_pairs(views[j], &jb.problem, qr.pair[j], qr.ranked[j], qr.rank[j], st));
+        CT_TRY(launch_row_roots(views[j], &jb.problem, first_slot[j], jb.n_trees, jb.first_tree, L.n_in, tv, L.list[0],
+                                L.tot[0], L.cap_list, L.s.ctr, L.mask[0], qr.vals[j], st));
+        account_row_roots(&jb.problem, jb.n_trees, 0);
+      }
+      current_prof()->end();
+      return grow_levels(&pb, vb, L, tv, st);
+    }
     CT_CUDA_TRY(cudaMemsetAsync(L.boot_ws, 0, 16, st));
     current_prof()->begin(CT_K_BOOTSTRAP);
     for (uint32_t j = 0; j < n_jobs; ++j) {
@@ -1488,35 +1572,7 @@ int fit_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o, 
     begin_level(L.s.ctr, st);
     for (uint32_t j = 0; j < n_jobs; ++j)
       CT_TRY(root(&jobs[j].problem, views[j], L, first_slot[j], jobs[j].n_trees, jobs[j].first_tree, tv, 0, st));
-    Counters h;
-    if (!current_prof()->timing && !L.host_loop) {
-      uint32_t n = 0;
-      uint64_t total = 0;
-      if (L.graph_samples != UINT64_MAX) {
-        CT_TRY(read_counters(L, &h, st));
-        n = h.n_next;
-        total = h.next_total;
-      }
-      int cur = 0;
-      while (n > 0 && total > L.graph_samples) {
-        begin_level(L.s.ctr, st);
-        CT_TRY(step(&pb, vb, L, tv, cur, n, total, st));
-        CT_TRY(read_counters(L, &h, st));
-        account_level(&pb, vb, h);
-        if (L.subtree_cut) L.small_bound = h.n_small;
-        n = h.n_next;
-        total = h.next_total;
-        cur = 1 - cur;
-      }
-      return graph_level_loop(&pb, vb, L, tv, cur, st);
-    }
-    CT_TRY(read_counters(L, &h, st));
-    CT_TRY(level_loop(&pb, vb, L, tv, 0, h.n_next, h.next_total, st));
-    if (L.small_bound) {
-      CT_TRY(flush_subtrees(&pb, vb, L, tv, st));
-      CT_TRY(read_counters(L, &h, st));
-    }
-    return CT_OK;
+    return grow_levels(&pb, vb, L, tv, st);
   };
   const int rc = run();
   pf->finish();

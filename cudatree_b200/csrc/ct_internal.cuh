@@ -303,6 +303,8 @@ struct View {
   View V##_job;                                               \
   if constexpr (Q) V##_job = (VB).jobs[(VB).slot_job[SLOT]];  \
   const View& V = Q ? V##_job : (VB)
+// The same by reference: the fields are read where they are used.
+#define CT_JOB_REF(V, VB, SLOT) const View& V = Q ? (VB).jobs[(VB).slot_job[SLOT]] : (VB)
 __device__ __forceinline__ bool two_valued(const View& v, uint32_t f) {
   return v.fbin && ((__ldg(v.fbin + (f >> 5)) >> (f & 31)) & 1u);
 }

@@ -328,7 +328,7 @@ __device__ __forceinline__ void row_select_item(const View& vb, const StepLists&
                                                 uint32_t w) {
   const uint32_t lane = lane_id();
   const ct_node nd = lists.nodes[w];
-  CT_JOB_VIEW(v, vb, nd.slot);
+  CT_JOB_REF(v, vb, nd.slot);
   const uint32_t m = v.max_features, n = nd.n;
   const bool writer = !CTA || threadIdx.x < 32;
   uint64_t* cmask = lists.node_mask ? const_cast<uint64_t*>(lists.node_mask) + (size_t)w * v.mask_stride : nullptr;
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(512) k_row_select_big(View v, LevelScratch s) 
   for (uint32_t i = blockIdx.x; i < zeros; i += gridDim.x) {
     const uint4 z = s.bzero[i];
     const ct_node nd = sl.nodes[z.x];
-    CT_JOB_VIEW(vj, v, nd.slot);
+    CT_JOB_REF(vj, v, nd.slot);
     zero_bits(vj, nd, z.y, s.carry + (size_t)z.z * v.n_classes, z.w * v.n_classes, threadIdx.x, blockDim.x);
   }
 }
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(BITS_THREADS, 2) k_row_bits(View vb, LevelScra
     const uint4 unit = s.bunits[s_item];
     const uint32_t slice = unit.z & 0xffffu, slices = unit.z >> 16;
     const ct_node nd = lists.nodes[unit.x];
-    CT_JOB_VIEW(v, vb, nd.slot);
+    CT_JOB_REF(v, vb, nd.slot);
     const uint32_t f = s.sel[(size_t)unit.x * v.sel_stride + unit.y];
     const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
     const uint32_t* rf = v.rank + (size_t)f * v.n_rows;
@@ -702,7 +702,7 @@ __device__ __forceinline__ void row_warp_item(const View& vb, const StepLists& l
                                               uint32_t* smem, uint32_t i) {
   const uint2 it = s.witems[i];
   const ct_node nd = lists.nodes[it.x];
-  CT_JOB_VIEW(v, vb, nd.slot);
+  CT_JOB_REF(v, vb, nd.slot);
   const uint32_t f = s.sel[(size_t)it.x * v.sel_stride + it.y];
   const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
   const uint2* pf = v.pair + (size_t)f * v.n_rows;
@@ -953,7 +953,7 @@ __device__ __forceinline__ void row_group_item(const View& vb, const StepLists& 
   constexpr uint32_t T = W * 32, K = (W == GROUP_SMALL_WARPS ? GROUP_SMALL_ROWS : GROUP_ROWS) / T;
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5, C = vb.n_classes;
   const ct_node nd = lists.nodes[item.x];
-  CT_JOB_VIEW(v, vb, nd.slot);
+  CT_JOB_REF(v, vb, nd.slot);
   const uint32_t n = nd.n;
   const uint32_t f = s.sel[(size_t)item.x * v.sel_stride + item.y];
   const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
@@ -1183,7 +1183,7 @@ __global__ void __launch_bounds__(ORDER_THREADS, 2) k_row_order(View vb, LevelSc
     if (it >= count) break;
     const uint2 item = s.oitems[it];
     const ct_node nd = lists.nodes[item.x];
-    CT_JOB_VIEW(v, vb, nd.slot);
+    CT_JOB_REF(v, vb, nd.slot);
     const uint32_t n = nd.n;
     const uint32_t f = s.sel[(size_t)item.x * v.sel_stride + item.y];
     const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
@@ -1354,7 +1354,7 @@ __device__ __forceinline__ void row_hist_item(const View& vb, const StepLists& l
   const RowPiece pc = s.rpieces[pi];
   if (pc.j + 1 >= pc.npieces) return;
   const ct_node nd = lists.nodes[pc.node];
-  CT_JOB_VIEW(v, vb, nd.slot);
+  CT_JOB_REF(v, vb, nd.slot);
   if (row_dense(nd.n, v.n_rows) && pc.npieces * C <= BITS_COUNTS) return;  // k_row_bits counted them
   const uint32_t f = s.sel[(size_t)pc.node * v.sel_stride + pc.slot];
   PieceStream ps = piece_stream(v, nd, pc, f, lists.scan_piece, smem);
@@ -1439,7 +1439,7 @@ __global__ void __launch_bounds__(256) k_row_bound(View vb, LevelScratch s) {
     const RowPiece pc = s.rpieces[pi];
     if (pc.j == 0) continue;
     const ct_node nd = lists.nodes[pc.node];
-    CT_JOB_VIEW(v, vb, nd.slot);
+    CT_JOB_REF(v, vb, nd.slot);
     const uint32_t* left = s.carry + (size_t)pi * C;
     uint32_t nl = 0;
     for (uint32_t c = 0; c < C; ++c) nl += left[c];
@@ -1503,7 +1503,7 @@ __device__ __forceinline__ void row_scan_item(const View& vb, const StepLists& l
   uint32_t* T = cnt + C;
   const RowPiece pc = s.rpieces[pi];
   const ct_node nd = lists.nodes[pc.node];
-  CT_JOB_VIEW(v, vb, nd.slot);
+  CT_JOB_REF(v, vb, nd.slot);
   const uint32_t* carry = pc.npieces > 1 ? s.carry + (size_t)pi * C : nullptr;
   const uint32_t* tot = lists.tot + (size_t)pc.node * C;
   const uint32_t n = nd.n;
@@ -1679,7 +1679,7 @@ __device__ __forceinline__ void row_reduce_item(const View& vb, const StepLists&
                                                 const TreeView& tv, uint32_t w) {
   const uint32_t lane = lane_id();
   const ct_node nd = lists.nodes[w];
-  CT_JOB_VIEW(v, vb, nd.slot);
+  CT_JOB_REF(v, vb, nd.slot);
   const uint32_t C = v.n_classes, nsel = s.nsel[w], n = nd.n;
   const uint32_t* sel = s.sel + (size_t)w * v.sel_stride;
   RowBest bb{dinf(), NONE, 0u, 0.f, 0.f};
@@ -1796,7 +1796,7 @@ __device__ __forceinline__ void row_mark_item(const View& vb, const StepLists& l
   const PartPiece pp = multi ? s.mpart[i] : s.part[i - nm];
   const RowSplit sr = s.rsplits[pp.split];
   const ct_node nd = lists.nodes[sr.node];
-  CT_JOB_VIEW(v, vb, nd.slot);
+  CT_JOB_REF(v, vb, nd.slot);
   const bool virt = is_virtual(v, sr.feature);
   const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
   const float* xf = v.x_fm + (size_t)sr.feature * v.n_rows;
@@ -1902,7 +1902,7 @@ __global__ void __launch_bounds__(THREADS_PER_BLOCK) k_row_move(View vb, LevelSc
     const PartPiece pp = s.mpart[i];
     const RowSplit sr = s.rsplits[pp.split];
     const ct_node nd = lists.nodes[sr.node];
-    CT_JOB_VIEW(v, vb, nd.slot);
+    CT_JOB_REF(v, vb, nd.slot);
     const uint32_t lo = pp.j * PART_PIECE, hi = min(lo + PART_PIECE, nd.n);
     const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
     uint32_t* dst = row_list(v, nd.buf ^ 1u, nd.slot) + nd.start;
@@ -1945,7 +1945,7 @@ __device__ __forceinline__ void row_children_item(const View& vb, const StepList
   const uint32_t lane = lane_id();
   const RowSplit sr = s.rsplits[w];
   const ct_node nd = lists.nodes[sr.node];
-  CT_JOB_VIEW(v, vb, nd.slot);
+  CT_JOB_REF(v, vb, nd.slot);
   const uint32_t C = v.n_classes;
   for (uint32_t side = 0; side < 2; ++side) {
     ct_node ch;
@@ -2168,7 +2168,7 @@ k_row_subtree(View vb, const ct_node* __restrict__ small, LevelScratch s, TreeVi
   const uint32_t count = live_count(s, s.ctr->n_small, cap_small);
   for_items(count, &s.ctr->claim[ITEM_SUBTREE], [&](uint32_t w) {
     const ct_node nd = small[w];
-    CT_JOB_VIEW(v, vb, nd.slot);
+    CT_JOB_REF(v, vb, nd.slot);
     const uint32_t* rows = row_list(v, nd.buf, nd.slot) + nd.start;
     const bool have = lane < nd.n;
     uint32_t e = have ? rows[lane] : 0u;
