@@ -402,7 +402,7 @@ int step(const ct_problem* p, const View& v, const FitLayout& L, const TreeView&
     if (L.subtree_cut && L.small_bound + 2ull * cn > L.cap_small) CT_TRY(flush_subtrees(p, v, L, tv, st));
     CT_TRY(launch_reset_step(L.s, cn, step_lists(L, cur, lo, C, total), st));
     if (L.rows) {
-      CT_TRY(launch_row_step(v, L.s, b, L.n_max, tv, L.cap_list, L.subtree_cut, L.small, L.cap_small, st));
+      CT_TRY(launch_row_step(v, L.s, b, L.n_max, tv, L.cap_list, L.subtree_cut, L.small, L.cap_small, nullptr, st));
       if (L.subtree_cut) L.small_bound += 2ull * cn;
       continue;
     }
@@ -576,6 +576,29 @@ cudaStream_t capture_stream() {
   return h.st;
 }
 
+// Branch streams and events of a capture, per thread; NULL when they cannot be
+// created (the capture then has no branches).
+const ForkStreams* fork_streams() {
+  static thread_local struct Holder {
+    ForkStreams f{};
+    bool ok = true;
+    Holder() {
+      for (auto& s : f.st) ok = ok && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
+      ok = ok && cudaEventCreateWithFlags(&f.fork, cudaEventDisableTiming) == cudaSuccess;
+      for (auto& e : f.join) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+      if (!ok) cudaGetLastError();
+    }
+    ~Holder() {
+      for (auto& s : f.st)
+        if (s) cudaStreamDestroy(s);
+      if (f.fork) cudaEventDestroy(f.fork);
+      for (auto& e : f.join)
+        if (e) cudaEventDestroy(e);
+    }
+  } h;
+  return h.ok ? &h.f : nullptr;
+}
+
 int build_loop_graph(const ct_problem* p, const View& v, const FitLayout& L, const TreeView& tv, cudaStream_t st,
                      LoopGraph& lg) {
   const uint32_t ib = p->index_bytes, lb = p->label_bytes, C = p->n_classes;
@@ -606,7 +629,8 @@ int build_loop_graph(const ct_problem* p, const View& v, const FitLayout& L, con
     k_loop_step<<<1, 1, 0, st>>>(L.ctl, L.s.ctr, L.s.step, ll, L.chunk, C, L.scan_piece, L.mat16);
     pf->launched(CT_K_CHILDREN);
     if (L.rows) {
-      CT_TRY(launch_row_step(v, L.s, b, L.n_max, tv, L.cap_list, L.subtree_cut, L.small, L.cap_small, st));
+      CT_TRY(launch_row_step(v, L.s, b, L.n_max, tv, L.cap_list, L.subtree_cut, L.small, L.cap_small, fork_streams(),
+                             st));
     } else {
       CT_TRY(launch_split(v, ib, lb, L.s, b, L.scan_piece, true, st));
       CT_TRY(launch_partition(v, ib, lb, L.s, b, tv, true, st));

@@ -585,6 +585,13 @@ struct LevelCaps {
 };
 LevelCaps level_caps(const View& v, uint32_t scan_piece, LevelBounds b);
 constexpr uint32_t VPIECE = 2048;  // rows per row-list piece (virtual features)
+// Row-list growth: pieces of MIN_VPIECE rows in levels whose scans take
+// pieces below 2,048 elements (few samples: 31 warps of 2,048 rows each held
+// a one-tree level of 63,000 rows for 25 us, pieces of 512 for 9).
+constexpr uint32_t MIN_VPIECE = 512;
+__device__ __forceinline__ uint32_t vpiece_rows(const View& v, uint32_t scan_piece) {
+  return v.rl[0] && scan_piece < VPIECE ? MIN_VPIECE : VPIECE;
+}
 // Scratch of virtual features: carved when `virt` (the fit may have some).
 bool virtual_possible(const ct_problem* p);
 bool carve_level_scratch(Arena& a, const View& v, const LevelCaps& c, LevelScratch* s, bool virt = false);
@@ -631,12 +638,21 @@ bool rows_have_large(uint32_t n_rows);  // some node may take a bitmap or an ord
 int launch_row_roots(const View& v, const ct_problem* p, uint32_t slot_lo, uint32_t n_slots, uint32_t tree_lo,
                      uint32_t* n_in, const TreeView& tv, ct_node* out, uint32_t* out_tot, uint32_t cap, Counters* ctr,
                      uint64_t* out_mask, const float2* vals, cudaStream_t st);
+// Streams and events that fork a step's independent kernels into branches;
+// used while a loop graph is captured (a step launched straight to a stream
+// runs them in order: NULL).
+struct ForkStreams {
+  static constexpr int N = 3;
+  cudaStream_t st[N];
+  cudaEvent_t fork;
+  cudaEvent_t join[N];
+};
 // One level step: selection, split search, split of the row lists, children.
 // n_max: the most rows of any tree (a step whose nodes all fit a warp item
 // launches no order and piece kernels).
 int launch_row_step(const View& v, const LevelScratch& s, LevelBounds b, uint32_t n_max,
                     const TreeView& tv, uint32_t cap_next, uint32_t small_cut, ct_node* small, uint32_t cap_small,
-                    cudaStream_t st);
+                    const ForkStreams* fork, cudaStream_t st);
 int launch_row_subtrees(const View& v, const ct_node* small, uint32_t cap_small, uint32_t bound, const LevelScratch& s,
                         const TreeView& tv, cudaStream_t st);
 // Virtual-feature counts of a step's nodes (ct_level.cu).

@@ -68,7 +68,7 @@ __device__ __forceinline__ void vpieces_item(const View& v, const StepLists& lis
   for (uint32_t f = lane; f < 64; f += 32) s.vcnt[(size_t)w * 64 + f] = 0;
   for (uint32_t i = lane; i < fc; i += 32) s.vcls[(size_t)w * fc + i] = 0;
   if (nd.n < 2) return;
-  const uint32_t np = ceil_div(nd.n, VPIECE);
+  const uint32_t np = ceil_div(nd.n, vpiece_rows(v, lists.scan_piece));
   uint32_t base = 0;
   if (lane == 0) {
     base = atomicAdd(&s.ctr->n_vpieces, np);
@@ -99,8 +99,8 @@ __device__ __forceinline__ void vcount_item(const View& v, const StepLists& list
   const IdxT* rl =
       (v.rl[0] ? reinterpret_cast<const IdxT*>(row_list(v, nd.buf, nd.slot)) : list_ptr<IdxT>(v, nd.buf, nd.slot, v.vslot)) +
       nd.start;
-  const uint32_t lo = pc.y * VPIECE;
-  const uint32_t hi = min(lo + VPIECE, nd.n);
+  const uint32_t lo = pc.y * vpiece_rows(v, lists.scan_piece);
+  const uint32_t hi = min(lo + vpiece_rows(v, lists.scan_piece), nd.n);
   for (uint32_t i = lane; i < fc; i += 32) cnt[i] = 0;
   __syncwarp();
   // VB rows per lane: their entry loads, then their value-bit gathers, are in

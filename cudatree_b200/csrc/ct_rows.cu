@@ -2292,7 +2292,8 @@ int launch_bitmap(K kernel, int threads, size_t smem, uint32_t items, cudaStream
 
 template <bool Q>
 int row_step(const View& v, const LevelScratch& s, LevelBounds b, uint32_t n_max, const TreeView& tv,
-             uint32_t cap_next, uint32_t small_cut, ct_node* small, uint32_t cap_small, cudaStream_t st) {
+             uint32_t cap_next, uint32_t small_cut, ct_node* small, uint32_t cap_small, const ForkStreams* fork,
+             cudaStream_t st) {
   Prof* pf = current_prof();
   const uint32_t C = v.n_classes;
   const size_t sm1 = (size_t)WARPS_PER_BLOCK * C * sizeof(uint32_t);
@@ -2312,6 +2313,20 @@ int row_step(const View& v, const LevelScratch& s, LevelBounds b, uint32_t n_max
     pf->launched(CT_K_SELECT);
   }
   pf->end();
+  // The orders and scans of the size classes are independent: in a graph they
+  // are branches, so the latency of one class's kernels (a level has few large
+  // nodes) hides behind the others'.  The bitmaps' chain is the longest and
+  // stays on st.
+  cudaStream_t br[ForkStreams::N];
+  for (int i = 0; i < ForkStreams::N; ++i) br[i] = fork ? fork->st[i] : st;
+  const bool forked = fork && n_max > GROUP_SMALL_ROWS;
+  if (forked) {
+    CT_CUDA_TRY(cudaEventRecord(fork->fork, st));
+    for (int i = 0; i < ForkStreams::N; ++i) CT_CUDA_TRY(cudaStreamWaitEvent(br[i], fork->fork, 0));
+  } else {
+    for (int i = 0; i < ForkStreams::N; ++i) br[i] = st;
+  }
+  const size_t smw = (size_t)WARPS_PER_BLOCK * warp_item_words(C) * sizeof(uint32_t);
   if (n_max > GROUP_ROWS) {
     pf->begin(CT_K_PARTITION);
     CT_TRY(launch_bitmap(k_row_bits<Q>, BITS_THREADS, (size_t)bits_words(n_max) * 4, s.cap_units, st, v, s, n_max));
@@ -2323,16 +2338,18 @@ int row_step(const View& v, const LevelScratch& s, LevelBounds b, uint32_t n_max
     pf->end();
   }
   pf->begin(CT_K_SCAN);
-  if (n_max > WARP_ROWS) {
-    CT_TRY(launch_bitmap(k_row_group<Q, GROUP_SMALL_WARPS>, 32 * GROUP_SMALL_WARPS,
-                         group_words<GROUP_SMALL_WARPS>(C, n_max) * sizeof(uint32_t), s.cap_order, st, v, s, n_max));
-    pf->launched(CT_K_SCAN);
-  }
   if (n_max > GROUP_SMALL_ROWS) {
     CT_TRY(launch_bitmap(k_row_group<Q, GROUP_WARPS>, 32 * GROUP_WARPS,
-                         group_words<GROUP_WARPS>(C, n_max) * sizeof(uint32_t), s.cap_order, st, v, s, n_max));
+                         group_words<GROUP_WARPS>(C, n_max) * sizeof(uint32_t), s.cap_order, br[0], v, s, n_max));
     pf->launched(CT_K_SCAN);
   }
+  if (n_max > WARP_ROWS) {
+    CT_TRY(launch_bitmap(k_row_group<Q, GROUP_SMALL_WARPS>, 32 * GROUP_SMALL_WARPS,
+                         group_words<GROUP_SMALL_WARPS>(C, n_max) * sizeof(uint32_t), s.cap_order, br[1], v, s, n_max));
+    pf->launched(CT_K_SCAN);
+  }
+  k_row_warp<Q><<<grid_for(k_row_warp<Q>, s.cap_w, smw, true), THREADS_PER_BLOCK, smw, br[2]>>>(v, s);
+  pf->launched(CT_K_SCAN);
   if (n_max > GROUP_ROWS) {
     const size_t smh = (size_t)WARPS_PER_BLOCK * hist_words(C) * sizeof(uint32_t);
     const size_t sms2 = (size_t)WARPS_PER_BLOCK * scan_words(C) * sizeof(uint32_t);
@@ -2348,10 +2365,12 @@ int row_step(const View& v, const LevelScratch& s, LevelBounds b, uint32_t n_max
     k_row_scan<Q><<<grid_for(k_row_scan<Q>, s.cap_scan, sms2, true), THREADS_PER_BLOCK, sms2, st>>>(v, s);
     pf->launched(CT_K_SCAN, hist ? 3 : 2);
   }
-  const size_t smw = (size_t)WARPS_PER_BLOCK * warp_item_words(C) * sizeof(uint32_t);
-  k_row_warp<Q><<<grid_for(k_row_warp<Q>, s.cap_w, smw, true), THREADS_PER_BLOCK, smw, st>>>(v, s);
   pf->end();
-  pf->launched(CT_K_SCAN);
+  if (forked)
+    for (int i = 0; i < ForkStreams::N; ++i) {
+      CT_CUDA_TRY(cudaEventRecord(fork->join[i], br[i]));
+      CT_CUDA_TRY(cudaStreamWaitEvent(st, fork->join[i], 0));
+    }
   pf->begin(CT_K_REDUCE);
   k_row_reduce<Q><<<grid_for(k_row_reduce<Q>, nodes, 0, true), THREADS_PER_BLOCK, 0, st>>>(v, s, tv);
   pf->end();
@@ -2425,7 +2444,7 @@ bool carve_row_scratch(Arena& a, const View& v, LevelBounds b, uint32_t scan_pie
   t.cap_part = t.cap_nodes;
   t.cap_mpart = clamp32(b.samples / PART_PIECE + b.samples / (PART_PIECE + 1) + 1);
   t.cap_big = clamp32(b.samples / SELECT_ROWS + 1);
-  t.cap_vpieces = virt ? clamp32(b.samples / VPIECE + b.nodes + 1) : 0u;
+  t.cap_vpieces = virt ? clamp32(b.samples / MIN_VPIECE + b.nodes + 1) : 0u;
   t.ctr = a.take<Counters>(1);
   t.step = a.take<StepLists>(1);
   t.sel = a.take<uint32_t>(t.cap_nodes * m);
@@ -2497,9 +2516,10 @@ int launch_row_roots(const View& v, const ct_problem* p, uint32_t slot_lo, uint3
 }
 
 int launch_row_step(const View& v, const LevelScratch& s, LevelBounds b, uint32_t n_max, const TreeView& tv,
-                    uint32_t cap_next, uint32_t small_cut, ct_node* small, uint32_t cap_small, cudaStream_t st) {
-  return v.jobs ? row_step<true>(v, s, b, n_max, tv, cap_next, small_cut, small, cap_small, st)
-                : row_step<false>(v, s, b, n_max, tv, cap_next, small_cut, small, cap_small, st);
+                    uint32_t cap_next, uint32_t small_cut, ct_node* small, uint32_t cap_small, const ForkStreams* fork,
+                    cudaStream_t st) {
+  return v.jobs ? row_step<true>(v, s, b, n_max, tv, cap_next, small_cut, small, cap_small, fork, st)
+                : row_step<false>(v, s, b, n_max, tv, cap_next, small_cut, small, cap_small, fork, st);
 }
 
 int launch_row_subtrees(const View& v, const ct_node* small, uint32_t cap_small, uint32_t bound, const LevelScratch& s,
