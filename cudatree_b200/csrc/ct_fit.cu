@@ -1106,11 +1106,17 @@ int autotune(const ct_problem* p, const ct_lists* l, uint32_t n_trees, uint32_t 
   return CT_OK;
 }
 
+// Workspace of list growth: what a fit needs at the least.
+size_t fit_least_workspace_bytes(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o) {
+  FitLayout L{};
+  list_layout(p, n_trees, o, nullptr, 0, &L);
+  return L.bytes;
+}
+
 // The larger of the two growth forms' workspaces: a fit takes the one it can.
 size_t fit_workspace_bytes(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o) {
   FitLayout L{};
-  list_layout(p, n_trees, o, nullptr, 0, &L);
-  size_t bytes = L.bytes;
+  size_t bytes = fit_least_workspace_bytes(p, n_trees, o);
   if (o->mode == CT_FIT_BATCHED && rows_possible(p)) {
     row_layout(p, n_trees, o, nullptr, 0, &L);
     bytes = std::max(bytes, L.bytes);
@@ -1197,10 +1203,113 @@ int canonicalize(const uint32_t* left, const uint32_t* right, const uint32_t* fe
 }
 
 // ---------------------------------------------------------------------------
-// Read-back of one fit call's trees: the used prefix of every tree's raw
-// arrays is gathered into contiguous device arrays (one kernel), copied to
-// the host in five transfers, and renumbered breadth-first on host threads.
+// Read-back of one fit call's trees.  One CTA per tree renumbers it breadth-first
+// on the device, level by level (a level's inner nodes, in order, get the next
+// ids two by two), and writes its columns in place; one copy brings all of
+// them to a page-locked staging buffer, and host threads (one per 64 Ki nodes)
+// copy them to the caller's arrays.  A tree of more than FETCH_LEVELS levels
+// (one step of the CTA each) is left to the host.  Renumbering on up to 16 host
+// threads took 0.45 ms for 738 nodes (thread starts) and 2.3 ms for 1.03 M
+// nodes of 100 trees; now 0.05 and 0.71 ms.
 namespace {
+
+constexpr uint32_t FETCH_LEVELS = 4096;
+constexpr uint32_t FETCH_THREADS = 512;
+enum : uint32_t { FETCH_OK = 0, FETCH_BAD = 1, FETCH_DEEP = 2 };
+
+// Canonical columns, each of `total` entries, tree after tree.
+struct TreeColumns {
+  uint32_t* left;
+  uint32_t* right;
+  float* threshold;
+  uint32_t* value;  // until a node is reached by the walk, its raw id
+  uint16_t* feature;
+  uint32_t* status;  // [n_trees], after the features (4-byte aligned)
+};
+__host__ __device__ __forceinline__ size_t column_bytes(size_t total, uint32_t n_trees) {
+  return 16 * total + ((2 * total + 3) & ~size_t(3)) + 4 * (size_t)n_trees;
+}
+__host__ __device__ __forceinline__ TreeColumns columns_at(char* base, size_t total) {
+  TreeColumns c;
+  c.left = reinterpret_cast<uint32_t*>(base);
+  c.right = c.left + total;
+  c.threshold = reinterpret_cast<float*>(c.right + total);
+  c.value = c.right + 2 * total;
+  c.feature = reinterpret_cast<uint16_t*>(c.right + 3 * total);
+  c.status = reinterpret_cast<uint32_t*>(base + 16 * total + ((2 * total + 3) & ~size_t(3)));
+  return c;
+}
+size_t seen_words(uint64_t total, uint32_t n_trees) { return total / 32 + n_trees + 1; }
+
+__global__ void __launch_bounds__(FETCH_THREADS)
+k_canonical(ct_tree_buffers tb, const uint32_t* __restrict__ off, TreeColumns c, uint32_t* seen_all) {
+  __shared__ uint32_t s_cnt[FETCH_THREADS / 32];
+  __shared__ uint32_t s_bad;
+  const uint32_t t = blockIdx.x, o = off[t], n = off[t + 1] - o;
+  const size_t src = (size_t)t * tb.capacity;
+  uint32_t* seen = seen_all + o / 32 + t;  // the trees' words do not overlap
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    s_bad = 0;
+    c.value[o] = 0;
+    seen[0] = 1;
+  }
+  __syncthreads();
+  uint32_t lo = 0, hi = 1, levels = 0;
+  while (lo < hi && levels < FETCH_LEVELS) {
+    uint32_t next = hi;
+    for (uint32_t i0 = lo; i0 < hi; i0 += FETCH_THREADS) {
+      const uint32_t i = i0 + threadIdx.x;
+      uint32_t l = 0, r = 0, f = 0, v = 0;
+      float th = 0.f;
+      if (i < hi) {
+        const size_t raw = src + c.value[o + i];
+        l = tb.left[raw];
+        r = tb.right[raw];
+        f = tb.feature[raw];
+        th = tb.threshold[raw];
+        v = tb.value[raw];
+      }
+      const bool inner = l != 0 && r != 0;
+      const unsigned m = __ballot_sync(FULL, inner);
+      if (lane == 0) s_cnt[warp] = __popc(m);
+      __syncthreads();
+      const uint32_t mine = lane < FETCH_THREADS / 32 ? s_cnt[lane] : 0u;
+      const uint32_t incl = (uint32_t)warp_incl_scan_i32((int32_t)mine);
+      const uint32_t before = __shfl_sync(FULL, incl - mine, warp), all = __shfl_sync(FULL, incl, 31);
+      const uint32_t id = next + 2 * (before + __popc(m & lanemask_lt()));
+      if (i < hi) {
+        bool ok = true;
+        if (inner) {
+          ok = l < n && r < n && l != r && id + 1 < n;
+          if (ok) {
+            ok = !((atomicOr(seen + (l >> 5), 1u << (l & 31)) >> (l & 31)) & 1u) &&
+                 !((atomicOr(seen + (r >> 5), 1u << (r & 31)) >> (r & 31)) & 1u);
+          }
+          if (ok) {
+            c.value[o + id] = l;
+            c.value[o + id + 1] = r;
+          } else {
+            s_bad = 1;
+          }
+        }
+        c.left[o + i] = inner ? id : 0u;
+        c.right[o + i] = inner ? id + 1 : 0u;
+        c.feature[o + i] = (uint16_t)f;
+        c.threshold[o + i] = th;
+        c.value[o + i] = v;
+      }
+      next += 2 * all;
+      __syncthreads();  // s_cnt is free; the next level's raw ids are written
+      if (s_bad) break;
+    }
+    if (s_bad) break;
+    lo = hi;
+    hi = next;
+    ++levels;
+  }
+  if (threadIdx.x == 0) c.status[t] = s_bad || (lo >= hi && hi != n) ? FETCH_BAD : lo < hi ? FETCH_DEEP : FETCH_OK;
+}
 
 __global__ void k_gather_trees(ct_tree_buffers tb, const uint32_t* __restrict__ off, uint32_t n_trees,
                                uint32_t total, uint32_t* __restrict__ out) {
@@ -1224,6 +1333,30 @@ __global__ void k_gather_trees(ct_tree_buffers tb, const uint32_t* __restrict__ 
 // the device and takes tens of ms for a 100-tree forest, so a server reserves
 // its largest size up front, and a growth takes half again the old size
 // (16 MiB steps): forests a little larger than the last do not reallocate.
+template <int N>
+struct EventSet {
+  cudaEvent_t e[N] = {};
+  bool ok = true;
+  EventSet() {
+    for (auto& x : e) ok = ok && cudaEventCreateWithFlags(&x, cudaEventDisableTiming) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+  }
+  ~EventSet() {
+    for (auto& x : e)
+      if (x) cudaEventDestroy(x);
+  }
+};
+// Threads joined at the end of their scope, also when starting one throws.
+struct ThreadSet {
+  std::vector<std::thread> v;
+  template <typename F>
+  void start(F f, uint32_t arg) {
+    v.emplace_back(f, arg);
+  }
+  ~ThreadSet() {
+    for (auto& t : v) t.join();
+  }
+};
 struct Staging {
   std::mutex mu;
   void* p = nullptr;
@@ -1250,8 +1383,13 @@ int fetch_trees_reserve(uint64_t total_nodes) {
 }
 
 size_t fetch_trees_scratch(uint64_t total_nodes, uint32_t n_trees) {
-  return 5 * total_nodes * sizeof(uint32_t) + ((size_t)n_trees + 1) * sizeof(uint32_t) + 256;
+  return 5 * total_nodes * sizeof(uint32_t) + (4 * (size_t)n_trees + 8) * sizeof(uint32_t) + 256;
 }
+
+// The trees as gathered by k_gather_trees, renumbered on host threads.
+static int fetch_trees_host(const ct_tree_buffers* tb, uint32_t n_trees, const uint32_t* counts,
+                            const std::vector<uint32_t>& off, uint32_t* d_cols, const uint32_t* d_off, uint32_t* ol,
+                            uint32_t* orr, uint16_t* of, float* ot, uint32_t* ov, cudaStream_t st);
 
 int fetch_trees(const ct_tree_buffers* tb, uint32_t n_trees, const uint32_t* counts, void* scratch,
                 size_t scratch_bytes, uint32_t* ol, uint32_t* orr, uint16_t* of, float* ot, uint32_t* ov,
@@ -1265,10 +1403,80 @@ int fetch_trees(const ct_tree_buffers* tb, uint32_t n_trees, const uint32_t* cou
   }
   const uint32_t total = off[n_trees];
   if (n_trees == 0) return CT_OK;
-  CT_ARG_CHECK(scratch_bytes >= fetch_trees_scratch(total, n_trees), "fetch trees: scratch too small");
-  uint32_t* d_cols = reinterpret_cast<uint32_t*>(scratch);
-  uint32_t* d_off = d_cols + 5 * (size_t)total;
+  // at the least what the gather for the host needs (a caller may have sized for that)
+  const size_t least = 5 * (size_t)total * sizeof(uint32_t) + ((size_t)n_trees + 1) * sizeof(uint32_t) + 256;
+  CT_ARG_CHECK(scratch_bytes >= least, "fetch trees: scratch too small");
+  // offsets, visited bits, then the columns (which a gather for the host may
+  // take whole: 20 bytes per node)
+  uint32_t* d_off = reinterpret_cast<uint32_t*>(scratch);
+  char* d_cols = reinterpret_cast<char*>(d_off + ((n_trees + 1 + 3) & ~3u));
+  const size_t cb = column_bytes(total, n_trees);
+  uint32_t* d_seen = reinterpret_cast<uint32_t*>(d_cols + ((cb + 3) & ~size_t(3)));
   CT_CUDA_TRY(cudaMemcpyAsync(d_off, off.data(), off.size() * 4, cudaMemcpyHostToDevice, st));
+  if (scratch_bytes < fetch_trees_scratch(total, n_trees))
+    return fetch_trees_host(tb, n_trees, counts, off, reinterpret_cast<uint32_t*>(d_cols), d_off, ol, orr, of, ot, ov,
+                            st);
+  CT_CUDA_TRY(cudaMemsetAsync(d_seen, 0, seen_words(total, n_trees) * 4, st));
+  k_canonical<<<n_trees, FETCH_THREADS, 0, st>>>(*tb, d_off, columns_at(d_cols, total), d_seen);
+  CT_CUDA_TRY(cudaGetLastError());
+  {
+    std::lock_guard<std::mutex> lk(g_staging.mu);
+    CT_TRY(g_staging.grow(std::max<size_t>(cb, (size_t)5 * total * sizeof(uint32_t))));
+    const TreeColumns h = columns_at(static_cast<char*>(g_staging.p), total);
+    // large forests: a copy per column, so that the host threads copy one
+    // column out while the next arrives
+    const uint32_t workers = std::max(1u, std::min({total >> 16, 16u, std::thread::hardware_concurrency()}));
+    const size_t col[6] = {0, 4 * (size_t)total, 8 * (size_t)total, 12 * (size_t)total, 16 * (size_t)total, cb};
+    EventSet<5> ev;
+    const int parts = workers > 1 && ev.ok ? 5 : 1;
+    char* to = static_cast<char*>(g_staging.p);
+    for (int k = 0; k < parts; ++k) {
+      const size_t lo = col[k], hi = parts == 1 ? cb : col[k + 1];
+      CT_CUDA_TRY(cudaMemcpyAsync(to + lo, d_cols + lo, hi - lo, cudaMemcpyDeviceToHost, st));
+      if (parts > 1) CT_CUDA_TRY(cudaEventRecord(ev.e[k], st));
+    }
+    std::vector<cudaError_t> arrived(workers, cudaSuccess);
+    if (parts == 1) CT_CUDA_TRY(cudaStreamSynchronize(st));
+    char* dst[5] = {reinterpret_cast<char*>(ol), reinterpret_cast<char*>(orr), reinterpret_cast<char*>(ot),
+                    reinterpret_cast<char*>(ov), reinterpret_cast<char*>(of)};
+    auto copy = [&](uint32_t w) {
+      const size_t lo = (size_t)total * w / workers, n = (size_t)total * (w + 1) / workers - lo;
+      for (int k = 0; k < 5; ++k) {
+        const size_t es = k == 4 ? 2 : 4;
+        if (parts > 1) {
+          const cudaError_t e = cudaEventSynchronize(ev.e[k]);
+          if (e != cudaSuccess) {
+            arrived[w] = e;
+            return;
+          }
+        }
+        std::memcpy(dst[k] + lo * es, to + col[k] + lo * es, n * es);
+      }
+    };
+    {
+      ThreadSet pool;
+      for (uint32_t w = 1; w < workers; ++w) pool.start(copy, w);
+      copy(0);
+    }
+    for (const cudaError_t e : arrived) CT_CUDA_TRY(e);
+    bool deep = false;
+    for (uint32_t t = 0; t < n_trees; ++t) {
+      if (h.status[t] == FETCH_BAD) {
+        set_last_error("tree " + std::to_string(t) + ": raw tree is not a binary tree rooted at node 0");
+        return CT_ERR_INTERNAL;
+      }
+      deep |= h.status[t] == FETCH_DEEP;
+    }
+    if (!deep) return CT_OK;
+  }
+  return fetch_trees_host(tb, n_trees, counts, off, reinterpret_cast<uint32_t*>(d_cols), d_off, ol, orr, of, ot, ov,
+                          st);
+}
+
+static int fetch_trees_host(const ct_tree_buffers* tb, uint32_t n_trees, const uint32_t* counts,
+                            const std::vector<uint32_t>& off, uint32_t* d_cols, const uint32_t* d_off, uint32_t* ol,
+                            uint32_t* orr, uint16_t* of, float* ot, uint32_t* ov, cudaStream_t st) {
+  const uint32_t total = off[n_trees];
   k_gather_trees<<<std::min<uint32_t>(ceil_div(total, 256), 148 * 16), 256, 0, st>>>(*tb, d_off, n_trees, total,
                                                                                     d_cols);
   CT_CUDA_TRY(cudaGetLastError());

@@ -45,6 +45,7 @@
 namespace ct {
 
 size_t fit_workspace_bytes(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o);
+size_t fit_least_workspace_bytes(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o);
 int fit(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uint32_t n_trees, const ct_fit_options* o,
         const ct_tree_buffers* trees, void* ws, size_t wsb, cudaStream_t st);
 size_t fetch_trees_scratch(uint64_t total_nodes, uint32_t n_trees);
@@ -238,14 +239,17 @@ class Server {
     // page-locked read-back staging for the largest fit job, taken now: a
     // page-locked allocation while requests run would stall every stream
     if (nfw) CT_TRY(fetch_trees_reserve((uint64_t)cfg.max_fit_trees * 2 * cfg.max_fit_rows));
-    const size_t arena = fit_arena_bytes();
+    // Room for row-list growth of the largest job when the budget has it (list
+    // growth, which needs less, otherwise: the fit takes what its arena holds).
+    size_t pool_bytes = cfg.forest_pool_bytes ? cfg.forest_pool_bytes : std::min<size_t>(4ull << 30, budget / 4);
+    pool_bytes = Pool::round(pool_bytes);
+    size_t arena = fit_arena_bytes(false);
+    if (nfw && used + (uint64_t)nfw * fit_arena_bytes(true) + pool_bytes <= budget) arena = fit_arena_bytes(true);
     for (auto& fw : fit_workers) {
       CT_CUDA_TRY(cudaStreamCreateWithPriority(&fw.st, cudaStreamNonBlocking, prio_lo));
       CT_TRY(take(arena, (void**)&fw.arena));
       fw.arena_bytes = arena;
     }
-    size_t pool_bytes = cfg.forest_pool_bytes ? cfg.forest_pool_bytes : std::min<size_t>(4ull << 30, budget / 4);
-    pool_bytes = Pool::round(pool_bytes);
     CT_TRY(take(pool_bytes, (void**)&pool_base));
     pool.reset(pool_bytes);
     CT_CUDA_TRY(cudaStreamCreateWithFlags(&upload_st, cudaStreamNonBlocking));
@@ -255,9 +259,12 @@ class Server {
   }
 
   // Device bytes of one fit job at the configured maximum size.
-  size_t fit_arena_bytes() const { return job_bytes(cfg.max_fit_rows, cfg.max_features, 255, cfg.max_fit_trees); }
+  size_t fit_arena_bytes(bool rows) const {
+    return job_bytes(cfg.max_fit_rows, cfg.max_features, 255, cfg.max_fit_trees, rows);
+  }
 
-  static size_t job_bytes(uint32_t n, uint32_t f, uint32_t c, uint32_t t) {
+  // rows: with the larger workspace of row-list growth.
+  static size_t job_bytes(uint32_t n, uint32_t f, uint32_t c, uint32_t t, bool rows = false) {
     ct_problem p{};
     p.n_rows = n;
     p.n_features = f;
@@ -286,7 +293,7 @@ class Server {
     add((size_t)t * 2 * n * 4 * 5);    // raw trees
     add((size_t)t * 4);                // node counts
     add(fetch_trees_scratch((uint64_t)t * 2 * n, t));  // tree read-back
-    add(fit_workspace_bytes(&p, t, &o));
+    add(rows ? fit_workspace_bytes(&p, t, &o) : fit_least_workspace_bytes(&p, t, &o));
     return b + 4096;
   }
 
@@ -731,7 +738,10 @@ class Server {
     // each job has its own shape and arena, so a loop graph would be built
     // for one fit and dropped: host-driven levels cost less here
     o.flags = CT_FIT_HOST_LOOP;
-    const size_t wsb = fit_workspace_bytes(&p, T, &o);
+    // the fit gets the rest of the arena, at least what list growth needs
+    const size_t ws_off = (a.used + 255) & ~size_t(255);
+    const size_t rest = ws_off < fw.arena_bytes ? fw.arena_bytes - ws_off : 0;
+    const size_t wsb = std::max(fit_least_workspace_bytes(&p, T, &o), rest);
     char* ws = a.take<char>(wsb);
     if (!ws || !a.ok()) {
       set_last_error("fit job: arena carve failed");
