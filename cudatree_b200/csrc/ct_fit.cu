@@ -667,7 +667,9 @@ int graph_level_loop(const ct_problem* p, const View& v, const FitLayout& L, con
   key_add(key, v);
   key_add(key, L.s);
   key_add(key, tv);
-  key_add(key, *p);
+  ct_problem kp = *p;
+  kp.seed = 0;  // only the roots, made outside the loop, depend on it
+  key_add(key, kp);
   for (int i = 0; i < 2; ++i) {
     key_add(key, L.list[i]);
     key_add(key, L.tot[i]);

@@ -2,6 +2,8 @@
 #pragma once
 
 #include <algorithm>
+#include <mutex>
+#include <set>
 
 #include "ct_internal.cuh"
 
@@ -55,6 +57,21 @@ uint32_t grid_for(K kernel, uint64_t warps, size_t smem, bool persistent) {
     cap = (uint32_t)std::max(1, sms) * (uint32_t)std::max(1, per);
   }
   return item_blocks(warps, cap);
+}
+
+// Raises a kernel's dynamic shared-memory limit once per device (kernels of
+// one signature share this function).
+template <typename K>
+int allow_smem(K kernel, int bytes) {
+  static std::mutex mu;
+  static std::set<std::pair<int, const void*>> done;
+  int dev = 0;
+  CT_CUDA_TRY(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  if (done.count({dev, (const void*)kernel})) return CT_OK;
+  CT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  done.insert({dev, (const void*)kernel});
+  return CT_OK;
 }
 
 }  // namespace ct

@@ -1897,6 +1897,55 @@ __global__ void k_ff_final(const uint2* __restrict__ mm, const uint32_t* __restr
     if (!((third[f >> 5] >> (f & 31)) & 1u)) atomicOr(bits + (f >> 5), 1u << (f & 31));
   }
 }
+// The same in one launch, a CTA per feature (few rows: the launches and
+// memsets of the grid above take longer than the reads).  bits is zeroed.
+constexpr uint32_t FLAG_CTA_ROWS = 32768;
+
+__global__ void __launch_bounds__(256) k_ff_cta(const float* __restrict__ x_fm, uint32_t n_rows, uint32_t n_features,
+                                                uint2* __restrict__ mm, uint32_t* __restrict__ bits, float2* vals) {
+  __shared__ uint32_t s_mn, s_mx;
+  for (uint32_t f = blockIdx.x; f < n_features; f += gridDim.x) {
+    const float* xr = x_fm + (size_t)f * n_rows;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_mn = 0xffffffffu;
+      s_mx = 0u;
+    }
+    __syncthreads();
+    uint32_t mn = 0xffffffffu, mx = 0u;
+    for (uint32_t i = threadIdx.x; i < n_rows; i += blockDim.x) {
+      const uint32_t o = f32_order(xr[i]);
+      mn = min(mn, o);
+      mx = max(mx, o);
+    }
+    mn = __reduce_min_sync(FULL, mn);
+    mx = __reduce_max_sync(FULL, mx);
+    if (lane_id() == 0) {
+      atomicMin(&s_mn, mn);
+      atomicMax(&s_mx, mx);
+    }
+    __syncthreads();
+    mn = s_mn;
+    mx = s_mx;
+    bool other = false;
+    for (uint32_t i0 = 0; i0 < n_rows && !other; i0 += blockDim.x * 8) {  // usually seen in the first rows
+      bool d = false;
+      for (uint32_t k = 0; k < 8; ++k) {
+        const uint32_t i = i0 + k * blockDim.x + threadIdx.x;
+        if (i < n_rows) {
+          const uint32_t o = f32_order(xr[i]);
+          d |= o != mn && o != mx;
+        }
+      }
+      other = __syncthreads_or(d);
+    }
+    if (threadIdx.x == 0) {
+      mm[f] = make_uint2(mn, mx);
+      if (vals) vals[f] = make_float2(f32_unorder(mn), f32_unorder(mx));
+      if (!other) atomicOr(bits + (f >> 5), 1u << (f & 31));
+    }
+  }
+}
 }  // namespace
 
 // work: feature_flags_work_bytes(n_features) of device scratch (the
@@ -1907,6 +1956,11 @@ int feature_flags(const float* x_fm, uint32_t n_rows, uint32_t n_features, uint3
   uint2* mm = reinterpret_cast<uint2*>(work);
   uint32_t* third = reinterpret_cast<uint32_t*>(mm + n_features);
   CT_CUDA_TRY(cudaMemsetAsync(bits, 0, words * sizeof(uint32_t), st));
+  if (n_rows <= FLAG_CTA_ROWS) {
+    k_ff_cta<<<std::min<uint32_t>(n_features, 148u * 8u), 256, 0, st>>>(x_fm, n_rows, n_features, mm, bits, vals);
+    CT_CUDA_TRY(cudaGetLastError());
+    return CT_OK;
+  }
   CT_CUDA_TRY(cudaMemsetAsync(third, 0, words * sizeof(uint32_t), st));
   CT_CUDA_TRY(cudaMemsetAsync(mm, 0xff, n_features * sizeof(uint2), st));  // min: all ones
   CT_CUDA_TRY(cudaMemset2DAsync(reinterpret_cast<char*>(mm) + 4, sizeof(uint2), 0, 4, n_features, st));  // max: 0

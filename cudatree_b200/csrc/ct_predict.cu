@@ -19,10 +19,8 @@
 //     kernel takes the majority, lowest class on ties
 //     (np.argmax(np.bincount(...)), random_forest.py:358).
 #include <cstring>
-#include <mutex>
-#include <set>
 
-#include "ct_internal.cuh"
+#include "ct_items.cuh"
 
 namespace ct {
 
@@ -291,20 +289,6 @@ int check_forest_device(const void* nodes, uint32_t n_nodes, const uint32_t* off
     set_last_error(std::string("predict: malformed forest: ") + forest_error_text(bad));
     return CT_ERR_ARG;
   }
-  return CT_OK;
-}
-
-// Raise a kernel's dynamic shared-memory limit once per device.
-template <typename K>
-int allow_smem(K kernel, int bytes) {
-  static std::mutex mu;
-  static std::set<int> done;
-  int dev = 0;
-  CT_CUDA_TRY(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(mu);
-  if (done.count(dev)) return CT_OK;
-  CT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  done.insert(dev);
   return CT_OK;
 }
 

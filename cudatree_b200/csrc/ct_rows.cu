@@ -2282,7 +2282,7 @@ inline uint32_t clamp32(uint64_t x) { return x > 0xffffffffull ? 0xffffffffu : (
 // A kernel of CTAs that claim bitmap work: as many as are resident at once.
 template <typename K, typename... A>
 int launch_bitmap(K kernel, int threads, size_t smem, uint32_t items, cudaStream_t st, const A&... args) {
-  CT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ORDER_SMEM_MAX));
+  CT_TRY(allow_smem(kernel, (int)ORDER_SMEM_MAX));
   int per = 1;
   CT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem));
   kernel<<<std::min<uint32_t>(items, sm_count() * (uint32_t)std::max(1, per)), threads, smem, st>>>(args...);
@@ -2499,15 +2499,11 @@ int launch_row_roots(const View& v, const ct_problem* p, uint32_t slot_lo, uint3
   const size_t smem = ((size_t)(p->n_rows + 31) / 32 + v.n_classes) * sizeof(uint32_t);
   const uint32_t threads = p->n_rows >= 8192 ? 1024u : p->n_rows >= 1024 ? 512u : 128u;
   if (p->label_bytes == 1) {
-    static const cudaError_t configured =
-        cudaFuncSetAttribute(k_row_roots<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ORDER_SMEM_MAX);
-    CT_CUDA_TRY(configured);
+    CT_TRY(allow_smem(k_row_roots<uint8_t>, (int)ORDER_SMEM_MAX));
     k_row_roots<uint8_t><<<n_slots, threads, smem, st>>>(v, p->seed, p->bootstrap, slot_lo, tree_lo, n_in, tv, out,
                                                          out_tot, cap, ctr, out_mask, vals);
   } else {
-    static const cudaError_t configured =
-        cudaFuncSetAttribute(k_row_roots<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ORDER_SMEM_MAX);
-    CT_CUDA_TRY(configured);
+    CT_TRY(allow_smem(k_row_roots<uint16_t>, (int)ORDER_SMEM_MAX));
     k_row_roots<uint16_t><<<n_slots, threads, smem, st>>>(v, p->seed, p->bootstrap, slot_lo, tree_lo, n_in, tv, out,
                                                           out_tot, cap, ctr, out_mask, vals);
   }
