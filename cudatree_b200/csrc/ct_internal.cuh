@@ -126,6 +126,7 @@ struct Counters {
   uint32_t ticket_huge;   // k_part_seg's unit counter
   uint32_t n_bchains;     // active chains of k_part_big's segments
   uint32_t n_tv;          // scan pieces of two-valued features
+  uint32_t n_live_pieces; // pieces left by k_row_limit
   uint32_t claim[16];     // item counters of persistent launches (ITEM_* slots)
   unsigned long long next_total;
   unsigned long long small_total;
@@ -142,7 +143,7 @@ struct Counters {
 // and its loop graph, not per step (subtrees run after the level loop).
 enum : uint32_t {
   ITEM_SELECT, ITEM_HIST, ITEM_CARRY, ITEM_SCAN, ITEM_TWO_VALUED, ITEM_REDUCE, ITEM_PLAN, ITEM_FILL,
-  ITEM_CHILDREN, ITEM_VPIECES, ITEM_VCOUNT, ITEM_MOVE, ITEM_BITS, ITEM_STEP_SLOTS, ITEM_SUBTREE = ITEM_STEP_SLOTS,
+  ITEM_CHILDREN, ITEM_VPIECES, ITEM_VCOUNT, ITEM_MOVE, ITEM_BITS, ITEM_LIMIT, ITEM_STEP_SLOTS, ITEM_SUBTREE = ITEM_STEP_SLOTS,
   ITEM_SUBTREE_WIDE
 };
 __device__ __forceinline__ void reset_step_counters(Counters* c, uint32_t n_nodes) {
@@ -156,6 +157,7 @@ __device__ __forceinline__ void reset_step_counters(Counters* c, uint32_t n_node
   c->n_scan_pieces = 0;
   c->n_carry = 0;
   c->n_tv = 0;
+  c->n_live_pieces = 0;
   c->n_splits = 0;
   c->n_part_pieces = 0;
   c->n_status = 0;
@@ -465,6 +467,8 @@ struct LevelScratch {
   uint2* citems;          // [cap_order] (first piece, pieces) of every list of several pieces
   RowPiece* rpieces;      // [cap_scan] pieces of sorted lists and bitmaps; carry rows are indexed alike
   RowBest* rbest;         // [cap_nodes][sel_stride] best of the warp items, then [cap_scan] of the pieces
+  uint2* rscan;           // [cap_scan] (piece, bits of its limit) of the pieces k_row_limit left
+  uint8_t* rlive;         // [cap_scan / 8 + 1] a bit for each piece: left
   uint32_t* node_q;       // [cap_nodes] bits of the largest gain known of the node's candidates (seq_scan)
   RowSplit* rsplits;      // [cap_nodes]
   PartPiece* mpart;       // [cap_mpart] row pieces of splits of more than PART_PIECE rows

@@ -18,8 +18,9 @@
 //   k_row_bits     larger nodes, by a bitmap over the feature's ranks, which
 //                  stands for the sorted list of a node with one row in 64
 //   k_row_order    larger nodes that are sparser: their list, from such a bitmap
-//   k_row_hist, k_row_carry, k_row_scan  the Gini scan of those lists and bitmaps
-//                  in pieces (reference compute_2d, dfs_module.cu:310-443)
+//   k_row_hist, k_row_carry, k_row_bound, k_row_limit, k_row_scan  the Gini scan
+//                  of those lists and bitmaps in pieces (reference compute_2d,
+//                  dfs_module.cu:310-443)
 //   k_row_reduce   best candidate of each node; node record, children, work list
 //   k_row_mark     left flags and class counts; moves the rows of small splits
 //   k_row_move     stable split of the row lists of larger ones
@@ -648,35 +649,6 @@ __device__ __forceinline__ void seq_totals(uint32_t* sq, const uint32_t* tot, ui
     reinterpret_cast<double*>(sq + SEQ_TAB)[lane] = (double)t;
     sq[SEQ_BEFORE + SEQ_CLASSES + lane] = t;
   }
-}
-
-// The largest gain any order of rows could reach at a position among them or
-// at their ends, a[] and b[] being the class counts before and after them: the
-// gain is a convex function of the left class counts, so it is largest where
-// every class's rows lie all left or all right.  One such corner per lane and
-// round.  Warp-collective.
-__device__ __forceinline__ float gain_limit(const uint32_t* a, const uint32_t* b, const uint32_t* total, uint32_t C,
-                                            uint32_t n) {
-  const uint32_t lane = lane_id();
-  const double inv = 1.0 / (double)n;
-  float best = 0.f;
-  for (uint32_t m = lane; m < (1u << C); m += 32) {
-    uint32_t nl = 0;
-#pragma unroll
-    for (uint32_t c = 0; c < SEQ_CLASSES; ++c)
-      if (c < C) nl += (m >> c) & 1u ? b[c] : a[c];
-    if (nl == 0 || nl >= n) continue;
-    const double t = (double)nl * inv;
-    double d = 0.0;
-#pragma unroll
-    for (uint32_t c = 0; c < SEQ_CLASSES; ++c) {
-      if (c >= C) break;
-      const double u = (double)((m >> c) & 1u ? b[c] : a[c]) - t * (double)total[c];
-      d += u * u;
-    }
-    best = fmaxf(best, gain_of(d, (float)nl, (float)(n - nl), (float)n));
-  }
-  return __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(best)));
 }
 
 // The scan of a run at positions p0.. of the node's order.  run: this lane's
@@ -1371,7 +1343,7 @@ struct PieceStream {
 // Shared memory of one warp of k_row_hist and k_row_scan, in words.
 __host__ __device__ __forceinline__ uint32_t hist_words(uint32_t n_classes) { return LIST_CAP / 2 + n_classes; }
 __host__ __device__ __forceinline__ uint32_t scan_words(uint32_t n_classes) {
-  return LIST_CAP / 2 + (n_classes <= SEQ_CLASSES ? 2 * SEQ_SLOTS + SEQ_WORDS : 2 * n_classes);
+  return LIST_CAP / 2 + 2 * n_classes;
 }
 
 __device__ __forceinline__ PieceStream piece_stream(const View& v, const ct_node& nd, const RowPiece& pc, uint32_t f,
@@ -1517,6 +1489,139 @@ __global__ void __launch_bounds__(256) k_row_bound(View vb, LevelScratch s) {
   }
 }
 
+// Which pieces to scan, with up to SEQ_CLASSES classes.  The gain is a convex
+// function of the left class counts, so no order of a piece's rows has a
+// candidate with a larger gain than the corners have at which every class's
+// rows lie all left or all right of it; a piece whose best corner is below the
+// best gain known for the node holds no split (98 pieces in 100 on
+// covtype-shaped data).  The counts' sums of squares and of products with the
+// totals that a gain takes (seq_scan) are sums over the classes, so a lane
+// adds up its five lowest classes' once and then only the others', corner by
+// corner.  A warp takes LIMIT_PIECES pieces together, whose records and counts
+// come in with one round of loads: checked by the scanning warp, one piece at
+// a time, the loads' latency was most of the scan (9.2 ms of 100
+// covtype-shaped trees, 0.7 here).
+constexpr uint32_t LIMIT_PIECES = 8;
+constexpr uint32_t LIMIT_BASE = 5;  // classes of a lane's own corner
+
+struct PieceLimit {
+  double2 add[SEQ_CLASSES];    // what a class's rows of the piece add to s and a when they lie left
+  uint32_t rows[SEQ_CLASSES];  // those rows
+  double s, a, t;              // sums of A^2, A T, T^2 over the classes, A the counts before the piece
+  uint32_t nl;                 // sum of A
+  uint32_t n_rows;             // rows of the piece
+};
+// From the class counts a before the piece, b after it, t of the node: one
+// class per lane of a group of SEQ_CLASSES lanes.  Warp-collective.
+__device__ __forceinline__ void limit_set(PieceLimit& pl, bool write, uint32_t a, uint32_t b, uint32_t t) {
+  const uint32_t c = lane_id() % SEQ_CLASSES;
+  double qs = (double)((uint64_t)a * a), qa = (double)((uint64_t)a * t), qt = (double)((uint64_t)t * t);
+  uint32_t nl = a, rows = b - a;
+  if (write) {
+    pl.add[c] = make_double2((double)((uint64_t)b * b - (uint64_t)a * a), (double)((uint64_t)(b - a) * t));
+    pl.rows[c] = b - a;
+  }
+#pragma unroll
+  for (uint32_t k = 1; k < SEQ_CLASSES; k <<= 1) {
+    qs += __shfl_xor_sync(FULL, qs, k);
+    qa += __shfl_xor_sync(FULL, qa, k);
+    qt += __shfl_xor_sync(FULL, qt, k);
+    nl += __shfl_xor_sync(FULL, nl, k);
+    rows += __shfl_xor_sync(FULL, rows, k);
+  }
+  if (write && c == 0) {
+    pl.s = qs;
+    pl.a = qa;
+    pl.t = qt;
+    pl.nl = nl;
+    pl.n_rows = rows;
+  }
+}
+// The largest estimated gain of the piece's corners (0: no rows, so no
+// candidate).  Warp-collective.
+__device__ __forceinline__ float limit_of(const PieceLimit& pl, uint32_t C, uint32_t n) {
+  const uint32_t lane = lane_id();
+  if (pl.n_rows == 0) return 0.f;
+  const double inv = 1.0 / (double)n, st2 = pl.t;
+  const float nf = (float)n;
+  double ls = pl.s, la = pl.a;
+  uint32_t nl = pl.nl;
+#pragma unroll
+  for (uint32_t c = 0; c < LIMIT_BASE; ++c)
+    if ((lane >> c) & 1u) {
+      const double2 d = pl.add[c];
+      ls += d.x;
+      la += d.y;
+      nl += pl.rows[c];
+    }
+  float best = 0.f;
+  for (uint32_t m = 0; m < (C > LIMIT_BASE ? 1u << (C - LIMIT_BASE) : 1u); ++m) {
+    double ms = ls, ma = la;
+    uint32_t k = nl;
+#pragma unroll
+    for (uint32_t c = 0; c < SEQ_CLASSES - LIMIT_BASE; ++c)
+      if ((m >> c) & 1u) {
+        const double2 d = pl.add[LIMIT_BASE + c];
+        ms += d.x;
+        ma += d.y;
+        k += pl.rows[LIMIT_BASE + c];
+      }
+    const double t = (double)k * inv;
+    const float g = gain_of(fma(t, fma(t, st2, -2.0 * ma), ms), (float)k, (float)(n - k), nf);
+    if (k > 0 && k < n) best = fmaxf(best, g);
+  }
+  return __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(best)));
+}
+
+__global__ void __launch_bounds__(THREADS_PER_BLOCK) k_row_limit(LevelScratch s, uint32_t C) {
+  __shared__ PieceLimit limits_all[WARPS_PER_BLOCK][LIMIT_PIECES];
+  const uint32_t lane = lane_id();
+  PieceLimit* limits = limits_all[threadIdx.x >> 5];
+  const uint32_t count = live_count(s, s.ctr->n_scan_pieces, s.cap_scan);
+  const StepLists lists = *s.step;
+  for_items(ceil_div(count, LIMIT_PIECES), &s.ctr->claim[ITEM_LIMIT], [&](uint32_t i) {
+    const uint32_t p0 = i * LIMIT_PIECES, np = min(LIMIT_PIECES, count - p0);
+    RowPiece pc{0u, 0u, 0u, 1u};
+    uint32_t n = 1;
+    float known = 0.f;
+    if (lane < np) {
+      pc = s.rpieces[p0 + lane];
+      n = lists.nodes[pc.node].n;
+      known = __uint_as_float(*reinterpret_cast<volatile uint32_t*>(s.node_q + pc.node));
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < LIMIT_PIECES * SEQ_CLASSES / 32; ++r) {
+      const uint32_t p = r * (32 / SEQ_CLASSES) + lane / SEQ_CLASSES, c = lane % SEQ_CLASSES;
+      const uint32_t node = __shfl_sync(FULL, pc.node, p), j = __shfl_sync(FULL, pc.j, p);
+      const uint32_t npieces = __shfl_sync(FULL, pc.npieces, p);
+      uint32_t a = 0, b = 0, t = 0;
+      if (p < np && c < C) {
+        const uint32_t* carry = s.carry + (size_t)(p0 + p) * C + c;
+        t = lists.tot[(size_t)node * C + c];
+        a = npieces > 1 ? *carry : 0u;
+        b = j + 1 < npieces ? carry[C] : t;
+      }
+      limit_set(limits[p], true, a, b, t);
+    }
+    __syncwarp();
+    uint32_t live = 0;
+    float limit = 0.f;
+    for (uint32_t p = 0; p < np; ++p) {
+      const uint32_t pn = __shfl_sync(FULL, n, p);
+      const float best = limit_of(limits[p], C, pn);
+      if (best > 0.f && best >= gain_bound(__shfl_sync(FULL, known, p), pn)) live |= 1u << p;
+      if (lane == p) limit = best;
+    }
+    uint32_t at = 0;
+    if (lane == 0) {
+      s.rlive[i] = (uint8_t)live;
+      if (live) at = atomicAdd(&s.ctr->n_live_pieces, (uint32_t)__popc(live));
+    }
+    at = __shfl_sync(FULL, at, 0) + (uint32_t)__popc(live & lanemask_lt());
+    if ((live >> lane) & 1u) s.rscan[at] = make_uint2(p0 + lane, __float_as_uint(limit));
+  });
+}
+
 // Value bits of the element before the piece (the last set bit before a
 // run of ranks).  The piece is not the node's first with elements.
 __device__ __forceinline__ uint32_t value_before(const View& v, const PieceStream& ps, const ct_node& nd,
@@ -1540,12 +1645,9 @@ __device__ __forceinline__ uint32_t value_before(const View& v, const PieceStrea
 
 // Gini scan of one piece.  The candidate between two neighbours is judged
 // when the upper one is met, so only the value before the piece comes from
-// outside it.  A piece whose values all equal that one has no candidate, and
-// with up to SEQ_CLASSES classes neither is a piece scanned whose gain_limit
-// is below the best known (three rows in four on covtype-shaped data).  Per
-// 100 covtype-shaped trees: class match and warp scans per round 19.4 ms,
-// lane-sequential 21.3, with gain_limit 13.5, with estimates precise enough
-// that few lanes score exactly 9.3.
+// outside it.  A piece whose values all equal that one has no candidate.
+// With more than SEQ_CLASSES classes one warp scans a piece; a round of 32
+// elements matches its classes and scans the sums' increments.
 template <bool Q>
 __device__ __forceinline__ void row_scan_item(const View& vb, const StepLists& lists, const LevelScratch& s,
                                               uint32_t* smem, uint32_t pi) {
@@ -1561,68 +1663,6 @@ __device__ __forceinline__ void row_scan_item(const View& vb, const StepLists& l
   RowBest* out = s.rbest + (size_t)s.cap_nodes * vb.sel_stride + pi;
   const uint32_t f = s.sel[(size_t)pc.node * v.sel_stride + pc.slot];
   PieceStream ps = piece_stream(v, nd, pc, f, lists.scan_piece, smem);
-  if (C <= SEQ_CLASSES) {
-    // staged in shared memory, SEQ_ROWS at a time, for the lane-sequential scan
-    uint2* ent = reinterpret_cast<uint2*>(smem + LIST_CAP / 2);
-    uint32_t* sq = smem + LIST_CAP / 2 + 2 * SEQ_SLOTS;
-    uint32_t* before = sq + SEQ_BEFORE;
-    const uint32_t mine = lane < C && carry ? carry[lane] : 0u;
-    const uint32_t last = lane >= C ? 0u : pc.j + 1 < pc.npieces ? carry[C + lane] : tot[lane];  // counts after the piece
-    const float known = __uint_as_float(*reinterpret_cast<volatile uint32_t*>(s.node_q + pc.node));
-    if (lane < SEQ_CLASSES) {
-      before[lane] = mine;
-      sq[lane] = last;
-    }
-    seq_totals(sq, tot, C);
-    uint32_t p0 = __reduce_add_sync(FULL, mine);
-    const bool empty = !__any_sync(FULL, last != mine);
-    __syncwarp();
-    // no candidate of the piece can reach the best known: nothing to scan
-    if (empty || gain_limit(before, sq, before + SEQ_CLASSES, C, n) < gain_bound(known, n)) {
-      if (lane == 0) *out = RowBest{dinf(), NONE, 0u, 0.f, 0.f};
-      return;
-    }
-    __syncwarp();
-    SeqBest bb{dinf(), NONE, 0u, 0.f, 0.f};
-    float x_last = 0.f;
-    bool first = true;
-    uint32_t keep = 0;
-    while (ps.fill(keep)) {
-      if (first && p0 > 0) {
-        x_last = __uint_as_float(value_before(v, ps, nd, pc, f, lists.scan_piece));
-        if (!ps.dense && __uint_as_float(ps.base[ps.count - 1].x) == x_last) break;  // no candidate in the piece
-      }
-      keep = 0;
-      for (uint32_t b = 0; b < ps.count; b += SEQ_ROWS) {
-        const uint32_t k = min(SEQ_ROWS, ps.count - b);
-        if (k < SEQ_ROWS && ps.more()) {  // with the next batch
-          keep = k;
-          break;
-        }
-        const uint32_t sh = seq_shift(k);
-#pragma unroll 4
-        for (uint32_t i = lane; i < k; i += 32) {
-          const uint2 e = ps.load(b + i);
-          ent[seq_at(i, sh)] = seq_entry(e.x, e.y);
-        }
-        __syncwarp();
-        if (first && p0 == 0) x_last = __uint_as_float(ent[0].x);  // no candidate before the node's first row
-        first = false;
-        const uint32_t i0 = min(lane << sh, k), m = min(k - i0, 1u << sh);
-        const uint2* run = ent + seq_at(i0, sh);
-        uint32_t w[4];
-        seq_count(run, m, w);
-        const float x_end = __uint_as_float(ent[seq_at(k - 1, sh)].x);
-        const float xp = i0 > 0 && m > 0 ? __uint_as_float(ent[seq_at(i0 - 1, sh)].x) : x_last;
-        seq_scan(run, m, sh, w, sq, C, xp, p0, n, s.node_q + pc.node, bb);
-        x_last = x_end;
-        p0 += k;
-      }
-    }
-    const uint32_t win = warp_best_lane(bb.score, bb.pos);
-    if (win == NONE ? lane == 0 : lane == win) *out = RowBest{bb.score, bb.pos, bb.pure, bb.xl, bb.xr};
-    return;
-  }
   int64_t sl = 0, st2 = 0, a = 0;
   uint32_t before = 0;
   for (uint32_t c = lane; c < C; c += 32) {
@@ -1722,6 +1762,182 @@ __global__ void __launch_bounds__(THREADS_PER_BLOCK, 7) k_row_scan(View v, Level
   for_items(count, &s.ctr->claim[ITEM_SCAN], [&](uint32_t i) { row_scan_item<Q>(v, sl, s, ws, i); });
 }
 
+// The scan of the pieces k_row_limit left, with up to SEQ_CLASSES classes.
+// They are few and may be long (a run of ranks can hold all of a node's rows),
+// so what bounds it is how long one piece takes: the warps of a CTA share a
+// piece.  Each counts the classes of its part, then knows the counts before
+// it, and walks only the runs of up to SEQ_ROWS rows whose own limit reaches
+// the bound.  One warp per piece took 120 us of a level of 20 covtype-shaped
+// trees with 7% of the warps in flight (100 trees: 8.3 ms, here 2.9).
+constexpr int SCAN_WARPS = 8;
+constexpr uint32_t SCAN_WORDS = LIST_CAP / 2 + 2 * SEQ_SLOTS + SEQ_WORDS + sizeof(PieceLimit) / 4;  // of one warp
+static_assert(SCAN_WORDS % 4 == 0 && (LIST_CAP / 2 + 2 * SEQ_SLOTS + SEQ_WORDS) % 4 == 0, "PieceLimit is aligned to 16 bytes");
+
+template <bool Q>
+__global__ void __launch_bounds__(32 * SCAN_WARPS, 3) k_row_scan_seq(View vb, LevelScratch s) {
+  extern __shared__ __align__(16) uint32_t scan_sm[];
+  __shared__ uint32_t s_piece;
+  __shared__ uint32_t s_cnt[SCAN_WARPS][SEQ_CLASSES], s_rows[SCAN_WARPS], s_last[SCAN_WARPS];
+  __shared__ RowBest s_best[SCAN_WARPS];
+  const uint32_t count = live_count(s, s.ctr->n_live_pieces, s.cap_scan);
+  const StepLists lists = *s.step;
+  const uint32_t C = vb.n_classes, lane = lane_id(), warp = threadIdx.x >> 5;
+  uint32_t* smem = scan_sm + warp * SCAN_WORDS;
+  uint2* ent = reinterpret_cast<uint2*>(smem + LIST_CAP / 2);
+  uint32_t* sq = smem + LIST_CAP / 2 + 2 * SEQ_SLOTS;
+  uint32_t* before = sq + SEQ_BEFORE;
+  PieceLimit& pl = *reinterpret_cast<PieceLimit*>(sq + SEQ_WORDS);
+  RowBest* best = s.rbest + (size_t)s.cap_nodes * vb.sel_stride;
+  uint32_t item = blockIdx.x;
+  while (true) {
+    if (threadIdx.x == 0) {
+      uint32_t pi = NONE;
+      for (; item < count; item = gridDim.x + atomicAdd(&s.ctr->claim[ITEM_SCAN], 1u)) {
+        const uint2 live = s.rscan[item];
+        const uint32_t node = s.rpieces[live.x].node;
+        const float known = __uint_as_float(*reinterpret_cast<volatile uint32_t*>(s.node_q + node));
+        if (__uint_as_float(live.y) >= gain_bound(known, lists.nodes[node].n)) {
+          pi = live.x;
+          item = gridDim.x + atomicAdd(&s.ctr->claim[ITEM_SCAN], 1u);
+          break;
+        }
+        best[live.x] = RowBest{dinf(), NONE, 0u, 0.f, 0.f};  // other pieces' scans have raised the bound
+      }
+      s_piece = pi;
+    }
+    __syncthreads();
+    const uint32_t pi = s_piece;
+    if (pi == NONE) break;
+    const RowPiece pc = s.rpieces[pi];
+    const ct_node nd = lists.nodes[pc.node];
+    CT_JOB_REF(v, vb, nd.slot);
+    const uint32_t n = nd.n, f = s.sel[(size_t)pc.node * v.sel_stride + pc.slot];
+    const uint32_t* tot = lists.tot + (size_t)pc.node * C;
+    const PieceStream whole = piece_stream(v, nd, pc, f, lists.scan_piece, smem);
+    PieceStream part = whole;  // this warp's part
+    if (part.dense) {
+      const uint32_t per = ceil_div(whole.n_words, (uint32_t)SCAN_WARPS), w0 = min(warp * per, whole.n_words);
+      part.base += w0 * 32;
+      part.words += w0;
+      part.n_words = min(per, whole.n_words - w0);
+    } else {
+      const uint32_t per = ceil_div(whole.count, (uint32_t)SCAN_WARPS), i0 = min(warp * per, whole.count);
+      part.base += i0;
+      part.count = min(per, whole.count - i0);
+    }
+    const uint32_t carry = lane < C && pc.npieces > 1 ? s.carry[(size_t)pi * C + lane] : 0u;
+    const uint32_t total = lane < C ? tot[lane] : 0u;
+    seq_totals(sq, tot, C);
+    auto stage = [&](const PieceStream& ps, uint32_t b, uint32_t k, uint32_t sh) {
+      __syncwarp();
+#pragma unroll 4
+      for (uint32_t i = lane; i < k; i += 32) {
+        const uint2 e = ps.load(b + i);
+        ent[seq_at(i, sh)] = seq_entry(e.x, e.y);
+      }
+      __syncwarp();
+    };
+    // counts of a staged run: by lane in w, in all on lane c for class c
+    auto count_run = [&](uint32_t k, uint32_t sh, uint32_t(&w)[4]) {
+      const uint32_t i0 = min(lane << sh, k);
+      seq_count(ent + seq_at(i0, sh), min(k - i0, 1u << sh), w);
+      uint32_t t[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) t[h] = h < 2 || C > 4 ? __reduce_add_sync(FULL, w[h]) : 0u;
+      return lane < C ? seq_field(t, lane) : 0u;
+    };
+    // classes, rows and last value of the part; one run of it stays staged
+    PieceStream ps = part;
+    bool more = ps.fill();
+    const bool staged = more && !ps.more() && ps.count <= SEQ_ROWS;
+    uint32_t w[4] = {0u, 0u, 0u, 0u}, mine = 0, x_last = 0;
+    while (more) {
+      for (uint32_t b = 0; b < ps.count; b += SEQ_ROWS) {
+        const uint32_t k = min(SEQ_ROWS, ps.count - b), sh = seq_shift(k);
+        stage(ps, b, k, sh);
+        mine += count_run(k, sh, w);
+        x_last = ent[seq_at(k - 1, sh)].x;
+      }
+      more = ps.more() && ps.fill();
+    }
+    const uint32_t rows = __reduce_add_sync(FULL, mine);
+    if (lane < SEQ_CLASSES) s_cnt[warp][lane] = mine;
+    if (lane == 0) {
+      s_rows[warp] = rows;
+      s_last[warp] = x_last;
+    }
+    __syncthreads();
+    uint32_t a = carry, prev = NONE;  // counts before the part; the nearest part before it with rows
+    for (uint32_t k = 0; k < warp; ++k) {
+      if (lane < SEQ_CLASSES) a += s_cnt[k][lane];
+      if (s_rows[k]) prev = k;
+    }
+    if (lane < SEQ_CLASSES) before[lane] = a;
+    __syncwarp();
+    const uint32_t* known = s.node_q + pc.node;
+    auto reaches = [&](uint32_t lo, uint32_t run) {  // may a candidate of the run win
+      __syncwarp();
+      limit_set(pl, lane < SEQ_CLASSES, lo, lo + run, total);
+      __syncwarp();
+      const float g = limit_of(pl, C, n);
+      return g > 0.f && g >= gain_bound(__uint_as_float(*reinterpret_cast<const volatile uint32_t*>(known)), n);
+    };
+    SeqBest bb{dinf(), NONE, 0u, 0.f, 0.f};
+    if (rows > 0 && reaches(a, mine)) {
+      uint32_t p0 = __reduce_add_sync(FULL, a);
+      // no candidate before the node's first row
+      x_last = prev != NONE ? s_last[prev] : p0 > 0 ? value_before(v, whole, nd, pc, f, lists.scan_piece) : NONE;
+      bool first = p0 == 0;
+      auto scan_run = [&](uint32_t k, uint32_t sh) {
+        if (first) x_last = ent[0].x;
+        first = false;
+        const uint32_t i0 = min(lane << sh, k), m = min(k - i0, 1u << sh);
+        const uint32_t x_end = ent[seq_at(k - 1, sh)].x;
+        const uint32_t xp = i0 > 0 && m > 0 ? ent[seq_at(i0 - 1, sh)].x : x_last;
+        seq_scan(ent + seq_at(i0, sh), m, sh, w, sq, C, __uint_as_float(xp), p0, n, s.node_q + pc.node, bb);
+        x_last = x_end;
+        p0 += k;
+      };
+      if (staged) {
+        scan_run(rows, seq_shift(rows));
+      } else {
+        ps = part;
+        uint32_t keep = 0;
+        while (ps.fill(keep)) {
+          keep = 0;
+          for (uint32_t b = 0; b < ps.count; b += SEQ_ROWS) {
+            const uint32_t k = min(SEQ_ROWS, ps.count - b);
+            if (k < SEQ_ROWS && ps.more()) {  // with the next batch
+              keep = k;
+              break;
+            }
+            const uint32_t sh = seq_shift(k);
+            stage(ps, b, k, sh);
+            const uint32_t run = count_run(k, sh, w), lo = lane < SEQ_CLASSES ? before[lane] : 0u;
+            if (reaches(lo, run)) {
+              scan_run(k, sh);
+            } else {
+              if (lane < SEQ_CLASSES) before[lane] = lo + run;
+              __syncwarp();
+              x_last = ent[seq_at(k - 1, sh)].x;
+              first = false;
+              p0 += k;
+            }
+          }
+        }
+      }
+    }
+    const uint32_t win = warp_best_lane(bb.score, bb.pos);
+    if (win == NONE ? lane == 0 : lane == win) s_best[warp] = RowBest{bb.score, bb.pos, bb.pure, bb.xl, bb.xr};
+    __syncthreads();
+    if (warp == 0) {
+      const RowBest rb = lane < SCAN_WARPS ? s_best[lane] : RowBest{dinf(), NONE, 0u, 0.f, 0.f};
+      const uint32_t wl = warp_best_lane(rb.score, rb.pos);
+      if (wl == NONE ? lane == 0 : lane == wl) best[pi] = rb;
+    }
+  }
+}
+
 // ------------------------------------------------------------------------
 // Best candidate of a node (lowest score, then feature, then position), its
 // record in the tree, and the pieces of its rows' split.
@@ -1747,7 +1963,9 @@ __device__ __forceinline__ void row_reduce_item(const View& vb, const StepLists&
   } else {
     const uint32_t pb = s.piece_base[w], pn = s.piece_cnt[w];
     const RowBest* best = s.rbest + (size_t)s.cap_nodes * vb.sel_stride;
-    for (uint32_t q = lane; q < pn; q += 32) take(best[pb + q], sel[s.rpieces[pb + q].slot]);
+    for (uint32_t q = pb + lane; q < pb + pn; q += 32)
+      if (C > SEQ_CLASSES || ((s.rlive[q / LIMIT_PIECES] >> (q % LIMIT_PIECES)) & 1u))
+        take(best[q], sel[s.rpieces[q].slot]);
   }
   if (v.vmask) {
     // a virtual feature's one candidate (the last low-value row), scored from
@@ -2360,9 +2578,14 @@ int row_step(const View& v, const LevelScratch& s, LevelBounds b, uint32_t n_max
     k_row_carry<<<grid_for(k_row_carry, (uint64_t)s.cap_order * C, 0, true), THREADS_PER_BLOCK, 0, st>>>(s, C);
     if (C <= SEQ_CLASSES) {
       k_row_bound<Q><<<sms * 8, 256, 0, st>>>(v, s);
-      pf->launched(CT_K_SCAN);
+      k_row_limit<<<grid_for(k_row_limit, ceil_div(s.cap_scan, LIMIT_PIECES), 0, true), THREADS_PER_BLOCK, 0, st>>>(s, C);
+      pf->launched(CT_K_SCAN, 2);
     }
-    k_row_scan<Q><<<grid_for(k_row_scan<Q>, s.cap_scan, sms2, true), THREADS_PER_BLOCK, sms2, st>>>(v, s);
+    if (C <= SEQ_CLASSES)
+      CT_TRY(launch_bitmap(k_row_scan_seq<Q>, 32 * SCAN_WARPS, SCAN_WARPS * SCAN_WORDS * sizeof(uint32_t), s.cap_scan, st,
+                           v, s));
+    else
+      k_row_scan<Q><<<grid_for(k_row_scan<Q>, s.cap_scan, sms2, true), THREADS_PER_BLOCK, sms2, st>>>(v, s);
     pf->launched(CT_K_SCAN, hist ? 3 : 2);
   }
   pf->end();
@@ -2461,6 +2684,8 @@ bool carve_row_scratch(Arena& a, const View& v, LevelBounds b, uint32_t scan_pie
   t.glarge = a.take<uint2>(t.cap_order);
   t.rpieces = a.take<RowPiece>(t.cap_scan);
   t.rbest = a.take<RowBest>((size_t)t.cap_nodes * m + t.cap_scan);
+  t.rscan = C <= SEQ_CLASSES ? a.take<uint2>(t.cap_scan) : nullptr;
+  t.rlive = C <= SEQ_CLASSES ? a.take<uint8_t>(t.cap_scan / LIMIT_PIECES + 1) : nullptr;
   t.carry = a.take<uint32_t>((size_t)t.cap_scan * C);
   t.rsplits = a.take<RowSplit>(t.cap_nodes);
   t.split_left = a.take<uint32_t>((size_t)t.cap_nodes * C);
