@@ -4,10 +4,10 @@
 // per warp, and random_forest.py:339-362 stacks per-tree labels on the host
 // and votes row by row in Python.  Here one launch walks every tree of the
 // forest:
-//   * blocks cover (row tile, tree group); the trees are cut into groups whose
-//     nodes fit comfortably in L2, and blocks are numbered group-major, so the
-//     blocks in flight walk one group and its nodes come from DRAM about once
-//     per launch instead of once per walk;
+//   * blocks cover (row tile, tree group); the trees are cut into groups of as
+//     many as a block walks at once, and blocks are numbered group-major, so the
+//     blocks in flight walk one group's trees and find much of them in L1
+//     (predict_group_size);
 //   * walks inside a block are numbered row-fastest: with 32 rows per tile a
 //     lane keeps one row and a warp's lanes walk the same tree (shared loads
 //     of its top levels); each thread keeps PRED_ILP walks in flight;
@@ -27,10 +27,16 @@ namespace ct {
 namespace {
 
 constexpr int PRED_THREADS = 256;
-constexpr int PRED_ILP = 8;
+// Walks in flight per thread.  4 at 6 blocks per SM against 8 at 4 blocks: fewer
+// trees in flight, whose nodes stay in L1 longer.  500 covtype-shaped trees
+// (37 MB of nodes), 65,536 rows, in groups of one round of walks each: 4 walks
+// 1.64 ms, 8 walks 1.82, 2 walks (8 blocks) 1.82.
+constexpr int PRED_ILP = 4;
 constexpr uint32_t X_SMEM_BYTES = 32 * 1024;     // rows of x staged per block when they fit
 constexpr uint32_t HIST_SMEM_BYTES = 64 * 1024;  // vote histogram [rows][classes]
-constexpr size_t GROUP_L2_BYTES = 32ull << 20;   // node bytes of one tree group
+constexpr size_t GROUP_L2_BYTES = 32ull << 20;   // node bytes of one tree group, at the most
+constexpr size_t GROUP_L1_BYTES = 192ull << 10;  // node bytes of one round of walks from which groups are single rounds
+constexpr uint32_t PRED_BLOCKS_PER_SM = 6;
 
 __host__ __device__ __forceinline__ bool predict_rows_staged(uint32_t rpb, uint32_t n_features) {
   return (size_t)rpb * n_features * sizeof(float) <= X_SMEM_BYTES;
@@ -193,7 +199,7 @@ __device__ __forceinline__ void tile_work(const void* nodes, const uint32_t* tre
 }
 
 template <typename Form>
-__global__ void __launch_bounds__(PRED_THREADS, 4)
+__global__ void __launch_bounds__(PRED_THREADS, PRED_BLOCKS_PER_SM)
 k_predict(const void* __restrict__ nodes, const uint32_t* __restrict__ tree_off, uint32_t n_trees, uint32_t fbits,
           uint32_t group, uint32_t tiles, const float* __restrict__ x, uint32_t n_rows, uint32_t n_features,
           uint32_t n_classes, uint32_t rpb, uint32_t* __restrict__ votes, uint32_t* __restrict__ pred) {
@@ -294,11 +300,13 @@ int check_forest_device(const void* nodes, uint32_t n_nodes, const uint32_t* off
 
 }  // namespace
 
-// Rows per tile: 32, halved until the [rows][classes] histogram and the
-// staged [features][rows] tile fit their shared-memory budgets.
-uint32_t predict_rows_per_block(uint32_t n_classes, uint32_t n_features) {
+// Rows per tile: 32, halved while half as many still hold all rows (a few
+// rows' trees are then spread over a block's threads instead of over rounds of
+// walks) or until the [rows][classes] histogram and the staged
+// [features][rows] tile fit their shared-memory budgets.
+uint32_t predict_rows_per_block(uint32_t n_classes, uint32_t n_features, uint32_t n_rows) {
   uint32_t r = 32;
-  while (r > 1 && ((size_t)r * n_classes * sizeof(uint32_t) > HIST_SMEM_BYTES ||
+  while (r > 1 && (r / 2 >= n_rows || (size_t)r * n_classes * sizeof(uint32_t) > HIST_SMEM_BYTES ||
                    (size_t)r * n_features * sizeof(float) > X_SMEM_BYTES))
     r >>= 1;
   return r;
@@ -314,6 +322,28 @@ uint32_t predict_group_size(uint32_t n_trees, uint64_t n_nodes, size_t node_byte
   uint64_t g = per_tree ? GROUP_L2_BYTES / per_tree : n_trees;
   if (g < 1) g = 1;
   return (uint32_t)std::min<uint64_t>(g, n_trees);
+}
+
+// Trees per group of a launch with a vote table.  A block's threads walk
+// `round` trees at once; with one round per group the blocks on an SM walk the
+// same few trees, whose nodes then come from L1 more often: 500 trees of 75 KB,
+// 65,536 rows: 1.64 ms in groups of 32 (one round of 32 rows), 1.81 of 64,
+// 2.20 of 128, 3.29 ungrouped, and 1.83 of 24 (a round not filled).  A group
+// costs each tile a staging of its rows and a flush of its votes, which is
+// more than short walks in trees that fit L1 anyway gain: 100 trees of 5.5 KB
+// take 193 us in groups of 32 and 189 us as one, of 8.4 KB 233 and 250 us.  (And
+// two groups of 20 take 174 us where one of 40 takes 167: from one and a half
+// rounds on.)  Fewer tiles than blocks the chip holds are cut further, down to 2
+// trees per thread column, when the trees are more than a round: 2,048 rows,
+// 100 trees of 24 KB: 96 us as one group, 61 of 32, 58 of 16; but 20,000 rows of
+// 20 small trees 53 us as one, 60 as two.
+uint32_t predict_group_size(uint32_t n_trees, uint64_t n_nodes, size_t node_bytes, uint32_t rpb, uint32_t tiles) {
+  const uint32_t columns = PRED_THREADS / rpb, round = columns * PRED_ILP;
+  uint32_t g = predict_group_size(n_trees, n_nodes, node_bytes);
+  if (n_nodes * node_bytes / n_trees * round > GROUP_L1_BYTES && n_trees >= round + round / 2) g = std::min(g, round);
+  const uint32_t fill = ceil_div(148u * PRED_BLOCKS_PER_SM, tiles);
+  if (fill > 1 && n_trees > round) g = std::min(g, std::max(ceil_div(n_trees, fill), 2 * columns));
+  return ceil_div(n_trees, ceil_div(n_trees, g));
 }
 
 uint32_t compact_feature_bits(uint32_t n_features) {
@@ -376,7 +406,7 @@ int compact_forest(const ct_packed_node* nodes, uint32_t n_nodes, uint32_t n_fea
   return CT_OK;
 }
 
-__global__ void __launch_bounds__(PRED_THREADS, 4)
+__global__ void __launch_bounds__(PRED_THREADS, PRED_BLOCKS_PER_SM)
 k_predict_batch(const BatchReq* __restrict__ reqs, uint32_t n_req) {
   extern __shared__ uint32_t smem[];
   uint32_t lo = 0, hi = n_req;  // the last request whose first block is <= blockIdx.x
@@ -440,12 +470,14 @@ int predict(const void* nodes, uint32_t n_nodes, uint32_t fbits, const uint32_t*
     CT_TRY(check_forest_device<CompactForm>(nodes, n_nodes, tree_off, n_trees, fbits, n_features, n_classes, pred, st));
   else
     CT_TRY(check_forest_device<PackedForm>(nodes, n_nodes, tree_off, n_trees, 0, n_features, n_classes, pred, st));
-  const uint32_t rpb = predict_rows_per_block(n_classes, n_features);
+  const uint32_t rpb = predict_rows_per_block(n_classes, n_features, n_rows);
   const uint32_t tiles = ceil_div(n_rows, rpb);
   // Tree groups need the vote table; without one every block walks all trees.
+  // Few rows are worth the table's zeroing and the votes' own launch from two
+  // rounds of walks on: a call with 40 rows and 500 trees 344 -> 155 us.
   uint32_t group = n_trees;
-  if (votes && n_trees >= 16 && n_rows >= 1024)
-    group = predict_group_size(n_trees, n_nodes, fbits ? CompactForm::BYTES : PackedForm::BYTES);
+  if (votes && n_trees >= (n_rows >= 1024 ? 16u : 2u * PRED_ILP * (PRED_THREADS / rpb)))
+    group = predict_group_size(n_trees, n_nodes, fbits ? CompactForm::BYTES : PackedForm::BYTES, rpb, tiles);
   const uint32_t groups = ceil_div(n_trees, group);
   const size_t smem = predict_tile_smem(rpb, n_classes, n_features);
   if (groups > 1) CT_CUDA_TRY(cudaMemsetAsync(votes, 0, (size_t)n_rows * n_classes * sizeof(uint32_t), st));

@@ -361,6 +361,7 @@ class Server {
     }
     const size_t node_bytes = Pool::round((size_t)n_nodes * elem), off_bytes = (size_t)n_trees * 4;
     f.bytes = Pool::round(node_bytes + off_bytes);
+    f.n_nodes = n_nodes;
     f.group = n_classes <= cfg.max_classes ? predict_group_size(n_trees, n_nodes, elem) : n_trees;
     {
       std::lock_guard<std::mutex> lk(mu);
@@ -596,7 +597,7 @@ class Server {
       ct_request* r = batch[i]->req;
       const Forest& f = fs[i];
       BatchReq& br = s.req_host[i];
-      const uint32_t rpb = predict_rows_per_block(f.n_classes, f.n_features);
+      const uint32_t rpb = predict_rows_per_block(f.n_classes, f.n_features, r->n_rows);
       smem = std::max(smem, predict_tile_smem(rpb, f.n_classes, f.n_features));
       // small requests whose rows are staged whole read and answer host
       // memory directly when the device can address it
@@ -615,15 +616,20 @@ class Server {
       br.n_trees = f.n_trees;
       br.block0 = blocks;
       br.tiles = ceil_div(r->n_rows, rpb);
+      // many rows: groups by the request's tiles (a few rows are answered
+      // soonest by one group, unless the forest is larger than L2's share)
       br.group = f.group;
+      if (r->n_rows >= 1024 && f.n_classes <= cfg.max_classes)
+        br.group = predict_group_size(f.n_trees, f.n_nodes, f.fbits ? sizeof(ct_compact_node) : sizeof(ct_packed_node),
+                                      rpb, br.tiles);
       br.row0 = (uint32_t)roff;
       br.votes = nullptr;  // a single-group request votes directly and must not touch the table
-      if (f.group < f.n_trees) {
+      if (br.group < f.n_trees) {
         grouped = true;
         br.votes = s.votes_dev + voff;
         voff += (uint64_t)r->n_rows * f.n_classes;
       }
-      blocks += br.tiles * ceil_div(f.n_trees, f.group);
+      blocks += br.tiles * ceil_div(f.n_trees, br.group);
       if (s.direct[i]) {
         ++zero;
       } else {
