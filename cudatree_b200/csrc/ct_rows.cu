@@ -28,10 +28,10 @@
 //   k_row_subtree  subtrees of at most 32 rows, one warp each
 //
 // Measured on one B200 (ct_fit): 581,012 x 54 covtype-shaped rows, 100 trees
-// 62.5 -> 42.6 ms; 10,000 x 3,000 rows, 100 classes, 200 trees 202 -> 46.7 ms
+// 62.5 -> 30.6 ms; 10,000 x 3,000 rows, 100 classes, 200 trees 202 -> 30.6 ms
 // (the lists of 3,000 features were partitioned per level for 55 scanned); 200,003 x
-// 28 continuous columns, 50 trees 14.2 -> 8.0 ms; 1,797 x 64, 50 trees 1.44 ->
-// 0.67 ms.  What bounds each kernel stands at it.
+// 28 continuous columns, 50 trees 14.2 -> 5.3 ms; 1,797 x 64, 50 trees 1.44 ->
+// 0.63 ms.  What bounds each kernel stands at it.
 //
 // Rows of equal value may come in any order in a sorted list: no candidate
 // lies between them, and a candidate's class counts depend only on the set of
@@ -941,21 +941,44 @@ __global__ void __launch_bounds__(THREADS_PER_BLOCK, 8) k_row_warp(View v, Level
 }
 
 // ------------------------------------------------------------------------
-// Nodes of WARP_ROWS + 1 .. GROUP_ROWS rows: one CTA per (node, feature).  The
-// rows set their rank's bit in a bitmap over all ranks and count themselves in
-// their group of 128 ranks; a prefix over the groups and the set bits below a
-// row's own give its sorted position, where its value and label are stored.
-// Only the words a node touched are cleared after it, so an item costs its
-// rows and the groups, not the ranks.  Each warp then scans a run of the
-// sorted rows, from the class counts of the warps before it.  Bound by latency
-// (two CTAs per SM at covtype's 581,012 ranks, barriers between the phases); a
-// bitonic sort of the ranks in registers took 13.7 ms per 100 covtype-shaped
-// trees against 8.5 ms.
+// Nodes of WARP_ROWS + 1 .. GROUP_ROWS rows: one CTA per (node, feature) finds
+// its rows' sorted positions, stores their values and labels there, and each
+// warp scans a run of them from the class counts of the warps before it.
+//
+// By bitmap: the rows set their rank's bit in a bitmap over all ranks and count
+// themselves in their group of 128 ranks; a prefix over the groups and the set
+// bits below a row's own give its position.  Only the words a node touched are
+// cleared after it, so an item costs its rows and the groups, not the ranks.
+// By buckets: the rows count themselves in their bucket of 32 ranks (a byte
+// each); a prefix over the buckets gives every bucket's first position, where a
+// word, in the place of the sorted rows, holds the bits of its ranks.  One
+// phase more, but a third of the bitmap's memory, which the scan's tables then
+// share.  Both are bound by latency, so by the CTAs that an SM holds: at 581,012
+// ranks the bitmap leaves two CTAs of 8 warps, the buckets four (the smaller
+// nodes of 100 covtype-shaped trees: 3.7 -> 2.6 ms); the larger nodes' rows
+// themselves leave one CTA or two of 16, and there the bitmap is faster (5.1
+// against 5.8 ms) up to about 640,000 ranks (700,000 x 20 rows, 4 classes: 20.6
+// against 19.8 ms; from 930,000 on it does not fit), as it is for both while it
+// leaves four CTAs (10,000 x 3,000 rows, ct_fit: 29.9 against 31.6 ms).  A
+// bitonic sort of the ranks in registers took 13.7 ms against 8.5 of the
+// bitmaps.
+constexpr uint32_t BUCKET_RANKS = 200000;  // more ranks: less than four CTAs of 8 warps by bitmap
+constexpr uint32_t BUCKET_RANKS_LARGE = 640000;
 __host__ __device__ __forceinline__ uint32_t group_count_words(uint32_t n_rows) {  // two 16-bit counts per word
   return ((order_words(n_rows) / 4 + 7) / 8) * 4;
 }
+__host__ __device__ __forceinline__ uint32_t bucket_words(uint32_t n_rows) {  // a word per 4 buckets
+  return ((order_words(n_rows) / 4 + 3) / 4) * 4;
+}
+// The bytes of a word added up (at most 4 x 32).
+__device__ __forceinline__ uint32_t byte_sum(uint32_t w) {
+  const uint32_t t = (w & 0x00ff00ffu) + ((w >> 8) & 0x00ff00ffu);
+  return (t & 0xffffu) + (t >> 16);
+}
 // Shared memory, in words: (value bits, 8 x label or label | class total << 16)
-// by position, bitmap, group counts, the warps' class counts or seq tables.
+// by position; the bitmap, group counts and the warps' class counts or seq
+// tables; or the buckets' bytes and the prefix of every word of them (16 bits),
+// in whose place the tables come.
 // With up to SEQ_CLASSES classes a warp's run is padded for seq_scan.
 template <int W>
 __host__ __device__ __forceinline__ uint32_t group_rows_words() {
@@ -965,11 +988,18 @@ __host__ __device__ __forceinline__ uint32_t group_class_words(uint32_t n_classe
   return n_classes <= SEQ_CLASSES ? SEQ_WORDS : (n_classes + 3u) & ~3u;
 }
 template <int W>
+__host__ __device__ __forceinline__ bool group_by_buckets(uint32_t n_rows) {
+  return n_rows > (W == GROUP_SMALL_WARPS ? BUCKET_RANKS : BUCKET_RANKS_LARGE);
+}
+template <int W>
 __host__ __device__ __forceinline__ uint32_t group_words(uint32_t n_classes, uint32_t n_rows) {
-  return group_rows_words<W>() + order_words(n_rows) + group_count_words(n_rows) + W * group_class_words(n_classes);
+  const uint32_t tables = W * group_class_words(n_classes);
+  if (!group_by_buckets<W>(n_rows)) return group_rows_words<W>() + order_words(n_rows) + group_count_words(n_rows) + tables;
+  const uint32_t buckets = bucket_words(n_rows) / 2 * 3;
+  return group_rows_words<W>() + (buckets > tables ? buckets : tables);
 }
 
-template <bool Q, int W>
+template <bool Q, int W, bool BUCKETS>
 __device__ __forceinline__ void row_group_item(const View& vb, const StepLists& lists, const LevelScratch& s,
                                                uint32_t* smem, uint32_t n_max, RowBest* s_best, uint32_t* s_wsum,
                                                uint2 item) {
@@ -983,12 +1013,16 @@ __device__ __forceinline__ void row_group_item(const View& vb, const StepLists& 
   const uint2* pf = v.pair + (size_t)f * v.n_rows;
   const uint32_t* tot = lists.tot + (size_t)item.x * C;
   uint2* ent = reinterpret_cast<uint2*>(smem);
-  uint32_t* bm = smem + group_rows_words<W>();
+  uint32_t* bits = smem;  // by buckets: of a bucket's ranks, at its first position
+  uint32_t* bm = smem + group_rows_words<W>();  // the bitmap or the buckets
   uint32_t* gc = bm + order_words(n_max);
-  uint32_t* cls = gc + group_count_words(n_max);
+  uint32_t* cls = BUCKETS ? bm : gc + group_count_words(n_max);
   uint32_t* cnt = cls + warp * group_class_words(C);
   const bool seq = C <= SEQ_CLASSES;
-  const uint32_t units = group_count_words(v.n_rows) / 4;  // of 8 groups
+  // 16-byte units: of 16 buckets, or of 8 groups
+  const uint32_t units = (BUCKETS ? bucket_words(v.n_rows) : group_count_words(v.n_rows)) / 4;
+  uint4* unit = reinterpret_cast<uint4*>(BUCKETS ? bm : gc);
+  uint16_t* prefix = reinterpret_cast<uint16_t*>(bm + bucket_words(v.n_rows));
   // rows of one warp's run, and where position p is kept: runs of 32 << sh
   // rows padded for seq_scan, else runs without padding
   const uint32_t sh = seq_shift(ceil_div(n, (uint32_t)W));
@@ -998,7 +1032,9 @@ __device__ __forceinline__ void row_group_item(const View& vb, const StepLists& 
   float xv[K];
 #pragma unroll
   for (uint32_t k = 0; k < K; ++k) lb[k] = k * T + threadIdx.x < n ? rows[k * T + threadIdx.x] : 0u;
-  for (uint32_t g = threadIdx.x; g < units; g += T) reinterpret_cast<uint4*>(gc)[g] = make_uint4(0u, 0u, 0u, 0u);
+  for (uint32_t g = threadIdx.x; g < units; g += T) unit[g] = make_uint4(0u, 0u, 0u, 0u);
+  if (BUCKETS)
+    for (uint32_t i = threadIdx.x; i < n; i += T) bits[i] = 0u;
 #pragma unroll
   for (uint32_t k = 0; k < K; ++k) {
     rk[k] = 0;
@@ -1009,24 +1045,32 @@ __device__ __forceinline__ void row_group_item(const View& vb, const StepLists& 
       xv[k] = __uint_as_float(pr.y);
     }
   }
-  if (!seq)
+  if (!BUCKETS && !seq)
     for (uint32_t c = lane; c < C; c += 32) cnt[c] = 0;
   __syncthreads();
 #pragma unroll
   for (uint32_t k = 0; k < K; ++k)
     if (k * T + threadIdx.x < n) {
-      atomicOr(&bm[rk[k] >> 5], 1u << (rk[k] & 31));
-      atomicAdd(&gc[rk[k] >> 8], 1u << ((rk[k] >> 3) & 16));
+      if (BUCKETS) {
+        atomicAdd(&bm[rk[k] >> 7], 1u << ((rk[k] >> 2) & 24));
+      } else {
+        atomicOr(&bm[rk[k] >> 5], 1u << (rk[k] & 31));
+        atomicAdd(&gc[rk[k] >> 8], 1u << ((rk[k] >> 3) & 16));
+      }
     }
   __syncthreads();
-  // exclusive prefix of the groups' counts (at most 8,192: 16 bits)
+  // exclusive prefix of the counts by 128 ranks (at most 9,216: 16 bits)
   const uint32_t per_w = ceil_div(ceil_div(units, 32u), (uint32_t)W) * 32;
   const uint32_t ulo = min(warp * per_w, units), uhi = min(ulo + per_w, units);
   uint32_t sum = 0;
   for (uint32_t u = ulo + lane; u < uhi; u += 32) {
-    const uint4 q = reinterpret_cast<const uint4*>(gc)[u];
-    const uint32_t t = q.x + q.y + q.z + q.w;  // 16-bit fields: at most 512 each
-    sum += (t & 0xffffu) + (t >> 16);
+    const uint4 q = unit[u];
+    if (BUCKETS) {
+      sum += byte_sum(q.x) + byte_sum(q.y) + byte_sum(q.z) + byte_sum(q.w);
+    } else {
+      const uint32_t t = q.x + q.y + q.z + q.w;  // 16-bit fields: at most 512 each
+      sum += (t & 0xffffu) + (t >> 16);
+    }
   }
   sum = __reduce_add_sync(FULL, sum);
   if (lane == 0) s_wsum[warp] = sum;
@@ -1034,39 +1078,63 @@ __device__ __forceinline__ void row_group_item(const View& vb, const StepLists& 
   uint32_t run = __reduce_add_sync(FULL, lane < warp ? s_wsum[lane & (W - 1)] : 0u);
   for (uint32_t u0 = ulo; u0 < uhi; u0 += 32) {
     const uint32_t u = u0 + lane;
-    const uint4 q = u < uhi ? reinterpret_cast<const uint4*>(gc)[u] : make_uint4(0u, 0u, 0u, 0u);
-    const uint32_t t4 = q.x + q.y + q.z + q.w, t = (t4 & 0xffffu) + (t4 >> 16);
-    const uint32_t incl = (uint32_t)warp_incl_scan_i32((int32_t)t);
-    uint32_t b = run + incl - t;
-    uint4 o;
-    // each word holds the groups 2 i (low half) and 2 i + 1
-    o.x = b | ((b + (q.x & 0xffffu)) << 16);
-    b += (q.x & 0xffffu) + (q.x >> 16);
-    o.y = b | ((b + (q.y & 0xffffu)) << 16);
-    b += (q.y & 0xffffu) + (q.y >> 16);
-    o.z = b | ((b + (q.z & 0xffffu)) << 16);
-    b += (q.z & 0xffffu) + (q.z >> 16);
-    o.w = b | ((b + (q.w & 0xffffu)) << 16);
-    if (u < uhi) reinterpret_cast<uint4*>(gc)[u] = o;
+    const uint4 q = u < uhi ? unit[u] : make_uint4(0u, 0u, 0u, 0u);
+    uint32_t tx, ty, tz, tw;  // by word
+    if (BUCKETS) {
+      tx = byte_sum(q.x), ty = byte_sum(q.y), tz = byte_sum(q.z), tw = byte_sum(q.w);
+    } else {
+      tx = (q.x & 0xffffu) + (q.x >> 16), ty = (q.y & 0xffffu) + (q.y >> 16);
+      tz = (q.z & 0xffffu) + (q.z >> 16), tw = (q.w & 0xffffu) + (q.w >> 16);
+    }
+    const uint32_t t = tx + ty + tz + tw, incl = (uint32_t)warp_incl_scan_i32((int32_t)t);
+    const uint32_t b0 = run + incl - t, b1 = b0 + tx, b2 = b1 + ty, b3 = b2 + tz;
+    if (u < uhi) {
+      if (BUCKETS)
+        reinterpret_cast<uint2*>(prefix)[u] = make_uint2(b0 | (b1 << 16), b2 | (b3 << 16));
+      else  // each word holds the groups 2 i (low half) and 2 i + 1
+        unit[u] = make_uint4(b0 | ((b0 + (q.x & 0xffffu)) << 16), b1 | ((b1 + (q.y & 0xffffu)) << 16),
+                             b2 | ((b2 + (q.z & 0xffffu)) << 16), b3 | ((b3 + (q.w & 0xffffu)) << 16));
+    }
     run += __shfl_sync(FULL, incl, 31);
   }
   __syncthreads();
+  if (BUCKETS) {
+#pragma unroll
+    for (uint32_t k = 0; k < K; ++k)
+      if (k * T + threadIdx.x < n) {
+        const uint32_t r = rk[k], first = prefix[r >> 7] + byte_sum(bm[r >> 7] & ((1u << ((r >> 2) & 24)) - 1u));
+        atomicOr(&bits[first], 1u << (r & 31));
+        rk[k] = (first << 5) | (r & 31);
+      }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t k = 0; k < K; ++k)
+      if (k * T + threadIdx.x < n) rk[k] = (rk[k] >> 5) + __popc(bits[rk[k] >> 5] & ((1u << (rk[k] & 31)) - 1u));
+    if (!seq)  // every row is done with the buckets
+      for (uint32_t c = lane; c < C; c += 32) cnt[c] = 0;
+    __syncthreads();
+  }
 #pragma unroll
   for (uint32_t k = 0; k < K; ++k)
     if (k * T + threadIdx.x < n) {
-      const uint32_t r = rk[k], in = (r >> 5) & 3u, below = (1u << (r & 31)) - 1u;
-      const uint4 q = reinterpret_cast<const uint4*>(bm)[r >> 7];
-      const uint32_t pos = reinterpret_cast<const uint16_t*>(gc)[r >> 7] + __popc(q.x & (in > 0 ? FULL : below)) +
-                           __popc(q.y & (in > 1 ? FULL : in == 1 ? below : 0u)) +
-                           __popc(q.z & (in > 2 ? FULL : in == 2 ? below : 0u)) + __popc(q.w & (in == 3 ? below : 0u));
+      uint32_t pos = rk[k];
+      if (!BUCKETS) {
+        const uint32_t r = rk[k], in = (r >> 5) & 3u, below = (1u << (r & 31)) - 1u;
+        const uint4 q = reinterpret_cast<const uint4*>(bm)[r >> 7];
+        pos = reinterpret_cast<const uint16_t*>(gc)[r >> 7] + __popc(q.x & (in > 0 ? FULL : below)) +
+              __popc(q.y & (in > 1 ? FULL : in == 1 ? below : 0u)) +
+              __popc(q.z & (in > 2 ? FULL : in == 2 ? below : 0u)) + __popc(q.w & (in == 3 ? below : 0u));
+      }
       const uint32_t lab = lb[k] >> v.lab_shift;
       ent[at(pos)] = seq ? seq_entry(__float_as_uint(xv[k]), lab)
                          : make_uint2(__float_as_uint(xv[k]), lab | (__ldg(tot + lab) << 16));
     }
   __syncthreads();
+  if (!BUCKETS) {
 #pragma unroll
-  for (uint32_t k = 0; k < K; ++k)  // every row is placed: clear the words it touched
-    if (k * T + threadIdx.x < n) bm[rk[k] >> 5] = 0u;
+    for (uint32_t k = 0; k < K; ++k)  // every row is placed: clear the words it touched
+      if (k * T + threadIdx.x < n) bm[rk[k] >> 5] = 0u;
+  }
   // this warp's run of sorted rows
   const uint32_t w0 = min(warp * len, n), w1 = min(w0 + len, n);
   RowBest rb{dinf(), NONE, 0u, 0.f, 0.f};
@@ -1106,7 +1174,7 @@ __device__ __forceinline__ void row_group_item(const View& vb, const StepLists& 
       }
     }
     __syncthreads();
-    // sums of squares stay at or below 2^26 (at most 8,192 rows)
+    // sums of squares stay below 2^27 (at most 9,216 rows)
     uint32_t sl = 0, a = 0, st2 = 0;
     for (uint32_t c = lane; c < C; c += 32) {
       const uint32_t k = cnt[c], t = __ldg(tot + c);
@@ -1161,7 +1229,7 @@ __device__ __forceinline__ void row_group_item(const View& vb, const StepLists& 
   }
 }
 
-template <bool Q, int W>
+template <bool Q, int W, bool BUCKETS>
 __global__ void __launch_bounds__(W * 32, W == GROUP_SMALL_WARPS ? 4 : 2) k_row_group(View v, LevelScratch s, uint32_t n_max) {
   extern __shared__ __align__(16) uint32_t group_sm[];
   __shared__ RowBest s_best[W];
@@ -1173,11 +1241,13 @@ __global__ void __launch_bounds__(W * 32, W == GROUP_SMALL_WARPS ? 4 : 2) k_row_
   const StepLists sl = *s.step;
   uint32_t i = blockIdx.x;
   if (i >= count) return;
-  uint4* bm4 = reinterpret_cast<uint4*>(group_sm + group_rows_words<W>());
-  for (uint32_t g = threadIdx.x; g < order_words(n_max) / 4; g += W * 32) bm4[g] = make_uint4(0u, 0u, 0u, 0u);
+  if (!BUCKETS) {
+    uint4* bm4 = reinterpret_cast<uint4*>(group_sm + group_rows_words<W>());
+    for (uint32_t g = threadIdx.x; g < order_words(n_max) / 4; g += W * 32) bm4[g] = make_uint4(0u, 0u, 0u, 0u);
+  }
   while (i < count) {
     if (threadIdx.x == 0) s_item = gridDim.x + atomicAdd(claim, 1u);  // the next item, claimed ahead
-    row_group_item<Q, W>(v, sl, s, group_sm, n_max, s_best, s_wsum, list[i]);
+    row_group_item<Q, W, BUCKETS>(v, sl, s, group_sm, n_max, s_best, s_wsum, list[i]);
     __syncthreads();
     i = s_item;
     __syncthreads();
@@ -2294,7 +2364,7 @@ k_row_children(View v, LevelScratch s, TreeView tv, uint32_t cap_next, uint32_t 
 // keeps its best candidate over all features; one reduction at the end gives
 // the node's.  A virtual feature's values come from the rows' value bits, read
 // once per subtree.  Wide data (55 features per node): 11.6 ms per 200 trees
-// with one feature at a time -> 6.9 ms.
+// with one feature at a time -> 4.6 ms.
 struct RowSub {
   uint32_t mask;
   uint32_t raw;
@@ -2557,13 +2627,21 @@ int row_step(const View& v, const LevelScratch& s, LevelBounds b, uint32_t n_max
   }
   pf->begin(CT_K_SCAN);
   if (n_max > GROUP_SMALL_ROWS) {
-    CT_TRY(launch_bitmap(k_row_group<Q, GROUP_WARPS>, 32 * GROUP_WARPS,
-                         group_words<GROUP_WARPS>(C, n_max) * sizeof(uint32_t), s.cap_order, br[0], v, s, n_max));
+    const size_t smg = group_words<GROUP_WARPS>(C, n_max) * sizeof(uint32_t);
+    if (group_by_buckets<GROUP_WARPS>(n_max))
+      CT_TRY(launch_bitmap(k_row_group<Q, GROUP_WARPS, true>, 32 * GROUP_WARPS, smg, s.cap_order, br[0], v, s, n_max));
+    else
+      CT_TRY(launch_bitmap(k_row_group<Q, GROUP_WARPS, false>, 32 * GROUP_WARPS, smg, s.cap_order, br[0], v, s, n_max));
     pf->launched(CT_K_SCAN);
   }
   if (n_max > WARP_ROWS) {
-    CT_TRY(launch_bitmap(k_row_group<Q, GROUP_SMALL_WARPS>, 32 * GROUP_SMALL_WARPS,
-                         group_words<GROUP_SMALL_WARPS>(C, n_max) * sizeof(uint32_t), s.cap_order, br[1], v, s, n_max));
+    const size_t smg = group_words<GROUP_SMALL_WARPS>(C, n_max) * sizeof(uint32_t);
+    if (group_by_buckets<GROUP_SMALL_WARPS>(n_max))
+      CT_TRY(launch_bitmap(k_row_group<Q, GROUP_SMALL_WARPS, true>, 32 * GROUP_SMALL_WARPS, smg, s.cap_order, br[1], v, s,
+                           n_max));
+    else
+      CT_TRY(launch_bitmap(k_row_group<Q, GROUP_SMALL_WARPS, false>, 32 * GROUP_SMALL_WARPS, smg, s.cap_order, br[1], v,
+                           s, n_max));
     pf->launched(CT_K_SCAN);
   }
   k_row_warp<Q><<<grid_for(k_row_warp<Q>, s.cap_w, smw, true), THREADS_PER_BLOCK, smw, br[2]>>>(v, s);
@@ -2637,9 +2715,25 @@ uint32_t rows_planes_in_lists(const ct_problem* p) {
   return 2 * k >= rows_planes_needed(p) ? k : 0u;
 }
 
+// Tables on which list growth is the faster of the two: row-list growth sorts
+// each selected feature anew, in shared memory that holds fewer items at once
+// the more rows there are, so with many rows, many classes (a scan by class
+// match) and a good part of the features selected it loses.  ct_fit and the
+// read-back of 8 trees, lists / rows: 700,000 x 20, 20 classes, 10 selected 30 /
+// 46 ms; 8 classes, 20 selected 39 / 52; 950,000 x 20, 20 classes, 5 selected 31 /
+// 42; 450,000 x 20, 20 classes, 20 selected 30 / 34; but 560,000 x 20, 20 classes,
+// 5 selected 22 / 17; 700,000 x 20, 4 classes, 10 selected 23 / 21; 581,012 x 54
+// covtype-shaped, all selected 32 / 19.
+static bool rows_slower(const ct_problem* p) {
+  const uint64_t m = std::min(p->max_features, p->n_features), F = p->n_features;
+  return (p->n_rows > 600000 && p->n_classes >= SEQ_CLASSES && 8 * m >= F) ||
+         (p->n_rows > 400000 && p->n_classes > SEQ_CLASSES && 2 * m >= F);
+}
+
 // A row id and a label share 32 bits, the row list fits a list buffer, and the
 // rank bitmap fits shared memory.
 bool rows_possible(const ct_problem* p) {
+  if (rows_slower(p)) return false;
   const uint32_t row_bits = p->n_rows > 1 ? 32u - (uint32_t)__builtin_clz(p->n_rows - 1) : 1u;
   const uint32_t lab_bits = p->n_classes > 1 ? 32u - (uint32_t)__builtin_clz(p->n_classes - 1) : 0u;
   return row_bits + lab_bits <= 32 && row_bits <= 22 && (uint64_t)p->n_features * p->index_bytes >= 4 &&

@@ -58,15 +58,18 @@ def test_options_match_oracle(cuda_device, kw, virtual):
     _assert_same_trees(forest._trees, ref.trees)
 
 
-@pytest.mark.parametrize("n,few", [(300000, 12000), (700000, 9800)])
+@pytest.mark.parametrize("n,few", [(300000, 12000), (590000, 9219), (700000, 9800)])
 @pytest.mark.parametrize("c", [2, 6, 8, 9])
 def test_crowded_runs_of_ranks_match_oracle(cuda_device, n, few, c):
     """The first split leaves a node of `few` rows that are neighbours in two
-    columns: one run of ranks holds them all (the larger share of rows), or the
-    node is too sparse for a bitmap (the smaller)."""
+    columns: one run of ranks holds them all (the first size), or the node is
+    too sparse for a bitmap (the others; at the last, 8 and 9 classes take
+    list growth).  Its descendants pass every size class with the sorts that
+    many ranks take."""
     rng = np.random.default_rng(n + c)
     u = rng.permutation(n).astype(np.float32)
-    x = np.stack([u, u + rng.normal(size=n).astype(np.float32), rng.normal(size=n).astype(np.float32)], axis=1)
+    x = np.stack([u, u + rng.normal(size=n).astype(np.float32), rng.normal(size=n).astype(np.float32)]
+                 + [np.ones(n, np.float32)] * 5, axis=1)
     y = np.where(u < few, (x[:, 2] * 3 + rng.integers(0, 2, size=n) + (u > few / 3)).astype(np.int64) % c, 0)
     kw = dict(n_estimators=1, bootstrap=False, seed=c, max_features=3)
     forest = RandomForestClassifier(**kw).fit(x, y)
