@@ -27,16 +27,19 @@ namespace ct {
 namespace {
 
 constexpr int PRED_THREADS = 256;
-// Walks in flight per thread.  4 at 6 blocks per SM against 8 at 4 blocks: fewer
-// trees in flight, whose nodes stay in L1 longer.  500 covtype-shaped trees
-// (37 MB of nodes), 65,536 rows, in groups of one round of walks each: 4 walks
-// 1.64 ms, 8 walks 1.82, 2 walks (8 blocks) 1.82.
+// Walks in flight per thread: 4 at 6 blocks per SM where a group is one round of
+// them, else 8 at 4 blocks.  Fewer trees in flight, whose nodes stay in L1
+// longer, but more rounds: 500 covtype-shaped trees (37 MB of nodes), 65,536
+// rows, in groups of 32: 4 walks 1.64 ms, 8 walks 1.82, 2 walks (8 blocks) 1.82;
+// all trees in one group: 3.29, 3.00 and 3.7 ms.
 constexpr int PRED_ILP = 4;
+constexpr int PRED_ILP_LONG = 8;
+constexpr int pred_blocks(int ilp) { return ilp == PRED_ILP ? 6 : 4; }
+__host__ __device__ __forceinline__ uint32_t walk_round(uint32_t rpb) { return PRED_THREADS / rpb * PRED_ILP; }
 constexpr uint32_t X_SMEM_BYTES = 32 * 1024;     // rows of x staged per block when they fit
 constexpr uint32_t HIST_SMEM_BYTES = 64 * 1024;  // vote histogram [rows][classes]
 constexpr size_t GROUP_L2_BYTES = 32ull << 20;   // node bytes of one tree group, at the most
 constexpr size_t GROUP_L1_BYTES = 192ull << 10;  // node bytes of one round of walks from which groups are single rounds
-constexpr uint32_t PRED_BLOCKS_PER_SM = 6;
 
 __host__ __device__ __forceinline__ bool predict_rows_staged(uint32_t rpb, uint32_t n_features) {
   return (size_t)rpb * n_features * sizeof(float) <= X_SMEM_BYTES;
@@ -79,9 +82,9 @@ struct CompactForm {
 // Walks are numbered w = t * rpb + row (row-fastest); rpb is a power of two
 // dividing blockDim.x, so a thread's row is fixed (threadIdx.x % rpb) and its
 // tree index advances by blockDim.x / rpb per walk.  Each thread keeps
-// PRED_ILP walks in flight; their node loads are issued together, then each
+// ILP walks in flight; their node loads are issued together, then each
 // walk steps or, at a leaf, votes and starts the thread's next tree.
-template <typename Form>
+template <typename Form, int ILP>
 __device__ __forceinline__ void walk_tile(const void* __restrict__ nodes, const uint32_t* __restrict__ tree_off,
                                           uint32_t t_lo, uint32_t n_t, uint32_t fbits, const float* x,
                                           uint32_t row_stride, uint32_t feat_stride, uint32_t rows, uint32_t rpb,
@@ -92,9 +95,9 @@ __device__ __forceinline__ void walk_tile(const void* __restrict__ nodes, const 
   const float* xr = x + (size_t)r * row_stride;
   uint32_t* hr = hist + r * n_classes;
   uint32_t t_next = threadIdx.x / rpb;
-  uint32_t base[PRED_ILP], pos[PRED_ILP];  // pos: absolute node index, NONE when the slot is idle
+  uint32_t base[ILP], pos[ILP];  // pos: absolute node index, NONE when the slot is idle
 #pragma unroll
-  for (int k = 0; k < PRED_ILP; ++k) {
+  for (int k = 0; k < ILP; ++k) {
     pos[k] = NONE;
     base[k] = 0;
     if (t_next < n_t) {
@@ -105,13 +108,13 @@ __device__ __forceinline__ void walk_tile(const void* __restrict__ nodes, const 
   }
   bool any = pos[0] != NONE;
   while (any) {
-    typename Form::Raw nd[PRED_ILP];
+    typename Form::Raw nd[ILP];
 #pragma unroll
-    for (int k = 0; k < PRED_ILP; ++k)
+    for (int k = 0; k < ILP; ++k)
       if (pos[k] != NONE) nd[k] = Form::load(nodes, pos[k]);
     any = false;
 #pragma unroll
-    for (int k = 0; k < PRED_ILP; ++k) {
+    for (int k = 0; k < ILP; ++k) {
       if (pos[k] == NONE) continue;
       any = true;
       if (Form::inner(nd[k])) {
@@ -167,7 +170,7 @@ __device__ __forceinline__ void stage_rows(const float* x, uint32_t rows, uint32
 
 // One tile of one tree group: walk, then either vote (single group) or add
 // the histogram into the global vote table.
-template <typename Form>
+template <typename Form, int ILP>
 __device__ __forceinline__ void tile_work(const void* nodes, const uint32_t* tree_off, uint32_t fbits, uint32_t t_lo,
                                           uint32_t n_t, bool single_group, const float* x, uint32_t n_rows,
                                           uint32_t n_features, uint32_t n_classes, uint32_t rpb, uint32_t row0,
@@ -180,9 +183,9 @@ __device__ __forceinline__ void tile_work(const void* nodes, const uint32_t* tre
   if (fits) stage_rows(x + (size_t)row0 * n_features, rows, rpb, n_features, xs);
   __syncthreads();
   if (fits)
-    walk_tile<Form>(nodes, tree_off, t_lo, n_t, fbits, xs, 1, rpb, rows, rpb, n_classes, hist);
+    walk_tile<Form, ILP>(nodes, tree_off, t_lo, n_t, fbits, xs, 1, rpb, rows, rpb, n_classes, hist);
   else
-    walk_tile<Form>(nodes, tree_off, t_lo, n_t, fbits, x + (size_t)row0 * n_features, n_features, 1, rows, rpb,
+    walk_tile<Form, ILP>(nodes, tree_off, t_lo, n_t, fbits, x + (size_t)row0 * n_features, n_features, 1, rows, rpb,
                     n_classes, hist);
   __syncthreads();
   if (single_group) {
@@ -198,15 +201,15 @@ __device__ __forceinline__ void tile_work(const void* nodes, const uint32_t* tre
   }
 }
 
-template <typename Form>
-__global__ void __launch_bounds__(PRED_THREADS, PRED_BLOCKS_PER_SM)
+template <typename Form, int ILP>
+__global__ void __launch_bounds__(PRED_THREADS, pred_blocks(ILP))
 k_predict(const void* __restrict__ nodes, const uint32_t* __restrict__ tree_off, uint32_t n_trees, uint32_t fbits,
           uint32_t group, uint32_t tiles, const float* __restrict__ x, uint32_t n_rows, uint32_t n_features,
           uint32_t n_classes, uint32_t rpb, uint32_t* __restrict__ votes, uint32_t* __restrict__ pred) {
   extern __shared__ uint32_t smem[];
   const uint32_t g = blockIdx.x / tiles, tile = blockIdx.x - g * tiles;  // group-major
   const uint32_t t_lo = g * group;
-  tile_work<Form>(nodes, tree_off, fbits, t_lo, min(group, n_trees - t_lo), group >= n_trees, x, n_rows, n_features,
+  tile_work<Form, ILP>(nodes, tree_off, fbits, t_lo, min(group, n_trees - t_lo), group >= n_trees, x, n_rows, n_features,
                   n_classes, rpb, tile * rpb, votes, pred, smem);
 }
 
@@ -338,13 +341,15 @@ uint32_t predict_group_size(uint32_t n_trees, uint64_t n_nodes, size_t node_byte
 // 100 trees of 24 KB: 96 us as one group, 61 of 32, 58 of 16; but 20,000 rows of
 // 20 small trees 53 us as one, 60 as two.
 uint32_t predict_group_size(uint32_t n_trees, uint64_t n_nodes, size_t node_bytes, uint32_t rpb, uint32_t tiles) {
-  const uint32_t columns = PRED_THREADS / rpb, round = columns * PRED_ILP;
+  const uint32_t columns = PRED_THREADS / rpb, round = walk_round(rpb);
   uint32_t g = predict_group_size(n_trees, n_nodes, node_bytes);
   if (n_nodes * node_bytes / n_trees * round > GROUP_L1_BYTES && n_trees >= round + round / 2) g = std::min(g, round);
-  const uint32_t fill = ceil_div(148u * PRED_BLOCKS_PER_SM, tiles);
+  const uint32_t fill = ceil_div(148u * (uint32_t)pred_blocks(PRED_ILP), tiles);
   if (fill > 1 && n_trees > round) g = std::min(g, std::max(ceil_div(n_trees, fill), 2 * columns));
   return ceil_div(n_trees, ceil_div(n_trees, g));
 }
+
+bool predict_one_round(uint32_t rpb, uint32_t group) { return group <= walk_round(rpb); }
 
 uint32_t compact_feature_bits(uint32_t n_features) {
   uint32_t b = 1;
@@ -406,7 +411,8 @@ int compact_forest(const ct_packed_node* nodes, uint32_t n_nodes, uint32_t n_fea
   return CT_OK;
 }
 
-__global__ void __launch_bounds__(PRED_THREADS, PRED_BLOCKS_PER_SM)
+template <int ILP>
+__global__ void __launch_bounds__(PRED_THREADS, pred_blocks(ILP))
 k_predict_batch(const BatchReq* __restrict__ reqs, uint32_t n_req) {
   extern __shared__ uint32_t smem[];
   uint32_t lo = 0, hi = n_req;  // the last request whose first block is <= blockIdx.x
@@ -421,10 +427,10 @@ k_predict_batch(const BatchReq* __restrict__ reqs, uint32_t n_req) {
   const uint32_t n_t = min(rq.group, rq.n_trees - t_lo);
   const uint32_t rpb = rq.rpb;
   if (rq.fbits)
-    tile_work<CompactForm>(rq.nodes, rq.tree_off, rq.fbits, t_lo, n_t, rq.group >= rq.n_trees, rq.x, rq.n_rows,
+    tile_work<CompactForm, ILP>(rq.nodes, rq.tree_off, rq.fbits, t_lo, n_t, rq.group >= rq.n_trees, rq.x, rq.n_rows,
                            rq.n_features, rq.n_classes, rpb, tile * rpb, rq.votes, rq.pred, smem);
   else
-    tile_work<PackedForm>(rq.nodes, rq.tree_off, 0, t_lo, n_t, rq.group >= rq.n_trees, rq.x, rq.n_rows,
+    tile_work<PackedForm, ILP>(rq.nodes, rq.tree_off, 0, t_lo, n_t, rq.group >= rq.n_trees, rq.x, rq.n_rows,
                           rq.n_features, rq.n_classes, rpb, tile * rpb, rq.votes, rq.pred, smem);
 }
 
@@ -445,11 +451,15 @@ __global__ void k_vote_batch(const BatchReq* __restrict__ reqs, uint32_t n_req, 
 }
 
 int predict_batch(const BatchReq* reqs_dev, uint32_t n_req, uint32_t total_blocks, uint32_t total_rows,
-                  size_t smem, bool any_grouped, cudaStream_t st) {
+                  size_t smem, bool any_grouped, bool one_round, cudaStream_t st) {
   if (n_req == 0 || total_blocks == 0) return CT_OK;
   CT_ARG_CHECK(smem <= HIST_SMEM_BYTES + X_SMEM_BYTES, "predict batch: tile shared memory too large");
-  CT_TRY(allow_smem(k_predict_batch, (int)(HIST_SMEM_BYTES + X_SMEM_BYTES)));
-  k_predict_batch<<<total_blocks, PRED_THREADS, smem, st>>>(reqs_dev, n_req);
+  auto launch = [&](auto kernel) -> int {
+    CT_TRY(allow_smem(kernel, (int)(HIST_SMEM_BYTES + X_SMEM_BYTES)));
+    kernel<<<total_blocks, PRED_THREADS, smem, st>>>(reqs_dev, n_req);
+    return CT_OK;
+  };
+  CT_TRY(one_round ? launch(k_predict_batch<PRED_ILP>) : launch(k_predict_batch<PRED_ILP_LONG>));
   if (any_grouped) k_vote_batch<<<ceil_div(total_rows, 8), 256, 0, st>>>(reqs_dev, n_req, total_rows);
   CT_CUDA_TRY(cudaGetLastError());
   return CT_OK;
@@ -476,21 +486,24 @@ int predict(const void* nodes, uint32_t n_nodes, uint32_t fbits, const uint32_t*
   // Few rows are worth the table's zeroing and the votes' own launch from two
   // rounds of walks on: a call with 40 rows and 500 trees 344 -> 155 us.
   uint32_t group = n_trees;
-  if (votes && n_trees >= (n_rows >= 1024 ? 16u : 2u * PRED_ILP * (PRED_THREADS / rpb)))
+  if (votes && n_trees >= (n_rows >= 1024 ? 16u : 2u * walk_round(rpb)))
     group = predict_group_size(n_trees, n_nodes, fbits ? CompactForm::BYTES : PackedForm::BYTES, rpb, tiles);
   const uint32_t groups = ceil_div(n_trees, group);
   const size_t smem = predict_tile_smem(rpb, n_classes, n_features);
   if (groups > 1) CT_CUDA_TRY(cudaMemsetAsync(votes, 0, (size_t)n_rows * n_classes * sizeof(uint32_t), st));
   const int most = (int)(HIST_SMEM_BYTES + X_SMEM_BYTES);
-  if (fbits) {
-    CT_TRY(allow_smem(k_predict<CompactForm>, most));
-    k_predict<CompactForm><<<tiles * groups, PRED_THREADS, smem, st>>>(
-        nodes, tree_off, n_trees, fbits, group, tiles, x, n_rows, n_features, n_classes, rpb, votes, pred);
-  } else {
-    CT_TRY(allow_smem(k_predict<PackedForm>, most));
-    k_predict<PackedForm><<<tiles * groups, PRED_THREADS, smem, st>>>(
-        nodes, tree_off, n_trees, 0, group, tiles, x, n_rows, n_features, n_classes, rpb, votes, pred);
-  }
+  auto launch = [&](auto kernel) -> int {
+    CT_TRY(allow_smem(kernel, most));
+    kernel<<<tiles * groups, PRED_THREADS, smem, st>>>(nodes, tree_off, n_trees, fbits, group, tiles, x, n_rows,
+                                                       n_features, n_classes, rpb, votes, pred);
+    return CT_OK;
+  };
+  // (short walks in trees that fit L1: 100 trees of 0.9 KB, 65,536 rows, 124 us with 4, 138 with 8)
+  const bool one_round =
+      predict_one_round(rpb, group) ||
+      (uint64_t)n_nodes * (fbits ? CompactForm::BYTES : PackedForm::BYTES) / n_trees * walk_round(rpb) <= GROUP_L1_BYTES;
+  if (fbits) CT_TRY(one_round ? launch(k_predict<CompactForm, PRED_ILP>) : launch(k_predict<CompactForm, PRED_ILP_LONG>));
+  else CT_TRY(one_round ? launch(k_predict<PackedForm, PRED_ILP>) : launch(k_predict<PackedForm, PRED_ILP_LONG>));
   if (groups > 1) k_vote_rows<<<ceil_div(n_rows, 8), 256, 0, st>>>(votes, n_rows, n_classes, pred);
   CT_CUDA_TRY(cudaGetLastError());
   return CT_OK;

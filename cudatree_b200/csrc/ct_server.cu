@@ -569,7 +569,7 @@ class Server {
     uint64_t xoff = 0, roff = 0, voff = 0, zero = 0;
     size_t smem = 0;
     uint32_t blocks = 0, max_c = 1;
-    bool grouped = false;
+    bool grouped = false, one_round = true;
     std::vector<Forest> fs;
     {
       // a forest removed after the request was queued: the request fails;
@@ -617,9 +617,10 @@ class Server {
       br.block0 = blocks;
       br.tiles = ceil_div(r->n_rows, rpb);
       // many rows: groups by the request's tiles (a few rows are answered
-      // soonest by one group, unless the forest is larger than L2's share)
+      // soonest by one group, unless the forest is larger than L2's share; rows
+      // in host memory would cross the link once per group)
       br.group = f.group;
-      if (r->n_rows >= 1024 && f.n_classes <= cfg.max_classes)
+      if (!s.direct[i] && r->n_rows >= 1024 && f.n_classes <= cfg.max_classes)
         br.group = predict_group_size(f.n_trees, f.n_nodes, f.fbits ? sizeof(ct_compact_node) : sizeof(ct_packed_node),
                                       rpb, br.tiles);
       br.row0 = (uint32_t)roff;
@@ -629,6 +630,7 @@ class Server {
         br.votes = s.votes_dev + voff;
         voff += (uint64_t)r->n_rows * f.n_classes;
       }
+      one_round = one_round && predict_one_round(rpb, std::min(br.group, f.n_trees));
       blocks += br.tiles * ceil_div(f.n_trees, br.group);
       if (s.direct[i]) {
         ++zero;
@@ -644,7 +646,7 @@ class Server {
     if (cudaMemcpyAsync(s.req_dev, s.req_host, batch.size() * sizeof(BatchReq), cudaMemcpyHostToDevice, ln.st) !=
         cudaSuccess)
       err = 1;
-    if (predict_batch(s.req_dev, (uint32_t)batch.size(), blocks, (uint32_t)roff, smem, grouped, ln.st) != CT_OK)
+    if (predict_batch(s.req_dev, (uint32_t)batch.size(), blocks, (uint32_t)roff, smem, grouped, one_round, ln.st) != CT_OK)
       err = 1;
     for (size_t i = 0; i < batch.size(); ++i) {
       ct_request* r = batch[i]->req;
