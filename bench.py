@@ -34,11 +34,6 @@ WORKLOAD = ("covtype-shaped synthetic 581012x54 f32 (10 Gaussian + 44 one-hot), 
             "100 trees, bootstrap, max_features=7, uint32 indices, fully grown")
 N_TREES = 100
 MAX_FEATURES = 7
-# DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) per
-# algorithmic byte of the partition and the split-scan kernel groups, over
-# every launch of one profiled 16-tree fit of this workload
-PARTITION_DRAM_PER_ALGORITHMIC_BYTE = 0.71
-SCAN_DRAM_PER_ALGORITHMIC_BYTE = 1.00
 
 
 def peaks():
@@ -528,17 +523,11 @@ def run_ours(args, world, rank, local):
     pi = groups.index("partition")
     p_ms = stats["ms"][pi]
     p_gbs = stats["bytes"][pi] / (p_ms * 1e6) if p_ms > 0 else None
-    # DRAM bytes per partition launch: the algorithmic bytes per launch times
-    # the DRAM/algorithmic ratio ncu measured on the 16-tree case of this
-    # workload (dram__bytes_read.sum + dram__bytes_write.sum of the partition
-    # launches of that capture)
     p_launches = stats["launches"][pi]
-    traffic = (PARTITION_DRAM_PER_ALGORITHMIC_BYTE * stats["bytes"][pi] / p_launches) if p_launches else None
     si = groups.index("scan")
     s_ms = stats["ms"][si]
     s_gbs = stats["bytes"][si] / (s_ms * 1e6) if s_ms > 0 else None
     s_launches = stats["launches"][si]
-    s_traffic = (SCAN_DRAM_PER_ALGORITHMIC_BYTE * stats["bytes"][si] / s_launches) if s_launches else None
     cpu = None
     if not args.skip_cpu:
         cores = len(os.sched_getaffinity(0))
@@ -551,7 +540,7 @@ def run_ours(args, world, rank, local):
         "warmup": args.warmup, "ms_per_step": job_s * 1000, "higher_is_better": False, "scaling": "weak",
         "vs_baseline": None, "dtype": "u32 indices, int64 counts, f64 impurity", "data": "synthetic",
         "config": {"workload": WORKLOAD, "form": "batched level-synchronous, all 100 trees in flight",
-                   "l2": "inputs larger than L2 (per-tree index lists 2x54x581012x4 B = 251 MB)",
+                   "l2": "inputs larger than L2 (row lists of 100 trees, 2x581012x4 B each = 465 MB)",
                    "parallelism": f"replicas x{world}"},
         "plain_fit_s": plain_s, "batched_speedup_vs_plain": (plain_s / step_s) if plain_s else None,
         "plain_trees_identical": same if plain_s else None,
@@ -559,18 +548,17 @@ def run_ours(args, world, rank, local):
         "fit_options": ({k: v for k, v in forest._tuned.items() if k != "sample_ms"} if forest._tuned else "defaults"),
         "autotune_s": tune_s,
         "kernels": kernels,
-        "roofline": {"bound": "hbm", "kernel": "k_partition", "achieved": round(p_gbs, 1) if p_gbs else None,
+        "roofline": {"bound": "hbm", "kernel": "k_row_bits + k_row_order + k_row_move (rank bitmaps, sorted lists, row-list split)", "achieved": round(p_gbs, 1) if p_gbs else None,
                      "peak": peak, "unit": "GB/s", "frac": round(p_gbs / peak, 4) if p_gbs else None,
-                     "peak_kind": peak_kind, "traffic": round(traffic) if traffic else None,
-                     "traffic_unit": f"DRAM bytes per launch (ncu ratio {PARTITION_DRAM_PER_ALGORITHMIC_BYTE} x algorithmic, 16-tree capture)",
+                     "peak_kind": peak_kind, "traffic": None,
+                     "traffic_unit": "DRAM bytes per launch (not captured for these kernels)",
                      "algorithmic_bytes_per_launch": round(stats["bytes"][pi] / p_launches) if p_launches else None,
-                     "algorithmic_bytes_per_element": "n_features x (2 x index_bytes + 1)"},
-        "scan_roofline": {"bound": "hbm", "kernel": "k_split_scan (+hist, carry, two-valued, virtual counts)",
+                     "algorithmic_bytes_per_element": "per (node above 9,216 rows, selected feature, row): 2 x index_bytes + 1"},
+        "scan_roofline": {"bound": "hbm", "kernel": "k_row_scan_seq, k_row_group, k_row_warp (+limit, bound, carry, virtual counts)",
                           "achieved": round(s_gbs, 1) if s_gbs else None, "peak": peak, "unit": "GB/s",
                           "frac": round(s_gbs / peak, 4) if s_gbs else None, "peak_kind": peak_kind,
-                          "traffic": round(s_traffic) if s_traffic else None,
-                          "traffic_unit": f"DRAM bytes per launch (ncu ratio {SCAN_DRAM_PER_ALGORITHMIC_BYTE} x "
-                                          f"algorithmic, 16-tree capture)",
+                          "traffic": None,
+                          "traffic_unit": "DRAM bytes per launch (not captured for these kernels)",
                           "algorithmic_bytes_per_launch": round(stats["bytes"][si] / s_launches) if s_launches else None,
                           "algorithmic_bytes_per_element": "per (node, selected feature, position): index_bytes "
                                                            "+ 4 (x gather) + label gather when labels are not packed"},

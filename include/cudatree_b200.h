@@ -119,7 +119,8 @@ typedef struct ct_fit_options {
   uint32_t bfs_threshold;   /* plain: nodes with n <= this go to the BFS queue
                                (random_tree.py:616-622); 0 = reference formula     */
   uint32_t subtree_cutoff;  /* nodes with n <= this are grown whole by one warp
-                               (<= 128; 0 disables); the trees do not change        */
+                               (<= 128; 0 disables; row-list growth: more than 32
+                               acts as 32); the trees do not change                 */
   uint32_t scan_piece;      /* elements per split-scan work item (0 = default)      */
   uint32_t flags;           /* CT_FIT_PROFILE | CT_FIT_HOST_LOOP                    */
   uint32_t step_nodes;      /* nodes per level step (0 = 2^20): a wider level takes
@@ -127,6 +128,8 @@ typedef struct ct_fit_options {
   uint32_t graph_samples;   /* batched: levels of at most this many samples run in
                                the loop graph, larger ones from the host (0 or
                                0xffffffff = every level in the graph)               */
+                            /* The next three steer list growth (see ct_fit) only;
+                               row-list growth takes them and has no use for them   */
   uint32_t part_shape;      /* partition of big segments: CT_PART_* (0 = default)   */
   uint32_t huge_rows;       /* nodes of at least this many rows partition with the
                                tree's mark bits in shared memory (0 = 4096, at
@@ -225,7 +228,17 @@ int ct_partition_nodes(const ct_problem* p, const ct_lists* lists, const ct_node
  * `trees` (replaces RandomForestClassifier.fit's tree loop + RandomClassifierTree.fit,
  * random_forest.py:292-336, random_tree.py:461-676).  Lists must hold n_trees slots
  * (one for CT_FIT_PLAIN); they are the fit's scratch, and while it runs their
- * entries may carry each row's label above its row id. */
+ * entries may carry each row's label above its row id.
+ * The batched form has two ways of growing, which give the same trees.  List
+ * growth keeps every feature's sorted list per node, as the per-node entry
+ * points do.  Row-list growth keeps one list of rows per tree (at the start of
+ * each list buffer; sorted orders of large nodes behind it or in the
+ * workspace) and sorts a node's rows only for the features it selects; it is
+ * taken when a row id and a label fit 32 bits, si0 and si1 are 16-byte aligned,
+ * the tables of its kernels fit shared memory (up to about 1.1 million rows),
+ * the workspace holds its scratch, and it is not the slower one.
+ * ct_fit_workspace_size gives the larger of the two sizes; a workspace that
+ * only list growth fits is accepted and used for that. */
 int ct_fit_workspace_size(const ct_problem* p, uint32_t n_trees, const ct_fit_options* opt,
                           size_t* bytes);
 int ct_fit(const ct_problem* p, const ct_lists* lists, uint32_t first_tree, uint32_t n_trees,
@@ -306,9 +319,11 @@ int ct_transpose_rows(const float* x_rm, uint32_t n_rows, uint32_t n_cols, float
 /* Reads back the trees of one ct_fit call in canonical order.  counts[t]
  * (host) is trees->n_nodes[t]; tree t lands at [o_t, o_t + counts[t]) of the
  * host output arrays, o_t = counts[0] + ... + counts[t-1].  The used nodes
- * are gathered on the device into scratch (ct_fetch_trees_scratch bytes),
- * copied in one transfer, and renumbered on host threads.  Replaces the
- * full-buffer readback of decorate (random_tree.py:50-63). */
+ * are numbered breadth-first and gathered on the device into scratch
+ * (ct_fetch_trees_scratch bytes) and copied column by column, each column's
+ * transfer beside the next one's copy out of the staging buffer.  Less scratch
+ * (a gather's) and trees deeper than 4,096 levels are numbered on host threads
+ * instead.  Replaces the full-buffer readback of decorate (random_tree.py:50-63). */
 size_t ct_fetch_trees_scratch(uint64_t total_nodes, uint32_t n_trees);
 int ct_fetch_trees(const ct_tree_buffers* trees, uint32_t n_trees, const uint32_t* counts,
                    void* scratch, size_t scratch_bytes, uint32_t* out_left, uint32_t* out_right,
