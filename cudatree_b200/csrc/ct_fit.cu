@@ -764,9 +764,10 @@ View fit_view(const ct_problem* p, const ct_lists* l, const FitLayout& L) {
 }
 
 // The view of row-list growth: 32-bit row lists at the front of the caller's
-// list buffers, the sorted planes behind them (or in the workspace).
-View row_view(const ct_problem* p, const ct_lists* l, const FitLayout& L, uint2* pair, uint2* ranked,
-              uint32_t* rank, uint2* planes) {
+// list buffers, the sorted planes behind them (or in the workspace, where they
+// have the n_trees slots and n_rows entries that it was sized for).
+View row_view(const ct_problem* p, const ct_lists* l, uint32_t n_trees, const FitLayout& L, uint2* pair,
+              uint2* ranked, uint32_t* rank, uint2* planes) {
   View v = make_view(p, l);
   v.lab_shift = p->n_rows > 1 ? 32u - (uint32_t)__builtin_clz(p->n_rows - 1) : 1u;
   v.row_mask = (1u << v.lab_shift) - 1u;
@@ -778,6 +779,8 @@ View row_view(const ct_problem* p, const ct_lists* l, const FitLayout& L, uint2*
   v.rank = rank;
   const size_t off = ((size_t)l->n_slots * l->stride * sizeof(uint32_t) + 15) & ~size_t(15);
   v.planes0 = planes ? rows_planes_needed(p) : rows_planes_in_lists(p);
+  v.sorted_slots = planes ? n_trees : l->n_slots;
+  v.sorted_stride = planes ? p->n_rows : l->stride;
   v.sorted0 = planes ? planes : reinterpret_cast<uint2*>(reinterpret_cast<char*>(l->si0) + off);
   v.sorted1 = planes ? planes : reinterpret_cast<uint2*>(reinterpret_cast<char*>(l->si1) + off);
   return v;
@@ -869,7 +872,7 @@ int grow_levels(const ct_problem* p, const View& v, const FitLayout& L, const Tr
 int fit_batched(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uint32_t n_trees,
                 const FitLayout& L0, const ct_tree_buffers* trees, cudaStream_t st) {
   FitLayout L = L0;
-  View v = L.rows ? row_view(p, l, L, L.pair, L.ranked, L.rank, L.planes) : fit_view(p, l, L);
+  View v = L.rows ? row_view(p, l, n_trees, L, L.pair, L.ranked, L.rank, L.planes) : fit_view(p, l, L);
   TreeView tv = tree_view(trees, 0);
   CT_TRY(prepare_features(p, &L, &v, st));
   CT_CUDA_TRY(cudaMemsetAsync(L.s.ctr, 0, sizeof(Counters), st));
@@ -1663,7 +1666,7 @@ bool layout_queue_rows(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_opt
     qr->ranked.push_back(large ? a.take<uint2>(cells) : nullptr);
     qr->rank.push_back(large ? a.take<uint32_t>(cells) : nullptr);
     qr->planes.push_back(planes && !rows_planes_in_lists(&p)
-                             ? a.take<uint2>((size_t)planes * jobs[j].lists.n_slots * jobs[j].lists.stride)
+                             ? a.take<uint2>((size_t)planes * jobs[j].n_trees * p.n_rows)
                              : nullptr);
     qr->vals.push_back(a.take<float2>(p.n_features));
   }
@@ -1748,7 +1751,8 @@ int fit_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o, 
     uint32_t slot = 0, fw = 0;
     for (uint32_t j = 0; j < n_jobs; ++j) {
       const ct_fit_job& jb = jobs[j];
-      View vj = L.rows ? row_view(&jb.problem, &jb.lists, L, qr.pair[j], qr.ranked[j], qr.rank[j], qr.planes[j])
+      View vj = L.rows ? row_view(&jb.problem, &jb.lists, jb.n_trees, L, qr.pair[j], qr.ranked[j], qr.rank[j],
+                                  qr.planes[j])
                        : fit_view(&jb.problem, &jb.lists, L);
       vj.fbin = L.fbin + fw;
       vj.n_classes = q.c_max;

@@ -285,10 +285,12 @@ struct View {
   // lists of buffer b, [n_slots][stride]; pair[f * n_rows + row] = (position
   // of row in feature f's presort, bits of x[f][row]) and ranked[f * n_rows +
   // p] = (bits of the p-th smallest value, its row's label), not written for
-  // virtual features; sorted plane k ([n_slots][stride] (value bits, label))
-  // holds the sorted lists of the nodes' k-th selected features: planes
-  // [0, planes0) at sorted0, the others at sorted1.  rl[0] NULL: the lists
-  // of every feature are kept (list growth).
+  // virtual features; sorted plane k ([sorted_slots][sorted_stride] (value
+  // bits, label)) holds the sorted lists of the nodes' k-th selected features:
+  // planes [0, planes0) at sorted0, the others at sorted1.  Planes behind the
+  // row lists have the lists' slots and stride, planes in the workspace the
+  // fit's own trees and rows (its size does not see the lists).  rl[0] NULL:
+  // the lists of every feature are kept (list growth).
   uint32_t* rl[2];
   const uint2* pair;
   const uint2* ranked;
@@ -296,6 +298,8 @@ struct View {
   uint2* sorted0;
   uint2* sorted1;
   uint32_t planes0;
+  uint32_t sorted_slots;
+  uint32_t sorted_stride;
 };
 // `const View& V`: the view of the job that owns tree slot SLOT.  In a
 // kernel instantiated for a queue (template flag Q) it is that job's entry
@@ -359,7 +363,7 @@ __device__ __forceinline__ uint32_t* row_list(const View& v, uint32_t buf, uint3
 __device__ __forceinline__ uint2* sorted_list(const View& v, uint32_t slot, uint32_t k) {
   uint2* base = k < v.planes0 ? v.sorted0 : v.sorted1;
   const size_t plane = k < v.planes0 ? k : k - v.planes0;
-  return base + (plane * v.n_slots + (slot - v.slot_base)) * v.stride;
+  return base + (plane * v.sorted_slots + (slot - v.slot_base)) * v.sorted_stride;
 }
 template <typename IdxT>
 __device__ __forceinline__ IdxT* list_ptr(const View& v, uint32_t buf, uint32_t slot, uint32_t f) {

@@ -2039,6 +2039,7 @@ View make_view(const ct_problem* p, const ct_lists* l) {
   v.rank = nullptr;
   v.sorted0 = v.sorted1 = nullptr;
   v.planes0 = 0;
+  v.sorted_slots = v.sorted_stride = 0;
   return v;
 }
 
