@@ -375,6 +375,9 @@ int flush_subtrees(const ct_problem* p, const View& v, const FitLayout& L, const
                            (uint32_t)std::min<uint64_t>(L.small_bound, L.cap_small), L.subtree_cut > 32, false, L.s,
                            tv, st));
   CT_CUDA_TRY(cudaMemsetAsync(&L.s.ctr->n_small, 0, sizeof(uint32_t), st));
+  // the next launch's warps claim its subtrees from the first one past the grid again
+  static_assert(ITEM_SUBTREE_WIDE == ITEM_SUBTREE + 1, "one memset clears both claim counters");
+  CT_CUDA_TRY(cudaMemsetAsync(&L.s.ctr->claim[ITEM_SUBTREE], 0, 2 * sizeof(uint32_t), st));
   L.small_bound = 0;
   return CT_OK;
 }
