@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "ct_internal.cuh"
+#include "ct_per_device.cuh"
 
 namespace ct {
 
@@ -566,23 +567,31 @@ int capture_into(cudaGraph_t g, const cudaGraphNode_t* dep, cudaStream_t st, F l
   return CT_OK;
 }
 
-// Stream the loop graph is captured on: capture cannot start on the legacy
-// default stream, which callers often pass; the graph runs on the caller's.
+// Stream the loop graph is captured on, per thread and device: capture cannot
+// start on the legacy default stream, which callers often pass; the graph runs
+// on the caller's.
 cudaStream_t capture_stream() {
-  static thread_local struct Holder {
+  struct Holder {
     cudaStream_t st = nullptr;
     ~Holder() {
       if (st) cudaStreamDestroy(st);
     }
-  } h;
-  if (!h.st) cudaStreamCreateWithFlags(&h.st, cudaStreamNonBlocking);
+  };
+  static thread_local PerDevice<Holder> all;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  Holder& h = all.on(dev);
+  if (!h.st && cudaStreamCreateWithFlags(&h.st, cudaStreamNonBlocking) != cudaSuccess) {
+    cudaGetLastError();
+    h.st = nullptr;
+  }
   return h.st;
 }
 
-// Branch streams and events of a capture, per thread; NULL when they cannot be
-// created (the capture then has no branches).
+// Branch streams and events of a capture, per thread and device; NULL when they
+// cannot be created (the capture then has no branches).
 const ForkStreams* fork_streams() {
-  static thread_local struct Holder {
+  struct Holder {
     ForkStreams f{};
     bool ok = true;
     Holder() {
@@ -598,7 +607,11 @@ const ForkStreams* fork_streams() {
       for (auto& e : f.join)
         if (e) cudaEventDestroy(e);
     }
-  } h;
+  };
+  static thread_local PerDevice<Holder> all;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  Holder& h = all.on(dev);
   return h.ok ? &h.f : nullptr;
 }
 
