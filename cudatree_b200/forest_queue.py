@@ -20,6 +20,7 @@ side from their own host threads and CUDA streams.
 from __future__ import annotations
 
 import ctypes as C
+import itertools
 import math
 import os
 import threading
@@ -83,34 +84,33 @@ def fit_forests(jobs, n_estimators=10, max_features=None, seeds=None, group_byte
     dev = _device()
     plans = [_GroupPlan([jobs[i] for i in g], fit_options or {}, profile) for g in groups]
     # waves of `streams` groups; a wave's buffers are one allocation (a queue
-    # of the same shape later reuses it from the caching allocator)
-    for w0 in range(0, len(groups), streams):
-        wave = list(range(w0, min(w0 + streams, len(groups))))
-        offs, total = {}, 0
-        for k in wave:
-            offs[k] = total
-            total += (plans[k].size + 255) & ~255
-        arena = torch.empty(total, dtype=torch.uint8, device=dev)
-        torch.cuda.current_stream(dev).synchronize()  # the allocation is ready for the groups' streams
+    # of the same shape later reuses it from the caching allocator).  The i-th
+    # group of every wave runs on the call's i-th worker thread.
+    workers = _take_workers(dev.index, min(streams, len(groups)))
+    try:
+        for w0 in range(0, len(groups), streams):
+            wave = list(range(w0, min(w0 + streams, len(groups))))
+            offs, total = {}, 0
+            for k in wave:
+                offs[k] = total
+                total += (plans[k].size + 255) & ~255
+            arena = torch.empty(total, dtype=torch.uint8, device=dev)
+            torch.cuda.current_stream(dev).synchronize()  # the allocation is ready for the groups' streams
 
-        def run(k):
-            g = groups[k]
-            st = torch.cuda.Stream(dev)
-            with torch.cuda.stream(st):
-                res = _fit_group([jobs[i] for i in g], [seeds[i] for i in g], n_estimators, max_features, plans[k],
-                                 arena, offs[k], k - w0)
-            st.synchronize()
-            for i, f in zip(g, res):
-                forests[i] = f
+            def run(worker, k):
+                g = groups[k]
+                st = torch.cuda.Stream(dev)
+                with torch.cuda.stream(st):
+                    res = _fit_group([jobs[i] for i in g], [seeds[i] for i in g], n_estimators, max_features,
+                                     plans[k], arena, offs[k], worker)
+                st.synchronize()
+                for i, f in zip(g, res):
+                    forests[i] = f
 
-        # each slot's groups run on the slot's own thread, kept between calls:
-        # the library's capture streams and loop graph are per thread, and a
-        # new thread pays 0.4 ms for the one and up to 0.5 ms for the other
-        work = [_slot_worker(k - w0).submit(run, k) for k in wave]
-        wait(work)
-        for f in work:
-            f.result()
-        del arena
+            _run_all(workers, run, wave)
+            del arena
+    finally:
+        _give_back(dev.index, workers)
     return forests
 
 
@@ -198,40 +198,80 @@ class _GroupPlan:
         self.size = ar.size
 
 
-_WORKERS = {}  # one thread per group slot, started on first use
-_WORKERS_LOCK = threading.Lock()
+class _Worker:
+    """A thread that fits groups one after another, with its page-locked upload
+    staging (kept, grow only).  The library's capture streams and loop graph
+    are per thread: a new thread pays 0.4 ms for the one and up to 0.5 ms for
+    the other, so idle workers are kept between calls."""
+
+    _numbers = itertools.count()
+
+    def __init__(self):
+        self.number = next(_Worker._numbers)
+        self._pool = ThreadPoolExecutor(max_workers=1, thread_name_prefix=f"forest-queue-{self.number}")
+        self._staging = None
+
+    def submit(self, fn, *args):
+        return self._pool.submit(fn, *args)
+
+    def staging(self, nbytes: int) -> torch.Tensor:
+        if self._staging is None or self._staging.numel() < nbytes:
+            self._staging = torch.empty(max(nbytes, 1), dtype=torch.uint8, pin_memory=True)
+        return self._staging
+
+    def close(self) -> None:
+        self._pool.shutdown(wait=False)
 
 
-def _slot_worker(slot: int) -> ThreadPoolExecutor:
-    with _WORKERS_LOCK:
-        if slot not in _WORKERS:
-            _WORKERS[slot] = ThreadPoolExecutor(max_workers=1, thread_name_prefix=f"forest-queue-{slot}")
-        return _WORKERS[slot]
+IDLE_WORKERS = 8  # kept per device; workers given back beyond them end
+_IDLE = {}  # device index -> idle workers, by number: a caller alone gets the same ones each time
+_IDLE_LOCK = threading.Lock()
+
+
+def _take_workers(device: int, k: int) -> list:
+    """k workers of the caller's own until it gives them back: calls of several
+    threads, or on several devices, run side by side."""
+    with _IDLE_LOCK:
+        idle = _IDLE.setdefault(device, [])
+        got = idle[:k]
+        del idle[:k]
+    return got + [_Worker() for _ in range(k - len(got))]
+
+
+def _give_back(device: int, workers: list) -> None:
+    with _IDLE_LOCK:
+        idle = sorted(_IDLE.get(device, []) + workers, key=lambda w: w.number)
+        _IDLE[device] = idle[:IDLE_WORKERS]
+    for w in idle[IDLE_WORKERS:]:
+        w.close()
+
+
+def _run_all(workers: list, fn, items: list) -> None:
+    """fn(worker, item) on the workers, one item each; returns or raises when all
+    have ended, also when it is interrupted (they use the caller's buffers)."""
+    work = []
+    try:
+        for w, item in zip(workers, items):
+            work.append(w.submit(fn, w, item))
+        wait(work)
+    finally:
+        wait(work)
+    for f in work:
+        f.result()
 
 
 def _after_fork() -> None:  # a forked child has none of the threads
-    global _WORKERS_LOCK
-    _WORKERS_LOCK = threading.Lock()
-    _WORKERS.clear()
+    global _IDLE_LOCK
+    _IDLE_LOCK = threading.Lock()
+    _IDLE.clear()
 
 
 os.register_at_fork(after_in_child=_after_fork)
 
 
-_PINNED = {}  # page-locked upload staging per group slot, kept across calls (grow only)
-
-
-def _staging(slot: int, nbytes: int) -> torch.Tensor:
-    buf = _PINNED.get(slot)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(max(nbytes, 1), dtype=torch.uint8, pin_memory=True)
-        _PINNED[slot] = buf
-    return buf
-
-
-def _fit_group(jobs, seeds, n_estimators, max_features, plan, arena, off, slot):
+def _fit_group(jobs, seeds, n_estimators, max_features, plan, arena, off, worker):
     """One group's shared fit in arena[off:off + plan.size], on the current
-    stream; returns its forests.  slot: the group's page-locked staging."""
+    stream; returns its forests.  worker: whose staging the uploads take."""
     dev = _device()
     mem = arena[off:off + plan.size]
     base = mem.data_ptr()
@@ -243,7 +283,7 @@ def _fit_group(jobs, seeds, n_estimators, max_features, plan, arena, off, slot):
     # stream, so the host copy of the next job overlaps this one's transfer
     up = [(j.x.view(np.uint8).reshape(-1), l["x_rm"]) for j, l in zip(jobs, lay)]
     up += [(j.labels.view(np.uint8), l["lab"]) for j, l in zip(jobs, lay)]
-    stage = _staging(slot, sum(a.nbytes for a, _ in up))
+    stage = worker.staging(sum(a.nbytes for a, _ in up))
     host = stage.numpy()
     o = 0
     for a, dst in up:
