@@ -11,8 +11,8 @@ max_features, seed=seeds[i]).fit(x, y)`` grows alone.
 
 Groups: jobs of one index width and label width share a call (the kernels
 are compiled per width), and a group's device memory (samples, presort,
-index lists, trees) stays within ``group_bytes`` (default 40 % of the free
-device memory).  A group's buffers are one allocation; each job is
+index lists, trees) stays within ``group_bytes`` (default 40 % of the device
+memory that this process can still allocate).  A group's buffers are one allocation; each job is
 uploaded, transposed and presorted on the device (the steps of
 ``fit_init``) before the shared fit, and several groups are fitted side by
 side from their own host threads and CUDA streams.
@@ -31,7 +31,7 @@ import torch
 
 from . import _lib
 from .random_forest import (PAD_BYTES, RandomForestClassifier, _device, _stream, best_index_bytes, compact_labels,
-                            fetch_tree_columns)
+                            fetch_tree_columns, free_bytes)
 
 
 def fit_forests(jobs, n_estimators=10, max_features=None, seeds=None, group_bytes=None, fit_options=None,
@@ -52,8 +52,7 @@ def fit_forests(jobs, n_estimators=10, max_features=None, seeds=None, group_byte
     if len(seeds) != len(jobs):
         raise ValueError("one seed per job")
     if group_bytes is None:
-        free, _ = torch.cuda.mem_get_info(_device())
-        group_bytes = int(0.4 * free)
+        group_bytes = int(0.4 * free_bytes(_device()))
     streams = max(1, int(streams))
     # groups of one (index width, label width): each within its share of the
     # memory budget (the groups of `streams` threads are in flight at once)

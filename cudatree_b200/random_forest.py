@@ -59,6 +59,15 @@ def _device() -> torch.device:
     return torch.device("cuda", torch.cuda.current_device())
 
 
+def free_bytes(dev: torch.device) -> int:
+    """Device memory that this process can allocate: what is free and what the
+    caching allocator holds unused.  (The free figure alone falls once a first
+    call's buffers are in the cache: a repeat of 256 queue jobs was cut into 5
+    groups where the first call had 4, with new loop graphs and staging.)"""
+    free, _ = torch.cuda.mem_get_info(dev)
+    return free + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+
+
 PAD_BYTES = 64  # index buffers are read up to 15 bytes past their end by 16-byte bulk copies
 
 
@@ -339,7 +348,7 @@ class RandomForestClassifier:
     def trees_in_flight(self, mode: str, query_free: bool = False) -> int:
         """Trees grown by one batched call: all of them when their lists and
         workspace take at most half of the device, else as many as fit in 70 %
-        of the free memory.  The free-memory query is skipped when the forest
+        of the memory that this process can still allocate.  The free-memory query is skipped when the forest
         is small against the device: it took 1-77 ms per call on B200."""
         if mode == "plain":
             return 1
@@ -355,8 +364,7 @@ class RandomForestClassifier:
         total = torch.cuda.get_device_properties(_device()).total_memory
         if not query_free and need(k) <= total // 2:
             return k
-        free, _ = torch.cuda.mem_get_info()
-        budget = int(free * 0.7)
+        budget = int(free_bytes(_device()) * 0.7)
         while k > 1 and need(k) > budget:
             k = max(1, k // 2)
         return k
