@@ -177,7 +177,7 @@ struct FitLayout {
   uint2* pair;           // [n_features][n_rows] (rank, value bits), by row
   uint2* ranked;         // [n_features][n_rows] (value bits, label), by rank, or NULL
   uint32_t* rank;        // [n_features][n_rows] ranks alone, by row, or NULL
-  uint2* planes;         // its sorted lists, or NULL: they fit the caller's list buffers
+  uint2* planes;         // its planes of sorted lists that do not fit the caller's list buffers, or NULL
   void* boot_ws;
   size_t boot_bytes;
   size_t bytes;
@@ -237,8 +237,8 @@ bool row_layout(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o, 
     L->ranked = a.take<uint2>((size_t)p->n_features * p->n_rows);
     L->rank = a.take<uint32_t>((size_t)p->n_features * p->n_rows);
   }
-  const uint32_t planes = rows_planes_needed(p);
-  L->planes = planes && !rows_planes_in_lists(p) ? a.take<uint2>((size_t)planes * S) : nullptr;
+  const uint32_t planes = rows_planes_in_workspace(p);
+  L->planes = planes ? a.take<uint2>((size_t)planes * S) : nullptr;
   carve_row_scratch(a, v, LevelBounds{L->chunk, S}, step_piece(0, L->scan_piece, 1), &L->s, L->virt);
   L->ctl = a.take<LoopCtl>(1);
   L->bytes = a.used + 256;
@@ -780,8 +780,8 @@ View fit_view(const ct_problem* p, const ct_lists* l, const FitLayout& L) {
 }
 
 // The view of row-list growth: 32-bit row lists at the front of the caller's
-// list buffers, the sorted planes behind them (or in the workspace, where they
-// have the n_trees slots and n_rows entries that it was sized for).
+// list buffers, as many sorted planes as fit behind them, and the others in the
+// workspace, with the n_trees slots and n_rows entries that it was sized for.
 View row_view(const ct_problem* p, const ct_lists* l, uint32_t n_trees, const FitLayout& L, uint2* pair,
               uint2* ranked, uint32_t* rank, uint2* planes) {
   View v = make_view(p, l);
@@ -794,11 +794,12 @@ View row_view(const ct_problem* p, const ct_lists* l, uint32_t n_trees, const Fi
   v.ranked = ranked;
   v.rank = rank;
   const size_t off = ((size_t)l->n_slots * l->stride * sizeof(uint32_t) + 15) & ~size_t(15);
-  v.planes0 = planes ? rows_planes_needed(p) : rows_planes_in_lists(p);
-  v.sorted_slots = planes ? n_trees : l->n_slots;
-  v.sorted_stride = planes ? p->n_rows : l->stride;
-  v.sorted0 = planes ? planes : reinterpret_cast<uint2*>(reinterpret_cast<char*>(l->si0) + off);
-  v.sorted1 = planes ? planes : reinterpret_cast<uint2*>(reinterpret_cast<char*>(l->si1) + off);
+  v.planes0 = rows_planes_in_lists(p);
+  v.sorted0 = reinterpret_cast<uint2*>(reinterpret_cast<char*>(l->si0) + off);
+  v.sorted1 = reinterpret_cast<uint2*>(reinterpret_cast<char*>(l->si1) + off);
+  v.sorted2 = planes;
+  v.sorted_slots = n_trees;
+  v.sorted_stride = p->n_rows;
   return v;
 }
 
@@ -1677,13 +1678,11 @@ bool layout_queue_rows(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_opt
     const ct_problem& p = jobs[j].problem;
     const size_t cells = (size_t)p.n_features * p.n_rows;
     const bool large = rows_have_large(p.n_rows);
-    const uint32_t planes = rows_planes_needed(&p);
+    const uint32_t planes = rows_planes_in_workspace(&p);
     qr->pair.push_back(a.take<uint2>(cells));
     qr->ranked.push_back(large ? a.take<uint2>(cells) : nullptr);
     qr->rank.push_back(large ? a.take<uint32_t>(cells) : nullptr);
-    qr->planes.push_back(planes && !rows_planes_in_lists(&p)
-                             ? a.take<uint2>((size_t)planes * jobs[j].n_trees * p.n_rows)
-                             : nullptr);
+    qr->planes.push_back(planes ? a.take<uint2>((size_t)planes * jobs[j].n_trees * p.n_rows) : nullptr);
     qr->vals.push_back(a.take<float2>(p.n_features));
   }
   View v = make_view(&pb, nullptr);

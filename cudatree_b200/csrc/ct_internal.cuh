@@ -285,11 +285,12 @@ struct View {
   // lists of buffer b, [n_slots][stride]; pair[f * n_rows + row] = (position
   // of row in feature f's presort, bits of x[f][row]) and ranked[f * n_rows +
   // p] = (bits of the p-th smallest value, its row's label), not written for
-  // virtual features; sorted plane k ([sorted_slots][sorted_stride] (value
-  // bits, label)) holds the sorted lists of the nodes' k-th selected features:
-  // planes [0, planes0) at sorted0, the others at sorted1.  Planes behind the
-  // row lists have the lists' slots and stride, planes in the workspace the
-  // fit's own trees and rows (its size does not see the lists).  rl[0] NULL:
+  // virtual features; sorted plane k ([slots][stride] (value bits, label))
+  // holds the sorted lists of the nodes' k-th selected features: planes
+  // [0, planes0) at sorted0 and [planes0, 2 planes0) at sorted1, behind the row
+  // lists and with the lists' slots and stride, the others at sorted2, in the
+  // workspace and with the fit's own trees and rows (sorted_slots,
+  // sorted_stride: the workspace's size does not see the lists).  rl[0] NULL:
   // the lists of every feature are kept (list growth).
   uint32_t* rl[2];
   const uint2* pair;
@@ -297,6 +298,7 @@ struct View {
   const uint32_t* rank;   // the ranks alone, [n_features][n_rows] by row
   uint2* sorted0;
   uint2* sorted1;
+  uint2* sorted2;
   uint32_t planes0;
   uint32_t sorted_slots;
   uint32_t sorted_stride;
@@ -361,9 +363,11 @@ __device__ __forceinline__ uint32_t* row_list(const View& v, uint32_t buf, uint3
 }
 // the sorted list of a node's k-th selected feature (row-list growth)
 __device__ __forceinline__ uint2* sorted_list(const View& v, uint32_t slot, uint32_t k) {
+  if (k >= 2 * v.planes0)
+    return v.sorted2 + ((size_t)(k - 2 * v.planes0) * v.sorted_slots + (slot - v.slot_base)) * v.sorted_stride;
   uint2* base = k < v.planes0 ? v.sorted0 : v.sorted1;
   const size_t plane = k < v.planes0 ? k : k - v.planes0;
-  return base + (plane * v.sorted_slots + (slot - v.slot_base)) * v.sorted_stride;
+  return base + (plane * v.n_slots + (slot - v.slot_base)) * v.stride;
 }
 template <typename IdxT>
 __device__ __forceinline__ IdxT* list_ptr(const View& v, uint32_t buf, uint32_t slot, uint32_t f) {
@@ -635,11 +639,11 @@ int launch_seg_partition(uint32_t index_bytes, const PartWork& w, uint64_t bound
 PartWork level_part_work(const View& v, const LevelScratch& s);
 
 // Row-list growth (ct_rows.cu).  Whether a problem's trees can grow that way,
-// and whether its sorted lists fit behind the row lists in the caller's list
-// buffers (else they take row_planes_bytes of workspace).
+// how many of its planes of sorted lists fit behind the row list in each of the
+// caller's two list buffers, and how many are left for the workspace.
 bool rows_possible(const ct_problem* p);
 uint32_t rows_planes_in_lists(const ct_problem* p);
-uint32_t rows_planes_needed(const ct_problem* p);
+uint32_t rows_planes_in_workspace(const ct_problem* p);
 bool carve_row_scratch(Arena& a, const View& v, LevelBounds b, uint32_t scan_piece, LevelScratch* s, bool virt);
 int launch_row_pairs(const View& v, const ct_problem* p, uint2* pair, uint2* ranked, uint32_t* rank, cudaStream_t st);
 bool rows_have_large(uint32_t n_rows);  // some node may take a bitmap or an order item (rank and ranked are needed)

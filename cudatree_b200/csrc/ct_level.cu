@@ -2037,7 +2037,7 @@ View make_view(const ct_problem* p, const ct_lists* l) {
   v.pair = nullptr;
   v.ranked = nullptr;
   v.rank = nullptr;
-  v.sorted0 = v.sorted1 = nullptr;
+  v.sorted0 = v.sorted1 = v.sorted2 = nullptr;
   v.planes0 = 0;
   v.sorted_slots = v.sorted_stride = 0;
   return v;

@@ -2701,18 +2701,18 @@ int row_step(const View& v, const LevelScratch& s, LevelBounds b, uint32_t n_max
 // ---------------------------------------------------------------------------
 // Sorted planes (8 bytes per row and slot) that fit behind the row list in
 // each of the two list buffers (4 bytes per row and slot of n_features *
-// index_bytes).
-static uint32_t planes_per_buffer(const ct_problem* p) {
+// index_bytes); the others take workspace.  (With all of them there as soon as
+// one did not fit, a fit of 1,000,000 x 100 rows, all features selected, 100
+// trees, asked for 97 GB of workspace instead of 18.)
+uint32_t rows_planes_in_lists(const ct_problem* p) {
   const uint64_t per_row = (uint64_t)p->n_features * p->index_bytes;
   return per_row < 16 ? 0u : (uint32_t)std::min<uint64_t>((per_row - 8) / 8, 1u << 20);
 }
 bool rows_have_large(uint32_t n_rows) { return n_rows > GROUP_ROWS; }
-uint32_t rows_planes_needed(const ct_problem* p) {
-  return rows_have_large(p->n_rows) ? std::min(p->max_features, p->n_features) : 0u;
-}
-uint32_t rows_planes_in_lists(const ct_problem* p) {
-  const uint32_t k = planes_per_buffer(p);
-  return 2 * k >= rows_planes_needed(p) ? k : 0u;
+uint32_t rows_planes_in_workspace(const ct_problem* p) {
+  const uint32_t needed = rows_have_large(p->n_rows) ? std::min(p->max_features, p->n_features) : 0u;
+  const uint32_t there = 2 * rows_planes_in_lists(p);
+  return needed > there ? needed - there : 0u;
 }
 
 // Tables on which list growth is the faster of the two: row-list growth sorts
@@ -2750,11 +2750,12 @@ bool carve_row_scratch(Arena& a, const View& v, LevelBounds b, uint32_t scan_pie
   LevelScratch& t = *s;
   t = LevelScratch{};
   t.cap_nodes = clamp32(b.nodes);
-  // A sparse node makes at most n / piece + 1 pieces per slot, a dense one at
-  // most 2 n / piece + 1 (its runs of ranks hold half a piece at the least) or,
-  // at the longest run and 64 n >= n_rows, n / 512 + 1.
+  // Nodes above the group size make pieces: a sparse one at most n / piece + 1
+  // per slot, a dense one at most 2 n / piece + 1 (its runs of ranks hold half a
+  // piece at the least) or, at the longest run and 64 n >= n_rows, n / 512 + 1.
   const uint64_t large = b.samples / (WARP_ROWS + 1);  // nodes above the warp size
-  t.cap_scan = clamp32(m * (2 * b.samples / scan_piece + b.samples / 512 + large) + 1);
+  t.cap_scan = clamp32(m * (std::max<uint64_t>(2 * b.samples / scan_piece, b.samples / 512) +
+                            b.samples / (GROUP_ROWS + 1)) + 1);
   t.cap_order = clamp32(m * large + 1);
   t.cap_units = clamp32(m * (b.samples / BITS_SLICE + large) + 1);
   t.cap_w = clamp32(m * b.nodes + 1);

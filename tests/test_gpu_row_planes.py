@@ -16,7 +16,7 @@ from . import gpu_utils as G
 from .test_gpu_fit import _assert_same_trees
 
 pytestmark = pytest.mark.gpu
-GUARD = 1 << 20  # bytes behind the workspace that must stay as they were
+GUARD = 1 << 20  # bytes behind the workspace and the lists that must stay as they were
 
 
 def _data(n, f, c, seed):
@@ -34,15 +34,17 @@ def _assert_columns(counts, cols, ref):
         np.testing.assert_array_equal(col, np.concatenate([getattr(t, name) for t in ref]), err_msg=name)
 
 
-# features, selected: no plane fits behind the row lists (5, 6 of 16 bits), one per buffer does (9)
-@pytest.mark.parametrize("f,m", [(5, 3), (6, 6), (9, 3)])
+# features, selected: no plane fits behind the row lists (5, 6 of 16 bits), one (9) or two (13) per
+# buffer do; the others lie in the workspace
+@pytest.mark.parametrize("f,m", [(5, 3), (6, 6), (9, 3), (9, 9), (13, 4), (13, 12)])
 @pytest.mark.parametrize("extra_slots,extra_stride", [(0, 0), (35, 0), (0, 4099), (3, 513)])
 def test_lists_larger_than_the_fit(cuda_device, f, m, extra_slots, extra_stride):
     n, trees = 20000, 2
     x, y = _data(n, f, 3, f)
     gp = G.GpuProblem(x, y, 3, m, bootstrap=True, seed=7)
     slots, stride = trees + extra_slots, n + extra_stride
-    si = [G.dev_bytes(slots * f * stride * gp.ib) for _ in range(2)]
+    size = slots * f * stride * gp.ib
+    si = [torch.full((size + GUARD,), 0x5A, dtype=torch.uint8, device=G.dev()) for _ in range(2)]
     mark = G.dev_bytes(_lib.mark_bytes(stride, slots))
     lists = _lib.Lists(si[0].data_ptr(), si[1].data_ptr(), mark.data_ptr(), stride, slots)
     raw = [torch.zeros(trees * 2 * n, dtype=torch.int32, device=G.dev()) for _ in range(5)]
@@ -55,7 +57,8 @@ def test_lists_larger_than_the_fit(cuda_device, f, m, extra_slots, extra_stride)
     _lib.call("ct_fit", C.byref(gp.prob), C.byref(lists), 0, trees, C.byref(opts), C.byref(tb), work.data_ptr(),
               ws.value, G.stream())
     counts, cols = fetch_tree_columns(tb, nn, trees, G.dev())
-    assert bool((work[ws.value:] == 0x5A).all())
+    for buf, used in ((work, ws.value), (si[0], size), (si[1], size)):
+        assert bool((buf[used:] == 0x5A).all())
     _assert_columns(counts, cols, O.fit_forest(x, y, n_estimators=trees, max_features=m, seed=7).trees)
 
 
