@@ -1021,18 +1021,21 @@ int fit_plain(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uint3
 // with the default partition; the partition shape of big segments (tile,
 // ring buffers, CTAs per SM) x the size from which a node partitions with
 // its tree's mark bits in shared memory; the size up to which a node
-// partitions one warp per (node, 8 features).  The plain form tunes the
+// partitions one warp per (node, 8 features).  Row-list growth (rows) has no
+// use for the partition's options and takes cutoffs above 32 as 32, so only its
+// scan pieces and cutoffs of 0 and 32 are timed.  The plain form tunes the
 // depth-first/breadth-first switch (the quantity the reference fits offline,
 // estimate_threshold.py, and predicts with random_forest.py:278-289).
 std::vector<ct_fit_options> tune_candidates(const ct_problem* p, uint32_t mode, int stage,
-                                            const ct_fit_options& base) {
+                                            const ct_fit_options& base, bool rows) {
   std::vector<ct_fit_options> c;
+  if (rows && stage > 0) return c;
   if (mode == CT_FIT_BATCHED && stage == 0) {
     // the defaults first: a later candidate must beat the current best by 1 %
     std::vector<std::pair<uint32_t, uint32_t>> pairs = {{2048u, 32u}};
     for (uint32_t sp : {1024u, 2048u, 4096u})
       for (uint32_t cut : {0u, 32u, 128u})
-        if (!(sp == 2048u && cut == 32u)) pairs.push_back({sp, cut});
+        if (!(sp == 2048u && cut == 32u) && !(rows && cut > 32u)) pairs.push_back({sp, cut});
     for (const auto& pc : pairs) {
       ct_fit_options o{};
       o.mode = CT_FIT_BATCHED;
@@ -1074,10 +1077,19 @@ size_t fit_workspace_bytes(const ct_problem* p, uint32_t n_trees, const ct_fit_o
 int fit(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uint32_t n_trees,
         const ct_fit_options* o, const ct_tree_buffers* trees, void* ws, size_t wsb, cudaStream_t st);
 
+// Row-list growth where the problem, the lists' alignment and the workspace
+// allow it (its layout in *L); a workspace sized for list growth alone still
+// takes that.
+static bool takes_rows(const ct_problem* p, const ct_lists* l, uint32_t n_trees, const ct_fit_options* o, char* ws,
+                       size_t wsb, FitLayout* L) {
+  return o->mode == CT_FIT_BATCHED && (((uintptr_t)l->si0 | (uintptr_t)l->si1) & 15u) == 0 && rows_possible(p) &&
+         row_layout(p, n_trees, o, ws, wsb, L);
+}
+
 // The second stage changes no capacity, so the first stage's candidates bound the workspace.
 size_t autotune_workspace_bytes(const ct_problem* p, uint32_t n_trees, uint32_t mode) {
   size_t most = 0;
-  for (const ct_fit_options& o : tune_candidates(p, mode, 0, ct_fit_options{}))
+  for (const ct_fit_options& o : tune_candidates(p, mode, 0, ct_fit_options{}, false))
     most = std::max(most, fit_workspace_bytes(p, n_trees, &o));
   return most;
 }
@@ -1091,11 +1103,17 @@ int autotune(const ct_problem* p, const ct_lists* l, uint32_t n_trees, uint32_t 
   float top = 3.0e38f;
   int rc = CT_OK;
   bool any = false;
+  // the form that the candidates' fits will take: it depends on no option that is tuned but the workspace's
+  FitLayout L{};
+  ct_fit_options o0{};
+  o0.mode = mode;
+  o0.subtree_cutoff = 32;
+  const bool rows = l && takes_rows(p, l, n_trees, &o0, static_cast<char*>(ws), wsb, &L);
   for (int stage = 0; stage < 3 && rc == CT_OK; ++stage) {
     if (stage > 0 && !any) break;
     const ct_fit_options base = *best;
     bool first = true;  // a stage's first candidate is its base (or the defaults), timed again
-    for (const ct_fit_options& o : tune_candidates(p, mode, stage, base)) {
+    for (const ct_fit_options& o : tune_candidates(p, mode, stage, base, rows)) {
       if (fit_workspace_bytes(p, n_trees, &o) > wsb) continue;
       float t = 3.0e38f;
       for (int rep = 0; rep < 2 && rc == CT_OK; ++rep) {
@@ -1163,13 +1181,9 @@ int fit(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uint32_t n_
   CT_ARG_CHECK(l->stride >= p->n_rows, "list stride must be >= n_rows");
   const uint32_t need_slots = (o->mode == CT_FIT_PLAIN) ? 1u : n_trees;
   CT_ARG_CHECK(l->n_slots >= need_slots, "lists hold too few tree slots");
-  // Row-list growth where the problem, the lists' alignment and the workspace
-  // allow it; a workspace sized for list growth alone still takes that.
   FitLayout L{};
   char* base = reinterpret_cast<char*>(ws);
-  const bool aligned = (((uintptr_t)l->si0 | (uintptr_t)l->si1) & 15u) == 0;
-  if (!(o->mode == CT_FIT_BATCHED && aligned && rows_possible(p) && row_layout(p, n_trees, o, base, wsb, &L)) &&
-      !list_layout(p, n_trees, o, base, wsb, &L)) {
+  if (!takes_rows(p, l, n_trees, o, base, wsb, &L) && !list_layout(p, n_trees, o, base, wsb, &L)) {
     set_last_error("fit workspace too small");
     return CT_ERR_OOM;
   }

@@ -477,7 +477,8 @@ class RandomForestClassifier:
         return o
 
     def _shape_key(self, mode):
-        return (mode, self.n_samples, self.n_features, self.n_labels, self._m, self.index_bytes,
+        # choices timed before the batched form grew row lists have the key "batched"
+        return ("batched, row lists" if mode == "batched" else mode, self.n_samples, self.n_features, self.n_labels, self._m, self.index_bytes,
                 bool(self.bootstrap), self.min_samples_split)
 
     def _tune_key(self, mode):

@@ -298,7 +298,8 @@ int ct_tree_canonicalize(const uint32_t* left, const uint32_t* right, const uint
  * speed only.  Batched, in two stages: scan piece length (1024, 2048, 4096)
  * x warp-subtree cutoff (0, 32, 128); then, around each choice, the
  * partition shape (CT_PART_*) x huge_rows (4096, 16384, never), then
- * small_rows (default, 512, 2048, 8192).  Plain: the
+ * small_rows (default, 512, 2048, 8192); where the fits take row-list growth,
+ * only the first stage, without cutoff 128.  Plain: the
  * depth-first/breadth-first switch, which the reference sets with an offline
  * regression (estimate_threshold.py, random_forest.py:278-289).  The
  * workspace must hold ct_autotune_workspace_size bytes; lists and trees as
