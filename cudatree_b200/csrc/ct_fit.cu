@@ -1074,6 +1074,7 @@ std::vector<ct_fit_options> tune_candidates(const ct_problem* p, uint32_t mode, 
 }
 
 size_t fit_workspace_bytes(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o);
+size_t fit_least_workspace_bytes(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o);
 int fit(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uint32_t n_trees,
         const ct_fit_options* o, const ct_tree_buffers* trees, void* ws, size_t wsb, cudaStream_t st);
 
@@ -1114,7 +1115,7 @@ int autotune(const ct_problem* p, const ct_lists* l, uint32_t n_trees, uint32_t 
     const ct_fit_options base = *best;
     bool first = true;  // a stage's first candidate is its base (or the defaults), timed again
     for (const ct_fit_options& o : tune_candidates(p, mode, stage, base, rows)) {
-      if (fit_workspace_bytes(p, n_trees, &o) > wsb) continue;
+      if (fit_least_workspace_bytes(p, n_trees, &o) > wsb) continue;  // (a fit takes the form that fits)
       float t = 3.0e38f;
       for (int rep = 0; rep < 2 && rc == CT_OK; ++rep) {
         cudaEventRecord(e0, st);
