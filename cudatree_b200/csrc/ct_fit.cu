@@ -128,8 +128,15 @@ void account_level(const ct_problem* p, const View& view, const Counters& h) {
   // row-list growth: 32-bit row entries and 8-byte (value, label) sorted entries
   const double w = view.rl[0] ? 4.0 : p->index_bytes, l = view.lab_shift ? 0.0 : p->label_bytes, v = sizeof(float);
   pf->stats.bytes[CT_K_SCAN] += (double)h.scan_elems * (w + l + v) + (double)h.vrows * (w + 8.0);
-  pf->stats.bytes[CT_K_MARK] += (double)h.split_total * (w + 1.0);
-  pf->stats.bytes[CT_K_PARTITION] += (double)h.part_elems * (2.0 * w + 1.0);  // chains actually partitioned
+  if (view.rl[0]) {
+    // k_row_mark reads an entry and its value and moves the rows of splits of
+    // one piece itself; the others' entries are read again and moved by k_row_move
+    pf->stats.bytes[CT_K_MARK] += (double)h.split_total * (w + v) + (double)(h.split_total - h.part_elems) * w;
+    pf->stats.bytes[CT_K_PARTITION] += (double)h.order_bytes + (double)h.part_elems * 2.0 * w;
+  } else {
+    pf->stats.bytes[CT_K_MARK] += (double)h.split_total * (w + 1.0);
+    pf->stats.bytes[CT_K_PARTITION] += (double)h.part_elems * (2.0 * w + 1.0);  // chains actually partitioned
+  }
   pf->stats.steps += 1;
 }
 
@@ -144,6 +151,7 @@ struct LoopCtl {
   unsigned long long scan_elems;   // totals of the finished levels
   unsigned long long split_total;
   unsigned long long part_elems;
+  unsigned long long order_bytes;
   unsigned long long vrows;
   unsigned long long level_samples;  // samples of the current level (its scan piece)
 };
@@ -471,6 +479,7 @@ __global__ void k_loop_init(LoopCtl* ctl, Counters* c, uint32_t cap_list, cudaGr
   ctl->scan_elems = 0;
   ctl->split_total = 0;
   ctl->part_elems = 0;
+  ctl->order_bytes = 0;
   ctl->vrows = 0;
   ctl->level_samples = c->next_total;
   reset_level_counters(c);
@@ -508,6 +517,7 @@ __global__ void k_loop_end(LoopCtl* ctl, Counters* c, uint32_t chunk, uint32_t c
   ctl->scan_elems += c->scan_elems;
   ctl->split_total += c->split_total;
   ctl->part_elems += c->part_elems;
+  ctl->order_bytes += c->order_bytes;
   ctl->vrows += c->vrows;
   ctl->levels += 1;
   const uint32_t n = min(c->n_next, cap_list);
@@ -734,6 +744,7 @@ int graph_level_loop(const ct_problem* p, const View& v, const FitLayout& L, con
   tot.scan_elems = ctl.scan_elems;
   tot.split_total = ctl.split_total;
   tot.part_elems = ctl.part_elems;
+  tot.order_bytes = ctl.order_bytes;
   tot.vrows = ctl.vrows;
   const uint64_t steps = pf->stats.steps;
   account_level(p, v, tot);

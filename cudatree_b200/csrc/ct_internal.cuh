@@ -132,13 +132,14 @@ struct Counters {
   unsigned long long small_total;
   unsigned long long split_total;  // samples in nodes partitioned this level
   unsigned long long scan_elems;   // (node, feature) elements scanned this level
-  unsigned long long part_elems;   // (node, feature) elements partitioned this level
+  unsigned long long part_elems;   // (node, feature) elements partitioned this level; row-list growth: rows k_row_move moves
+  unsigned long long order_bytes;  // row-list growth: bytes of k_row_bits and k_row_order this level (ORDER_BYTES_*)
   unsigned long long vrows;        // row-list rows read by the virtual-feature counts this level
 };
 
 // Counters of one step, zeroed at its start (n_nodes set); the level totals
-// (n_next, next_total, small_total, split_total, scan_elems, part_elems) are
-// zeroed once per level by reset_level_counters.
+// (n_next, next_total, small_total, split_total, scan_elems, part_elems,
+// order_bytes, vrows) are zeroed once per level by reset_level_counters.
 // Slots of Counters::claim.  The subtree slots are zeroed by a fit's start
 // and its loop graph, not per step (subtrees run after the level loop).
 enum : uint32_t {
@@ -173,6 +174,7 @@ __device__ __forceinline__ void reset_level_counters(Counters* c) {
   c->split_total = 0;
   c->scan_elems = 0;
   c->part_elems = 0;
+  c->order_bytes = 0;
   c->vrows = 0;
 }
 

@@ -73,6 +73,10 @@ __device__ __forceinline__ uint32_t dense_chunk(uint32_t n, uint32_t n_rows, uin
   const uint64_t ranks = (uint64_t)scan_piece * n_rows / n;
   return ranks >= 32768u ? 32768u : ranks <= 1024u ? 1024u : 1u << (31 - __clz((int)ranks));
 }
+// Bytes per (node, selected feature, row) that the two cannot do without: a
+// row's entry and its rank; its entry, its (rank, value) and its place in the list.
+constexpr uint32_t ORDER_BYTES_BITS = 8;
+constexpr uint32_t ORDER_BYTES_LIST = 20;
 constexpr uint32_t BITS_SLICE = 32768;   // rows per k_row_bits unit
 constexpr int BITS_THREADS = 512;
 constexpr uint32_t BITS_COUNTS = 4096;   // pieces x classes that k_row_bits counts itself (else k_row_hist does)
@@ -421,7 +425,7 @@ __device__ __forceinline__ void row_select_item(const View& vb, const StepLists&
       } else {
         base = atomicAdd(&s.ctr->n_scan_pieces, tmat * pps);
         ok = base + (uint64_t)tmat * pps <= s.cap_scan;
-        atomicAdd(&s.ctr->part_elems, (unsigned long long)tmat * n);
+        atomicAdd(&s.ctr->order_bytes, (unsigned long long)tmat * n * (dense ? ORDER_BYTES_BITS : ORDER_BYTES_LIST));
         if (pps > 1) {
           cbase = atomicAdd(&s.ctr->n_bchains, tmat);
           ok = ok && cbase + (uint64_t)tmat <= s.cap_order;
@@ -2086,7 +2090,7 @@ __device__ __forceinline__ void row_reduce_item(const View& vb, const StepLists&
       tv.value[at] = 0;
       sidx = atomicAdd(&s.ctr->n_splits, 1u);
       atomicAdd(&s.ctr->split_total, (unsigned long long)n);
-      atomicAdd(&s.ctr->part_elems, (unsigned long long)n);
+      if (npp > 1) atomicAdd(&s.ctr->part_elems, (unsigned long long)n);
       base = npp == 1 ? atomicAdd(&s.ctr->n_part_pieces, 1u) : atomicAdd(&s.ctr->n_status, npp);
       if (sidx >= s.cap_nodes || (npp == 1 ? base >= s.cap_part : base + (uint64_t)npp > s.cap_mpart)) {
         atomicOr(&s.ctr->error, DEV_ERR_CAPACITY);
