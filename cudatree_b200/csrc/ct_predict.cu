@@ -346,6 +346,8 @@ uint32_t predict_group_size(uint32_t n_trees, uint64_t n_nodes, size_t node_byte
   if (n_nodes * node_bytes / n_trees * round > GROUP_L1_BYTES && n_trees >= round + round / 2) g = std::min(g, round);
   const uint32_t fill = ceil_div(148u * (uint32_t)pred_blocks(PRED_ILP), tiles);
   if (fill > 1 && n_trees > round) g = std::min(g, std::max(ceil_div(n_trees, fill), 2 * columns));
+  // a grid holds 2^31 - 1 blocks (from 2.1 billion rows on with 32 groups)
+  g = std::max(g, ceil_div(n_trees, std::max(1u, 0x7fffffffu / tiles)));
   return ceil_div(n_trees, ceil_div(n_trees, g));
 }
 
@@ -481,7 +483,7 @@ int predict(const void* nodes, uint32_t n_nodes, uint32_t fbits, const uint32_t*
   else
     CT_TRY(check_forest_device<PackedForm>(nodes, n_nodes, tree_off, n_trees, 0, n_features, n_classes, pred, st));
   const uint32_t rpb = predict_rows_per_block(n_classes, n_features, n_rows);
-  const uint32_t tiles = ceil_div(n_rows, rpb);
+  const uint32_t tiles = (uint32_t)(((uint64_t)n_rows + rpb - 1) / rpb);  // (not 0 for the last rows of 32 bits)
   // Tree groups need the vote table; without one every block walks all trees.
   // Few rows are worth the table's zeroing and the votes' own launch from two
   // rounds of walks on: a call with 40 rows and 500 trees 344 -> 155 us.
