@@ -1089,13 +1089,17 @@ size_t fit_least_workspace_bytes(const ct_problem* p, uint32_t n_trees, const ct
 int fit(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uint32_t n_trees,
         const ct_fit_options* o, const ct_tree_buffers* trees, void* ws, size_t wsb, cudaStream_t st);
 
-// Row-list growth where the problem, the lists' alignment and the workspace
-// allow it (its layout in *L); a workspace sized for list growth alone still
-// takes that.
+// Row-list growth reads the list buffers and the workspace in 16-byte words;
+// list growth takes a workspace at any multiple of 8 bytes.
+static bool rows_aligned(const ct_lists& l, const void* ws) {
+  return (((uintptr_t)l.si0 | (uintptr_t)l.si1 | (uintptr_t)ws) & 15u) == 0;
+}
+
+// Row-list growth where the problem, the alignment and the workspace allow it
+// (its layout in *L); a workspace sized for list growth alone still takes that.
 static bool takes_rows(const ct_problem* p, const ct_lists* l, uint32_t n_trees, const ct_fit_options* o, char* ws,
                        size_t wsb, FitLayout* L) {
-  return o->mode == CT_FIT_BATCHED && (((uintptr_t)l->si0 | (uintptr_t)l->si1) & 15u) == 0 && rows_possible(p) &&
-         row_layout(p, n_trees, o, ws, wsb, L);
+  return o->mode == CT_FIT_BATCHED && rows_aligned(*l, ws) && rows_possible(p) && row_layout(p, n_trees, o, ws, wsb, L);
 }
 
 // The second stage changes no capacity, so the first stage's candidates bound the workspace.
@@ -1670,13 +1674,12 @@ struct QueueRows {
   std::vector<float2*> vals;
 };
 
-bool queue_rows_possible(const ct_fit_job* jobs, uint32_t n_jobs) {
+bool queue_rows_possible(const ct_fit_job* jobs, uint32_t n_jobs, const void* ws) {
   const QueueShape q = queue_shape(jobs, n_jobs);
   const ct_problem pb = batch_problem(jobs, q);  // the kernels' shared memory is sized by the batch's largest N and C
   if (!rows_possible(&pb)) return false;
   for (uint32_t j = 0; j < n_jobs; ++j)
-    if (!rows_possible(&jobs[j].problem) || (((uintptr_t)jobs[j].lists.si0 | (uintptr_t)jobs[j].lists.si1) & 15u))
-      return false;
+    if (!rows_possible(&jobs[j].problem) || !rows_aligned(jobs[j].lists, ws)) return false;
   return true;
 }
 
@@ -1728,7 +1731,7 @@ size_t fit_queue_workspace_bytes(const ct_fit_job* jobs, uint32_t n_jobs, const 
   uint32_t* sj = nullptr;
   layout_queue(jobs, n_jobs, o, nullptr, 0, &L, &vd, &sj);
   size_t bytes = L.bytes;
-  if (queue_rows_possible(jobs, n_jobs)) {
+  if (queue_rows_possible(jobs, n_jobs, nullptr)) {
     QueueRows qr;
     layout_queue_rows(jobs, n_jobs, o, nullptr, 0, &L, &vd, &sj, &qr);
     bytes = std::max(bytes, L.bytes);
@@ -1771,7 +1774,7 @@ int fit_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o, 
   uint32_t* slot_job_dev = nullptr;
   QueueRows qr;
   char* base = reinterpret_cast<char*>(ws);
-  if (!(queue_rows_possible(jobs, n_jobs) &&
+  if (!(queue_rows_possible(jobs, n_jobs, ws) &&
         layout_queue_rows(jobs, n_jobs, o, base, wsb, &L, &views_dev, &slot_job_dev, &qr)) &&
       !layout_queue(jobs, n_jobs, o, base, wsb, &L, &views_dev, &slot_job_dev)) {
     set_last_error("queue fit workspace too small");

@@ -234,9 +234,9 @@ int ct_partition_nodes(const ct_problem* p, const ct_lists* lists, const ct_node
  * points do.  Row-list growth keeps one list of rows per tree (at the start of
  * each list buffer; sorted orders of large nodes behind it or in the
  * workspace) and sorts a node's rows only for the features it selects; it is
- * taken when a row id and a label fit 32 bits, si0 and si1 are 16-byte aligned,
- * the tables of its kernels fit shared memory (up to about 1.1 million rows),
- * the workspace holds its scratch, and it is not the slower one.
+ * taken when a row id and a label fit 32 bits, si0, si1 and the workspace are
+ * 16-byte aligned, the tables of its kernels fit shared memory (up to about 1.1
+ * million rows), the workspace holds its scratch, and it is not the slower one.
  * ct_fit_workspace_size gives the larger of the two sizes; a workspace that
  * only list growth fits is accepted and used for that. */
 int ct_fit_workspace_size(const ct_problem* p, uint32_t n_trees, const ct_fit_options* opt,
