@@ -126,10 +126,14 @@ PROTOTYPES = {
                                      C.c_size_t, P]),
     "ct_fit_workspace_size": (C.c_int, [C.POINTER(Problem), C.c_uint32, C.POINTER(FitOptions),
                                         C.POINTER(C.c_size_t)]),
+    "ct_fit_least_workspace_size": (C.c_int, [C.POINTER(Problem), C.c_uint32, C.POINTER(FitOptions),
+                                              C.POINTER(C.c_size_t)]),
     "ct_fit": (C.c_int, [C.POINTER(Problem), C.POINTER(Lists), C.c_uint32, C.c_uint32,
                          C.POINTER(FitOptions), C.POINTER(TreeBuffers), P, C.c_size_t, P]),
     "ct_fit_queue_workspace_size": (C.c_int, [C.POINTER(FitJob), C.c_uint32, C.POINTER(FitOptions),
                                               C.POINTER(C.c_size_t)]),
+    "ct_fit_queue_least_workspace_size": (C.c_int, [C.POINTER(FitJob), C.c_uint32, C.POINTER(FitOptions),
+                                                    C.POINTER(C.c_size_t)]),
     "ct_fit_queue": (C.c_int, [C.POINTER(FitJob), C.c_uint32, C.POINTER(FitOptions), C.POINTER(TreeBuffers), P,
                                C.c_size_t, P]),
     "ct_fit_stats": (C.c_int, [C.c_void_p]),
@@ -194,10 +198,15 @@ def call(name: str, *args) -> None:
     check(getattr(load(), name)(*args))
 
 
-def mark_bytes(n_rows: int, n_slots: int) -> int:
+def size_of(name: str, *args) -> int:
+    """What the size function `name` stores in its last argument."""
     out = C.c_size_t()
-    call("ct_mark_bytes", n_rows, n_slots, C.byref(out))
+    call(name, *args, C.byref(out))
     return out.value
+
+
+def mark_bytes(n_rows: int, n_slots: int) -> int:
+    return size_of("ct_mark_bytes", n_rows, n_slots)
 
 
 def version() -> str:

@@ -17,7 +17,9 @@ size_t bootstrap_scratch_bytes(uint32_t n_rows, uint32_t n_features, uint32_t n_
 int bootstrap_compact(const ct_problem* p, const ct_lists* l, uint32_t slot, uint32_t tree,
                       uint32_t* n_in_dev, void* ws, size_t wsb, cudaStream_t st);
 size_t fit_workspace_bytes(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o);
+size_t fit_least_workspace_bytes(const ct_problem* p, uint32_t n_trees, const ct_fit_options* o);
 size_t fit_queue_workspace_bytes(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o);
+size_t fit_queue_least_workspace_bytes(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o);
 int fit_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o, const ct_tree_buffers* trees,
               void* ws, size_t wsb, cudaStream_t st);
 int fit(const ct_problem* p, const ct_lists* l, uint32_t first_tree, uint32_t n_trees,
@@ -213,6 +215,12 @@ int ct_fit_workspace_size(const ct_problem* p, uint32_t n_trees, const ct_fit_op
   return CT_OK;
 }
 
+int ct_fit_least_workspace_size(const ct_problem* p, uint32_t n_trees, const ct_fit_options* opt, size_t* bytes) {
+  CT_ARG_CHECK(p && opt && bytes, "NULL argument");
+  *bytes = fit_least_workspace_bytes(p, n_trees, opt);
+  return CT_OK;
+}
+
 int ct_fit(const ct_problem* p, const ct_lists* lists, uint32_t first_tree, uint32_t n_trees,
            const ct_fit_options* opt, const ct_tree_buffers* trees, void* workspace, size_t workspace_bytes,
            void* stream) {
@@ -224,6 +232,12 @@ int ct_fit_queue_workspace_size(const ct_fit_job* jobs, uint32_t n_jobs, const c
                                 size_t* bytes) {
   CT_ARG_CHECK(jobs && n_jobs >= 1 && opt && bytes, "NULL argument");
   CT_GUARD(*bytes = fit_queue_workspace_bytes(jobs, n_jobs, opt); return CT_OK;)
+}
+
+int ct_fit_queue_least_workspace_size(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* opt,
+                                      size_t* bytes) {
+  CT_ARG_CHECK(jobs && n_jobs >= 1 && opt && bytes, "NULL argument");
+  CT_GUARD(*bytes = fit_queue_least_workspace_bytes(jobs, n_jobs, opt); return CT_OK;)
 }
 
 int ct_fit_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* opt, const ct_tree_buffers* trees,

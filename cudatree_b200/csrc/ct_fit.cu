@@ -1725,13 +1725,21 @@ bool layout_queue_rows(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_opt
 
 }  // namespace
 
-size_t fit_queue_workspace_bytes(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o) {
+// As fit_least_workspace_bytes and fit_workspace_bytes.
+size_t fit_queue_least_workspace_bytes(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o) {
   FitLayout L{};
   View* vd = nullptr;
   uint32_t* sj = nullptr;
   layout_queue(jobs, n_jobs, o, nullptr, 0, &L, &vd, &sj);
-  size_t bytes = L.bytes;
+  return L.bytes;
+}
+
+size_t fit_queue_workspace_bytes(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o) {
+  size_t bytes = fit_queue_least_workspace_bytes(jobs, n_jobs, o);
   if (queue_rows_possible(jobs, n_jobs, nullptr)) {
+    FitLayout L{};
+    View* vd = nullptr;
+    uint32_t* sj = nullptr;
     QueueRows qr;
     layout_queue_rows(jobs, n_jobs, o, nullptr, 0, &L, &vd, &sj, &qr);
     bytes = std::max(bytes, L.bytes);

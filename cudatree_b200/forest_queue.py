@@ -89,11 +89,7 @@ def fit_forests(jobs, n_estimators=10, max_features=None, seeds=None, group_byte
     try:
         for w0 in range(0, len(groups), streams):
             wave = list(range(w0, min(w0 + streams, len(groups))))
-            offs, total = {}, 0
-            for k in wave:
-                offs[k] = total
-                total += (plans[k].size + 255) & ~255
-            arena = torch.empty(total, dtype=torch.uint8, device=dev)
+            arena, offs = _wave_memory({k: plans[k] for k in wave}, dev)
             torch.cuda.current_stream(dev).synchronize()  # the allocation is ready for the groups' streams
 
             def run(worker, k):
@@ -111,6 +107,26 @@ def fit_forests(jobs, n_estimators=10, max_features=None, seeds=None, group_byte
     finally:
         _give_back(dev.index, workers)
     return forests
+
+
+def _wave_memory(plans, dev):
+    """One allocation for a wave's groups and each group's offset in it.  Where
+    the workspaces of row lists are not to be had, the groups take the least."""
+    def allocate():
+        offs, total = {}, 0
+        for k, p in plans.items():
+            offs[k] = total
+            total += (p.size + 255) & ~255
+        return torch.empty(total, dtype=torch.uint8, device=dev), offs
+
+    try:
+        return allocate()
+    except torch.OutOfMemoryError:
+        pass
+    torch.cuda.empty_cache()
+    for p in plans.values():
+        p.take_least_workspace()
+    return allocate()
 
 
 class _HostJob:
@@ -190,11 +206,14 @@ class _GroupPlan:
                                                1, 1, 0)
             self.arr[k].lists = _lib.Lists(None, None, None, j.n, j.trees)
             self.arr[k].n_trees = j.trees
-        ws = C.c_size_t()
-        _lib.call("ct_fit_queue_workspace_size", self.arr, len(jobs), C.byref(self.opts), C.byref(ws))
-        self.ws_bytes = ws.value
-        self.work = ar.take(ws.value)
+        self.ws_bytes = _lib.size_of("ct_fit_queue_workspace_size", self.arr, len(jobs), C.byref(self.opts))
+        self.work = ar.take(self.ws_bytes)  # last: its size may change
         self.size = ar.size
+
+    def take_least_workspace(self):
+        least = _lib.size_of("ct_fit_queue_least_workspace_size", self.arr, len(self.arr), C.byref(self.opts))
+        self.size -= self.ws_bytes - least
+        self.ws_bytes = least
 
 
 class _Worker:

@@ -75,6 +75,19 @@ def _dev_bytes(nbytes: int, dev) -> torch.Tensor:
     return torch.empty(max(int(nbytes), 1) + PAD_BYTES, dtype=torch.uint8, device=dev)
 
 
+def first_that_fits(sizes, dev):
+    """(buffer, bytes) of the first of the sizes, most wanted first, that can be
+    allocated.  (A fit runs faster with the workspace of row lists, up to 20
+    bytes per cell of the table more than it needs at the least.)"""
+    for nbytes in sizes[:-1]:
+        try:
+            return _dev_bytes(nbytes, dev), nbytes
+        except torch.OutOfMemoryError:
+            pass
+        torch.cuda.empty_cache()
+    return _dev_bytes(sizes[-1], dev), sizes[-1]
+
+
 def _to_dev(a: np.ndarray, dev) -> torch.Tensor:
     a = np.ascontiguousarray(a)
     return torch.from_numpy(a.view(np.uint8).reshape(-1)).to(dev, non_blocking=False)
@@ -356,9 +369,8 @@ class RandomForestClassifier:
         opts = self._fit_options(_lib.CT_FIT_BATCHED, 0)
 
         def need(k):
-            ws = C.c_size_t()
-            _lib.call("ct_fit_workspace_size", C.byref(prob), k, C.byref(opts), C.byref(ws))
-            return k * self._slot_bytes() + ws.value
+            ws = _lib.size_of("ct_fit_workspace_size", C.byref(prob), k, C.byref(opts))
+            return k * self._slot_bytes() + ws
 
         k = self.n_estimators
         total = torch.cuda.get_device_properties(_device()).total_memory
@@ -396,15 +408,15 @@ class RandomForestClassifier:
                               _ptr(raw["threshold"]), _ptr(raw["value"]), _ptr(n_nodes), cap)
         opts = self._fit_options(mode_id, bfs_threshold)
         opts.flags |= (_lib.CT_FIT_PROFILE if self.profile else 0) | (_lib.CT_FIT_HOST_LOOP if self.host_level_loop else 0)
-        ws = C.c_size_t()
-        _lib.call("ct_fit_workspace_size", C.byref(prob), per_call, C.byref(opts), C.byref(ws))
-        work = _dev_bytes(ws.value, dev)
+        sizes = [_lib.size_of(f"ct_fit_{least}workspace_size", C.byref(prob), per_call, C.byref(opts))
+                 for least in ("", "least_")]
+        work, ws_bytes = first_that_fits(sizes, dev)
         trees = []
         stats = None
         for t0 in range(first, first + count, per_call):
             kk = min(per_call, first + count - t0)
             _lib.call("ct_fit", C.byref(prob), C.byref(lists), t0, kk, C.byref(opts), C.byref(tb),
-                      _ptr(work), ws.value, _stream())
+                      _ptr(work), ws_bytes, _stream())
             st = _lib.fit_stats()
             if stats is None:
                 stats = st
@@ -498,13 +510,14 @@ class RandomForestClassifier:
         raw = [torch.empty(sample_trees * cap, dtype=torch.int32, device=dev) for _ in range(5)]
         n_nodes = torch.zeros(sample_trees, dtype=torch.int32, device=dev)
         tb = _lib.TreeBuffers(*[_ptr(r) for r in raw], _ptr(n_nodes), cap)
-        wsb = C.c_size_t()
-        _lib.call("ct_autotune_workspace_size", C.byref(prob), sample_trees, mode_id, C.byref(wsb))
-        work = _dev_bytes(wsb.value, dev)
+        least = _lib.FitOptions(mode_id, 0, 128, 1024)  # the candidate that takes the most
+        sizes = [_lib.size_of("ct_autotune_workspace_size", C.byref(prob), sample_trees, mode_id),
+                 _lib.size_of("ct_fit_least_workspace_size", C.byref(prob), sample_trees, C.byref(least))]
+        work, ws_bytes = first_that_fits(sizes, dev)
         best = _lib.FitOptions()
         ms = C.c_float()
         _lib.call("ct_autotune", C.byref(prob), C.byref(lists), sample_trees, mode_id, C.byref(tb), _ptr(work),
-                  wsb.value, C.byref(best), C.byref(ms), _stream())
+                  ws_bytes, C.byref(best), C.byref(ms), _stream())
         self._tuned = {"scan_piece": int(best.scan_piece), "subtree_cutoff": int(best.subtree_cutoff),
                        "bfs_threshold": int(best.bfs_threshold) or self.bfs_threshold,
                        "part_shape": int(best.part_shape), "huge_rows": int(best.huge_rows),

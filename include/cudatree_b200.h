@@ -238,9 +238,12 @@ int ct_partition_nodes(const ct_problem* p, const ct_lists* lists, const ct_node
  * 16-byte aligned, the tables of its kernels fit shared memory (up to about 1.1
  * million rows), the workspace holds its scratch, and it is not the slower one.
  * ct_fit_workspace_size gives the larger of the two sizes; a workspace that
- * only list growth fits is accepted and used for that. */
+ * only list growth fits (ct_fit_least_workspace_size) is accepted and used for
+ * that. */
 int ct_fit_workspace_size(const ct_problem* p, uint32_t n_trees, const ct_fit_options* opt,
                           size_t* bytes);
+int ct_fit_least_workspace_size(const ct_problem* p, uint32_t n_trees, const ct_fit_options* opt,
+                                size_t* bytes);
 int ct_fit(const ct_problem* p, const ct_lists* lists, uint32_t first_tree, uint32_t n_trees,
            const ct_fit_options* opt, const ct_tree_buffers* trees, void* workspace,
            size_t workspace_bytes, void* stream);
@@ -254,8 +257,9 @@ int ct_fit(const ct_problem* p, const ct_lists* lists, uint32_t first_tree, uint
  * after the slots of the jobs before it; trees->capacity must be at least
  * 2 * every job's n_rows.  Every job has the same index_bytes and
  * label_bytes; opt->mode must be CT_FIT_BATCHED (huge_rows is ignored: the
- * partition of big nodes reads marks from global memory).  ct_fit_stats
- * reports the whole queue. */
+ * partition of big nodes reads marks from global memory).  Growth and the two
+ * workspace sizes are as in ct_fit; the jobs of a queue grow alike.
+ * ct_fit_stats reports the whole queue. */
 typedef struct ct_fit_job {
   ct_problem problem;
   ct_lists lists;            /* n_slots >= n_trees                            */
@@ -264,6 +268,8 @@ typedef struct ct_fit_job {
 } ct_fit_job;
 int ct_fit_queue_workspace_size(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* opt,
                                 size_t* bytes);
+int ct_fit_queue_least_workspace_size(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* opt,
+                                      size_t* bytes);
 int ct_fit_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* opt,
                  const ct_tree_buffers* trees, void* workspace, size_t workspace_bytes, void* stream);
 
