@@ -709,6 +709,7 @@ size_t predict_tile_smem(uint32_t rpb, uint32_t n_classes, uint32_t n_features);
 uint32_t predict_group_size(uint32_t n_trees, uint64_t n_nodes, size_t node_bytes);  // by the nodes' share of L2
 uint32_t predict_group_size(uint32_t n_trees, uint64_t n_nodes, size_t node_bytes, uint32_t rpb, uint32_t tiles);
 bool predict_one_round(uint32_t rpb, uint32_t group);  // a block walks the group's trees at once
+bool predict_few_in_flight(uint32_t rpb, uint32_t group, uint64_t tree_bytes);
 uint32_t compact_feature_bits(uint32_t n_features);
 bool compact_fits(uint32_t n_features, uint64_t max_tree_nodes);
 void compact_host(const ct_packed_node* in, uint32_t n, uint32_t fbits, ct_compact_node* out);

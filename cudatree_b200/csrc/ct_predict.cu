@@ -28,7 +28,7 @@ namespace {
 
 constexpr int PRED_THREADS = 256;
 // Walks in flight per thread: 4 at 6 blocks per SM where a group is one round of
-// them, else 8 at 4 blocks.  Fewer trees in flight, whose nodes stay in L1
+// them or small (predict_few_in_flight), else 8 at 4 blocks.  Fewer trees in flight, whose nodes stay in L1
 // longer, but more rounds: 500 covtype-shaped trees (37 MB of nodes), 65,536
 // rows, in groups of 32: 4 walks 1.64 ms, 8 walks 1.82, 2 walks (8 blocks) 1.82;
 // all trees in one group: 3.29, 3.00 and 3.7 ms.
@@ -40,6 +40,7 @@ constexpr uint32_t X_SMEM_BYTES = 32 * 1024;     // rows of x staged per block w
 constexpr uint32_t HIST_SMEM_BYTES = 64 * 1024;  // vote histogram [rows][classes]
 constexpr size_t GROUP_L2_BYTES = 32ull << 20;   // node bytes of one tree group, at the most
 constexpr size_t GROUP_L1_BYTES = 192ull << 10;  // node bytes of one round of walks from which groups are single rounds
+constexpr size_t GROUP_SHORT_BYTES = 768ull << 10;  // node bytes of a group of several rounds of short walks
 
 __host__ __device__ __forceinline__ bool predict_rows_staged(uint32_t rpb, uint32_t n_features) {
   return (size_t)rpb * n_features * sizeof(float) <= X_SMEM_BYTES;
@@ -353,6 +354,17 @@ uint32_t predict_group_size(uint32_t n_trees, uint64_t n_nodes, size_t node_byte
 
 bool predict_one_round(uint32_t rpb, uint32_t group) { return group <= walk_round(rpb); }
 
+// Which of the two forms of the walk.  Several rounds of trees that fit L1 are
+// short walks while the whole group is not far beyond L1 either, and then more
+// blocks hide more (65,536 rows, 4 walks / 8 walks: 100 trees of 1.2 KB 135 / 169
+// us, of 5.6 KB 219 / 251; 300 trees of 1.9 KB 428 / 442, of 2.8 KB 514 / 514).
+// Past that most nodes come from L2 and more walks in flight do (300 trees of 4
+// KB 619 / 599; 1,000 of 1.2 KB 1,536 / 1,419; 5,000 rows, 1,000 of 4 KB 254 / 200).
+bool predict_few_in_flight(uint32_t rpb, uint32_t group, uint64_t tree_bytes) {
+  return predict_one_round(rpb, group) ||
+         (tree_bytes * walk_round(rpb) <= GROUP_L1_BYTES && tree_bytes * group <= GROUP_SHORT_BYTES);
+}
+
 uint32_t compact_feature_bits(uint32_t n_features) {
   uint32_t b = 1;
   while (b < 31 && (1u << b) < n_features) ++b;
@@ -500,12 +512,10 @@ int predict(const void* nodes, uint32_t n_nodes, uint32_t fbits, const uint32_t*
                                                        n_features, n_classes, rpb, votes, pred);
     return CT_OK;
   };
-  // (short walks in trees that fit L1: 100 trees of 0.9 KB, 65,536 rows, 124 us with 4, 138 with 8)
-  const bool one_round =
-      predict_one_round(rpb, group) ||
-      (uint64_t)n_nodes * (fbits ? CompactForm::BYTES : PackedForm::BYTES) / n_trees * walk_round(rpb) <= GROUP_L1_BYTES;
-  if (fbits) CT_TRY(one_round ? launch(k_predict<CompactForm, PRED_ILP>) : launch(k_predict<CompactForm, PRED_ILP_LONG>));
-  else CT_TRY(one_round ? launch(k_predict<PackedForm, PRED_ILP>) : launch(k_predict<PackedForm, PRED_ILP_LONG>));
+  const bool few =
+      predict_few_in_flight(rpb, group, (uint64_t)n_nodes * (fbits ? CompactForm::BYTES : PackedForm::BYTES) / n_trees);
+  if (fbits) CT_TRY(few ? launch(k_predict<CompactForm, PRED_ILP>) : launch(k_predict<CompactForm, PRED_ILP_LONG>));
+  else CT_TRY(few ? launch(k_predict<PackedForm, PRED_ILP>) : launch(k_predict<PackedForm, PRED_ILP_LONG>));
   if (groups > 1) k_vote_rows<<<ceil_div(n_rows, 8), 256, 0, st>>>(votes, n_rows, n_classes, pred);
   CT_CUDA_TRY(cudaGetLastError());
   return CT_OK;
