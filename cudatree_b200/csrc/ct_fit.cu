@@ -1491,7 +1491,11 @@ int fetch_trees(const ct_tree_buffers* tb, uint32_t n_trees, const uint32_t* cou
     if (parts == 1) CT_CUDA_TRY(cudaStreamSynchronize(st));
     char* dst[5] = {reinterpret_cast<char*>(ol), reinterpret_cast<char*>(orr), reinterpret_cast<char*>(ot),
                     reinterpret_cast<char*>(ov), reinterpret_cast<char*>(of)};
+    int dev = 0;
+    CT_CUDA_TRY(cudaGetDevice(&dev));
     auto copy = [&](uint32_t w) {
+      // (a thread starts on device 0, where its first call would make a context)
+      if (parts > 1 && w > 0 && (arrived[w] = cudaSetDevice(dev)) != cudaSuccess) return;
       const size_t lo = (size_t)total * w / workers, n = (size_t)total * (w + 1) / workers - lo;
       for (int k = 0; k < 5; ++k) {
         const size_t es = k == 4 ? 2 : 4;
