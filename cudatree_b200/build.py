@@ -46,7 +46,7 @@ def nvcc() -> str:
 
 
 def _deps() -> list[Path]:
-    return sorted(CSRC.glob("*.cu*")) + sorted(INCLUDE.glob("*.h")) + [Path(__file__)]
+    return sorted(CSRC.glob("*.cu*")) + sorted(CSRC.glob("*.h")) + sorted(INCLUDE.glob("*.h")) + [Path(__file__)]
 
 
 def _compile(src: Path, ptxas_verbose: bool) -> tuple[Path, str]:

@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "ct_internal.cuh"
+#include "ct_parts.h"
 #include "ct_per_device.cuh"
 
 namespace ct {
@@ -1380,11 +1381,6 @@ __global__ void k_gather_trees(ct_tree_buffers tb, const uint32_t* __restrict__ 
   }
 }
 
-// Page-locked staging for the raw read-back, shared by the process and grown
-// on demand (portable across devices).  Page-locked allocation synchronizes
-// the device and takes tens of ms for a 100-tree forest, so a server reserves
-// its largest size up front, and a growth takes half again the old size
-// (16 MiB steps): forests a little larger than the last do not reallocate.
 template <int N>
 struct EventSet {
   cudaEvent_t e[N] = {};
@@ -1398,17 +1394,11 @@ struct EventSet {
       if (x) cudaEventDestroy(x);
   }
 };
-// Threads joined at the end of their scope, also when starting one throws.
-struct ThreadSet {
-  std::vector<std::thread> v;
-  template <typename F>
-  void start(F f, uint32_t arg) {
-    v.emplace_back(f, arg);
-  }
-  ~ThreadSet() {
-    for (auto& t : v) t.join();
-  }
-};
+// Page-locked staging for the raw read-back, shared by the process and grown
+// on demand (portable across devices).  Page-locked allocation synchronizes
+// the device and takes tens of ms for a 100-tree forest, so a server reserves
+// its largest size up front, and a growth takes half again the old size
+// (16 MiB steps): forests a little larger than the last do not reallocate.
 struct Staging {
   std::mutex mu;
   void* p = nullptr;
@@ -1509,11 +1499,7 @@ int fetch_trees(const ct_tree_buffers* tb, uint32_t n_trees, const uint32_t* cou
         std::memcpy(dst[k] + lo * es, to + col[k] + lo * es, n * es);
       }
     };
-    {
-      ThreadSet pool;
-      for (uint32_t w = 1; w < workers; ++w) pool.start(copy, w);
-      copy(0);
-    }
+    run_parts(workers, copy);  // (all transfers have ended when it returns)
     for (const cudaError_t e : arrived) CT_CUDA_TRY(e);
     bool deep = false;
     for (uint32_t t = 0; t < n_trees; ++t) {
@@ -1560,10 +1546,7 @@ static int fetch_trees_host(const ct_tree_buffers* tb, uint32_t n_trees, const u
       }
     }
   };
-  std::vector<std::thread> pool;
-  for (uint32_t w = 1; w < workers; ++w) pool.emplace_back(run, w);
-  run(0);
-  for (auto& th : pool) th.join();
+  run_parts(workers, run);
   for (uint32_t w = 0; w < workers; ++w)
     if (status[w] != CT_OK) {
       set_last_error(errors[w]);
