@@ -1628,7 +1628,7 @@ __device__ __forceinline__ float limit_of(const PieceLimit& pl, uint32_t C, uint
       la += d.y;
       nl += pl.rows[c];
     }
-  float best = 0.f;
+  float best = 1.f;  // no gain: a piece that holds all rows of a node of one class has no corner with rows on both sides
   for (uint32_t m = 0; m < (C > LIMIT_BASE ? 1u << (C - LIMIT_BASE) : 1u); ++m) {
     double ms = ls, ma = la;
     uint32_t k = nl;
