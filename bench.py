@@ -34,6 +34,12 @@ WORKLOAD = ("covtype-shaped synthetic 581012x54 f32 (10 Gaussian + 44 one-hot), 
             "100 trees, bootstrap, max_features=7, uint32 indices, fully grown")
 N_TREES = 100
 MAX_FEATURES = 7
+# DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum, caches cold at
+# every launch) per algorithmic byte of the partition and the split-scan kernel
+# groups of row-list growth, over every launch of one profiled 16-tree fit of
+# this workload
+PARTITION_DRAM_PER_ALGORITHMIC_BYTE = 0.80
+SCAN_DRAM_PER_ALGORITHMIC_BYTE = 1.38
 
 
 def peaks():
@@ -523,11 +529,15 @@ def run_ours(args, world, rank, local):
     pi = groups.index("partition")
     p_ms = stats["ms"][pi]
     p_gbs = stats["bytes"][pi] / (p_ms * 1e6) if p_ms > 0 else None
+    # DRAM bytes per launch: the algorithmic bytes per launch times the ratio
+    # measured on the 16-tree case
     p_launches = stats["launches"][pi]
+    traffic = (PARTITION_DRAM_PER_ALGORITHMIC_BYTE * stats["bytes"][pi] / p_launches) if p_launches else None
     si = groups.index("scan")
     s_ms = stats["ms"][si]
     s_gbs = stats["bytes"][si] / (s_ms * 1e6) if s_ms > 0 else None
     s_launches = stats["launches"][si]
+    s_traffic = (SCAN_DRAM_PER_ALGORITHMIC_BYTE * stats["bytes"][si] / s_launches) if s_launches else None
     cpu = None
     if not args.skip_cpu:
         cores = len(os.sched_getaffinity(0))
@@ -550,18 +560,21 @@ def run_ours(args, world, rank, local):
         "kernels": kernels,
         "roofline": {"bound": "hbm", "kernel": "k_row_bits + k_row_order + k_row_move (rank bitmaps, sorted lists, row-list split)", "achieved": round(p_gbs, 1) if p_gbs else None,
                      "peak": peak, "unit": "GB/s", "frac": round(p_gbs / peak, 4) if p_gbs else None,
-                     "peak_kind": peak_kind, "traffic": None,
-                     "traffic_unit": "DRAM bytes per launch (not captured for these kernels)",
+                     "peak_kind": peak_kind, "traffic": round(traffic) if traffic else None,
+                     "traffic_unit": f"DRAM bytes per launch (ncu ratio {PARTITION_DRAM_PER_ALGORITHMIC_BYTE} x "
+                                     f"algorithmic, 16-tree capture)",
                      "algorithmic_bytes_per_launch": round(stats["bytes"][pi] / p_launches) if p_launches else None,
-                     "algorithmic_bytes_per_element": "per (node above 9,216 rows, selected feature, row): 2 x index_bytes + 1"},
+                     "algorithmic_bytes_per_element": "per (node above 9,216 rows, selected feature, row): 8 (bitmap) or 20 "
+                                                      "(list); per row of a split above 512 rows: 8"},
         "scan_roofline": {"bound": "hbm", "kernel": "k_row_scan_seq, k_row_group, k_row_warp (+limit, bound, carry, virtual counts)",
                           "achieved": round(s_gbs, 1) if s_gbs else None, "peak": peak, "unit": "GB/s",
                           "frac": round(s_gbs / peak, 4) if s_gbs else None, "peak_kind": peak_kind,
-                          "traffic": None,
-                          "traffic_unit": "DRAM bytes per launch (not captured for these kernels)",
+                          "traffic": round(s_traffic) if s_traffic else None,
+                          "traffic_unit": f"DRAM bytes per launch (ncu ratio {SCAN_DRAM_PER_ALGORITHMIC_BYTE} x "
+                                          f"algorithmic, 16-tree capture)",
                           "algorithmic_bytes_per_launch": round(stats["bytes"][si] / s_launches) if s_launches else None,
-                          "algorithmic_bytes_per_element": "per (node, selected feature, position): index_bytes "
-                                                           "+ 4 (x gather) + label gather when labels are not packed"},
+                          "algorithmic_bytes_per_element": "per (node, selected feature, row): 8 (entry and value, or sorted "
+                                                           "entry); per row of a node's virtual counts: 12"},
         "predict": serving,
         "configs": configs,
         "cpu_baseline": cpu,

@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(BITS_THREADS, 2) k_row_bits(View vb, LevelScra
 // fields of two registers; a prefix over the lanes gives each its left class
 // counts and sums at its first row; then each updates them row by row, with no
 // exchange between lanes.  The exact score costs more than the rest of a step,
-// so a step only estimates the candidate's gain (see Gain) and the walk keeps
+// so a step only estimates the candidate's gain (gain_of) and the walk keeps
 // the largest.  Only a lane whose largest gain reaches the best known for the
 // node within the estimate's error walks again, and there the candidates
 // within that error are scored exactly: one further below can neither win nor

@@ -307,9 +307,10 @@ int ct_tree_canonicalize(const uint32_t* left, const uint32_t* right, const uint
  * small_rows (default, 512, 2048, 8192); where the fits take row-list growth,
  * only the first stage, without cutoff 128.  Plain: the
  * depth-first/breadth-first switch, which the reference sets with an offline
- * regression (estimate_threshold.py, random_forest.py:278-289).  The
- * workspace must hold ct_autotune_workspace_size bytes; lists and trees as
- * for ct_fit with n_trees. */
+ * regression (estimate_threshold.py, random_forest.py:278-289).  With
+ * ct_autotune_workspace_size bytes of workspace every candidate is timed; those
+ * that a smaller one does not fit are skipped.  Lists and trees as for ct_fit
+ * with n_trees. */
 int ct_autotune_workspace_size(const ct_problem* p, uint32_t n_trees, uint32_t mode, size_t* bytes);
 int ct_autotune(const ct_problem* p, const ct_lists* lists, uint32_t n_trees, uint32_t mode,
                 const ct_tree_buffers* trees, void* workspace, size_t workspace_bytes,
