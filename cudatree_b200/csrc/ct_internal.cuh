@@ -707,9 +707,13 @@ struct BatchReq {
 uint32_t predict_rows_per_block(uint32_t n_classes, uint32_t n_features, uint32_t n_rows);
 size_t predict_tile_smem(uint32_t rpb, uint32_t n_classes, uint32_t n_features);
 uint32_t predict_group_size(uint32_t n_trees, uint64_t n_nodes, size_t node_bytes);  // by the nodes' share of L2
-uint32_t predict_group_size(uint32_t n_trees, uint64_t n_nodes, size_t node_bytes, uint32_t rpb, uint32_t tiles);
 bool predict_one_round(uint32_t rpb, uint32_t group);  // a block walks the group's trees at once
-bool predict_few_in_flight(uint32_t rpb, uint32_t group, uint64_t tree_bytes);
+struct WalkPlan {
+  uint32_t group;          // trees per group
+  bool few_in_flight;      // which form of the walk
+};
+WalkPlan predict_plan(uint32_t n_trees, uint64_t n_nodes, size_t node_bytes, uint32_t n_rows, uint32_t n_features,
+                      uint32_t n_classes, bool votes);
 uint32_t compact_feature_bits(uint32_t n_features);
 bool compact_fits(uint32_t n_features, uint64_t max_tree_nodes);
 void compact_host(const ct_packed_node* in, uint32_t n, uint32_t fbits, ct_compact_node* out);
@@ -719,7 +723,7 @@ void compact_host(const ct_packed_node* in, uint32_t n, uint32_t fbits, ct_compa
 int check_forest_host(const ct_packed_node* nodes, uint32_t n_nodes, const uint32_t* off, uint32_t n_trees,
                       uint32_t n_features, uint32_t n_classes);
 int predict_batch(const BatchReq* reqs_dev, uint32_t n_req, uint32_t total_blocks, uint32_t total_rows,
-                  size_t smem, bool any_grouped, bool one_round, cudaStream_t st);
+                  size_t smem, bool any_grouped, bool few_in_flight, cudaStream_t st);
 // Bit f of bits ([ceil(n_features / 32)] words, zeroed here): feature f takes
 // at most two distinct values (-0.0 and +0.0 count as one, as in the scan's
 // comparisons).

@@ -18,6 +18,7 @@
 //     histograms are added into a global [rows][classes] table and a second
 //     kernel takes the majority, lowest class on ties
 //     (np.argmax(np.bincount(...)), random_forest.py:358).
+#include <cmath>
 #include <cstring>
 
 #include "ct_items.cuh"
@@ -28,7 +29,7 @@ namespace {
 
 constexpr int PRED_THREADS = 256;
 // Walks in flight per thread: 4 at 6 blocks per SM where a group is one round of
-// them or small (predict_few_in_flight), else 8 at 4 blocks.  Fewer trees in flight, whose nodes stay in L1
+// them or small (predict_plan), else 8 at 4 blocks.  Fewer trees in flight, whose nodes stay in L1
 // longer, but more rounds: 500 covtype-shaped trees (37 MB of nodes), 65,536
 // rows, in groups of 32: 4 walks 1.64 ms, 8 walks 1.82, 2 walks (8 blocks) 1.82;
 // all trees in one group: 3.29, 3.00 and 3.7 ms.
@@ -39,8 +40,14 @@ __host__ __device__ __forceinline__ uint32_t walk_round(uint32_t rpb) { return P
 constexpr uint32_t X_SMEM_BYTES = 32 * 1024;     // rows of x staged per block when they fit
 constexpr uint32_t HIST_SMEM_BYTES = 64 * 1024;  // vote histogram [rows][classes]
 constexpr size_t GROUP_L2_BYTES = 32ull << 20;   // node bytes of one tree group, at the most
-constexpr size_t GROUP_L1_BYTES = 192ull << 10;  // node bytes of one round of walks from which groups are single rounds
-constexpr size_t GROUP_SHORT_BYTES = 768ull << 10;  // node bytes of a group of several rounds of short walks
+// predict_plan
+constexpr uint32_t SMS = 148;
+constexpr uint32_t FILL_BLOCKS = 416;                  // blocks a launch of few tiles is cut into
+constexpr size_t GROUP_L1_BYTES = 864ull << 10;        // node bytes of a group of several rounds
+constexpr size_t ROUND_L1_BYTES = 192ull << 10;        // node bytes of a round that L1 holds
+constexpr size_t SMALL_FOREST_BYTES = 256ull << 10;    // node bytes up to which a forest is one group
+constexpr size_t SHORT_GROUP_BYTES = 704ull << 10;     // node bytes of a group of several rounds, few walks in flight
+constexpr size_t SIX_BLOCKS_SMEM = 26000;              // rows and votes of a block when six are on an SM
 
 __host__ __device__ __forceinline__ bool predict_rows_staged(uint32_t rpb, uint32_t n_features) {
   return (size_t)rpb * n_features * sizeof(float) <= X_SMEM_BYTES;
@@ -328,41 +335,67 @@ uint32_t predict_group_size(uint32_t n_trees, uint64_t n_nodes, size_t node_byte
   return (uint32_t)std::min<uint64_t>(g, n_trees);
 }
 
-// Trees per group of a launch with a vote table.  A block's threads walk
-// `round` trees at once; with one round per group the blocks on an SM walk the
-// same few trees, whose nodes then come from L1 more often: 500 trees of 75 KB,
-// 65,536 rows: 1.64 ms in groups of 32 (one round of 32 rows), 1.81 of 64,
-// 2.20 of 128, 3.29 ungrouped, and 1.83 of 24 (a round not filled).  A group
-// costs each tile a staging of its rows and a flush of its votes, which is
-// more than short walks in trees that fit L1 anyway gain: 100 trees of 5.5 KB
-// take 193 us in groups of 32 and 189 us as one, of 8.4 KB 233 and 250 us.  (And
-// two groups of 20 take 174 us where one of 40 takes 167: from one and a half
-// rounds on.)  Fewer tiles than blocks the chip holds are cut further, down to 2
-// trees per thread column, when the trees are more than a round: 2,048 rows,
-// 100 trees of 24 KB: 96 us as one group, 61 of 32, 58 of 16; but 20,000 rows of
-// 20 small trees 53 us as one, 60 as two.
-uint32_t predict_group_size(uint32_t n_trees, uint64_t n_nodes, size_t node_bytes, uint32_t rpb, uint32_t tiles) {
-  const uint32_t columns = PRED_THREADS / rpb, round = walk_round(rpb);
-  uint32_t g = predict_group_size(n_trees, n_nodes, node_bytes);
-  if (n_nodes * node_bytes / n_trees * round > GROUP_L1_BYTES && n_trees >= round + round / 2) g = std::min(g, round);
-  const uint32_t fill = ceil_div(148u * (uint32_t)pred_blocks(PRED_ILP), tiles);
-  if (fill > 1 && n_trees > round) g = std::min(g, std::max(ceil_div(n_trees, fill), 2 * columns));
-  // a grid holds 2^31 - 1 blocks (from 2.1 billion rows on with 32 groups)
-  g = std::max(g, ceil_div(n_trees, std::max(1u, 0x7fffffffu / tiles)));
-  return ceil_div(n_trees, ceil_div(n_trees, g));
-}
-
 bool predict_one_round(uint32_t rpb, uint32_t group) { return group <= walk_round(rpb); }
 
-// Which of the two forms of the walk.  Several rounds of trees that fit L1 are
-// short walks while the whole group is not far beyond L1 either, and then more
-// blocks hide more (65,536 rows, 4 walks / 8 walks: 100 trees of 1.2 KB 135 / 169
-// us, of 5.6 KB 219 / 251; 300 trees of 1.9 KB 428 / 442, of 2.8 KB 514 / 514).
-// Past that most nodes come from L2 and more walks in flight do (300 trees of 4
-// KB 619 / 599; 1,000 of 1.2 KB 1,536 / 1,419; 5,000 rows, 1,000 of 4 KB 254 / 200).
-bool predict_few_in_flight(uint32_t rpb, uint32_t group, uint64_t tree_bytes) {
-  return predict_one_round(rpb, group) ||
-         (tree_bytes * walk_round(rpb) <= GROUP_L1_BYTES && tree_bytes * group <= GROUP_SHORT_BYTES);
+// Tree groups and form of a walk over n_rows rows; votes: there is a vote table.
+// A block's threads walk a round of trees at once.  Groups are for two things:
+//   * the blocks on an SM walk the same few trees, whose nodes then come from L1
+//     more often: groups of one to six rounds with at most 864 KB of nodes (65,536
+//     rows, 500 trees of 75 KB: 1.64 ms in groups of 32, 1.81 of 64, 2.20 of 128,
+//     3.29 as one; 7,800 rows, 1,000 trees of 4.8 KB: 247 us in groups of 63, 337 of
+//     250, 480 as one; 16,600 rows, 1,174 trees of 9.1 KB: 1.84 ms in groups of one
+//     round, 1.55 of two, 4.0 as one).
+//   * a launch of fewer tiles than two per SM is cut into about as many blocks as
+//     the chip takes at once (2,048 rows, 100 trees of 24 KB: 96 us as one group,
+//     58 of 16; but 16,000 rows, 36 trees of 8 KB 66 us as one, 87 as three).
+// A group costs every tile a staging of its rows, and grouping at all the vote
+// table's zeroing, filling and reading: in steps of a walk (the left side: those
+// of a round, times the rounds and the waves of blocks) about 7, half of one per
+// MB of rows read again and 2.7 per MB of the table.  Below that one group is
+// faster (4,600 rows of 1,023 features, 202 trees of 17 KB: 108 us, 145 as two
+// groups; 64,000 rows of 896, 300 classes, 308 trees of 16 KB: 1.77 ms, 2.32 as
+// three; 18,000 rows, 36 trees of 8 KB: 70 and 98 us).
+// Of 1,640 calls (60 to 30,000 training rows, 3 to 3,000 features, 2 to 300
+// classes, 12 to 1,200 trees, 1 to 70,000 rows) 1 in 100 takes more than 1.03
+// times what one group with 8 walks in flight takes; the geometric mean is 0.74.
+//
+// Few walks in flight (PRED_ILP) for a group of one round; for more rounds where
+// the launch fills the SMs, a block's rows and votes leave room for six blocks
+// and the group is small (two rounds, or 704 KB: 65,536 rows, 4 / 8 walks: 100
+// trees of 1.2 KB 135 / 169 us, 300 trees of 1.9 KB 428 / 442; but 300 trees of 4 KB
+// 619 / 599, 1,000 of 1.2 KB 1,536 / 1,419, 900 rows of 54 trees 57 / 47).
+WalkPlan predict_plan(uint32_t n_trees, uint64_t n_nodes, size_t node_bytes, uint32_t n_rows, uint32_t n_features,
+                      uint32_t n_classes, bool votes) {
+  const uint32_t rpb = predict_rows_per_block(n_classes, n_features, n_rows);
+  const uint32_t tiles = (uint32_t)(((uint64_t)n_rows + rpb - 1) / rpb);  // (not 0 for the last rows of 32 bits)
+  const uint32_t columns = PRED_THREADS / rpb, round = walk_round(rpb);
+  const double tree = std::max(1.0, (double)n_nodes * (double)node_bytes / n_trees);
+  uint32_t g = n_trees;
+  if (votes && n_trees >= (n_rows >= 1024 ? 16u : 2u * round)) {
+    const uint32_t most = predict_group_size(n_trees, n_nodes, node_bytes);
+    g = most;
+    const uint32_t few = std::max(round, (uint32_t)std::min(6.0 * round, GROUP_L1_BYTES / tree));
+    if (tree * n_trees > SMALL_FOREST_BYTES && n_trees >= 1.6 * few) g = std::min(g, few);
+    const uint32_t fill = tiles <= 2 * SMS ? ceil_div(FILL_BLOCKS, tiles) : 1u;
+    if (fill > 1 && tree * round > ROUND_L1_BYTES && n_trees >= round + round / 2) g = std::min(g, round);
+    if (fill > 1 && n_trees > round) g = std::min(g, std::max(ceil_div(n_trees, fill), columns));
+    const uint32_t groups = ceil_div(n_trees, g), least = ceil_div(n_trees, most);
+    g = ceil_div(n_trees, groups);
+    if (groups > least) {
+      const double mb = 4e-6 * n_rows;
+      const double steps = (double)n_trees / round * std::log2(tree / node_bytes + 2) * std::max(1.0, tiles / (4.5 * SMS));
+      if (steps < 7 + 0.5 * (groups - least) * mb * n_features + 2.7 * mb * n_classes)
+        g = n_rows >= 1024 ? ceil_div(n_trees, least) : n_trees;
+    }
+    // a grid holds 2^31 - 1 blocks (from 2.1 billion rows on with 32 groups)
+    g = std::max(g, ceil_div(n_trees, std::max(1u, 0x7fffffffu / tiles)));
+    g = ceil_div(n_trees, ceil_div(n_trees, g));
+  }
+  const size_t smem = (size_t)rpb * (n_features + n_classes) * sizeof(float);
+  const bool few_walks = predict_one_round(rpb, g) ||
+                         ((uint64_t)tiles * ceil_div(n_trees, g) > SMS && smem <= SIX_BLOCKS_SMEM &&
+                          (tree * g <= SHORT_GROUP_BYTES || g <= 2 * round));
+  return WalkPlan{g, few_walks};
 }
 
 uint32_t compact_feature_bits(uint32_t n_features) {
@@ -465,7 +498,7 @@ __global__ void k_vote_batch(const BatchReq* __restrict__ reqs, uint32_t n_req, 
 }
 
 int predict_batch(const BatchReq* reqs_dev, uint32_t n_req, uint32_t total_blocks, uint32_t total_rows,
-                  size_t smem, bool any_grouped, bool one_round, cudaStream_t st) {
+                  size_t smem, bool any_grouped, bool few_in_flight, cudaStream_t st) {
   if (n_req == 0 || total_blocks == 0) return CT_OK;
   CT_ARG_CHECK(smem <= HIST_SMEM_BYTES + X_SMEM_BYTES, "predict batch: tile shared memory too large");
   auto launch = [&](auto kernel) -> int {
@@ -473,7 +506,7 @@ int predict_batch(const BatchReq* reqs_dev, uint32_t n_req, uint32_t total_block
     kernel<<<total_blocks, PRED_THREADS, smem, st>>>(reqs_dev, n_req);
     return CT_OK;
   };
-  CT_TRY(one_round ? launch(k_predict_batch<PRED_ILP>) : launch(k_predict_batch<PRED_ILP_LONG>));
+  CT_TRY(few_in_flight ? launch(k_predict_batch<PRED_ILP>) : launch(k_predict_batch<PRED_ILP_LONG>));
   if (any_grouped) k_vote_batch<<<ceil_div(total_rows, 8), 256, 0, st>>>(reqs_dev, n_req, total_rows);
   CT_CUDA_TRY(cudaGetLastError());
   return CT_OK;
@@ -497,11 +530,9 @@ int predict(const void* nodes, uint32_t n_nodes, uint32_t fbits, const uint32_t*
   const uint32_t rpb = predict_rows_per_block(n_classes, n_features, n_rows);
   const uint32_t tiles = (uint32_t)(((uint64_t)n_rows + rpb - 1) / rpb);  // (not 0 for the last rows of 32 bits)
   // Tree groups need the vote table; without one every block walks all trees.
-  // Few rows are worth the table's zeroing and the votes' own launch from two
-  // rounds of walks on: a call with 40 rows and 500 trees 344 -> 155 us.
-  uint32_t group = n_trees;
-  if (votes && n_trees >= (n_rows >= 1024 ? 16u : 2u * walk_round(rpb)))
-    group = predict_group_size(n_trees, n_nodes, fbits ? CompactForm::BYTES : PackedForm::BYTES, rpb, tiles);
+  const WalkPlan plan = predict_plan(n_trees, n_nodes, fbits ? CompactForm::BYTES : PackedForm::BYTES, n_rows, n_features,
+                                     n_classes, votes != nullptr);
+  const uint32_t group = plan.group;
   const uint32_t groups = ceil_div(n_trees, group);
   const size_t smem = predict_tile_smem(rpb, n_classes, n_features);
   if (groups > 1) CT_CUDA_TRY(cudaMemsetAsync(votes, 0, (size_t)n_rows * n_classes * sizeof(uint32_t), st));
@@ -512,10 +543,8 @@ int predict(const void* nodes, uint32_t n_nodes, uint32_t fbits, const uint32_t*
                                                        n_features, n_classes, rpb, votes, pred);
     return CT_OK;
   };
-  const bool few =
-      predict_few_in_flight(rpb, group, (uint64_t)n_nodes * (fbits ? CompactForm::BYTES : PackedForm::BYTES) / n_trees);
-  if (fbits) CT_TRY(few ? launch(k_predict<CompactForm, PRED_ILP>) : launch(k_predict<CompactForm, PRED_ILP_LONG>));
-  else CT_TRY(few ? launch(k_predict<PackedForm, PRED_ILP>) : launch(k_predict<PackedForm, PRED_ILP_LONG>));
+  if (fbits) CT_TRY(plan.few_in_flight ? launch(k_predict<CompactForm, PRED_ILP>) : launch(k_predict<CompactForm, PRED_ILP_LONG>));
+  else CT_TRY(plan.few_in_flight ? launch(k_predict<PackedForm, PRED_ILP>) : launch(k_predict<PackedForm, PRED_ILP_LONG>));
   if (groups > 1) k_vote_rows<<<ceil_div(n_rows, 8), 256, 0, st>>>(votes, n_rows, n_classes, pred);
   CT_CUDA_TRY(cudaGetLastError());
   return CT_OK;

@@ -569,7 +569,7 @@ class Server {
     uint64_t xoff = 0, roff = 0, voff = 0, zero = 0;
     size_t smem = 0;
     uint32_t blocks = 0, max_c = 1;
-    bool grouped = false, one_round = true;
+    bool grouped = false, few = true;
     std::vector<Forest> fs;
     {
       // a forest removed after the request was queued: the request fails;
@@ -619,10 +619,11 @@ class Server {
       // many rows: groups by the request's tiles (a few rows are answered
       // soonest by one group, unless the forest is larger than L2's share; rows
       // in host memory would cross the link once per group)
-      br.group = f.group;
+      WalkPlan plan{f.group, predict_one_round(rpb, std::min(f.group, f.n_trees))};
       if (!s.direct[i] && r->n_rows >= 1024 && f.n_classes <= cfg.max_classes)
-        br.group = predict_group_size(f.n_trees, f.n_nodes, f.fbits ? sizeof(ct_compact_node) : sizeof(ct_packed_node),
-                                      rpb, br.tiles);
+        plan = predict_plan(f.n_trees, f.n_nodes, f.fbits ? sizeof(ct_compact_node) : sizeof(ct_packed_node), r->n_rows,
+                            f.n_features, f.n_classes, true);
+      br.group = plan.group;
       br.row0 = (uint32_t)roff;
       br.votes = nullptr;  // a single-group request votes directly and must not touch the table
       if (br.group < f.n_trees) {
@@ -630,7 +631,7 @@ class Server {
         br.votes = s.votes_dev + voff;
         voff += (uint64_t)r->n_rows * f.n_classes;
       }
-      one_round = one_round && predict_one_round(rpb, std::min(br.group, f.n_trees));
+      few = few && plan.few_in_flight;
       blocks += br.tiles * ceil_div(f.n_trees, br.group);
       if (s.direct[i]) {
         ++zero;
@@ -646,7 +647,7 @@ class Server {
     if (cudaMemcpyAsync(s.req_dev, s.req_host, batch.size() * sizeof(BatchReq), cudaMemcpyHostToDevice, ln.st) !=
         cudaSuccess)
       err = 1;
-    if (predict_batch(s.req_dev, (uint32_t)batch.size(), blocks, (uint32_t)roff, smem, grouped, one_round, ln.st) != CT_OK)
+    if (predict_batch(s.req_dev, (uint32_t)batch.size(), blocks, (uint32_t)roff, smem, grouped, few, ln.st) != CT_OK)
       err = 1;
     for (size_t i = 0; i < batch.size(); ++i) {
       ct_request* r = batch[i]->req;
