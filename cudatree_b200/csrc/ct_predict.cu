@@ -42,12 +42,13 @@ constexpr uint32_t HIST_SMEM_BYTES = 64 * 1024;  // vote histogram [rows][classe
 constexpr size_t GROUP_L2_BYTES = 32ull << 20;   // node bytes of one tree group, at the most
 // predict_plan
 constexpr uint32_t SMS = 148;
-constexpr uint32_t FILL_BLOCKS = 416;                  // blocks a launch of few tiles is cut into
-constexpr size_t GROUP_L1_BYTES = 864ull << 10;        // node bytes of a group of several rounds
-constexpr size_t ROUND_L1_BYTES = 192ull << 10;        // node bytes of a round that L1 holds
+constexpr uint32_t FILL_TILES = 300;                   // fewer tiles are cut
+constexpr uint32_t FILL_BLOCKS = 400;                  // into about as many blocks
+constexpr size_t GROUP_L1_BYTES = 424ull << 10;        // node bytes of a group of several rounds
+constexpr size_t ROUND_L1_BYTES = 113ull << 10;        // node bytes of a round that L1 holds
 constexpr size_t SMALL_FOREST_BYTES = 256ull << 10;    // node bytes up to which a forest is one group
-constexpr size_t SHORT_GROUP_BYTES = 704ull << 10;     // node bytes of a group of several rounds, few walks in flight
-constexpr size_t SIX_BLOCKS_SMEM = 26000;              // rows and votes of a block when six are on an SM
+constexpr size_t SHORT_GROUP_BYTES = 2000ull << 10;    // node bytes of a group of several rounds, few walks in flight
+constexpr size_t SIX_BLOCKS_SMEM = 31500;              // rows and votes of a block when six are on an SM
 
 __host__ __device__ __forceinline__ bool predict_rows_staged(uint32_t rpb, uint32_t n_features) {
   return (size_t)rpb * n_features * sizeof(float) <= X_SMEM_BYTES;
@@ -340,30 +341,30 @@ bool predict_one_round(uint32_t rpb, uint32_t group) { return group <= walk_roun
 // Tree groups and form of a walk over n_rows rows; votes: there is a vote table.
 // A block's threads walk a round of trees at once.  Groups are for two things:
 //   * the blocks on an SM walk the same few trees, whose nodes then come from L1
-//     more often: groups of one to six rounds with at most 864 KB of nodes (65,536
-//     rows, 500 trees of 75 KB: 1.64 ms in groups of 32, 1.81 of 64, 2.20 of 128,
-//     3.29 as one; 7,800 rows, 1,000 trees of 4.8 KB: 247 us in groups of 63, 337 of
-//     250, 480 as one; 16,600 rows, 1,174 trees of 9.1 KB: 1.84 ms in groups of one
-//     round, 1.55 of two, 4.0 as one).
-//   * a launch of fewer tiles than two per SM is cut into about as many blocks as
-//     the chip takes at once (2,048 rows, 100 trees of 24 KB: 96 us as one group,
-//     58 of 16; but 16,000 rows, 36 trees of 8 KB 66 us as one, 87 as three).
+//     more often: groups of one round, or of up to six with at most 424 KB of
+//     nodes (65,536 rows, 500 trees of 75 KB: 1.64 ms in groups of 32, 1.81 of 64,
+//     2.20 of 128, 3.29 as one; 7,800 rows, 1,000 trees of 4.8 KB: 247 us in groups
+//     of 63, 337 of 250, 480 as one);
+//   * a launch of fewer tiles than about two per SM is cut into some 400 blocks
+//     (2,048 rows, 100 trees of 24 KB: 96 us as one group, 58 of 16; but 16,000
+//     rows, 36 trees of 8 KB 66 us as one, 87 as three).
 // A group costs every tile a staging of its rows, and grouping at all the vote
 // table's zeroing, filling and reading: in steps of a walk (the left side: those
-// of a round, times the rounds and the waves of blocks) about 7, half of one per
-// MB of rows read again and 2.7 per MB of the table.  Below that one group is
-// faster (4,600 rows of 1,023 features, 202 trees of 17 KB: 108 us, 145 as two
-// groups; 64,000 rows of 896, 300 classes, 308 trees of 16 KB: 1.77 ms, 2.32 as
-// three; 18,000 rows, 36 trees of 8 KB: 70 and 98 us).
-// Of 1,640 calls (60 to 30,000 training rows, 3 to 3,000 features, 2 to 300
-// classes, 12 to 1,200 trees, 1 to 70,000 rows) 1 in 100 takes more than 1.03
-// times what one group with 8 walks in flight takes; the geometric mean is 0.74.
+// of a round, times the rounds and the waves of blocks) about 7.5, half of one
+// per MB of rows read again and 2.4 per MB of the table.  Below that one group is
+// faster (64,000 rows of 896 features, 300 classes, 308 trees of 16 KB: 1.77 ms,
+// 2.32 as three groups; 18,000 rows, 36 trees of 8 KB: 70 and 98 us).
+// The constants were fitted to 4,759 calls (60 to 30,000 training rows, 3 to 3,000
+// features, 2 to 300 classes, 12 to 1,200 trees, 1 to 70,000 rows), each timed with
+// groups of n / 1 to n / 64 trees in both forms: 2 in 100 take more than 1.03 times
+// what one group with 8 walks in flight takes, the geometric mean is 0.75 of it
+// and 1.03 of the best.
 //
 // Few walks in flight (PRED_ILP) for a group of one round; for more rounds where
-// the launch fills the SMs, a block's rows and votes leave room for six blocks
-// and the group is small (two rounds, or 704 KB: 65,536 rows, 4 / 8 walks: 100
-// trees of 1.2 KB 135 / 169 us, 300 trees of 1.9 KB 428 / 442; but 300 trees of 4 KB
-// 619 / 599, 1,000 of 1.2 KB 1,536 / 1,419, 900 rows of 54 trees 57 / 47).
+// the launch gives most SMs a block, the block's rows and votes leave room for
+// six and the group is not far beyond L1 (65,536 rows, 4 / 8 walks: 100 trees of
+// 1.2 KB 135 / 169 us, 300 trees of 1.9 KB 428 / 442; but 63,000 rows of 165 features,
+// 100 classes, 279 trees of 1 KB 528 / 448, 900 rows, 54 trees of 8 KB 57 / 47).
 WalkPlan predict_plan(uint32_t n_trees, uint64_t n_nodes, size_t node_bytes, uint32_t n_rows, uint32_t n_features,
                       uint32_t n_classes, bool votes) {
   const uint32_t rpb = predict_rows_per_block(n_classes, n_features, n_rows);
@@ -375,16 +376,16 @@ WalkPlan predict_plan(uint32_t n_trees, uint64_t n_nodes, size_t node_bytes, uin
     const uint32_t most = predict_group_size(n_trees, n_nodes, node_bytes);
     g = most;
     const uint32_t few = std::max(round, (uint32_t)std::min(6.0 * round, GROUP_L1_BYTES / tree));
-    if (tree * n_trees > SMALL_FOREST_BYTES && n_trees >= 1.6 * few) g = std::min(g, few);
-    const uint32_t fill = tiles <= 2 * SMS ? ceil_div(FILL_BLOCKS, tiles) : 1u;
+    if (tree * n_trees > SMALL_FOREST_BYTES && n_trees >= 1.64 * few) g = std::min(g, few);
+    const uint32_t fill = tiles <= FILL_TILES ? ceil_div(FILL_BLOCKS, tiles) : 1u;
     if (fill > 1 && tree * round > ROUND_L1_BYTES && n_trees >= round + round / 2) g = std::min(g, round);
     if (fill > 1 && n_trees > round) g = std::min(g, std::max(ceil_div(n_trees, fill), columns));
     const uint32_t groups = ceil_div(n_trees, g), least = ceil_div(n_trees, most);
     g = ceil_div(n_trees, groups);
     if (groups > least) {
       const double mb = 4e-6 * n_rows;
-      const double steps = (double)n_trees / round * std::log2(tree / node_bytes + 2) * std::max(1.0, tiles / (4.5 * SMS));
-      if (steps < 7 + 0.5 * (groups - least) * mb * n_features + 2.7 * mb * n_classes)
+      const double steps = (double)n_trees / round * std::log2(tree / node_bytes + 2) * std::max(1.0, tiles / (3.5 * SMS));
+      if (steps < 7.5 + 0.5 * (groups - least) * mb * n_features + 2.35 * mb * n_classes)
         g = n_rows >= 1024 ? ceil_div(n_trees, least) : n_trees;
     }
     // a grid holds 2^31 - 1 blocks (from 2.1 billion rows on with 32 groups)
@@ -393,8 +394,8 @@ WalkPlan predict_plan(uint32_t n_trees, uint64_t n_nodes, size_t node_bytes, uin
   }
   const size_t smem = (size_t)rpb * (n_features + n_classes) * sizeof(float);
   const bool few_walks = predict_one_round(rpb, g) ||
-                         ((uint64_t)tiles * ceil_div(n_trees, g) > SMS && smem <= SIX_BLOCKS_SMEM &&
-                          (tree * g <= SHORT_GROUP_BYTES || g <= 2 * round));
+                         ((uint64_t)tiles * ceil_div(n_trees, g) > SMS * 3 / 4 && smem <= SIX_BLOCKS_SMEM &&
+                          (tree * g <= SHORT_GROUP_BYTES || 5 * g <= 9 * round));
   return WalkPlan{g, few_walks};
 }
 

@@ -56,9 +56,9 @@ def test_no_groups_without_a_vote_table(rows):
     assert _plan(700, 30_000, rows, votes=False).group == 700
 
 
-@pytest.mark.parametrize("n_trees,tree_bytes,rows,features,few", [
-    (32, 75_000, 65536, 10, True), (500, 75_000, 65536, 54, True),            # one round
-    (100, 1_200, 65536, 20, True), (300, 1_900, 65536, 20, True),             # small groups, every SM at work
-    (370, 1_100, 18270, 425, False), (54, 8_400, 901, 24, False)])            # no room for six blocks; few blocks
-def test_form(n_trees, tree_bytes, rows, features, few):
-    assert _plan(n_trees, tree_bytes, rows, features).few_in_flight == few
+@pytest.mark.parametrize("n_trees,tree_bytes,rows,features,classes,few", [
+    (32, 75_000, 65536, 10, 2, True), (500, 75_000, 65536, 54, 7, True),            # one round
+    (100, 1_200, 65536, 20, 2, True), (300, 1_900, 65536, 20, 2, True),             # small groups, every SM at work
+    (279, 1_000, 63112, 165, 100, False), (54, 8_400, 901, 24, 7, False)])          # no room for six blocks; few blocks
+def test_form(n_trees, tree_bytes, rows, features, classes, few):
+    assert _plan(n_trees, tree_bytes, rows, features, classes).few_in_flight == few
