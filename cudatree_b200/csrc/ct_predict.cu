@@ -4,10 +4,10 @@
 // per warp, and random_forest.py:339-362 stacks per-tree labels on the host
 // and votes row by row in Python.  Here one launch walks every tree of the
 // forest:
-//   * blocks cover (row tile, tree group); the trees are cut into groups of as
-//     many as a block walks at once, and blocks are numbered group-major, so the
-//     blocks in flight walk one group's trees and find much of them in L1
-//     (predict_group_size);
+//   * blocks cover (row tile, tree group); the trees are cut into groups of one
+//     or a few rounds of a block's walks where that pays, and blocks are numbered
+//     group-major, so the blocks in flight walk one group's trees and find much
+//     of them in L1 (predict_plan);
 //   * walks inside a block are numbered row-fastest: with 32 rows per tile a
 //     lane keeps one row and a warp's lanes walk the same tree (shared loads
 //     of its top levels); each thread keeps PRED_ILP walks in flight;
@@ -29,10 +29,10 @@ namespace {
 
 constexpr int PRED_THREADS = 256;
 // Walks in flight per thread: 4 at 6 blocks per SM where a group is one round of
-// them or small (predict_plan), else 8 at 4 blocks.  Fewer trees in flight, whose nodes stay in L1
-// longer, but more rounds: 500 covtype-shaped trees (37 MB of nodes), 65,536
-// rows, in groups of 32: 4 walks 1.64 ms, 8 walks 1.82, 2 walks (8 blocks) 1.82;
-// all trees in one group: 3.29, 3.00 and 3.7 ms.
+// them or small (predict_plan), else 8 at 4 blocks.  Fewer trees in flight, whose
+// nodes stay in L1 longer, but more rounds: 500 covtype-shaped trees (37 MB of
+// nodes), 65,536 rows, in groups of 32: 4 walks 1.64 ms, 8 walks 1.82, 2 walks (8
+// blocks) 1.82; all trees in one group: 3.29, 3.00 and 3.7 ms.
 constexpr int PRED_ILP = 4;
 constexpr int PRED_ILP_LONG = 8;
 constexpr int pred_blocks(int ilp) { return ilp == PRED_ILP ? 6 : 4; }
