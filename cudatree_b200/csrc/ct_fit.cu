@@ -1816,6 +1816,7 @@ int fit_queue(const ct_fit_job* jobs, uint32_t n_jobs, const ct_fit_options* o, 
     vb.slot_job = slot_job_dev;
     vb.sel_stride = q.m_max;
     vb.mask_stride = L.mask_words;
+    vb.fbin = L.fbin;  // (some job may have two-valued features: their scan is launched)
     vb.bit_words = 0;  // per job (the shared-memory staging of marks is off)
     vb.lab_shift = views[0].lab_shift;
     vb.row_mask = views[0].row_mask;
