@@ -530,15 +530,9 @@ __global__ void k_loop_end(LoopCtl* ctl, Counters* c, uint32_t chunk, uint32_t c
   cudaGraphSetConditional(h, n > 0 ? 1u : 0u);
 }
 
-// Making, launching and destroying loop graphs is one thread's work at a time:
-// each thread has its own, but while one thread's graph was destroyed beside
-// another's being made or launched, the process crashed inside
-// cudaGraphDestroy (fits of new shapes from three threads at once).
-std::mutex g_graphs;
-
 // The instantiated loop graph of the last batched fit on this thread, reused
 // while every kernel argument is the same (same problem, workspace, lists and
-// options).  Its functions are called with g_graphs held.
+// options).
 struct LoopGraph {
   std::vector<unsigned char> key;
   cudaGraph_t graph = nullptr;
@@ -553,10 +547,7 @@ struct LoopGraph {
     graph = nullptr;
     key.clear();
   }
-  ~LoopGraph() {
-    std::lock_guard<std::mutex> lk(g_graphs);
-    reset();
-  }
+  ~LoopGraph() { reset(); }
 };
 thread_local LoopGraph t_loop_graph;
 
@@ -723,7 +714,6 @@ int graph_level_loop(const ct_problem* p, const View& v, const FitLayout& L, con
   key_add(key, L.rows);
   key_add(key, L.n_max);
   LoopGraph& lg = t_loop_graph;
-  std::unique_lock<std::mutex> lk(g_graphs);
   if (!lg.exec || lg.key != key) {
     lg.reset();
     cudaStream_t cs = capture_stream();
@@ -743,7 +733,6 @@ int graph_level_loop(const ct_problem* p, const View& v, const FitLayout& L, con
   CT_CUDA_TRY(cudaMemsetAsync(&L.ctl->cur, 0, sizeof(uint32_t), st));
   if (cur) CT_CUDA_TRY(cudaMemsetAsync(&L.ctl->cur, 1, 1, st));
   CT_CUDA_TRY(cudaGraphLaunch(lg.exec, st));
-  lk.unlock();
   LoopCtl ctl;
   Counters h;
   CT_CUDA_TRY(cudaMemcpyAsync(&ctl, L.ctl, sizeof(ctl), cudaMemcpyDeviceToHost, st));

@@ -470,7 +470,9 @@ class RandomForestClassifier:
         self._trees = self._fit_trees(0, self.n_estimators, self.fit_mode, self.bfs_threshold)
         self._packed = None
         self.fit_release()
-        torch.cuda.synchronize()
+        # this stream only: a wait for the device is not allowed while another
+        # thread's fit captures its loop graph, and broke that graph
+        torch.cuda.current_stream().synchronize()
         self.last_fit_timing["fit_s"] = time.perf_counter() - t0
         return self
 

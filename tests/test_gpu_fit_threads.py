@@ -1,5 +1,5 @@
 """Fits and small queues of several threads at once, each call of another shape
-(so that every thread makes, launches and destroys loop graphs beside the
+(so that every thread makes and destroys loop graphs beside the
 others), give the trees of the same calls one after another."""
 import threading
 
@@ -47,3 +47,15 @@ def test_threads_with_graphs_of_their_own(cuda_device):
             np.testing.assert_array_equal(a.left_children, b.left_children)
             np.testing.assert_array_equal(a.feature_threshold_array, b.feature_threshold_array)
             np.testing.assert_array_equal(a.values_array, b.values_array)
+
+
+def test_fit_waits_for_its_own_stream_only(cuda_device, monkeypatch):
+    """A device-wide wait is forbidden while any stream captures: with one in fit,
+    a thread that was making its loop graph was left with a broken one."""
+    import torch
+
+    def refuse(*a):
+        raise AssertionError("device-wide wait")
+
+    monkeypatch.setattr(torch.cuda, "synchronize", refuse)
+    assert len(_call(2)) == 3 and len(_call(3)) == 4
