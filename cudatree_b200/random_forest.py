@@ -75,17 +75,17 @@ def _dev_bytes(nbytes: int, dev) -> torch.Tensor:
     return torch.empty(max(int(nbytes), 1) + PAD_BYTES, dtype=torch.uint8, device=dev)
 
 
-def first_that_fits(sizes, dev):
-    """(buffer, bytes) of the first of the sizes, most wanted first, that can be
+def wanted_or_least(wanted, least, dev):
+    """(buffer, bytes) of the wanted size, or of least() where that cannot be
     allocated.  (A fit runs faster with the workspace of row lists, up to 20
     bytes per cell of the table more than it needs at the least.)"""
-    for nbytes in sizes[:-1]:
-        try:
-            return _dev_bytes(nbytes, dev), nbytes
-        except torch.OutOfMemoryError:
-            pass
-        torch.cuda.empty_cache()
-    return _dev_bytes(sizes[-1], dev), sizes[-1]
+    try:
+        return _dev_bytes(wanted, dev), wanted
+    except torch.OutOfMemoryError:
+        pass
+    torch.cuda.empty_cache()
+    nbytes = least()
+    return _dev_bytes(nbytes, dev), nbytes
 
 
 def _to_dev(a: np.ndarray, dev) -> torch.Tensor:
@@ -408,9 +408,9 @@ class RandomForestClassifier:
                               _ptr(raw["threshold"]), _ptr(raw["value"]), _ptr(n_nodes), cap)
         opts = self._fit_options(mode_id, bfs_threshold)
         opts.flags |= (_lib.CT_FIT_PROFILE if self.profile else 0) | (_lib.CT_FIT_HOST_LOOP if self.host_level_loop else 0)
-        sizes = [_lib.size_of(f"ct_fit_{least}workspace_size", C.byref(prob), per_call, C.byref(opts))
-                 for least in ("", "least_")]
-        work, ws_bytes = first_that_fits(sizes, dev)
+        args = (C.byref(prob), per_call, C.byref(opts))
+        work, ws_bytes = wanted_or_least(_lib.size_of("ct_fit_workspace_size", *args),
+                                         lambda: _lib.size_of("ct_fit_least_workspace_size", *args), dev)
         trees = []
         stats = None
         for t0 in range(first, first + count, per_call):
@@ -513,9 +513,9 @@ class RandomForestClassifier:
         n_nodes = torch.zeros(sample_trees, dtype=torch.int32, device=dev)
         tb = _lib.TreeBuffers(*[_ptr(r) for r in raw], _ptr(n_nodes), cap)
         least = _lib.FitOptions(mode_id, 0, 128, 1024)  # the candidate that takes the most
-        sizes = [_lib.size_of("ct_autotune_workspace_size", C.byref(prob), sample_trees, mode_id),
-                 _lib.size_of("ct_fit_least_workspace_size", C.byref(prob), sample_trees, C.byref(least))]
-        work, ws_bytes = first_that_fits(sizes, dev)
+        work, ws_bytes = wanted_or_least(
+            _lib.size_of("ct_autotune_workspace_size", C.byref(prob), sample_trees, mode_id),
+            lambda: _lib.size_of("ct_fit_least_workspace_size", C.byref(prob), sample_trees, C.byref(least)), dev)
         best = _lib.FitOptions()
         ms = C.c_float()
         _lib.call("ct_autotune", C.byref(prob), C.byref(lists), sample_trees, mode_id, C.byref(tb), _ptr(work),
